@@ -310,8 +310,9 @@ def work(case):
 def tolerance(case):
     """bf16 activations between the kernels.  Served requests are 0.007 to 0.013 off the 64-bit values (2-norm, each output) at
     every size, rounding of stored activations through 8 layers, so two correct evaluations with unrelated roundings
-    differ by up to 0.018; one expert block is 0.003 off."""
-    return {"rel": 0.03, "max": 0.3} if case["kind"] == "serve" else {"rel": 0.01, "max": 0.1, "differ": 0.001}
+    differ by up to 0.018, and their largest single difference, over the millions of values of an output, was 0.24 to 0.38 of
+    its root mean square; one expert block is 0.003 off."""
+    return {"rel": 0.03, "max": 0.8} if case["kind"] == "serve" else {"rel": 0.01, "max": 0.1, "differ": 0.001}
 
 
 # ------------------------------------------------------------------------------------------------ 64-bit statement
