@@ -13,7 +13,8 @@ namespace pocket {
 
 namespace {
 constexpr int kHead = 128;          // head width of both attention kinds (the kernels are specialised for it)
-constexpr int kStreamMaxT = 32;     // largest batch the weight-streaming decode GEMM serves
+constexpr int kFusedMaxT = 64;      // largest decode batch whose activations stay E4M3 terms between the kernels
+constexpr int kTermsMaxT = 2047;    // longest batch whose FP8 products take the activations as E4M3 terms
 constexpr int kSMs = 148;
 
 double now_s() {
@@ -36,7 +37,7 @@ TensorView need(WeightSource& ws, const std::string& name) {
 // Split count for the tile-decoding GEMM at small T (same rule as the Python front end: the split count that
 // wastes least of the last wave, at least 8 k-blocks per split).
 int pick_splits(int t, int n, int k) {
-  if (t > 128) return 1;
+  if (t > 128 || (t > 32 && (long long)n * k <= (1 << 21))) return 1;      // as ops/gemm.py
   const int bn = t <= 16 ? 16 : t <= 32 ? 32 : t <= 64 ? 64 : 128;
   const int tiles = ((n + 127) / 128) * ((t + bn - 1) / bn);
   const int kb = (k + 63) / 64;
@@ -53,31 +54,26 @@ int pick_splits(int t, int n, int k) {
   return best;
 }
 
-// Split count for the weight-streaming GEMM: smallest count that fills 85% of the waves.
-int pick_splits_stream(int n, int k) {
-  const int tiles = (n + 127) / 128, kblk = k / 128;
-  int best = 1;
-  double best_eff = 0;
-  for (int s = 1; s <= std::max(1, std::min(kblk / 4, 16)); ++s) {
-    const int per = (kblk + s - 1) / s;
-    if ((kblk + per - 1) / per != s) continue;
-    const int waves = (tiles * s + kSMs - 1) / kSMs;
-    const double eff = double(tiles) * kblk / (double(waves) * kSMs * per);
-    if (eff > best_eff + 0.05) { best = s; best_eff = eff; }
-    if (best_eff >= 0.85) break;
-  }
-  return best;
-}
 }  // namespace
 
 // Activation and workspace buffers, sized once for the prefill chunk and the decode batch.
+// bf16 activations as E4M3 terms (kernels/gemm_fp8_terms.cu)
+struct QwenNativeEngine::TermsBuffer {
+  DeviceBuffer xq, sx;
+  void reset(size_t rows, size_t width) {
+    const size_t tiled = (rows + 255) / 256 * 256;
+    xq.reset(tiled * width * 2);
+    sx.reset(tiled * (width / 128 + 1) * 4);
+  }
+};
+
 struct QwenNativeEngine::Scratch {
   int rows = 0;                       // capacity in token rows
   DeviceBuffer ids, pos, kv_slots, meta, slot_ids, kv_len, bt_batch;
   DeviceBuffer h, x, d_attn, d_mlp, proj, mixed, core, y, ab, g, beta, q, gate, attn, gu, act;
   DeviceBuffer logits, next_idx, next_val, status, merge;
   DeviceBuffer gdn_ws, splitk_ws, counters, dec_ws;
-  DeviceBuffer xq, inv_c, xq2, inv_c2;
+  TermsBuffer norm_terms, act_terms;  // operands of the FP8 products: a norm's result; a mixer's or activation's
   size_t splitk_floats = 0;
   std::vector<int32_t> host_i32;
 };
@@ -164,7 +160,7 @@ QwenNativeEngine::QwenNativeEngine(const QwenConfig& cfg, WeightSource& weights,
   // ---- scratch
   s_ = std::make_unique<Scratch>();
   Scratch& s = *s_;
-  const size_t R = size_t(std::max(opt_.prefill_chunk, kStreamMaxT));
+  const size_t R = size_t(std::max(opt_.prefill_chunk, kFusedMaxT));
   s.rows = int(R);
   const size_t H = size_t(cfg_.hidden_size), I = size_t(inter_), V = size_t(vocab_n_);
   const size_t gate_mul = cfg_.attn_output_gate ? 2 : 1;
@@ -185,8 +181,8 @@ QwenNativeEngine::QwenNativeEngine(const QwenConfig& cfg, WeightSource& weights,
   s.counters.reset(size_t(1 << 16) * 4, true);
   s.dec_ws.reset(size_t(64) * hq_ * 64 * (kHead + 2) * 4);
   const size_t maxk = std::max({H, I, size_t(vd_), size_t(hq_) * kHead});
-  s.xq.reset(size_t(kStreamMaxT) * 3 * maxk); s.inv_c.reset(64 * 4);
-  s.xq2.reset(size_t(kStreamMaxT) * 3 * maxk); s.inv_c2.reset(64 * 4);
+  s.norm_terms.reset(kFusedMaxT, H);
+  s.act_terms.reset(std::min<size_t>(R, kTermsMaxT), maxk);
 
   // the fused decode path needs every FP8 reduction width to be a multiple of the 128-wide scale block
   stream_ok_ = (H % 128 == 0) && (I % 128 == 0) && (vd_ % 128 == 0) && ((hq_ * kHead) % 128 == 0) && kw == 4 && hk_ > 0 &&
@@ -441,6 +437,11 @@ void QwenNativeEngine::linear(const void* x, const PackedMatrix& w, void* out, i
                          nullptr, s.status.as<int>(), stream_), "gemm(f32)");
     return;
   }
+  if (const int tok = terms_tile(T, w)) {
+    rc(b200_split_terms(x, T, w.k, tok, s.act_terms.xq.get(), s.act_terms.sx.as<float>(), stream_), "split_terms");
+    linear_terms(s.act_terms, w, out, T);
+    return;
+  }
   int splits = pick_splits(T, w.n, w.k);
   while (splits > 1 && size_t(splits) * T * w.n > s.splitk_floats) --splits;
   const int bn = b200_gemm_pick_bn(T);
@@ -449,12 +450,17 @@ void QwenNativeEngine::linear(const void* x, const PackedMatrix& w, void* out, i
                        nullptr, T, w.n, w.k, splits, s.counters.as<int>(), s.status.as<int>(), stream_), "gemm");
 }
 
-void QwenNativeEngine::linear_stream(const void* xq, const float* inv_c, const PackedMatrix& w, void* out, int T) {
+int QwenNativeEngine::terms_tile(int T, const PackedMatrix& w) {
+  int tok = 0, counters = 0;
+  long long floats = 0;
+  if (w.wfmt != 1 || w.k % 128 || T > kTermsMaxT || b200_fp8_terms_plan(T, w.n, w.k, &tok, &floats, &counters)) return 0;
+  return size_t(floats) <= s_->splitk_floats && counters <= (1 << 16) ? tok : 0;
+}
+
+void QwenNativeEngine::linear_terms(const TermsBuffer& x, const PackedMatrix& w, void* out, int T) {
   Scratch& s = *s_;
-  int splits = pick_splits_stream(w.n, w.k);
-  while (splits > 1 && size_t(splits) * T * w.n > s.splitk_floats) --splits;
-  rc(b200_gemm_w8a8s(w.weight.get(), w.scales.as<float>(), xq, inv_c, out, nullptr, T, w.n, w.k, splits,
-                     s.splitk_ws.as<float>(), s.counters.as<int>(), s.status.as<int>(), stream_), "gemm_stream");
+  rc(b200_gemm_fp8_terms(w.weight.get(), w.scales.as<float>(), x.xq.get(), x.sx.as<float>(), out, nullptr, T, w.n, w.k,
+                         s.splitk_ws.as<float>(), s.counters.as<int>(), s.status.as<int>(), stream_), "gemm_fp8_terms");
 }
 
 // ------------------------------------------------------------------------------------------------ prefill
@@ -574,9 +580,8 @@ void QwenNativeEngine::forward_decode(const std::vector<int>& slots, const std::
   cuda_check(cudaMemcpyAsync(s.slot_ids.get(), hb.data() + 3 * B, size_t(B) * 4, cudaMemcpyHostToDevice, stream_), "slot ids");
   cuda_check(cudaMemcpyAsync(s.kv_len.get(), hb.data() + 4 * B, size_t(B) * 4, cudaMemcpyHostToDevice, stream_), "kv len");
 
-  const bool fused = stream_ok_ && B <= kStreamMaxT;
-  int terms = 2;
-  if (fused) b200_gemm_w8a8s_layout(B, &terms);
+  const int tok = B <= kFusedMaxT ? terms_tile(B, layers_[0].proj) : 0;
+  const bool fused = stream_ok_ && tok > 0;
   const int att_splits = int(std::max<int64_t>(1, std::min<int64_t>({64, (2 * kSMs) / std::max(1, B * hkv_), (max_kv + 255) / 256})));
   const float scale = 1.0f / std::sqrt(float(kHead));
   const int gate_mul = cfg_.attn_output_gate ? 2 : 1;
@@ -593,9 +598,9 @@ void QwenNativeEngine::forward_decode(const std::vector<int>& slots, const std::
     uint8_t* kc = k_cache_.as<uint8_t>() + kv_layer_stride_ * L.cache_index * 2;
     uint8_t* vc = v_cache_.as<uint8_t>() + kv_layer_stride_ * L.cache_index * 2;
     if (fused) {
-      rc(b200_rmsnorm_split(s.h.get(), delta, L.in_ln.get(), L.linear ? s.x.get() : nullptr, s.xq.get(), s.inv_c.as<float>(),
-                            B, H, eps, 1, terms, stream_), "rmsnorm_split");
-      linear_stream(s.xq.get(), s.inv_c.as<float>(), L.proj, s.proj.get(), B);
+      rc(b200_rmsnorm_terms(s.h.get(), delta, L.in_ln.get(), L.linear ? s.x.get() : nullptr, B, H, eps, 1, tok,
+                            s.norm_terms.xq.get(), s.norm_terms.sx.as<float>(), stream_), "rmsnorm_terms");
+      linear_terms(s.norm_terms, L.proj, s.proj.get(), B);
     } else {
       rc(b200_rmsnorm(s.h.get(), delta, nullptr, 0, L.in_ln.get(), s.x.get(), B, H, eps, 1, delta ? 1 : 0, stream_), "rmsnorm");
       linear(s.x.get(), L.proj, s.proj.get(), B);
@@ -605,8 +610,8 @@ void QwenNativeEngine::forward_decode(const std::vector<int>& slots, const std::
       if (fused) {
         rc(b200_gdn_decode_fused(s.proj.get(), ldp, s.x.get(), H, L.ab.weight.get(), L.a_log.as<float>(),
                                  L.dt_bias.as<float>(), L.conv_w.get(), kw, tails, (long long)tail_slot_stride_, states,
-                                 (long long)state_slot_stride_, s.slot_ids.as<int>(), L.gdn_norm.get(), s.y.get(), B, hv_,
-                                 hk_, eps, stream_), "gdn_decode_fused");
+                                 (long long)state_slot_stride_, s.slot_ids.as<int>(), L.gdn_norm.get(), nullptr, B, hv_,
+                                 hk_, eps, s.act_terms.xq.get(), s.act_terms.sx.as<float>(), tok, stream_), "gdn_decode_fused");
       } else {
         linear(s.x.get(), L.ab, s.ab.get(), B);
         rc(b200_gdn_gates(s.ab.get(), 2 * hv_, 0, hv_, L.a_log.as<float>(), L.dt_bias.as<float>(), s.g.as<float>(),
@@ -631,14 +636,15 @@ void QwenNativeEngine::forward_decode(const std::vector<int>& slots, const std::
       mix_out = s.attn.get();
     }
     if (fused) {
-      rc(b200_act_split_e4m3(mix_out, B, L.out.k, terms, s.xq2.get(), s.inv_c2.as<float>(), stream_), "act_split");
-      linear_stream(s.xq2.get(), s.inv_c2.as<float>(), L.out, s.d_attn.get(), B);
+      if (!L.linear)
+        rc(b200_split_terms(mix_out, B, L.out.k, tok, s.act_terms.xq.get(), s.act_terms.sx.as<float>(), stream_), "split_terms");
+      linear_terms(s.act_terms, L.out, s.d_attn.get(), B);
       reduce_rows(s.d_attn.get(), B);
-      rc(b200_rmsnorm_split(s.h.get(), s.d_attn.get(), L.post_ln.get(), nullptr, s.xq.get(), s.inv_c.as<float>(), B, H, eps,
-                            1, terms, stream_), "rmsnorm_split");
-      linear_stream(s.xq.get(), s.inv_c.as<float>(), L.gate_up, s.gu.get(), B);
-      rc(b200_silu_mul_split(s.gu.get(), s.xq2.get(), s.inv_c2.as<float>(), B, I, terms, stream_), "silu_mul_split");
-      linear_stream(s.xq2.get(), s.inv_c2.as<float>(), L.down, s.d_mlp.get(), B);
+      rc(b200_rmsnorm_terms(s.h.get(), s.d_attn.get(), L.post_ln.get(), nullptr, B, H, eps, 1, tok, s.norm_terms.xq.get(),
+                            s.norm_terms.sx.as<float>(), stream_), "rmsnorm_terms");
+      linear_terms(s.norm_terms, L.gate_up, s.gu.get(), B);
+      rc(b200_silu_mul_terms(s.gu.get(), B, I, tok, s.act_terms.xq.get(), s.act_terms.sx.as<float>(), stream_), "silu_mul_terms");
+      linear_terms(s.act_terms, L.down, s.d_mlp.get(), B);
     } else {
       linear(mix_out, L.out, s.d_attn.get(), B);
       reduce_rows(s.d_attn.get(), B);

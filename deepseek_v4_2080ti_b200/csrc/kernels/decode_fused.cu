@@ -14,6 +14,7 @@
 #include <cuda_bf16.h>
 #include <cuda_fp8.h>
 #include <stdint.h>
+#include "fp8_terms.cuh"
 #include "ops.h"
 #include "launch.h"
 
@@ -53,62 +54,86 @@ struct GdnDecodeParams {
   __nv_bfloat16* out;          // [B, Hv*128]
   int Hv, Hk;
   float eps, q_scale;
+  b200::f8t::TermsOut terms;   // where the result goes as E4M3 terms (xq set) instead of `out`: a head is one block of 128
 };
 
-// One conv step for channel c of row b: y = silu(sum_k w[c][k] * hist[k]); shifts the tail.
+// One channel of the causal convolution: the tail's values and the new one.
 template <int KW>
-__device__ __forceinline__ float conv_step(const GdnDecodeParams& p, __nv_bfloat16* tail, int C, int c, float cur,
-                                           bool write_tail) {
-  float h[KW - 1];
+struct ConvStep {
+  float v[KW];
+  __device__ __forceinline__ void load(const __nv_bfloat16* tail, int C, int c, __nv_bfloat16 cur) {
 #pragma unroll
-  for (int k = 0; k < KW - 1; ++k) h[k] = __bfloat162float(tail[(size_t)k * C + c]);
-  float acc = cur * __bfloat162float(p.conv_w[(size_t)c * KW + KW - 1]);
-#pragma unroll
-  for (int k = 0; k < KW - 1; ++k) acc += h[k] * __bfloat162float(p.conv_w[(size_t)c * KW + k]);
-  if (write_tail) {
-#pragma unroll
-    for (int k = 0; k + 1 < KW - 1; ++k) tail[(size_t)k * C + c] = __float2bfloat16(h[k + 1]);
-    tail[(size_t)(KW - 2) * C + c] = __float2bfloat16(cur);
+    for (int k = 0; k < KW - 1; ++k) v[k] = __bfloat162float(tail[(size_t)k * C + c]);
+    v[KW - 1] = __bfloat162float(cur);
   }
-  // the unfused path stores the conv output as bf16 before the recurrence reads it
-  return bf16_round(silu_f(acc));
-}
+  // y = silu(sum_k w[c][k] * v[k]), rounded as the unfused path stores it
+  __device__ __forceinline__ float result(const __nv_bfloat16* w, int c) const {
+    float acc = v[KW - 1] * __bfloat162float(w[(size_t)c * KW + KW - 1]);
+#pragma unroll
+    for (int k = 0; k < KW - 1; ++k) acc += v[k] * __bfloat162float(w[(size_t)c * KW + k]);
+    return bf16_round(silu_f(acc));
+  }
+  __device__ __forceinline__ void store(__nv_bfloat16* tail, int C, int c) const {
+#pragma unroll
+    for (int k = 0; k < KW - 1; ++k) tail[(size_t)k * C + c] = __float2bfloat16(v[k + 1]);
+  }
+};
 
-// grid (Hk, B); block = 128 * R * RG threads (R = Hv / Hk value heads per key head, RG row groups).
-// Thread (grp, rg, j) owns rows [rg*128/RG, (rg+1)*128/RG) of state column j of value head kh*R + grp; the row
-// groups cut the serial length of the recurrence per thread, their partial dot products meet in shared memory.
-// The q/k channels of key head kh are convolved once, by the threads with grp == 0 and rg == 0.
-template <int KW, int R, int RG>
-__global__ void __launch_bounds__(128 * R * RG)
+// grid (Hv, B), clusters of the R = Hv / Hk value heads that share a key head; block = 16 warps.  Warp w owns rows 8 w .. 8 w + 7
+// of the head's state, a lane four columns of them; the warps' partial dot products meet in shared memory.
+//
+// The kernel is bound by the state, 64 KB in and out per head, and by the length of its chain.  The state is asked for first,
+// 16 bytes per load, and arrives while the projections, the convolution and the gates are computed; a block holds one head and
+// two blocks fit an SM, so one block's loads run beside another's arithmetic.  The code is kept short: the weights of a layer
+// pass through L2 between two launches, so its instructions come from HBM.  (With the R heads of a key head in one block of
+// 1024 threads, the state loaded last, four bytes per load: 45 us at 32 rows of 32 heads, where its bytes take 20, and 13.8 us
+// at one row.)
+// Every block convolves the q and k channels of its key head itself; the first of the cluster moves their tail on when all of
+// them have read it.
+template <int KW, int R>
+__global__ void __launch_bounds__(512, 2)
 gdn_decode_fused_kernel(GdnDecodeParams p) {
-  constexpr int ROWS = DK / RG;
-  constexpr int WPH = 4 * RG;              // warps per value head
-  __shared__ float sq[DK], sk[DK];
-  __shared__ float s_v[R][DV];
-  __shared__ float s_part[R][RG][DV];
-  __shared__ float red_ab[R][WPH][2];
+  constexpr int WARPS = 16, ROWS = DK / WARPS;
+  __shared__ __align__(16) float sq[DK], sk[DK], s_delta[DV];
+  __shared__ __align__(16) float s_part[WARPS][DV];
+  __shared__ float red_ab[WARPS][2];
   __shared__ float red_qk[8];
-  __shared__ float red_o[R][4];
-  __shared__ float s_gate[R][2];
+  __shared__ float red_o[4];
+  __shared__ uint32_t red_m[4];
+  __shared__ float s_gate[2];
   b200::pdl_grid_trigger();
   b200::pdl_grid_wait();
-  const int kh = blockIdx.x, b = blockIdx.y;
-  const int j = threadIdx.x & 127;
-  const int rg = (threadIdx.x >> 7) % RG;
-  const int grp = threadIdx.x / (128 * RG);
-  const int h = kh * R + grp;
+  const int h = blockIdx.x, b = blockIdx.y, kh = h / R;
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int j = threadIdx.x;                 // channel / column of the first 128 threads
   const int kd = p.Hk * DK, vd = p.Hv * DV, C = 2 * kd + vd;
   const int slot = p.slot_ids ? p.slot_ids[b] : b;
   __nv_bfloat16* tail = p.tails + (size_t)slot * p.tail_stride;
   const __nv_bfloat16* row = p.proj + (size_t)b * p.ldp;
 
-  // ---- a/b projections of this value head: two dot products of length hidden over the head's 128*RG threads
+  float4* S = reinterpret_cast<float4*>(p.states + (size_t)slot * p.state_stride + ((size_t)h * DK + warp * ROWS) * DV) + lane;
+  float4 st[ROWS];
+#pragma unroll
+  for (int i = 0; i < ROWS; ++i) st[i] = S[i * (DV / 4)];
+
+  // ---- convolution (first 128 threads)
+  const int cq = kh * DK + j, ck = kd + kh * DK + j, cv = 2 * kd + h * DV + j;
+  ConvStep<KW> tq, tk, tv;
+  if (j < DK) {
+    tq.load(tail, C, cq, row[cq]);
+    tk.load(tail, C, ck, row[ck]);
+    tv.load(tail, C, cv, row[cv]);
+  }
+  if constexpr (R > 1) asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory");
+
+  // ---- a/b projections of this value head: two dot products of length hidden
   {
     const __nv_bfloat16* xr = p.x + (size_t)b * p.hidden;
     const __nv_bfloat16* wa = p.w_ab + (size_t)h * p.hidden;
     const __nv_bfloat16* wb = p.w_ab + (size_t)(p.Hv + h) * p.hidden;
     float da = 0.f, db = 0.f;
-    for (int i = (rg * 128 + j) * 8; i < p.hidden; i += 128 * RG * 8) {
+#pragma unroll 1
+    for (int i = (int)threadIdx.x * 8; i < p.hidden; i += 512 * 8) {
       const uint4 xv = *reinterpret_cast<const uint4*>(xr + i);
       const uint4 av = *reinterpret_cast<const uint4*>(wa + i);
       const uint4 bv = *reinterpret_cast<const uint4*>(wb + i);
@@ -124,90 +149,126 @@ gdn_decode_fused_kernel(GdnDecodeParams p) {
     }
     da = warp_sum(da);
     db = warp_sum(db);
-    if ((j & 31) == 0) {
-      red_ab[grp][rg * 4 + (j >> 5)][0] = da;
-      red_ab[grp][rg * 4 + (j >> 5)][1] = db;
+    if (lane == 0) {
+      red_ab[warp][0] = da;
+      red_ab[warp][1] = db;
     }
   }
-  // ---- conv step (row group 0 only): q/k channels by value head 0 of the block, v channel by every head
-  float qv = 0.f, kv = 0.f;
-  if (rg == 0) {
-    if (grp == 0) {
-      qv = conv_step<KW>(p, tail, C, kh * DK + j, __bfloat162float(row[kh * DK + j]), true);
-      kv = conv_step<KW>(p, tail, C, kd + kh * DK + j, __bfloat162float(row[kd + kh * DK + j]), true);
-      const float qs = warp_sum(qv * qv), ks = warp_sum(kv * kv);
-      if ((j & 31) == 0) {
-        red_qk[j >> 5] = qs;
-        red_qk[4 + (j >> 5)] = ks;
-      }
+  float qv = 0.f, kv = 0.f, vv = 0.f;
+  if (j < DK) {
+    qv = tq.result(p.conv_w, cq);
+    kv = tk.result(p.conv_w, ck);
+    vv = tv.result(p.conv_w, cv);
+    tv.store(tail, C, cv);
+    const float qs = warp_sum(qv * qv), ks = warp_sum(kv * kv);
+    if ((j & 31) == 0) {
+      red_qk[j >> 5] = qs;
+      red_qk[4 + (j >> 5)] = ks;
     }
-    s_v[grp][j] = conv_step<KW>(p, tail, C, 2 * kd + h * DV + j, __bfloat162float(row[2 * kd + h * DV + j]), true);
   }
   __syncthreads();
-  if (rg == 0 && j == 0) {
-    float a = 0.f, bb = 0.f;
-#pragma unroll
-    for (int w = 0; w < WPH; ++w) {
-      a += red_ab[grp][w][0];
-      bb += red_ab[grp][w][1];
-    }
+  if (warp == 4) {
+    float a = warp_sum(lane < WARPS ? red_ab[lane][0] : 0.f), bb = warp_sum(lane < WARPS ? red_ab[lane][1] : 0.f);
     // the unfused path rounds the a/b projection outputs to bf16 before the gate math
     a = bf16_round(a);
     bb = bf16_round(bb);
     const float av = a + p.dt_bias[h];
     const float sp = av > 20.f ? av : log1pf(expf(av));
-    s_gate[grp][0] = __expf(-expf(p.a_log[h]) * sp);   // decay = exp(g)
-    s_gate[grp][1] = sigmoid_f(bb);
+    if (lane == 0) {
+      s_gate[0] = __expf(-expf(p.a_log[h]) * sp);   // decay = exp(g)
+      s_gate[1] = sigmoid_f(bb);
+    }
   }
-  if (grp == 0 && rg == 0) {
+  if (j < DK) {
     const float qn = rsqrtf(red_qk[0] + red_qk[1] + red_qk[2] + red_qk[3] + 1e-6f);
     const float kn = rsqrtf(red_qk[4] + red_qk[5] + red_qk[6] + red_qk[7] + 1e-6f);
     sq[j] = qv * qn * p.q_scale;
     sk[j] = kv * kn;
   }
   __syncthreads();
-  // ---- gated delta rule on rows [rg*ROWS, (rg+1)*ROWS) of state column j of head h
-  float* S = p.states + (size_t)slot * p.state_stride + (size_t)h * DK * DV + (size_t)rg * ROWS * DV;
-  const float decay = s_gate[grp][0], bt = s_gate[grp][1];
-  float col[ROWS];
-  float part = 0.f;
+  // ---- gated delta rule
+  const float decay = s_gate[0], bt = s_gate[1];
+  float4 part = make_float4(0.f, 0.f, 0.f, 0.f);
 #pragma unroll
   for (int i = 0; i < ROWS; ++i) {
-    col[i] = S[(size_t)i * DV + j] * decay;
-    part += col[i] * sk[rg * ROWS + i];
+    const float k = sk[warp * ROWS + i];
+    st[i].x *= decay; st[i].y *= decay; st[i].z *= decay; st[i].w *= decay;
+    part.x += st[i].x * k; part.y += st[i].y * k; part.z += st[i].z * k; part.w += st[i].w * k;
   }
-  s_part[grp][rg][j] = part;
+  *reinterpret_cast<float4*>(&s_part[warp][lane * 4]) = part;
   __syncthreads();
-  float kv_mem = 0.f;
+  if (j < DV) {
+    float kv_mem = 0.f;
 #pragma unroll
-  for (int g2 = 0; g2 < RG; ++g2) kv_mem += s_part[grp][g2][j];
-  const float delta = (s_v[grp][j] - kv_mem) * bt;
+    for (int w = 0; w < WARPS; ++w) kv_mem += s_part[w][j];
+    s_delta[j] = (vv - kv_mem) * bt;
+  }
   __syncthreads();   // s_part is reused for the read-out partials
-  part = 0.f;
+  const float4 delta = *reinterpret_cast<const float4*>(&s_delta[lane * 4]);
+  part = make_float4(0.f, 0.f, 0.f, 0.f);
 #pragma unroll
   for (int i = 0; i < ROWS; ++i) {
-    col[i] += sk[rg * ROWS + i] * delta;
-    S[(size_t)i * DV + j] = col[i];
-    part += col[i] * sq[rg * ROWS + i];
+    const float k = sk[warp * ROWS + i], q = sq[warp * ROWS + i];
+    st[i].x += k * delta.x; st[i].y += k * delta.y; st[i].z += k * delta.z; st[i].w += k * delta.w;
+    S[i * (DV / 4)] = st[i];
+    part.x += st[i].x * q; part.y += st[i].y * q; part.z += st[i].z * q; part.w += st[i].w * q;
   }
-  s_part[grp][rg][j] = part;
+  *reinterpret_cast<float4*>(&s_part[warp][lane * 4]) = part;
+  if constexpr (R > 1) asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");   // every head has read the q and k tails
+  if (j < DK && h % R == 0) {
+    tq.store(tail, C, cq);
+    tk.store(tail, C, ck);
+  }
   __syncthreads();
-  // ---- per-head gated RMSNorm by row group 0 (the unfused path stores o as bf16 first)
+  if (j >= DV) return;
+  // ---- per-head gated RMSNorm by the first 128 threads (the unfused path stores o as bf16 first)
   float o = 0.f;
-  if (rg == 0) {
 #pragma unroll
-    for (int g2 = 0; g2 < RG; ++g2) o += s_part[grp][g2][j];
-    o = bf16_round(o);
-    const float ss = warp_sum(o * o);
-    if ((j & 31) == 0) red_o[grp][j >> 5] = ss;
-  }
-  __syncthreads();
-  if (rg == 0) {
-    const float inv = rsqrtf((red_o[grp][0] + red_o[grp][1] + red_o[grp][2] + red_o[grp][3]) / (float)DV + p.eps);
-    const float z = __bfloat162float(row[2 * kd + vd + h * DV + j]);
-    const float y = o * inv * __bfloat162float(p.gamma[j]) * silu_f(z);
+  for (int w = 0; w < WARPS; ++w) o += s_part[w][j];
+  o = bf16_round(o);
+  const float ss = warp_sum(o * o);
+  if ((j & 31) == 0) red_o[j >> 5] = ss;
+  asm volatile("bar.sync 1, 128;" ::: "memory");
+  const float inv = rsqrtf((red_o[0] + red_o[1] + red_o[2] + red_o[3]) / (float)DV + p.eps);
+  const float z = __bfloat162float(row[2 * kd + vd + h * DV + j]);
+  const float y = bf16_round(o * inv * __bfloat162float(p.gamma[j]) * silu_f(z));
+  if (!p.terms.xq) {
     p.out[((size_t)b * p.Hv + h) * DV + j] = __float2bfloat16(y);
+    return;
   }
+  s_part[0][j] = y;
+  const uint32_t m = __reduce_max_sync(0xffffffffu, b200::f8t::bf16_magnitude(y));
+  if ((j & 31) == 0) red_m[j >> 5] = m;
+  asm volatile("bar.sync 1, 128;" ::: "memory");
+  if (j < 32) {
+    const b200::f8t::TermScale ts(max(max(red_m[0], red_m[1]), max(red_m[2], red_m[3])));
+    uint32_t hi, mid;
+    ts.split4(&s_part[0][j * 4], hi, mid);
+    int r;
+    uint8_t* dst = p.terms.hi_row(b, h, r);
+    dst += b200::f8t::term_offset(r, j);
+    *reinterpret_cast<uint32_t*>(dst) = hi;
+    *reinterpret_cast<uint32_t*>(dst + p.terms.cap * 128) = mid;
+    if (j == 0) *p.terms.scale(b, h) = ts.inv;
+  }
+}
+
+template <int R>
+static int launch_gdn(const GdnDecodeParams& p, int B, cudaStream_t stream) {
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = dim3(p.Hv, B);
+  cfg.blockDim = dim3(512);
+  cfg.stream = stream;
+  cudaLaunchAttribute attr[2];
+  attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attr[0].val.programmaticStreamSerializationAllowed = 1;
+  attr[1].id = cudaLaunchAttributeClusterDimension;
+  attr[1].val.clusterDim.x = R;
+  attr[1].val.clusterDim.y = 1;
+  attr[1].val.clusterDim.z = 1;
+  cfg.attrs = attr;
+  cfg.numAttrs = R > 1 ? 2 : 1;
+  return (int)cudaLaunchKernelEx(&cfg, gdn_decode_fused_kernel<4, R>, p);
 }
 
 // ------------------------------------------------------------------------------------------------
@@ -385,12 +446,13 @@ extern "C" {
 // proj: [B, ldp] bf16 holding q | k | v | z at offsets 0, kd, 2kd, 2kd+vd (kd = Hk*128, vd = Hv*128);
 // x: [B, hidden] bf16; w_ab: [2*Hv, hidden] bf16; conv_w: [2kd+vd, kw] bf16; tails: [slots, kw-1, 2kd+vd] bf16
 // (tail_stride elements per slot); states: fp32 [slots, Hv, 128, 128] (state_stride floats per slot);
-// out: [B, Hv*128] bf16.  Hv / Hk must be 1, 2 or 4 and kw == 4.
+// out: [B, Hv*128] bf16, or null with terms_xq / terms_sx: the result as E4M3 terms (gemm_fp8_terms.cu, tok tokens per tile, no
+// pair).  Hv / Hk must be 1, 2 or 4 and kw == 4.
 int b200_gdn_decode_fused(const void* proj, int ldp, const void* x, int hidden, const void* w_ab, const float* a_log,
                           const float* dt_bias, const void* conv_w, int kw, void* tails, long long tail_stride,
                           float* states, long long state_stride, const int* slot_ids, const void* gamma, void* out,
-                          int B, int Hv, int Hk, float eps, cudaStream_t stream) {
-  if (B <= 0 || Hv <= 0 || Hk <= 0 || Hv % Hk != 0 || kw != 4 || hidden % 8 != 0) return -6;
+                          int B, int Hv, int Hk, float eps, void* terms_xq, float* terms_sx, int tok, cudaStream_t stream) {
+  if ((!out && (!terms_xq || !terms_sx || tok < B || tok > b200::f8t::MAX_SINGLE)) || B <= 0 || Hv <= 0 || Hk <= 0 || Hv % Hk != 0 || kw != 4 || hidden % 8 != 0) return -6;
   GdnDecodeParams p;
   p.proj = reinterpret_cast<const __nv_bfloat16*>(proj);
   p.ldp = ldp;
@@ -402,6 +464,7 @@ int b200_gdn_decode_fused(const void* proj, int ldp, const void* x, int hidden, 
   p.conv_w = reinterpret_cast<const __nv_bfloat16*>(conv_w);
   p.tails = reinterpret_cast<__nv_bfloat16*>(tails);
   p.tail_stride = (size_t)tail_stride;
+  if ((reinterpret_cast<uintptr_t>(states) & 15) != 0 || state_stride % 4 != 0) return -6;      // rows are read 16 bytes at a time
   p.states = states;
   p.state_stride = (size_t)state_stride;
   p.slot_ids = slot_ids;
@@ -411,11 +474,14 @@ int b200_gdn_decode_fused(const void* proj, int ldp, const void* x, int hidden, 
   p.Hk = Hk;
   p.eps = eps;
   p.q_scale = rsqrtf((float)DK);
-  const dim3 grid(Hk, B);
+  p.terms.xq = out ? nullptr : reinterpret_cast<uint8_t*>(terms_xq);
+  p.terms.sx = terms_sx;
+  p.terms.tok = p.terms.cap = tok;
+  p.terms.kb = Hv;
   switch (Hv / Hk) {
-    case 1: return (int)b200::launch_pdl(gdn_decode_fused_kernel<4, 1, 4>, grid, dim3(512), 0, stream, p);
-    case 2: return (int)b200::launch_pdl(gdn_decode_fused_kernel<4, 2, 4>, grid, dim3(1024), 0, stream, p);
-    case 4: return (int)b200::launch_pdl(gdn_decode_fused_kernel<4, 4, 2>, grid, dim3(1024), 0, stream, p);
+    case 1: return launch_gdn<1>(p, B, stream);
+    case 2: return launch_gdn<2>(p, B, stream);
+    case 4: return launch_gdn<4>(p, B, stream);
     default: return -6;
   }
 }

@@ -483,8 +483,9 @@ class QwenHybridRuntime(PagedSequences):
         self._graphs: dict[int, tuple] = {}
         self.launches = 0  # kernels launched by the last forward (for the bench record)
         self._sp = False   # set while a sequence-parallel prefill chunk is in flight
-        # decode batches of <= 32 rows take the fused path; needs every FP8 K dimension to be a multiple of 128
+        # decode batches of up to fused_rows rows take the fused path; needs every FP8 K dimension to be a multiple of 128
         from ..ops.gemm import WF_FP8_B128
+        self.fused_rows = gemm.TERMS_SINGLE_T if W == 1 else gemm.STREAM_MAX_T
         self.fused_decode = all(l.proj.k % 128 == 0 and l.out.k % 128 == 0 and l.down.k % 128 == 0 and
                                 l.gate_up.k % 128 == 0 and l.gate_up.wfmt == WF_FP8_B128 and l.down.wfmt == WF_FP8_B128
                                 for l in weights.layers) and \
@@ -548,8 +549,9 @@ class QwenHybridRuntime(PagedSequences):
         return gemm.linear(x, w)
 
     def _expand_ahead(self, x: torch.Tensor, w: PackedLinear) -> None:
-        if x.shape[0] >= gemm.PREDECODE_MIN_T:
-            nxt = self._next_w.get(id(w))
+        nxt = self._next_w.get(id(w))
+        # a sequence-parallel product expands whatever its size
+        if x.shape[0] >= gemm.PREDECODE_MIN_T and nxt is not None and (self._sp or gemm.expands(x.shape[0], nxt)):
             fused = nxt is not None and id(nxt) in self._gate_up_ids and self._swiglu_fused(x.shape[0], nxt)
             gemm.prefetch_bf16(nxt, x.device, w, gate_up=fused)
 
@@ -575,6 +577,30 @@ class QwenHybridRuntime(PagedSequences):
         self._expand_ahead(x, w)
         return self.comm.all_reduce(gemm.linear(x, w))
 
+    # Projections of a decode step.  On one rank an activation goes to its matrix as the exact E4M3 terms the matrix is
+    # multiplied with (``gemm.Terms``); under tensor parallelism as E4M3 terms of the weight-streaming GEMM whose epilogue
+    # carries the all-reduce.
+    def _decode_norm(self, h: torch.Tensor, delta: torch.Tensor | None, gamma: torch.Tensor, want_bf16: bool):
+        """(h += delta) -> (its norm in bf16 or None, the norm as an operand of ``_decode_linear``)."""
+        eps = self.cfg.rms_norm_eps
+        if self.comm.world == 1:
+            return basic.rmsnorm_terms(h, delta, gamma, eps, True, want_bf16)
+        return basic.rmsnorm_split(h, delta, gamma, gemm.stream_layout(h.shape[0])[1], eps, True, want_bf16)
+
+    def _decode_linear(self, a, w: PackedLinear) -> torch.Tensor:
+        return gemm.linear_terms(a, w) if isinstance(a, gemm.Terms) else gemm.linear_stream(None, w, xsplit=a)
+
+    def _decode_row_linear(self, x, w: PackedLinear) -> torch.Tensor:
+        """Row-parallel projection of ``x``: bf16 rows or an operand of ``_decode_linear``."""
+        if self.comm.world == 1:
+            return gemm.linear_terms(x if isinstance(x, gemm.Terms) else gemm.split_terms(x), w)
+        return self._stream_row_parallel(x, w) if isinstance(x, torch.Tensor) else self._stream_row_parallel(None, w, x)
+
+    def _decode_act(self, gu: torch.Tensor):
+        if self.comm.world == 1:
+            return basic.silu_mul_terms(gu)
+        return basic.silu_mul_split(gu, gemm.stream_layout(gu.shape[0])[1])
+
     def _stream_row_parallel(self, x: torch.Tensor | None, w: PackedLinear, xsplit=None) -> torch.Tensor:
         """Row-parallel projection of a decode step (T <= 32): with a peer-memory communicator the all-reduce is done
         in the epilogue of the weight-streaming GEMM, otherwise GEMM then all-reduce."""
@@ -583,8 +609,20 @@ class QwenHybridRuntime(PagedSequences):
             return fused(x, w, xsplit=xsplit)
         return self.comm.all_reduce(gemm.linear_stream(x, w, xsplit=xsplit))
 
+    def _terms_rows(self, t: int, lw: LayerWeights) -> bool:
+        """Do the FP8 products of a ``t``-row batch through layer ``lw`` take their activations as E4M3 terms, straight from
+        the kernels that make them?"""
+        return self.comm.world == 1 and self.fused_decode and \
+            not any(gemm.expands(t, m) or not gemm.terms_fit(t, m) for m in (lw.proj, lw.out, lw.gate_up, lw.down))
+
     def _mlp(self, lw: LayerWeights, h: torch.Tensor, delta: torch.Tensor) -> torch.Tensor:
         cfg = self.cfg
+        if self._terms_rows(h.shape[0], lw):
+            _, a = basic.rmsnorm_terms(h, delta, lw.post_ln, cfg.rms_norm_eps, True, want_bf16=False)
+            with PROFILER.scope("lin.gate_up"):
+                act = basic.silu_mul_terms(gemm.linear_terms(a, lw.gate_up))
+            with PROFILER.scope("lin.down+ar.mlp"):
+                return gemm.linear_terms(act, lw.down)
         if self._sp:
             x = self.comm.reduce_norm_gather(h, lw.post_ln, cfg.rms_norm_eps, True)
         else:
@@ -599,10 +637,10 @@ class QwenHybridRuntime(PagedSequences):
             return self._row_parallel(act, lw.down)
 
     def _linear_attn(self, li: int, lw: LayerWeights, x: torch.Tensor, t: int, slots_t: torch.Tensor | None,
-                     slot: int | None) -> torch.Tensor:
+                     slot: int | None, terms: gemm.Terms | None = None) -> torch.Tensor:
         cfg = self.cfg
         with PROFILER.scope("lin.qkvz"):
-            proj = self._col_parallel(x, lw.proj)            # [T, 2kd + vd + vd]
+            proj = self._col_parallel(x, lw.proj) if terms is None else gemm.linear_terms(terms, lw.proj)    # [T, 2kd + vd + vd]
         ab = gemm.linear(x, lw.ab)                           # [T, 2 hv]
         cw = 2 * self.kd + self.vd
         idx = self.lin_layers.index(li)
@@ -656,9 +694,10 @@ class QwenHybridRuntime(PagedSequences):
         return attention.decode_kv8(c.fmt, q, k8, v8, ks, vs, meta["block_table"], meta["kv_len"], gate=gate,
                                     max_kv_len=meta["max_kv_len"], window=win, sinks=sinks, v_min=vm)
 
-    def _full_attn(self, li: int, lw: LayerWeights, x: torch.Tensor, t: int, positions, kv_slots, meta) -> torch.Tensor:
+    def _full_attn(self, li: int, lw: LayerWeights, x: torch.Tensor, t: int, positions, kv_slots, meta,
+                   terms: gemm.Terms | None = None) -> torch.Tensor:
         idx = self.full_layers.index(li)
-        proj = self._col_parallel(x, lw.proj)
+        proj = self._col_parallel(x, lw.proj) if terms is None else gemm.linear_terms(terms, lw.proj)
         o = self._attend(idx, lw, proj, t, positions, kv_slots, meta, self.cfg.rms_norm_eps)
         return self._row_parallel(o.view(t, self.hq * 128), lw.out)
 
@@ -672,14 +711,17 @@ class QwenHybridRuntime(PagedSequences):
         h = self._embed(ids)
         delta = None
         for i, lw in enumerate(w.layers):
-            if delta is None:
+            a = None
+            if self._terms_rows(t, lw):
+                x, a = basic.rmsnorm_terms(h, delta, lw.in_ln, cfg.rms_norm_eps, True, want_bf16=lw.kind == "linear")
+            elif delta is None:
                 x = basic.rmsnorm(h, lw.in_ln, cfg.rms_norm_eps, True)
             else:
                 x = basic.add_rmsnorm(h, delta, lw.in_ln, cfg.rms_norm_eps, True)
             if lw.kind == "linear":
-                d_attn = self._linear_attn(i, lw, x, t, slots_t, slot)
+                d_attn = self._linear_attn(i, lw, x, t, slots_t, slot, a)
             else:
-                d_attn = self._full_attn(i, lw, x, t, positions, kv_slots, meta)
+                d_attn = self._full_attn(i, lw, x, t, positions, kv_slots, meta, a)
             delta = self._mlp(lw, h, d_attn)
         if logits_rows is not None and self.keep_hidden:
             self.hidden_rows = basic.add_rmsnorm(h, delta, w.final_norm, cfg.rms_norm_eps, True)
@@ -728,29 +770,27 @@ class QwenHybridRuntime(PagedSequences):
         return gemm.linear(x.index_select(0, logits_rows), w.lm_head, out_f32=True)
 
     def _forward_decode(self, ids, positions, kv_slots, meta, slots_t) -> torch.Tensor:
-        """Decode step for up to 32 sequences: FP8 projections through the weight-streaming kernel (activations
-        handed over as E4M3 terms by the fused norm / activation kernels), one fused launch for the whole
-        Gated-DeltaNet token mixer.  Same math as ``_forward``; 9 launches per linear layer instead of 16."""
+        """Decode step for up to 64 sequences (32 under tensor parallelism): activations are handed to the FP8 products as E4M3
+        terms by the kernels that make them, one fused launch for the whole Gated-DeltaNet token mixer.  Same math as
+        ``_forward``; 8 launches per linear layer instead of 16."""
         cfg, w = self.cfg, self.w
         t = ids.numel()
-        _, terms = gemm.stream_layout(t)
         eps = cfg.rms_norm_eps
         h = self._embed(ids)
         delta = None
         for i, lw in enumerate(w.layers):
-            x, xs = basic.rmsnorm_split(h, delta, lw.in_ln, terms, eps, True, want_bf16=lw.kind == "linear")
-            proj = gemm.linear_stream(None, lw.proj, xsplit=xs)
+            x, a = self._decode_norm(h, delta, lw.in_ln, lw.kind == "linear")
+            proj = self._decode_linear(a, lw.proj)
             if lw.kind == "linear":
                 idx = self.lin_layers.index(i)
+                terms = gemm.empty_terms(t, self.vd, self.device) if self.comm.world == 1 else None
                 y = gdn.decode_fused(proj, x, lw.ab.weight, lw.a_log, lw.dt_bias, lw.conv_w, self.tails[:, idx],
-                                     self.states[:, idx], slots_t, lw.gdn_norm, self.hv_lin, self.hk_lin, eps)
-                d_attn = self._stream_row_parallel(y, lw.out)
+                                     self.states[:, idx], slots_t, lw.gdn_norm, self.hv_lin, self.hk_lin, eps, terms=terms)
             else:
-                o = self._attend(self.full_layers.index(i), lw, proj, t, positions, kv_slots, meta, eps)
-                d_attn = self._stream_row_parallel(o.view(t, self.hq * 128), lw.out)
-            _, xs2 = basic.rmsnorm_split(h, d_attn, lw.post_ln, terms, eps, True, want_bf16=False)
-            gu = gemm.linear_stream(None, lw.gate_up, xsplit=xs2)
-            delta = self._stream_row_parallel(None, lw.down, basic.silu_mul_split(gu, terms))
+                y = self._attend(self.full_layers.index(i), lw, proj, t, positions, kv_slots, meta, eps).view(t, self.hq * 128)
+            d_attn = self._decode_row_linear(y, lw.out)
+            _, a = self._decode_norm(h, d_attn, lw.post_ln, False)
+            delta = self._decode_row_linear(self._decode_act(self._decode_linear(a, lw.gate_up)), lw.down)
         x = basic.add_rmsnorm(h, delta, w.final_norm, eps, True)
         return gemm.linear(x, w.lm_head, out_f32=True)
 
@@ -827,7 +867,7 @@ class QwenHybridRuntime(PagedSequences):
 
     def _decode_body(self, buf, max_kv_len: int) -> torch.Tensor:
         meta = {"mode": "decode", "block_table": buf["bt"], "kv_len": buf["kv_len"], "max_kv_len": max_kv_len}
-        if buf["ids"].numel() <= gemm.STREAM_MAX_T and self.fused_decode:
+        if buf["ids"].numel() <= self.fused_rows and self.fused_decode:
             logits = self._forward_decode(buf["ids"], buf["pos"], buf["kv_slots"], meta, buf["slots"])
         else:
             logits = self._forward(buf["ids"], buf["pos"], buf["kv_slots"], meta, None, buf["slots"], None)

@@ -108,13 +108,12 @@ class QwenSpeculator:
         r_rows = ids.numel()
         pos, kv_slots, meta = self._rows_meta(st, r_rows)
         slot1 = torch.tensor([st.slot], dtype=torch.int32, device=rt.device)
-        _, terms = gemm.stream_layout(r_rows)
         eps = cfg.rms_norm_eps
         h = rt._embed(ids)
         delta = None
         for i, lw in enumerate(w.layers):
-            x, xs = basic.rmsnorm_split(h, delta, lw.in_ln, terms, eps, True, want_bf16=lw.kind == "linear")
-            proj = gemm.linear_stream(None, lw.proj, xsplit=xs)
+            x, a = rt._decode_norm(h, delta, lw.in_ln, lw.kind == "linear")
+            proj = rt._decode_linear(a, lw.proj)
             if lw.kind == "linear":
                 idx = rt.lin_layers.index(i)
                 ys = []
@@ -126,13 +125,11 @@ class QwenSpeculator:
                         self.ck_states[r, idx].copy_(rt.states[st.slot, idx])
                         self.ck_tails[r, idx].copy_(rt.tails[st.slot, idx])
                 y = torch.cat(ys) if r_rows > 1 else ys[0]
-                d_attn = rt._stream_row_parallel(y, lw.out)
             else:
-                o = rt._attend(rt.full_layers.index(i), lw, proj, r_rows, pos, kv_slots, meta, eps)
-                d_attn = rt._stream_row_parallel(o.view(r_rows, rt.hq * 128), lw.out)
-            _, xs2 = basic.rmsnorm_split(h, d_attn, lw.post_ln, terms, eps, True, want_bf16=False)
-            gu = gemm.linear_stream(None, lw.gate_up, xsplit=xs2)
-            delta = rt._stream_row_parallel(None, lw.down, basic.silu_mul_split(gu, terms))
+                y = rt._attend(rt.full_layers.index(i), lw, proj, r_rows, pos, kv_slots, meta, eps).view(r_rows, rt.hq * 128)
+            d_attn = rt._decode_row_linear(y, lw.out)
+            _, a = rt._decode_norm(h, d_attn, lw.post_ln, False)
+            delta = rt._decode_row_linear(rt._decode_act(rt._decode_linear(a, lw.gate_up)), lw.down)
         x = basic.add_rmsnorm(h, delta, w.final_norm, eps, True)
         logits = gemm.linear(x, w.lm_head, out_f32=True)
         return rt._next_tokens(logits), x

@@ -218,6 +218,14 @@ def _expanded_bf16(w: "PackedLinear", device, gate_up: bool = False) -> "PackedL
     return PackedLinear(WF_BF16, _expander(device).get(w, gate_up), None, w.n, w.k)
 
 
+def expands(t: int, w: "PackedLinear") -> bool:
+    """Does a ``t``-token product expand FP8 matrix ``w`` to bf16 first?  Prefill-sized batches that the CTA-pair kernel tiles
+    evenly (it reaches 1.6 PFLOP/s at 8192 tokens, and the expansion hides under the product before it); other batches
+    multiply the FP8 weights as they are (``linear_terms``: 1.2 PFLOP/s at 1000 tokens)."""
+    return (w.wfmt == WF_FP8_B128 and t >= PREDECODE_MIN_T and
+            (bool(_lib.lib().b200_gemm_2cta_supported(t, w.n, w.k)) or not terms_fit(t, w)))
+
+
 def swiglu_fusable(t: int, w: "PackedLinear") -> bool:
     """Can ``linear_swiglu`` take [gate | up] matrix ``w`` for ``t`` tokens?  FP8 weights (they are re-laid-out while
     being expanded), a prefill-sized batch, and a shape the CTA-pair kernel tiles evenly."""
@@ -254,7 +262,9 @@ def pick_splits(t: int, n: int, k: int) -> int:
     The persistent grid runs ceil(units / 148) waves of (tile, split) units; the split count that wastes
     the least of the last wave wins, subject to at least 8 k-blocks (512 columns) per split so the
     pipeline fill is amortised, and to a bound on the fp32 partial traffic for larger T."""
-    if t > 128:
+    if t > 128 or (t > 32 and n * k <= 1 << 21):
+        # a matrix of a megabyte or two (gate projections, 64 x 5120) is no stream to spread over the SMs: adding up eight
+        # splits of 64 tokens takes longer (57 us) than walking its K
         return 1
     tiles = ((n + 127) // 128) * ((t + _bn(t) - 1) // _bn(t))
     kb = (k + 63) // 64
@@ -275,6 +285,7 @@ def pick_splits(t: int, n: int, k: int) -> int:
 
 
 STREAM_MAX_T = 32   # token counts served by the weight-streaming FP8 kernel (csrc/kernels/gemm_w8a8s.cu)
+TERMS_SINGLE_T = 64  # token counts the one-CTA form of ``linear_terms`` serves
 
 
 def stream_layout(t: int) -> tuple[int, int]:
@@ -357,24 +368,84 @@ def linear_stream(x: torch.Tensor, w: PackedLinear, residual: torch.Tensor | Non
     return out
 
 
+@dataclass
+class Terms:
+    """bf16 activations as two E4M3 terms per value, in the order ``linear_terms`` streams them
+    (csrc/kernels/gemm_fp8_terms.cu): blocks of 256 x ``tok`` bytes per (token tile, 128 inputs), and their scales."""
+    xq: torch.Tensor              # uint8 [ceil(t / tok), k / 128, 2 tok, 128]
+    sx: torch.Tensor              # fp32 [ceil(t / tok), k / 128, tok], powers of two
+    t: int
+    k: int
+
+
+def _terms_plan(t: int, n: int, k: int) -> tuple[int, int, int]:
+    """(tokens per tile, floats of partial sums, tile counters) of a ``linear_terms`` product."""
+    tok, part, cnt = ctypes.c_int(), ctypes.c_longlong(), ctypes.c_int()
+    _lib.check(_lib.lib().b200_fp8_terms_plan(t, n, k, ctypes.byref(tok), ctypes.byref(part), ctypes.byref(cnt)), "fp8_terms_plan", 0)
+    return tok.value, part.value, cnt.value
+
+
+def empty_terms(t: int, k: int, device) -> Terms:
+    tok = _terms_plan(t, 128, k)[0]
+    blocks = ((t + tok - 1) // tok, k // 128)
+    return Terms(torch.empty(*blocks, 2 * tok, 128, dtype=torch.uint8, device=device),
+                 torch.empty(*blocks, tok, dtype=torch.float32, device=device), t, k)
+
+
+def split_terms(x: torch.Tensor) -> Terms:
+    """bf16 [T, K] (K % 128 == 0) as exact E4M3 terms."""
+    assert x.dtype == torch.bfloat16 and x.is_contiguous()
+    xt = empty_terms(*x.shape, x.device)
+    rc = _lib.lib().b200_split_terms(_lib.ptr(x), xt.t, xt.k, xt.sx.shape[2], _lib.ptr(xt.xq), _lib.ptr(xt.sx), _lib.stream())
+    _lib.check(rc, "split_terms")
+    return xt
+
+
+def terms_fit(t: int, w: "PackedLinear") -> bool:
+    """Can ``linear_terms`` take FP8 matrix ``w`` for ``t`` tokens?"""
+    tiles = ((w.n + 255) // 256 * 2) * ((t + 255) // 256)
+    return w.wfmt == WF_FP8_B128 and w.k % 128 == 0 and t <= 65535 and tiles <= MAX_TILE_COUNTERS
+
+
+def linear_terms(xt: Terms, w: PackedLinear, residual: torch.Tensor | None = None, out: torch.Tensor | None = None) -> torch.Tensor:
+    """``x @ w^T`` (+ residual) for FP8 block-128 weights: bf16 [T, N]."""
+    assert w.wfmt == WF_FP8_B128 and xt.k == w.k
+    dev = xt.xq.device
+    if out is None:
+        out = torch.empty(xt.t, w.n, dtype=torch.bfloat16, device=dev)
+    _, part, cnt = _terms_plan(xt.t, w.n, w.k)
+    assert cnt <= MAX_TILE_COUNTERS
+    ws, counters = _workspace(part, dev)
+    rc = _lib.lib().b200_gemm_fp8_terms(_lib.ptr(w.weight), _lib.ptr(w.scales), _lib.ptr(xt.xq), _lib.ptr(xt.sx), _lib.ptr(out),
+                                        _lib.ptr(residual), xt.t, w.n, w.k, _lib.ptr(ws), _lib.ptr(counters),
+                                        _lib.ptr(_lib.status_word(dev)), _lib.stream())
+    _lib.check(rc, "gemm_fp8_terms")
+    return out
+
+
 def linear(x: torch.Tensor, w: PackedLinear, residual: torch.Tensor | None = None,
            out: torch.Tensor | None = None, splits: int | None = None,
            out_f32: bool = False, stream: bool | None = None) -> torch.Tensor:
-    """``x [T, K] bf16`` -> ``[T, N]`` bf16 (or fp32 when ``out_f32``).  FP8 weights with T <= 32 go to the
-    weight-streaming kernel (``stream=False`` forces the decode-warp kernel); split-K partials are
-    reduced inside the kernel by the last-arriving CTA of each output tile."""
+    """``x [T, K] bf16`` -> ``[T, N]`` bf16 (or fp32 when ``out_f32``).  FP8 weights go to the FP8 tensor pipe with the
+    activations as exact E4M3 terms, or, in prefill-sized batches that the CTA-pair kernel tiles evenly, are expanded to
+    bf16 first; ``stream=False``, or a number of ``splits``, asks for the decode-warp kernel (up to 32 tokens and not
+    ``stream=False``: the weight-streaming kernel), whose split-K partials are reduced by the last-arriving CTA of each
+    output tile."""
     assert x.dtype == torch.bfloat16 and x.is_cuda and x.dim() == 2 and x.is_contiguous()
     t, k = x.shape
     assert k == w.k, (k, w.k)
     n = w.n
-    if w.wfmt == WF_FP8_B128 and t <= STREAM_MAX_T and k % 128 == 0 and not out_f32 and stream is not False:
-        return linear_stream(x, w, residual, out, splits)
-    if w.wfmt == WF_FP8_B128 and t >= PREDECODE_MIN_T and not out_f32 and n % 128 == 0 and k % 64 == 0:
-        # prefill-sized batch: every weight tile would be decoded once per 256-token tile of the batch, so the matrix is
-        # expanded to bf16 once (one pass over the weights, ~3 % of the GEMM) and multiplied by the bf16 path, which
-        # has no decode traffic through shared memory (1.17 / 1.38 PFLOP/s against 1.09 / 1.16 at 8192 x 17408 x 5120
-        # and 8192 x 5120 x 17408)
-        w = _expanded_bf16(w, x.device)
+    if w.wfmt == WF_FP8_B128 and not out_f32:
+        if splits is not None and t <= STREAM_MAX_T and k % 128 == 0 and stream is not False:
+            return linear_stream(x, w, residual, out, splits)
+        if splits is None and stream is not False and terms_fit(t, w) and not expands(t, w):
+            return linear_terms(split_terms(x), w, residual, out)
+        if t >= PREDECODE_MIN_T and n % 128 == 0 and k % 64 == 0:
+            # every weight tile would be decoded once per 256-token tile of the batch, so the matrix is expanded to bf16
+            # once (one pass over the weights, ~3 % of the GEMM) and multiplied by the bf16 path, which has no decode
+            # traffic through shared memory (1.17 / 1.38 PFLOP/s against 1.09 / 1.16 at 8192 x 17408 x 5120 and
+            # 8192 x 5120 x 17408)
+            w = _expanded_bf16(w, x.device)
     if splits is None:
         splits = 1 if out_f32 else pick_splits(t, n, k)
     L = _lib.lib()

@@ -1,0 +1,153 @@
+"""FP8 block-128 products from exact E4M3 terms (csrc/kernels/gemm_fp8_terms.cu, gemm_fp8_pair.cu)."""
+import pytest
+import torch
+
+from deepseek_v4_2080ti_b200.formats import fp8 as fp8fmt
+
+# (tokens, features, inputs): both sides of every tile width (16, 32, 64 tokens; 256 on pairs), ragged feature counts, an odd
+# number of weight tiles, one K block, runs that cut tiles several times, more runs than one per tile
+SHAPES = [(1, 128, 128), (1, 5120, 4096), (16, 384, 512), (17, 1000, 1280), (32, 1536, 4096), (33, 201, 640), (64, 12288, 512),
+          (65, 128, 128), (100, 384, 1024), (128, 200, 384), (129, 640, 2560), (256, 1024, 4096), (257, 5120, 1024),
+          (300, 33, 256), (700, 3072, 1152)]
+
+
+def _terms(xt, t, k):
+    """hi + mid of every activation, times its block's scale, from the stored layout."""
+    tok = xt.sx.shape[2]
+    cap = tok // 2 if tok == 256 else tok
+    n, kb = xt.sx.shape[:2]
+    b = xt.xq.reshape(n, kb, tok // cap, 2, cap, 8, 16)
+    rows = torch.arange(cap, device=b.device)[:, None]
+    src = torch.arange(8, device=b.device)[None] ^ (rows & 7)
+    b = torch.gather(b, 5, src[None, None, None, None, :, :, None].expand_as(b))
+    v = b.reshape(n, kb, tok // cap, 2, cap, 32, 4)[..., [0, 2, 1, 3]].contiguous().view(torch.float8_e4m3fn).float()
+    v = v.sum(3).reshape(n, kb, tok, 128) * xt.sx[..., None]
+    return v.permute(0, 2, 1, 3).reshape(n * tok, k)[:t]
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("t", [1, 20, 64, 65, 200, 300])
+def test_terms_are_exact(t):
+    from deepseek_v4_2080ti_b200.ops import gemm
+    torch.manual_seed(t)
+    x = (torch.randn(t, 384, device="cuda") * torch.exp(2 * torch.randn(t, 384, device="cuda"))).bfloat16()
+    x[0, :128] = 0
+    got, xf = _terms(gemm.split_terms(x), t, 384), x.float()
+    top = xf.view(t, 3, 128).abs().amax(-1, keepdim=True).expand(t, 3, 128).reshape(t, 384)
+    small = xf.abs() < top * 2.0 ** -9
+    assert torch.equal(got[~small], xf[~small])
+    assert ((got - xf).abs() <= top * 2.0 ** -17).all()
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("t,n,k", SHAPES)
+def test_product_matches_64_bit(t, n, k):
+    from deepseek_v4_2080ti_b200.ops import _lib, gemm
+    torch.manual_seed(t + n + k)
+    q, s = fp8fmt.quantize_block128(torch.randn(n, k, device="cuda") * 0.05)
+    w = gemm.PackedLinear.from_fp8(q, s)
+    x = torch.randn(t, k, device="cuda").bfloat16()
+    x[:, ::7] *= 8.0
+    r = torch.randn(t, n, device="cuda").bfloat16()
+    wide = torch.empty(t, n + 1, dtype=torch.bfloat16, device="cuda")
+    out = wide.view(-1)[1:t * n + 1].view(t, n)                      # rows that no 16-byte access fits
+    xt = gemm.split_terms(x)
+    y, z, u = gemm.linear_terms(xt, w), gemm.linear_terms(xt, w, residual=r), gemm.linear_terms(xt, w, out=out)
+    again = gemm.linear_terms(xt, w)
+    torch.cuda.synchronize()
+    _lib.check_status()
+    ref = x.double() @ fp8fmt.dequantize_block128(q, s).double().t()
+    rel = lambda a, b: ((a.double() - b).norm() / b.norm()).item()
+    # rounding the result to bf16 is at most 2^-9 of each value; fp32 sums and subnormal terms stay far below
+    assert rel(y, ref) < 2.0 ** -9 and rel(z, ref + r.double()) < 2.0 ** -9
+    assert torch.equal(y, again) and torch.equal(y, u)
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("t", [3, 80])
+def test_infinities_and_nans_stay_in_their_row(t):
+    from deepseek_v4_2080ti_b200.ops import gemm
+    torch.manual_seed(t)
+    q, s = fp8fmt.quantize_block128(torch.randn(256, 256, device="cuda"))
+    w, wd = gemm.PackedLinear.from_fp8(q, s), fp8fmt.dequantize_block128(q, s)
+    x = torch.randn(t, 256, device="cuda").bfloat16()
+    clean = gemm.linear_terms(gemm.split_terms(x), w)
+    x[0, 5], x[1, 200] = float("inf"), float("nan")
+    y = gemm.linear_terms(gemm.split_terms(x), w)
+    ref = x[:1].float() @ wd.t()
+    assert torch.equal(y[2:], clean[2:]) and y[1].isnan().all()
+    assert torch.equal(y[0].float().isinf(), ref[0].isinf()) and torch.equal(y[0].float()[ref[0].isinf()], ref[0][ref[0].isinf()])
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("t,cols", [(1, 128), (3, 5120), (16, 8192), (33, 8320), (65, 20480), (300, 384)])
+def test_norm_leaves_its_result_as_terms(t, cols):
+    from deepseek_v4_2080ti_b200.ops import basic
+    torch.manual_seed(t + cols)
+    h, d = (torch.randn(t, cols, device="cuda").bfloat16() for _ in range(2))
+    g = (torch.randn(cols, device="cuda") * 0.1).bfloat16()
+    stream = h.clone()
+    out, xt = basic.rmsnorm_terms(stream, d, g, 1e-6, True)
+    assert torch.equal(stream, (h.float() + d.float()).bfloat16())
+    ref = basic.rmsnorm_ref(stream, g, 1e-6, True)
+    assert ((out.float() - ref).abs() <= ref.abs() * 2.0 ** -8 + 1e-6).all()        # bf16 rounding, fp32 sums in any order
+    got = _terms(xt, t, cols)
+    assert ((got - out.float()).abs() <= out.float().view(t, -1, 128).abs().amax(-1).repeat_interleave(128, 1) * 2.0 ** -17).all()
+    none, alone = basic.rmsnorm_terms(stream, None, g, 1e-6, True, want_bf16=False)
+    assert none is None and torch.equal(_terms(alone, t, cols), got)
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("t,inter", [(1, 128), (7, 17408), (64, 2176), (70, 384)])
+def test_activation_leaves_its_result_as_terms(t, inter):
+    from deepseek_v4_2080ti_b200.ops import basic
+    torch.manual_seed(t + inter)
+    gu = (torch.randn(t, 2 * inter, device="cuda") * 2).bfloat16()
+    ref, got = basic.silu_mul_ref(gu), _terms(basic.silu_mul_terms(gu), t, inter)
+    top = ref.view(t, -1, 128).abs().amax(-1).repeat_interleave(128, 1)
+    assert ((got - ref).abs() <= ref.abs() * 2.0 ** -8 + top * 2.0 ** -17).all()
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("b,hv,hk", [(1, 4, 2), (20, 4, 4), (33, 8, 2)])
+def test_decode_mixer_leaves_its_result_as_terms(b, hv, hk):
+    from deepseek_v4_2080ti_b200.ops import gdn, gemm
+    torch.manual_seed(b)
+    kd, vd, hidden = hk * 128, hv * 128, 512
+    bf = lambda *s, std=1.0: (torch.randn(*s, device="cuda") * std).bfloat16()
+    proj, x, w_ab, conv, gamma = bf(b, 2 * kd + 2 * vd), bf(b, hidden), bf(2 * hv, hidden, std=0.03), bf(2 * kd + vd, 4, std=0.3), bf(128)
+    a_log, dt = torch.rand(hv, device="cuda"), torch.rand(hv, device="cuda")
+    tails, states = bf(b, 3, 2 * kd + vd), torch.randn(b, hv, 128, 128, device="cuda") * 0.1
+    slots = torch.randperm(b, device="cuda").int()
+    args = lambda: (proj, x, w_ab, a_log, dt, conv, tails.clone(), states.clone(), slots, gamma, hv, hk)
+    y = gdn.decode_fused(*args()).float()
+    got = _terms(gdn.decode_fused(*args(), terms=gemm.empty_terms(b, vd, "cuda")), b, vd)
+    assert ((got - y).abs() <= y.view(b, hv, 128).abs().amax(-1).repeat_interleave(128, 1) * 2.0 ** -17).all()
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("t,n,k", [(65, 64, 5120), (129, 200, 1024), (333, 64, 5120), (700, 256, 512)])
+def test_narrow_bf16_matrices(t, n, k):
+    """Few feature tiles: the tokens are tiled finer."""
+    from deepseek_v4_2080ti_b200.ops import gemm
+    torch.manual_seed(t + n)
+    x, w = torch.randn(t, k, device="cuda").bfloat16(), (torch.randn(n, k, device="cuda") * 0.05).bfloat16()
+    ref = x.double() @ w.double().t()
+    y, f = gemm.linear(x, gemm.PackedLinear.from_bf16(w)), gemm.linear(x, gemm.PackedLinear.from_bf16(w), out_f32=True)
+    assert ((y.double() - ref).norm() / ref.norm()).item() < 2.0 ** -9
+    assert ((f.double() - ref).norm() / ref.norm()).item() < 1e-5
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("t,k,h", [(1, 6, 4096), (3, 1, 8), (5, 9, 1032), (2, 4, 100)])
+def test_expert_rows_are_combined(t, k, h):
+    """Eight columns per thread, and rows that do not divide into eights; routes held elsewhere are skipped."""
+    from deepseek_v4_2080ti_b200.ops import _lib
+    torch.manual_seed(h)
+    y, base = torch.randn(t * k, h, device="cuda").bfloat16(), torch.randn(t, h, device="cuda").bfloat16()
+    rows = torch.randperm(t * k, device="cuda").int().view(t, k)
+    rows[0, 0] = -1
+    w, out = torch.rand(t, k, device="cuda"), torch.empty(t, h, dtype=torch.bfloat16, device="cuda")
+    _lib.check(_lib.lib().b200_moe_combine(_lib.ptr(y), _lib.ptr(rows), _lib.ptr(w), _lib.ptr(base), _lib.ptr(out), t, k, h, _lib.stream()), "moe_combine")
+    ref = base.double() + torch.where(rows[..., None] >= 0, w.double()[..., None] * y.double()[rows.clamp_min(0).long()], 0.0).sum(1)
+    assert ((out.double() - ref).abs() <= ref.abs() * 2.0 ** -8 + 1e-5).all()
