@@ -1,13 +1,13 @@
 // Weight-decoding tensor-core GEMM for sm_100a:  Y[T, N] = X[T, K] * W[N, K]^T.
 //
-// Design (one persistent CTA per SM, 14 warps, warp-specialised):
+// Design (one persistent CTA per SM, 6 warps and those that decode, warp-specialised):
 //   * W is the UMMA "A" operand (M = 128 output features per tile) and the
 //     activations are the "B" operand (N = BN tokens, 16..256), so the same
 //     kernel serves prefill (BN = 256) and decode batches (BN = 16..64) while
 //     the weight tile is always a full 128-row MMA.
 //   * warp 4 streams raw weight bytes and bf16 activations with TMA
 //     (cp.async.bulk.tensor, destination = this CTA only, never multicast);
-//   * warps 6..13 decode the raw weight tile (FP8 E4M3 with one scale per
+//   * warps 6.. decode the raw weight tile (FP8 E4M3 with one scale per
 //     128x128 block) into bf16, written in the 128-byte-swizzled K-major layout
 //     the tensor core reads; the quantised matrix is never expanded in HBM;
 //   * warp 5 issues tcgen05.mma (kind::f16, fp32 accumulate in TMEM, two
@@ -25,6 +25,7 @@
 // instantiate it for their weight formats so the formats compile in parallel.)
 #pragma once
 #include <cuda_bf16.h>
+#include "launch.h"
 #include "per_device.h"
 #include <cuda_fp8.h>
 #include <cuda_fp16.h>
@@ -43,8 +44,6 @@ constexpr int NUM_EPI_WARPS = 4;
 constexpr int TMA_WARP = 4;
 constexpr int MMA_WARP = 5;
 constexpr int DEC_WARP0 = 6;
-constexpr int NUM_DEC_WARPS = 8;
-constexpr int NUM_THREADS = (DEC_WARP0 + NUM_DEC_WARPS) * 32;  // 448
 
 // WF_FP4: E2M1 nibbles (low nibble first) with one UE8M0 scale per 32 inputs, stored tile-major as
 // [m_tile][kb][128 rows x 32 code bytes | 128 rows x 2 scale bytes] (4352 bytes per stage).
@@ -178,16 +177,21 @@ struct SmemLayout {
   static constexpr int EPI_BYTES =
       ((WFMT == WF_BF16 && BN >= 128) || (WFMT == WF_FP8_B128 && BN == 128)) ? 16384 : 0;
   static constexpr int BUDGET = 232448 - 1024 /*align slack*/ - 512 /*barriers*/ - EPI_BYTES;
-  static constexpr int SA = (WFMT == WF_BF16) ? 0 : 4;
   static constexpr int W_STAGE_BYTES = (WFMT == WF_BF16) ? A_BYTES : RAW_BYTES;
   static constexpr int STAGE_BYTES = W_STAGE_BYTES + X_BYTES;
-  static constexpr int SR_RAW = (BUDGET - SA * A_BYTES) / STAGE_BYTES;
-  static constexpr int SR = SR_RAW > 16 ? 16 : SR_RAW;
-  static constexpr int TOTAL = SR * STAGE_BYTES + SA * A_BYTES + EPI_BYTES + 1024 + 512;
+  static constexpr int fit(int sa) { return (BUDGET - sa * A_BYTES) / STAGE_BYTES; }
   // Decode warps work in GROUPS independent groups; group g owns decoded slot g and every
-  // GROUPS-th k-block, so barrier/fence latency of one stage overlaps another's ALU work.
-  static constexpr int GROUPS = 4;
-  static constexpr int WARPS_PER_GROUP = NUM_DEC_WARPS / GROUPS;
+  // GROUPS-th k-block, so barrier/fence latency of one stage overlaps another's ALU work.  A slot's round - decode, product,
+  // commit, free - is some 2500 cycles for the formats with a long unpacking, so those take as many slots as shared memory
+  // holds beside a raw ring of as many stages, and more warps; FP8, a shift and a mask, keeps four slots and eight warps.
+  static constexpr bool LONG_UNPACK = WFMT != WF_BF16 && WFMT != WF_FP8_B128;
+  static constexpr int GROUPS = !LONG_UNPACK ? 4 : fit(8) >= 8 ? 8 : fit(6) >= 6 ? 6 : 4;
+  static constexpr int WARPS_PER_GROUP = LONG_UNPACK && GROUPS == 4 ? 4 : 2;
+  static constexpr int DEC_WARPS = WFMT == WF_BF16 ? 0 : GROUPS * WARPS_PER_GROUP;
+  static constexpr int THREADS = (DEC_WARP0 + DEC_WARPS) * 32;
+  static constexpr int SA = (WFMT == WF_BF16) ? 0 : GROUPS;
+  static constexpr int SR = fit(SA) > 16 ? 16 : fit(SA);
+  static constexpr int TOTAL = SR * STAGE_BYTES + SA * A_BYTES + EPI_BYTES + 1024 + 512;
   static_assert(SR >= 2, "pipeline needs at least two raw stages");
 };
 
@@ -198,6 +202,21 @@ __device__ __forceinline__ void fp8x4_to_bf16x4_raw(uint32_t q, uint32_t& w01, u
   uint32_t q2 = q << 8;
   w01 = (q2 & 0x80008000u) | ((q2 & 0x7F007F00u) >> 4);
 }
+// Four E2M1 codes (low 16 bits, low nibble first) -> two bf16x2 words.  The upper and lower bytes of the eight bf16 magnitudes
+// are tables in registers that one byte permutation reads for four codes at a time: 2 instructions per weight where placing
+// exponent and mantissa bits one byte at a time took 5.
+__device__ __forceinline__ void e2m1x4_to_bf16x4(uint32_t q, uint32_t& w01, uint32_t& w23) {
+  const uint32_t sel = q & 0x7777u;
+  const uint32_t lo = __byte_perm(0xC0800000u, 0xC0804000u, sel);        // 0, .5, 1, 1.5 | 2, 3, 4, 6
+  uint32_t hi = __byte_perm(0x3F3F3F00u, 0x40404040u, sel);
+  hi |= __byte_perm(q << 4, q, 0x5140) & 0x80808080u;                    // bit 3 of each code to its byte's sign
+  w01 = __byte_perm(lo, hi, 0x5140);
+  w23 = __byte_perm(lo, hi, 0x7362);
+}
+// Byte i of four small integers -> float, without the conversion unit (a quarter of the rate): 2^23 + v has v in its low bits.
+__device__ __forceinline__ float byte_to_float(uint32_t four, int i) {
+  return __uint_as_float(__byte_perm(four, 0x4B000000u, 0x7440 | i)) - 8388608.f;
+}
 __device__ __forceinline__ uint32_t bf16x2_mul(uint32_t a, uint32_t b) {
   uint32_t d;
   asm("mul.rn.bf16x2 %0, %1, %2;" : "=r"(d) : "r"(a), "r"(b));
@@ -205,7 +224,7 @@ __device__ __forceinline__ uint32_t bf16x2_mul(uint32_t a, uint32_t b) {
 }
 
 template <int BN, int WFMT>
-__global__ void __launch_bounds__(NUM_THREADS, 1)
+__global__ void __launch_bounds__((SmemLayout<BN, WFMT>::THREADS), 1)
 gemm_wdec_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constant__ CUtensorMap tmX,
                  GemmParams p) {
   using L = SmemLayout<BN, WFMT>;
@@ -263,7 +282,11 @@ gemm_wdec_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constant_
   __syncthreads();
   tc_fence_after();
   const uint32_t tmem_base = *tmem_slot;
-  const uint32_t ar_epoch_at_entry = p.ar_mode ? p.comm.ctrl[0] + 1 : 0;
+  // launched as a programmatic dependent: barriers and tensor memory are set up while the previous kernel drains
+  pdl_wait();
+  pdl_launch_dependents();
+  const int ar_mode = WFMT <= WF_FP4 ? p.ar_mode : 0;      // the GGUF entry points have no collective form
+  const uint32_t ar_epoch_at_entry = ar_mode ? p.comm.ctrl[0] + 1 : 0;
 
   const int total_work = p.work_table ? *p.num_work : p.m_tiles * p.n_tiles * p.splits;
   const int kb_per_split = (p.kb_total + p.splits - 1) / p.splits;
@@ -332,59 +355,52 @@ gemm_wdec_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constant_
     }
   } else if (warp == MMA_WARP) {
     // -------------------------------------------------------------- MMA issuer
-    if (lane == 0) {
-      constexpr uint32_t idesc = umma_idesc_bf16(BM, BN);
-      uint32_t it = 0;
-      uint32_t tile_i = 0;
-      for (int w = blockIdx.x; w < total_work && !*abort_flag; w += gridDim.x, ++tile_i) {
-        const int split = get_work<BN>(p, w).split;
-        const int kb0 = split * kb_per_split;
-        const int kb1 = min(p.kb_total, kb0 + kb_per_split);
-        const int buf = tile_i & 1;
-        const uint32_t acc_ph = (tile_i >> 1) & 1;
-        if (!mbar_wait(&acc_empty[buf], acc_ph ^ 1)) {
-          atomicExch(p.status, ERR_WAIT_ACC);
-          *abort_flag = 1;
-          break;
+    // The whole warp walks the pipeline and its elected lane issues: from a lane that branched off alone the operands do not
+    // sit in uniform registers and each instruction costs some 120 cycles, which bounded every k-block of small token tiles.
+    const uint32_t on = elect_one();
+    constexpr uint32_t idesc = umma_idesc_bf16(BM, BN);
+    uint32_t it = 0;
+    uint32_t tile_i = 0;
+    int err = 0;
+    for (int w = blockIdx.x; w < total_work; w += gridDim.x, ++tile_i) {
+      const int split = get_work<BN>(p, w).split;
+      const int kb0 = split * kb_per_split;
+      const int kb1 = min(p.kb_total, kb0 + kb_per_split);
+      const int buf = tile_i & 1;
+      const uint32_t acc_ph = (tile_i >> 1) & 1;
+      if (!mbar_wait(&acc_empty[buf], acc_ph ^ 1)) err = ERR_WAIT_ACC;
+      if (__any_sync(0xffffffffu, err != 0 || *abort_flag != 0)) break;
+      tc_fence_after();
+      const uint32_t tmem_d = tmem_base + buf * BN;
+      for (int kb = kb0; kb < kb1; ++kb, ++it) {
+        const int s = it % S;
+        const uint32_t ph = (it / S) & 1;
+        if (!mbar_wait(&tma_full[s], ph)) err = ERR_WAIT_TMA;
+        const int sa = (WFMT == WF_BF16) ? s : (int)(it % SAB);
+        if (WFMT != WF_BF16) {
+          if (!err && !mbar_wait(&a_full[sa], (it / SAB) & 1)) err = ERR_WAIT_DEQUANT;
         }
+        if (__any_sync(0xffffffffu, err != 0)) break;
         tc_fence_after();
-        const uint32_t tmem_d = tmem_base + buf * BN;
-        bool failed = false;
-        for (int kb = kb0; kb < kb1; ++kb, ++it) {
-          const int s = it % S;
-          const uint32_t ph = (it / S) & 1;
-          if (!mbar_wait(&tma_full[s], ph)) {
-            atomicExch(p.status, ERR_WAIT_TMA);
-            failed = true;
-            break;
-          }
-          const int sa = (WFMT == WF_BF16) ? s : (int)(it % SAB);
-          if (WFMT != WF_BF16) {
-            if (!mbar_wait(&a_full[sa], (it / SAB) & 1)) {
-              atomicExch(p.status, ERR_WAIT_DEQUANT);
-              failed = true;
-              break;
-            }
-          }
-          tc_fence_after();
-          const uint64_t da = umma_desc_sw128(sA + sa * L::A_BYTES);
-          const uint64_t db = umma_desc_sw128(sX + s * L::X_BYTES);
+        const uint64_t da = umma_desc_sw128(sA + sa * L::A_BYTES);
+        const uint64_t db = umma_desc_sw128(sX + s * L::X_BYTES);
 #pragma unroll
-          for (int k = 0; k < BK / 16; ++k) {
-            // advance 16 bf16 = 32 bytes inside the swizzle row: +2 in 16-byte units
-            umma_bf16_ss(tmem_d, da + 2 * k, db + 2 * k, idesc, (kb > kb0 || k > 0) ? 1u : 0u);
-          }
-          // One commit per k-block frees the raw stage for the producer and, SA k-blocks later, the
-          // decoded slot for the decode warps (they wait on the same barrier): tcgen05.commit occupies
-          // the tensor pipe for a few hundred cycles, so a second commit per k-block would cap the rate.
-          umma_commit(&empty[s]);
+        for (int k = 0; k < BK / 16; ++k) {
+          // advance 16 bf16 = 32 bytes inside the swizzle row: +2 in 16-byte units
+          umma_bf16_ss_warp(on, tmem_d, da + 2 * k, db + 2 * k, idesc, (kb > kb0 || k > 0) ? 1u : 0u);
         }
-        if (failed) {
-          *abort_flag = 1;
-          break;
-        }
-        umma_commit(&acc_full[buf]);
+        // One commit per k-block frees the raw stage for the producer and, SA k-blocks later, the
+        // decoded slot for the decode warps (they wait on the same barrier): tcgen05.commit occupies
+        // the tensor pipe for a few hundred cycles, so a second commit per k-block would cap the rate.
+        umma_commit_warp(on, &empty[s]);
       }
+      if (__any_sync(0xffffffffu, err != 0)) break;
+      umma_commit_warp(on, &acc_full[buf]);
+    }
+    err = (int)__reduce_max_sync(0xffffffffu, (unsigned)err);
+    if (err) {
+      if (lane == 0) atomicExch(p.status, err);
+      *abort_flag = 1;
     }
   } else if (warp >= DEC_WARP0) {
     // ------------------------------------------------- weight decode (FP8 -> bf16)
@@ -485,10 +501,9 @@ gemm_wdec_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constant_
               const int i = d + rep * GT;
               const int r = i >> 1, hh = i & 1;       // row, which half of the 64-wide K tile
               const uint4 qv = *reinterpret_cast<const uint4*>(raw + r * 32 + hh * 16);
-              // The code bits placed at exponent/mantissa positions of a bf16 read as value * 2^-126, so the
-              // multiplier is 2^(e-127) * 2^126 = 2^(e-1): a bf16 with biased exponent e + 126, built directly.
+              // 2^(e-127) is a bf16 with biased exponent e; 2^-127 is below the normal numbers
               const uint32_t e = sc_bytes[r * 2 + hh];
-              const uint32_t s1 = min(e + 126u, 254u) << 7;
+              const uint32_t s1 = e ? min(e, 254u) << 7 : 0x40u;
               const uint32_t sw2 = s1 | (s1 << 16);
               const uint32_t qq[4] = {qv.x, qv.y, qv.z, qv.w};
               uint8_t* rowp = A + (r >> 3) * 1024 + (r & 7) * 128;
@@ -496,14 +511,10 @@ gemm_wdec_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constant_
 #pragma unroll
               for (int wd = 0; wd < 4; ++wd) {        // 4 bytes = 8 values = one 16-byte output chunk
                 uint4 o;
-                uint32_t* ow = reinterpret_cast<uint32_t*>(&o);
-#pragma unroll
-                for (int b = 0; b < 4; ++b) {
-                  const uint32_t by = (qq[wd] >> (8 * b)) & 0xFFu;
-                  const uint32_t t = by | (by << 12);   // low nibble at bits 0..3, high nibble at bits 16..19
-                  const uint32_t v = ((t & 0x00070007u) << 6) | ((t & 0x00080008u) << 12);
-                  ow[b] = bf16x2_mul(v, sw2);
-                }
+                e2m1x4_to_bf16x4(qq[wd], o.x, o.y);
+                e2m1x4_to_bf16x4(qq[wd] >> 16, o.z, o.w);
+                o.x = bf16x2_mul(o.x, sw2); o.y = bf16x2_mul(o.y, sw2);
+                o.z = bf16x2_mul(o.z, sw2); o.w = bf16x2_mul(o.w, sw2);
                 *reinterpret_cast<uint4*>(rowp + (((hh * 4 + wd) ^ sw) << 4)) = o;
               }
             }
@@ -531,21 +542,18 @@ gemm_wdec_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constant_
                 const int4 a = *reinterpret_cast<const int4*>(qrow), b = *reinterpret_cast<const int4*>(qrow + 16);
                 const int w8[8] = {a.x, a.y, a.z, a.w, b.x, b.y, b.z, b.w};
 #pragma unroll
-                for (int e = 0; e < 32; ++e) {
-                  const int by = (w8[e >> 2] >> (8 * (e & 3))) & 0xFF;
-                  v[e] = sc * (float)(hh ? (by >> 4) : (by & 15)) - mn;
-                }
+                for (int e = 0; e < 32; ++e) v[e] = sc * byte_to_float((w8[e >> 2] >> (4 * hh)) & 0x0F0F0F0Fu, e & 3) - mn;
               } else if constexpr (WFMT == WF_Q2_K) {
                 const float dd = __half2float(*reinterpret_cast<const __half*>(srow));
                 const float dm = __half2float(*reinterpret_cast<const __half*>(srow + 2));
                 const int4 a = *reinterpret_cast<const int4*>(qrow);
-                const int w4[4] = {a.x, a.y, a.z, a.w};
+                const uint32_t w4[4] = {(uint32_t)a.x, (uint32_t)a.y, (uint32_t)a.z, (uint32_t)a.w};
 #pragma unroll
-                for (int e = 0; e < 32; ++e) {
-                  const int by = (w4[(e & 15) >> 2] >> (8 * (e & 3))) & 0xFF;
-                  const int nib = e < 16 ? (by & 15) : (by >> 4);
-                  const int sb = srow[4 + 2 * hh + (e >> 4)];
-                  v[e] = dd * (float)(sb & 15) * (float)((nib >> (2 * hh)) & 3) - dm * (float)(sb >> 4);
+                for (int g = 0; g < 2; ++g) {           // 16 inputs of one scale: the low, then the high nibbles
+                  const int sb = srow[4 + 2 * hh + g];
+                  const float sc = dd * (float)(sb & 15), mn = dm * (float)(sb >> 4);
+#pragma unroll
+                  for (int e = 0; e < 16; ++e) v[16 * g + e] = sc * byte_to_float((w4[e >> 2] >> (4 * g + 2 * hh)) & 0x03030303u, e & 3) - mn;
                 }
               } else if constexpr (WFMT == WF_Q5_K) {
                 const float dd = __half2float(*reinterpret_cast<const __half*>(srow));
@@ -688,10 +696,10 @@ gemm_wdec_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constant_
     // ---------------------------------------------------------------- epilogue
     uint32_t tile_i = 0;
     const int row_in_tile = warp * 32 + lane;  // TMEM lane == output feature within the tile
-    const uint32_t ar_epoch = p.ar_mode ? p.comm.ctrl[0] + 1 : 0;   // read before any CTA can finish
+    const uint32_t ar_epoch = ar_mode ? p.comm.ctrl[0] + 1 : 0;   // read before any CTA can finish
     // Modes whose epilogue uses a named barrier must leave the loop together: the decision to stop is
     // taken from epi_abort, which only epilogue threads write and always before a barrier.
-    const bool sync_mode = p.ar_mode != 0 || (p.splits > 1 && p.out != nullptr);
+    const bool sync_mode = ar_mode != 0 || (p.splits > 1 && p.out != nullptr);
     for (int w = blockIdx.x; w < total_work; w += gridDim.x, ++tile_i) {
       if (sync_mode) {
         if (threadIdx.x == 0 && *abort_flag) *epi_abort = 1;
@@ -723,7 +731,7 @@ gemm_wdec_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constant_
       const bool f_ok = f < p.N;
       const uint32_t taddr = tmem_base + (uint32_t(warp * 32) << 16) + buf * BN;
       constexpr int CH = BN >= 32 ? 32 : 16;
-      if (p.ar_mode == 3) {
+      if (ar_mode == 3) {
         // ---- reduce-scatter push: partial tile -> the owner's slot for source = this rank ----------------------
         if constexpr (L::EPI_BYTES > 0) {
           const B200Comm& cm = p.comm;
@@ -771,7 +779,7 @@ gemm_wdec_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constant_
         }
         continue;
       }
-      if (p.ar_mode != 0) {
+      if (ar_mode != 0) {
         // ---- fused all-reduce over peer memory --------------------------------------------------
         // The accumulator is first written as bf16 into this rank's own slot (a thread owns one feature, so these
         // are 2-byte stores, 64 bytes wide per warp: fine locally, far too fine for NVLink).  Everything that
@@ -779,7 +787,7 @@ gemm_wdec_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constant_
         // bytes of one token row with 16-byte accesses, several rows in flight per thread.
         const B200Comm& cm = p.comm;
         const int parity = ar_epoch & 1;
-        const bool two_shot = p.ar_mode == 2;
+        const bool two_shot = ar_mode == 2;
         const int owner = two_shot ? (w % cm.world) : cm.rank;
         const bool reduce_here = owner == cm.rank;
         const size_t slot_elems = cm.slot_elems;
@@ -984,14 +992,29 @@ gemm_wdec_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constant_
           __threadfence();
           const int t_lo = wk.row0;
           const int t_hi = wk.row0 + wk.rows;
-          for (int t = t_lo; t < t_hi; ++t) {
+          // eight tokens at a time: one after the other, every split's partial is a round trip to L2 of its own (80 us
+          // for 64 tokens of a 64 x 5120 matrix in eight splits)
+          constexpr int U = 8;
+          for (int t = t_lo; t < t_hi; t += U) {
             const size_t off = (size_t)t * p.ldo + f;
-            float acc = p.residual ? __bfloat162float(p.residual[off]) : 0.f;
-            for (int sp = 0; sp < p.splits; ++sp)
-              acc += __ldcg(p.out_f32 + (size_t)sp * p.T * p.ldo + off);
-            if (WFMT == WF_BF16 && p.act.on)
-              acc = xielu_bf16(acc + (p.act.bias ? __ldg(p.act.bias + f) : 0.f), p.act.ap, p.act.an);
-            p.out[off] = __float2bfloat16(acc);
+            float acc[U];
+#pragma unroll
+            for (int j = 0; j < U; ++j) acc[j] = p.residual && t + j < t_hi ? __bfloat162float(p.residual[off + (size_t)j * p.ldo]) : 0.f;
+            for (int sp = 0; sp < p.splits; ++sp) {
+              const float* src = p.out_f32 + (size_t)sp * p.T * p.ldo + off;
+              float v[U];
+#pragma unroll
+              for (int j = 0; j < U; ++j) v[j] = t + j < t_hi ? __ldcg(src + (size_t)j * p.ldo) : 0.f;
+#pragma unroll
+              for (int j = 0; j < U; ++j) acc[j] += v[j];
+            }
+#pragma unroll
+            for (int j = 0; j < U; ++j) {
+              if (t + j >= t_hi) continue;
+              if (WFMT == WF_BF16 && p.act.on)
+                acc[j] = xielu_bf16(acc[j] + (p.act.bias ? __ldg(p.act.bias + f) : 0.f), p.act.ap, p.act.an);
+              p.out[off + (size_t)j * p.ldo] = __float2bfloat16(acc[j]);
+            }
           }
         }
         asm volatile("bar.sync 1, 128;" ::: "memory");   // fix_last is rewritten by the next tile
@@ -999,7 +1022,7 @@ gemm_wdec_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constant_
     }
   }
 
-  if (warp < NUM_EPI_WARPS && p.ar_mode == 2 && !*abort_flag) {
+  if (warp < NUM_EPI_WARPS && ar_mode == 2 && !*abort_flag) {
     // two-shot: the tiles this CTA handed to other owners must have come back before the grid may finish
     const B200Comm& cm = p.comm;
     const uint32_t epoch = ar_epoch_at_entry;
@@ -1029,7 +1052,7 @@ gemm_wdec_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constant_
     tc_fence_after();
     tmem_dealloc(tmem_base, TMEM_COLS);
   }
-  if (p.ar_mode && threadIdx.x == 0) {
+  if (ar_mode && threadIdx.x == 0) {
     // the last CTA to leave publishes the new epoch (every CTA read the old one before the first barrier)
     __threadfence();
     const uint32_t done = atomicAdd(&p.comm.ctrl[1], 1u) + 1;
@@ -1067,7 +1090,8 @@ static int launch_one(const CUtensorMap& tmW, const CUtensorMap& tmX, const Gemm
   if (p.ar_mode == 3 && L::EPI_BYTES == 0) return -ERR_BAD_ARG;   // this instance has no epilogue staging
   const int total = p.work_table ? sm_count() : p.m_tiles * p.n_tiles * p.splits;
   const int grid = total < sm_count() ? total : sm_count();
-  gemm_wdec_kernel<BN, WFMT><<<grid, NUM_THREADS, L::TOTAL, stream>>>(tmW, tmX, p);
+  const cudaError_t le = launch_pdl(gemm_wdec_kernel<BN, WFMT>, dim3(grid), dim3(L::THREADS), L::TOTAL, stream, tmW, tmX, p);
+  if (le != cudaSuccess) return (int)le;
   return (int)cudaGetLastError();
 }
 
