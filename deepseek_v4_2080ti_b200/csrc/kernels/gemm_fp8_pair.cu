@@ -7,6 +7,12 @@
 // 32 shared-memory reads of 16 bytes per block and thread, beside operand traffic that already fills shared memory (112 KB
 // per 1024 tensor cycles), doubled the time (978 against 670 us for 1920 x 34816 x 5120).
 //
+// Measured, us per product (12288 x 5120, 5120 x 4096, 34816 x 5120, 5120 x 17408): 128 tokens 46, 36, 88, 60; 333 tokens 67, 37,
+// 153, 82; 1901 tokens 216, 84, 616, 320.  The decode-warp kernel before: 128 tokens 121, 103, 84, 135; 333 tokens 91, 43, 182,
+// 146; 1901 tokens 256, 102, 681, 409.  The split of the activations into terms, which that kernel had no need of, is not
+// counted: 3 to 5 us at 128 tokens, 11 to 36 at 1901, once for all products of the same input.  At 128 tokens the 34816 x 5120
+// product alone is slower than before; the other three outweigh it.
+//
 // Same work list and treatment of cut tiles as the one-CTA kernel; the tokens past the last one of a tile are not staged when
 // they fill a CTA, and not read back.  Roles: warps 0-7 epilogue (group of four: one weight tile of the pair), warp 8 weight
 // copies, warp 9 MMA issuer (first CTA), warp 10 activation copies.  All waits are bounded.

@@ -25,7 +25,8 @@
 //
 // Measured, us per product in a chain (weights 63, 21, 178, 89 MB: 12288 x 5120, 5120 x 4096, 34816 x 5120, 5120 x 17408;
 // a plain read of as many bytes takes 9.7, 3.7, 25.3, 13.2):
-//   1 token 18.4, 11.3, 37.0, 23.4;  32 tokens 20.0, 13.1, 39.7, 25.7;  64 tokens 22.5, 15.3, 45.4, 28.7.
+//   1 token 17.3, 11.6, 34.5, 22.5;  32 tokens 20.0, 13.1, 39.7, 25.7;  64 tokens 23.3, 16.8, 46.8, 30.2
+//   (the 32-token figures are those of an earlier build, whose 64-token ones were 22.5, 15.3, 45.4, 28.7)
 // The kernels this one took over from: gemm_w8a8s.cu at 1 token 20.6, 12.0, 38.7, 29.8, at 32 tokens 47.6, 52.6, 45.9, 71.8;
 // the decode-warp kernel at 64 tokens 77.9, 83.1, 188, 111.
 //
