@@ -79,23 +79,24 @@ struct ConvStep {
   }
 };
 
-// grid (Hv, B), clusters of the R = Hv / Hk value heads that share a key head; block = 16 warps.  Warp w owns rows 8 w .. 8 w + 7
-// of the head's state, a lane four columns of them; the warps' partial dot products meet in shared memory.
+// grid (Hv, B), clusters of the R = Hv / Hk value heads that share a key head; block = 128 * RG threads.  Thread (rg, j) owns
+// rows [rg*128/RG, (rg+1)*128/RG) of column j of the head's state; the row groups cut the serial length of the recurrence per
+// thread, their partial dot products meet in shared memory.
 //
-// The kernel is bound by the state, 64 KB in and out per head, and by the length of its chain.  The state is asked for first,
-// 16 bytes per load, and arrives while the projections, the convolution and the gates are computed; a block holds one head and
-// two blocks fit an SM, so one block's loads run beside another's arithmetic.  The code is kept short: the weights of a layer
-// pass through L2 between two launches, so its instructions come from HBM.  (With the R heads of a key head in one block of
-// 1024 threads, the state loaded last, four bytes per load: 45 us at 32 rows of 32 heads, where its bytes take 20, and 13.8 us
-// at one row.)
+// The state, 64 KB in and out per head, is asked for first and arrives while the projections, the convolution and the gates are
+// computed; a block holds one head and two blocks fit an SM.  At 32 rows of 32 heads that takes 41 to 42 us, where the bytes take 20;
+// what the rest goes on has not been measured.  (All heads of a key head in one block of 1024 threads, one block per
+// SM, the state loaded last: 45.6.  Four columns per thread, 16 bytes per load: 46.6.  Weights fetched before the wait for the
+// previous kernel: 48.4.  One row takes 14 us in every form.)
 // Every block convolves the q and k channels of its key head itself; the first of the cluster moves their tail on when all of
 // them have read it.
-template <int KW, int R>
-__global__ void __launch_bounds__(512, 2)
+template <int KW, int R, int RG>
+__global__ void __launch_bounds__(128 * RG, 2)
 gdn_decode_fused_kernel(GdnDecodeParams p) {
-  constexpr int WARPS = 16, ROWS = DK / WARPS;
-  __shared__ __align__(16) float sq[DK], sk[DK], s_delta[DV];
-  __shared__ __align__(16) float s_part[WARPS][DV];
+  constexpr int ROWS = DK / RG;
+  constexpr int WARPS = 4 * RG;
+  __shared__ float sq[DK], sk[DK], s_v[DV];
+  __shared__ float s_part[RG][DV];
   __shared__ float red_ab[WARPS][2];
   __shared__ float red_qk[8];
   __shared__ float red_o[4];
@@ -104,22 +105,21 @@ gdn_decode_fused_kernel(GdnDecodeParams p) {
   b200::pdl_grid_trigger();
   b200::pdl_grid_wait();
   const int h = blockIdx.x, b = blockIdx.y, kh = h / R;
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const int j = threadIdx.x;                 // channel / column of the first 128 threads
+  const int j = threadIdx.x & 127, rg = threadIdx.x >> 7;
   const int kd = p.Hk * DK, vd = p.Hv * DV, C = 2 * kd + vd;
   const int slot = p.slot_ids ? p.slot_ids[b] : b;
   __nv_bfloat16* tail = p.tails + (size_t)slot * p.tail_stride;
   const __nv_bfloat16* row = p.proj + (size_t)b * p.ldp;
 
-  float4* S = reinterpret_cast<float4*>(p.states + (size_t)slot * p.state_stride + ((size_t)h * DK + warp * ROWS) * DV) + lane;
-  float4 st[ROWS];
+  float* S = p.states + (size_t)slot * p.state_stride + (size_t)h * DK * DV + (size_t)rg * ROWS * DV;
+  float col[ROWS];
 #pragma unroll
-  for (int i = 0; i < ROWS; ++i) st[i] = S[i * (DV / 4)];
+  for (int i = 0; i < ROWS; ++i) col[i] = S[(size_t)i * DV + j];
 
-  // ---- convolution (first 128 threads)
+  // ---- convolution (row group 0)
   const int cq = kh * DK + j, ck = kd + kh * DK + j, cv = 2 * kd + h * DV + j;
   ConvStep<KW> tq, tk, tv;
-  if (j < DK) {
+  if (rg == 0) {
     tq.load(tail, C, cq, row[cq]);
     tk.load(tail, C, ck, row[ck]);
     tv.load(tail, C, cv, row[cv]);
@@ -132,8 +132,7 @@ gdn_decode_fused_kernel(GdnDecodeParams p) {
     const __nv_bfloat16* wa = p.w_ab + (size_t)h * p.hidden;
     const __nv_bfloat16* wb = p.w_ab + (size_t)(p.Hv + h) * p.hidden;
     float da = 0.f, db = 0.f;
-#pragma unroll 1
-    for (int i = (int)threadIdx.x * 8; i < p.hidden; i += 512 * 8) {
+    for (int i = (int)threadIdx.x * 8; i < p.hidden; i += 128 * RG * 8) {
       const uint4 xv = *reinterpret_cast<const uint4*>(xr + i);
       const uint4 av = *reinterpret_cast<const uint4*>(wa + i);
       const uint4 bv = *reinterpret_cast<const uint4*>(wb + i);
@@ -149,16 +148,16 @@ gdn_decode_fused_kernel(GdnDecodeParams p) {
     }
     da = warp_sum(da);
     db = warp_sum(db);
-    if (lane == 0) {
-      red_ab[warp][0] = da;
-      red_ab[warp][1] = db;
+    if ((j & 31) == 0) {
+      red_ab[threadIdx.x >> 5][0] = da;
+      red_ab[threadIdx.x >> 5][1] = db;
     }
   }
-  float qv = 0.f, kv = 0.f, vv = 0.f;
-  if (j < DK) {
+  float qv = 0.f, kv = 0.f;
+  if (rg == 0) {
     qv = tq.result(p.conv_w, cq);
     kv = tk.result(p.conv_w, ck);
-    vv = tv.result(p.conv_w, cv);
+    s_v[j] = tv.result(p.conv_w, cv);
     tv.store(tail, C, cv);
     const float qs = warp_sum(qv * qv), ks = warp_sum(kv * kv);
     if ((j & 31) == 0) {
@@ -167,64 +166,62 @@ gdn_decode_fused_kernel(GdnDecodeParams p) {
     }
   }
   __syncthreads();
-  if (warp == 4) {
-    float a = warp_sum(lane < WARPS ? red_ab[lane][0] : 0.f), bb = warp_sum(lane < WARPS ? red_ab[lane][1] : 0.f);
+  if (threadIdx.x == 0) {
+    float a = 0.f, bb = 0.f;
+#pragma unroll
+    for (int w = 0; w < WARPS; ++w) {
+      a += red_ab[w][0];
+      bb += red_ab[w][1];
+    }
     // the unfused path rounds the a/b projection outputs to bf16 before the gate math
     a = bf16_round(a);
     bb = bf16_round(bb);
     const float av = a + p.dt_bias[h];
     const float sp = av > 20.f ? av : log1pf(expf(av));
-    if (lane == 0) {
-      s_gate[0] = __expf(-expf(p.a_log[h]) * sp);   // decay = exp(g)
-      s_gate[1] = sigmoid_f(bb);
-    }
+    s_gate[0] = __expf(-expf(p.a_log[h]) * sp);   // decay = exp(g)
+    s_gate[1] = sigmoid_f(bb);
   }
-  if (j < DK) {
+  if (rg == 0) {
     const float qn = rsqrtf(red_qk[0] + red_qk[1] + red_qk[2] + red_qk[3] + 1e-6f);
     const float kn = rsqrtf(red_qk[4] + red_qk[5] + red_qk[6] + red_qk[7] + 1e-6f);
     sq[j] = qv * qn * p.q_scale;
     sk[j] = kv * kn;
   }
   __syncthreads();
-  // ---- gated delta rule
+  // ---- gated delta rule on rows [rg*ROWS, (rg+1)*ROWS) of state column j
   const float decay = s_gate[0], bt = s_gate[1];
-  float4 part = make_float4(0.f, 0.f, 0.f, 0.f);
+  float part = 0.f;
 #pragma unroll
   for (int i = 0; i < ROWS; ++i) {
-    const float k = sk[warp * ROWS + i];
-    st[i].x *= decay; st[i].y *= decay; st[i].z *= decay; st[i].w *= decay;
-    part.x += st[i].x * k; part.y += st[i].y * k; part.z += st[i].z * k; part.w += st[i].w * k;
+    col[i] *= decay;
+    part += col[i] * sk[rg * ROWS + i];
   }
-  *reinterpret_cast<float4*>(&s_part[warp][lane * 4]) = part;
+  s_part[rg][j] = part;
   __syncthreads();
-  if (j < DV) {
-    float kv_mem = 0.f;
+  float kv_mem = 0.f;
 #pragma unroll
-    for (int w = 0; w < WARPS; ++w) kv_mem += s_part[w][j];
-    s_delta[j] = (vv - kv_mem) * bt;
-  }
+  for (int g2 = 0; g2 < RG; ++g2) kv_mem += s_part[g2][j];
+  const float delta = (s_v[j] - kv_mem) * bt;
   __syncthreads();   // s_part is reused for the read-out partials
-  const float4 delta = *reinterpret_cast<const float4*>(&s_delta[lane * 4]);
-  part = make_float4(0.f, 0.f, 0.f, 0.f);
+  part = 0.f;
 #pragma unroll
   for (int i = 0; i < ROWS; ++i) {
-    const float k = sk[warp * ROWS + i], q = sq[warp * ROWS + i];
-    st[i].x += k * delta.x; st[i].y += k * delta.y; st[i].z += k * delta.z; st[i].w += k * delta.w;
-    S[i * (DV / 4)] = st[i];
-    part.x += st[i].x * q; part.y += st[i].y * q; part.z += st[i].z * q; part.w += st[i].w * q;
+    col[i] += sk[rg * ROWS + i] * delta;
+    S[(size_t)i * DV + j] = col[i];
+    part += col[i] * sq[rg * ROWS + i];
   }
-  *reinterpret_cast<float4*>(&s_part[warp][lane * 4]) = part;
+  s_part[rg][j] = part;
   if constexpr (R > 1) asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");   // every head has read the q and k tails
-  if (j < DK && h % R == 0) {
+  if (rg == 0 && h % R == 0) {
     tq.store(tail, C, cq);
     tk.store(tail, C, ck);
   }
   __syncthreads();
-  if (j >= DV) return;
-  // ---- per-head gated RMSNorm by the first 128 threads (the unfused path stores o as bf16 first)
+  if (rg != 0) return;
+  // ---- per-head gated RMSNorm by row group 0 (the unfused path stores o as bf16 first)
   float o = 0.f;
 #pragma unroll
-  for (int w = 0; w < WARPS; ++w) o += s_part[w][j];
+  for (int g2 = 0; g2 < RG; ++g2) o += s_part[g2][j];
   o = bf16_round(o);
   const float ss = warp_sum(o * o);
   if ((j & 31) == 0) red_o[j >> 5] = ss;
@@ -268,7 +265,7 @@ static int launch_gdn(const GdnDecodeParams& p, int B, cudaStream_t stream) {
   attr[1].val.clusterDim.z = 1;
   cfg.attrs = attr;
   cfg.numAttrs = R > 1 ? 2 : 1;
-  return (int)cudaLaunchKernelEx(&cfg, gdn_decode_fused_kernel<4, R>, p);
+  return (int)cudaLaunchKernelEx(&cfg, gdn_decode_fused_kernel<4, R, 4>, p);
 }
 
 // ------------------------------------------------------------------------------------------------
@@ -464,7 +461,6 @@ int b200_gdn_decode_fused(const void* proj, int ldp, const void* x, int hidden, 
   p.conv_w = reinterpret_cast<const __nv_bfloat16*>(conv_w);
   p.tails = reinterpret_cast<__nv_bfloat16*>(tails);
   p.tail_stride = (size_t)tail_stride;
-  if ((reinterpret_cast<uintptr_t>(states) & 15) != 0 || state_stride % 4 != 0) return -6;      // rows are read 16 bytes at a time
   p.states = states;
   p.state_stride = (size_t)state_stride;
   p.slot_ids = slot_ids;
