@@ -426,8 +426,11 @@ gemm_wdec_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constant_
     if constexpr (WFMT != WF_BF16) {
       constexpr int G = L::GROUPS;
       static_assert(G == SAB, "one decode group per decoded slot");
-      // A group's parity wait on raw stage it % S assumes k-block it - S has landed; the only ordering a group has
-      // with the producer is through its own previous k-block it - G, so the ring must hold at least G stages.
+      // A parity wait tells a phase only from its neighbours, and copies land in any order: the wait for raw stage it % S
+      // means k-block `it` only once k-block it - S is known to have landed.  The products give that: they are issued in order,
+      // so the commit of k-block it - G, which frees this group's decoded slot, says that everything up to it - G has landed
+      // and, with S >= G, that it - S is among it.  Hence the slot is waited for first, the raw stage second.  (The commit's own
+      // parity is unambiguous because the group saw the commit of it - 2 G at its previous k-block.)
       static_assert(S >= G, "raw ring shallower than the decode groups' look-ahead");
       constexpr int WPG = L::WARPS_PER_GROUP;
       constexpr int GT = WPG * 32;             // threads per group
@@ -469,12 +472,13 @@ gemm_wdec_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constant_
             __nv_bfloat162 sc2 = __float2bfloat162_rn(sc);
             scw = *reinterpret_cast<uint32_t*>(&sc2);
           }
-          bool ok = mbar_wait(&tma_full[s], ph);
+          bool ok = true;
           if (it >= (uint32_t)SAB) {
             // decoded slot `grp` was last read by the MMAs of k-block it - SA
             const uint32_t prev = it - SAB;
-            ok = ok && mbar_wait(&empty[prev % S], (prev / S) & 1);
+            ok = mbar_wait(&empty[prev % S], (prev / S) & 1);
           }
+          ok = ok && mbar_wait(&tma_full[s], ph);
           ok = __all_sync(0xffffffffu, ok);
           if (!ok) {
             if (lane == 0) atomicExch(p.status, ERR_WAIT_TMA);
