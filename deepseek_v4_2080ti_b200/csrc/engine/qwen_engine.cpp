@@ -13,8 +13,8 @@ namespace pocket {
 
 namespace {
 constexpr int kHead = 128;          // head width of both attention kinds (the kernels are specialised for it)
-constexpr int kFusedMaxT = 64;      // largest decode batch whose activations stay E4M3 terms between the kernels
-constexpr int kTermsMaxT = 2047;    // longest batch whose FP8 products take the activations as E4M3 terms
+constexpr int kFusedMaxT = 64;      // largest decode batch whose activations stay FP8 terms between the kernels
+constexpr int kTermsMaxT = 2047;    // longest batch whose FP8 products take the activations as FP8 terms
 constexpr int kSMs = 148;
 
 double now_s() {
@@ -56,17 +56,18 @@ int pick_splits(int t, int n, int k) {
 
 }  // namespace
 
-// Activation and workspace buffers, sized once for the prefill chunk and the decode batch.
-// bf16 activations as E4M3 terms (kernels/gemm_fp8_terms.cu)
+// bf16 activations as FP8 terms (kernels/gemm_fp8_terms.cu)
 struct QwenNativeEngine::TermsBuffer {
-  DeviceBuffer xq, sx;
+  DeviceBuffer xq, sx, rest;
   void reset(size_t rows, size_t width) {
     const size_t tiled = (rows + 255) / 256 * 256;
     xq.reset(tiled * width * 2);
     sx.reset(tiled * (width / 128 + 1) * 4);
+    rest.reset(rows * width * 2);
   }
 };
 
+// Activation and workspace buffers, sized once for the prefill chunk and the decode batch.
 struct QwenNativeEngine::Scratch {
   int rows = 0;                       // capacity in token rows
   DeviceBuffer ids, pos, kv_slots, meta, slot_ids, kv_len, bt_batch;
@@ -438,7 +439,8 @@ void QwenNativeEngine::linear(const void* x, const PackedMatrix& w, void* out, i
     return;
   }
   if (const int tok = terms_tile(T, w)) {
-    rc(b200_split_terms(x, T, w.k, tok, s.act_terms.xq.get(), s.act_terms.sx.as<float>(), stream_), "split_terms");
+    rc(b200_split_terms(x, T, w.k, tok, s.act_terms.xq.get(), s.act_terms.sx.as<float>(), s.act_terms.rest.get(), stream_),
+       "split_terms");
     linear_terms(s.act_terms, w, out, T);
     return;
   }
@@ -459,7 +461,7 @@ int QwenNativeEngine::terms_tile(int T, const PackedMatrix& w) {
 
 void QwenNativeEngine::linear_terms(const TermsBuffer& x, const PackedMatrix& w, void* out, int T) {
   Scratch& s = *s_;
-  rc(b200_gemm_fp8_terms(w.weight.get(), w.scales.as<float>(), x.xq.get(), x.sx.as<float>(), out, nullptr, T, w.n, w.k,
+  rc(b200_gemm_fp8_terms(w.weight.get(), w.scales.as<float>(), x.xq.get(), x.sx.as<float>(), x.rest.get(), out, nullptr, T, w.n, w.k,
                          s.splitk_ws.as<float>(), s.counters.as<int>(), s.status.as<int>(), stream_), "gemm_fp8_terms");
 }
 
@@ -599,7 +601,7 @@ void QwenNativeEngine::forward_decode(const std::vector<int>& slots, const std::
     uint8_t* vc = v_cache_.as<uint8_t>() + kv_layer_stride_ * L.cache_index * 2;
     if (fused) {
       rc(b200_rmsnorm_terms(s.h.get(), delta, L.in_ln.get(), L.linear ? s.x.get() : nullptr, B, H, eps, 1, tok,
-                            s.norm_terms.xq.get(), s.norm_terms.sx.as<float>(), stream_), "rmsnorm_terms");
+                            s.norm_terms.xq.get(), s.norm_terms.sx.as<float>(), s.norm_terms.rest.get(), stream_), "rmsnorm_terms");
       linear_terms(s.norm_terms, L.proj, s.proj.get(), B);
     } else {
       rc(b200_rmsnorm(s.h.get(), delta, nullptr, 0, L.in_ln.get(), s.x.get(), B, H, eps, 1, delta ? 1 : 0, stream_), "rmsnorm");
@@ -611,7 +613,8 @@ void QwenNativeEngine::forward_decode(const std::vector<int>& slots, const std::
         rc(b200_gdn_decode_fused(s.proj.get(), ldp, s.x.get(), H, L.ab.weight.get(), L.a_log.as<float>(),
                                  L.dt_bias.as<float>(), L.conv_w.get(), kw, tails, (long long)tail_slot_stride_, states,
                                  (long long)state_slot_stride_, s.slot_ids.as<int>(), L.gdn_norm.get(), nullptr, B, hv_,
-                                 hk_, eps, s.act_terms.xq.get(), s.act_terms.sx.as<float>(), tok, stream_), "gdn_decode_fused");
+                                 hk_, eps, s.act_terms.xq.get(), s.act_terms.sx.as<float>(), s.act_terms.rest.get(), tok,
+                                 stream_), "gdn_decode_fused");
       } else {
         linear(s.x.get(), L.ab, s.ab.get(), B);
         rc(b200_gdn_gates(s.ab.get(), 2 * hv_, 0, hv_, L.a_log.as<float>(), L.dt_bias.as<float>(), s.g.as<float>(),
@@ -637,13 +640,15 @@ void QwenNativeEngine::forward_decode(const std::vector<int>& slots, const std::
     }
     if (fused) {
       if (!L.linear)
-        rc(b200_split_terms(mix_out, B, L.out.k, tok, s.act_terms.xq.get(), s.act_terms.sx.as<float>(), stream_), "split_terms");
+        rc(b200_split_terms(mix_out, B, L.out.k, tok, s.act_terms.xq.get(), s.act_terms.sx.as<float>(), s.act_terms.rest.get(),
+                            stream_), "split_terms");
       linear_terms(s.act_terms, L.out, s.d_attn.get(), B);
       reduce_rows(s.d_attn.get(), B);
       rc(b200_rmsnorm_terms(s.h.get(), s.d_attn.get(), L.post_ln.get(), nullptr, B, H, eps, 1, tok, s.norm_terms.xq.get(),
-                            s.norm_terms.sx.as<float>(), stream_), "rmsnorm_terms");
+                            s.norm_terms.sx.as<float>(), s.norm_terms.rest.get(), stream_), "rmsnorm_terms");
       linear_terms(s.norm_terms, L.gate_up, s.gu.get(), B);
-      rc(b200_silu_mul_terms(s.gu.get(), B, I, tok, s.act_terms.xq.get(), s.act_terms.sx.as<float>(), stream_), "silu_mul_terms");
+      rc(b200_silu_mul_terms(s.gu.get(), B, I, tok, s.act_terms.xq.get(), s.act_terms.sx.as<float>(), s.act_terms.rest.get(),
+                             stream_), "silu_mul_terms");
       linear_terms(s.act_terms, L.down, s.d_mlp.get(), B);
     } else {
       linear(mix_out, L.out, s.d_attn.get(), B);

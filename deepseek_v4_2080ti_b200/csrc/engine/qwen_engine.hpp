@@ -149,7 +149,7 @@ class QwenNativeEngine : public InferenceEngine {
   void reduce_rows(void* buf, int T);
   void linear(const void* x, const PackedMatrix& w, void* out, int T, float* out_f32 = nullptr);
   struct TermsBuffer;
-  int terms_tile(int T, const PackedMatrix& w);       // tokens of a tile when `w` takes T rows as E4M3 terms, else 0
+  int terms_tile(int T, const PackedMatrix& w);       // tokens of a tile when `w` takes T rows as FP8 terms, else 0
   void linear_terms(const TermsBuffer& x, const PackedMatrix& w, void* out, int T);
   int32_t forward_prefill(int slot, const int32_t* tokens, int T, int64_t pos0, bool want_token);
   void forward_decode(const std::vector<int>& slots, const std::vector<int32_t>& tokens, std::vector<int32_t>& next);

@@ -54,7 +54,7 @@ struct GdnDecodeParams {
   __nv_bfloat16* out;          // [B, Hv*128]
   int Hv, Hk;
   float eps, q_scale;
-  b200::f8t::TermsOut terms;   // where the result goes as E4M3 terms (xq set) instead of `out`: a head is one block of 128
+  b200::f8t::TermsOut terms;   // where the result goes as FP8 terms (xq set) instead of `out`: a head is one block of 128
 };
 
 // One channel of the causal convolution: the tail's values and the new one.
@@ -96,11 +96,10 @@ gdn_decode_fused_kernel(GdnDecodeParams p) {
   constexpr int ROWS = DK / RG;
   constexpr int WARPS = 4 * RG;
   __shared__ float sq[DK], sk[DK], s_v[DV];
-  __shared__ float s_part[RG][DV];
+  __shared__ __align__(16) float s_part[RG][DV];
   __shared__ float red_ab[WARPS][2];
   __shared__ float red_qk[8];
   __shared__ float red_o[4];
-  __shared__ uint32_t red_m[4];
   __shared__ float s_gate[2];
   b200::pdl_grid_trigger();
   b200::pdl_grid_wait();
@@ -234,19 +233,11 @@ gdn_decode_fused_kernel(GdnDecodeParams p) {
     return;
   }
   s_part[0][j] = y;
-  const uint32_t m = __reduce_max_sync(0xffffffffu, b200::f8t::bf16_magnitude(y));
-  if ((j & 31) == 0) red_m[j >> 5] = m;
   asm volatile("bar.sync 1, 128;" ::: "memory");
   if (j < 32) {
-    const b200::f8t::TermScale ts(max(max(red_m[0], red_m[1]), max(red_m[2], red_m[3])));
-    uint32_t hi, mid;
-    ts.split4(&s_part[0][j * 4], hi, mid);
-    int r;
-    uint8_t* dst = p.terms.hi_row(b, h, r);
-    dst += b200::f8t::term_offset(r, j);
-    *reinterpret_cast<uint32_t*>(dst) = hi;
-    *reinterpret_cast<uint32_t*>(dst + p.terms.cap * 128) = mid;
-    if (j == 0) *p.terms.scale(b, h) = ts.inv;
+    const float4 f = *reinterpret_cast<const float4*>(&s_part[0][j * 4]);
+    const float v[4] = {f.x, f.y, f.z, f.w};
+    b200::f8t::put_terms(p.terms, b, h * DV + j * 4, v, true);
   }
 }
 
@@ -443,13 +434,14 @@ extern "C" {
 // proj: [B, ldp] bf16 holding q | k | v | z at offsets 0, kd, 2kd, 2kd+vd (kd = Hk*128, vd = Hv*128);
 // x: [B, hidden] bf16; w_ab: [2*Hv, hidden] bf16; conv_w: [2kd+vd, kw] bf16; tails: [slots, kw-1, 2kd+vd] bf16
 // (tail_stride elements per slot); states: fp32 [slots, Hv, 128, 128] (state_stride floats per slot);
-// out: [B, Hv*128] bf16, or null with terms_xq / terms_sx: the result as E4M3 terms (gemm_fp8_terms.cu, tok tokens per tile, no
-// pair).  Hv / Hk must be 1, 2 or 4 and kw == 4.
+// out: [B, Hv*128] bf16, or null with terms_xq / terms_sx / terms_rest: the result as FP8 terms (gemm_fp8_terms.cu,
+// tok tokens per tile, no pair).  Hv / Hk must be 1, 2 or 4 and kw == 4.
 int b200_gdn_decode_fused(const void* proj, int ldp, const void* x, int hidden, const void* w_ab, const float* a_log,
                           const float* dt_bias, const void* conv_w, int kw, void* tails, long long tail_stride,
                           float* states, long long state_stride, const int* slot_ids, const void* gamma, void* out,
-                          int B, int Hv, int Hk, float eps, void* terms_xq, float* terms_sx, int tok, cudaStream_t stream) {
-  if ((!out && (!terms_xq || !terms_sx || tok < B || tok > b200::f8t::MAX_SINGLE)) || B <= 0 || Hv <= 0 || Hk <= 0 || Hv % Hk != 0 || kw != 4 || hidden % 8 != 0) return -6;
+                          int B, int Hv, int Hk, float eps, void* terms_xq, float* terms_sx, void* terms_rest, int tok,
+                          cudaStream_t stream) {
+  if ((!out && (!terms_xq || !terms_sx || !terms_rest || tok < B || tok > b200::f8t::MAX_SINGLE)) || B <= 0 || Hv <= 0 || Hk <= 0 || Hv % Hk != 0 || kw != 4 || hidden % 8 != 0) return -6;
   GdnDecodeParams p;
   p.proj = reinterpret_cast<const __nv_bfloat16*>(proj);
   p.ldp = ldp;
@@ -472,6 +464,7 @@ int b200_gdn_decode_fused(const void* proj, int ldp, const void* x, int hidden, 
   p.q_scale = rsqrtf((float)DK);
   p.terms.xq = out ? nullptr : reinterpret_cast<uint8_t*>(terms_xq);
   p.terms.sx = terms_sx;
+  p.terms.rest = reinterpret_cast<__nv_bfloat16*>(terms_rest);
   p.terms.tok = p.terms.cap = tok;
   p.terms.kb = Hv;
   switch (Hv / Hk) {

@@ -1,5 +1,5 @@
 // The products of gemm_fp8_terms.cu for more than 64 tokens, on CTA pairs (tcgen05.mma.cta_group::2):
-//   Y[T, N] = X[T, K] * W[N, K]^T,  W = E4M3 with one scale per 128 x 128 block, X as two exact E4M3 terms.
+//   Y[T, N] = X[T, K] * W[N, K]^T,  W = E4M3 with one scale per 128 x 128 block, X as two FP8 terms.
 //
 // Here the tokens are the MMA's M dimension: a pair computes 256 tokens x 256 features, each CTA its own 128 tokens, and a
 // TMEM lane is a token.  The scale of a K block is then one number per thread (activation scale of its token x weight scale
@@ -168,7 +168,7 @@ gemm_fp8_pair_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_const
     } else if (warp == WARP_MMA && rank == 0) {
       // ---------------------------------------------------------- MMA issuer
       const uint32_t on = elect_one();
-      constexpr uint32_t idesc = umma_idesc_e4m3(2 * ROWS, 2 * BM);
+      constexpr uint32_t idesc_hi = umma_idesc_f8(2 * ROWS, 2 * BM, true), idesc_mid = umma_idesc_f8(2 * ROWS, 2 * BM);
       for (int blk = 0; blk < u1 - u0; ++blk) {
         const int b = blk % S, a = blk % A;
         int err = 0;
@@ -185,7 +185,8 @@ gemm_fp8_pair_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_const
         // one instruction covers 32 K bytes: +32 bytes = +2 in 16-byte units
 #pragma unroll
         for (int k = 0; k < 8; ++k)
-          umma_f8_pair_warp(on, tmem_base + a * 2 * BM, da + (k >> 2) * (X_BYTES / 2 / 16) + 2 * (k & 3), db + w_step(k & 3), idesc, k > 0);
+          umma_f8_pair_warp(on, tmem_base + a * 2 * BM, da + (k >> 2) * (X_BYTES / 2 / 16) + 2 * (k & 3), db + w_step(k & 3),
+                            k < 4 ? idesc_hi : idesc_mid, k > 0);
         commit_pair_warp(on, &done[b]);
       }
     }
@@ -220,7 +221,7 @@ gemm_fp8_pair_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_const
       f2 acc[BM / 2];
 #pragma unroll
       for (int i = 0; i < BM / 2; ++i) acc[i] = 0;
-      bool ok = true;
+      bool ok = true, outside = false;
       for (int c = 0; c < len; ++c) {
         const int blk = u - u0 + c, b = blk % S, a = blk % A;
         const float sw = c < RUN ? sc_run[c] : __ldg(srow + c);
@@ -239,7 +240,8 @@ gemm_fp8_pair_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_const
           }
         };
         if (busy) {
-          const float sv = sSx[b * ROWS + row] * sw;
+          const float sr = sSx[b * ROWS + row], sv = fabsf(sr) * sw;
+          outside |= sr < 0.f;
           const f2 s = pack2f(sv, sv);
           const uint32_t taddr = tmem_base + (uint32_t((warp & 3) * 32) << 16) + a * 2 * BM + group * BM;
 #pragma unroll
@@ -261,6 +263,25 @@ gemm_fp8_pair_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_const
         if (lane == 0) atomicExch(p.status, ERR_WAIT_ACC);
         *abort_flag = 1;
         *epi_abort = 1;
+      } else if (__any_sync(0xffffffffu, outside && row < rows)) {
+        // values outside the terms, on the CUDA cores: as a rule there are none, and in a block that has them a few
+        for (int c = 0; c < len; ++c) {
+          const float* sx = p.sx + ((size_t)n * p.kb + c0 + c) * PAIR_TOK + rank * ROWS;
+          uint32_t tokens = __ballot_sync(0xffffffffu, row < rows && __ldcg(sx + row) < 0.f);
+          const uint8_t* wb = p.w + ((size_t)m * p.kb + c0 + c) * W_BYTES;
+          const float sw = __ldg(srow + c);
+          for (; tokens; tokens &= tokens - 1) {
+            const int src = __ffs(tokens) - 1;
+            for_each_outside(p.rest, p.kb, n * PAIR_TOK + rank * ROWS + (warp & 3) * 32 + src, c0 + c, [&](int k, float x) {
+              const float mine = lane == src ? x : 0.f;
+#pragma unroll
+              for (int i = 0; i < BM / 2; ++i) {
+                const float2 w = e4m3x2_to_float2(wb[w_offset(2 * i, k)] | wb[w_offset(2 * i + 1, k)] << 8);
+                acc[i] = fma2(pack2f(w.x * sw, w.y * sw), pack2f(mine, mine), acc[i]);
+              }
+            });
+          }
+        }
       }
       epi_sync();
       if (*epi_abort) break;

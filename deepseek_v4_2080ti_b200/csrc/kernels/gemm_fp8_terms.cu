@@ -2,15 +2,15 @@
 //   Y[T, N] = X[T, K] * W[N, K]^T,  W = E4M3 with one scale per 128 x 128 block.
 //
 // Weights go from HBM to the tensor core untouched; the activations are adapted.  A bf16 number has 8 significant bits, an
-// E4M3 number 4, so with a power-of-two scale c per (token, 128 inputs) an activation is exactly
-//   x c = hi + mid,   hi, mid in E4M3
-// (for values above 2^-9 of the block's largest; below, off by at most 2^-18 of it).  Both terms have the same scale, so the
-// tensor core adds them: two products per K block into one accumulator, at twice the bf16 rate - the tensor time of bf16, half
-// the weight bytes, no decode warps, and no rounding of the scaled weights to bf16, which the decode-warp kernel
-// (gemm_wdec_kernel.cuh) needs and which costs 1.6e-3 of a result.  The scales are applied outside the tensor core: each
-// 128-wide K block is accumulated into its own TMEM buffer; one warp multiplies the weight scale into the block's activation
-// scales, and the epilogue warps add scale x block into fp32 registers, two tokens per instruction, while the tensor core is
-// on the next blocks.
+// E5M2 number 3, an E4M3 number 4, so with a power-of-two scale c per (token, 128 inputs) an activation is
+//   x c = hi + mid,   hi in E5M2, mid in E4M3
+// exactly where it is above 2^-13 of the block's largest (fp8_terms.cuh has what lies below, and what happens to blocks where
+// that is much).  Both terms have the same scale, so the tensor core adds them: two products per K block into one accumulator, at
+// twice the bf16 rate - the tensor time of bf16, half the weight bytes, no decode warps, and no rounding of the scaled weights to
+// bf16, which the decode-warp kernel (gemm_wdec_kernel.cuh) needs and which costs 1.6e-3 of a result.  The scales are applied
+// outside the tensor core: each 128-wide K block is accumulated into its own TMEM buffer; one warp multiplies the weight scale
+// into the block's activation scales, and the epilogue warps add scale x block into fp32 registers, two tokens per instruction,
+// while the tensor core is on the next blocks.
 //
 // This file: up to 64 tokens, one CTA per worker, weights as the MMA's M operand; bound by the weight stream, up to 190 KB in
 // flight per SM.  More tokens: gemm_fp8_pair.cu.
@@ -103,6 +103,7 @@ gemm_fp8_terms_kernel(Params p) {
   volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_slot + 1);
   volatile int* epi_abort = abort_flag + 1;     // written by epilogue threads only, always before a barrier
   int* fix_last = const_cast<int*>(abort_flag) + 2;
+  volatile int* last_outside = abort_flag + 3;  // the last block so far in which a token has values outside its terms
 
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   if (threadIdx.x == 0) {
@@ -116,6 +117,7 @@ gemm_fp8_terms_kernel(Params p) {
     for (int a = 0; a < A; ++a) mbar_init(&acc_free[a], READERS);
     *abort_flag = 0;
     *epi_abort = 0;
+    *last_outside = -1;
     mbar_fence_init();
   }
   if (warp == WARP_MMA) {
@@ -170,7 +172,8 @@ gemm_fp8_terms_kernel(Params p) {
     // -------------------------------------------------------------- MMA issuer
     {
       const uint32_t on = elect_one();
-      const uint32_t idesc = umma_idesc_e4m3(BM, round16(p.T));      // as many columns as there are tokens
+      // as many columns as there are tokens
+      const uint32_t idesc_hi = umma_idesc_f8(BM, round16(p.T), false, true), idesc_mid = umma_idesc_f8(BM, round16(p.T));
       for (int blk = 0; blk < u1 - u0; ++blk) {
         const int b = blk % S, a = blk % A;
         int err = 0;
@@ -189,7 +192,7 @@ gemm_fp8_terms_kernel(Params p) {
 #pragma unroll
         for (int k = 0; k < 8; ++k) {
           const uint64_t dbk = db + (k >> 2) * (L::X_BYTES / 2 / 16) + 2 * (k & 3);
-          umma_f8_warp(on, d, da + w_step(k & 3), dbk, idesc, k > 0);
+          umma_f8_warp(on, d, da + w_step(k & 3), dbk, k < 4 ? idesc_hi : idesc_mid, k > 0);
         }
         umma_commit_warp(on, &done[b]);
       }
@@ -219,7 +222,13 @@ gemm_fp8_terms_kernel(Params p) {
         ok = __all_sync(0xffffffffu, mbar_wait(&sx_full[b], (blk / S) & 1));
         if (!ok) break;
         float* sx = sSx + b * TOK;
-        for (int i = lane; i < TOK; i += 32) sx[i] *= sc;
+        bool outside = false;
+        for (int i = lane; i < TOK; i += 32) {
+          const float v = sx[i];
+          outside |= i < p.T && v < 0.f;
+          sx[i] = fabsf(v) * sc;
+        }
+        if (__any_sync(0xffffffffu, outside) && lane == 0) *last_outside = blk;
         fence_proxy_async_smem();          // the next copy into this slot comes after these writes
         __syncwarp();
         if (lane == 0) mbar_arrive(&sc_full[b]);
@@ -278,6 +287,23 @@ gemm_fp8_terms_kernel(Params p) {
         if (lane == 0) atomicExch(p.status, ERR_WAIT_ACC);
         *abort_flag = 1;
         *epi_abort = 1;
+      } else if (*last_outside >= u - u0) {
+        // values outside the terms, on the CUDA cores: as a rule there are none, and in a block that has them a few
+        for (int c = L::BY_TOKENS ? 0 : (group ^ ((u - u0) & 1)); c < len; c += L::BY_TOKENS ? 1 : 2) {
+          const float* sx = p.sx + (size_t)(c0 + c) * TOK + w0;
+          uint32_t tokens = __ballot_sync(0xffffffffu, lane < WT && w0 + lane < w1 && __ldcg(sx + lane) < 0.f);
+          if (!tokens) continue;
+          const uint8_t* wb = p.w + (size_t)(u + c) * W_BYTES;
+          const float sc = __ldg(p.scales + u + c);
+          for (; tokens; tokens &= tokens - 1) {
+            const int t = __ffs(tokens) - 1;
+            float sum = 0.f;
+            for_each_outside(p.rest, p.kb, w0 + t, c0 + c,
+                             [&](int k, float x) { sum += x * (e4m3x2_to_float2(wb[w_offset(row, k)]).x * sc); });
+#pragma unroll
+            for (int i = 0; i < WT / 2; ++i) acc[i] = add2(acc[i], pack2f(t == 2 * i ? sum : 0.f, t == 2 * i + 1 ? sum : 0.f));
+          }
+        }
       }
       if constexpr (!L::BY_TOKENS) {
         if (group == 1) {
@@ -434,26 +460,6 @@ struct Eight {
     }
     return u;
   }
-  // values i0 .. i0 + 7 of token t, for threads that are `on`; the whole warp takes part
-  __device__ __forceinline__ void put(const TermsOut& o, int t, int i0, bool on) const {
-    uint32_t m = 0;
-#pragma unroll
-    for (int i = 0; i < 8; ++i) m = max(m, bf16_magnitude(v[i]));
-#pragma unroll
-    for (int d = 8; d > 0; d >>= 1) m = max(m, __shfl_xor_sync(0xffffffffu, m, d));
-    if (!on) return;
-    const TermScale ts(m);
-    uint2 hi, mid;
-    ts.split4(v, hi.x, mid.x);
-    ts.split4(v + 4, hi.y, mid.y);
-    const int c = i0 >> 7, g = (i0 & 127) >> 2;
-    int row;
-    uint8_t* dst = o.hi_row(t, c, row);
-    dst += term_offset(row, g);
-    *reinterpret_cast<uint2*>(dst) = hi;
-    *reinterpret_cast<uint2*>(dst + o.cap * 128) = mid;
-    if ((i0 & 127) == 0) *o.scale(t, c) = ts.inv;
-  }
 };
 
 __global__ void __launch_bounds__(256) split_terms_kernel(const __nv_bfloat16* __restrict__ x, int K, TermsOut o) {
@@ -462,7 +468,7 @@ __global__ void __launch_bounds__(256) split_terms_kernel(const __nv_bfloat16* _
   const int i = (blockIdx.x * 256 + threadIdx.x) * 8, t = blockIdx.y;
   Eight e = {};
   if (i < K) e.load(x + (size_t)t * K + i);
-  e.put(o, t, i, i < K);
+  put_terms(o, t, i, e.v, i < K);
 }
 
 // silu(gate) up of rows [gate | up], rounded to bf16, as terms.
@@ -478,7 +484,7 @@ __global__ void __launch_bounds__(256) silu_mul_terms_kernel(const __nv_bfloat16
     for (int k = 0; k < 8; ++k) g.v[k] = g.v[k] / (1.f + __expf(-g.v[k])) * u.v[k];
     g.round();
   }
-  g.put(o, t, i, i < I);
+  put_terms(o, t, i, g.v, i < I);
 }
 
 // x (+= delta, written back) -> rmsnorm(x) (1 +) gamma in bf16: stored (out, optional) and as terms.  One block per row, V
@@ -534,7 +540,7 @@ __global__ void __launch_bounds__(1024) rmsnorm_terms_kernel(__nv_bfloat16* __re
       const uint4 r = e[j].round();
       if (out) *reinterpret_cast<uint4*>(out + (size_t)t * cols + i) = r;
     }
-    e[j].put(o, t, i, i < cols);
+    put_terms(o, t, i, e[j].v, i < cols);
   }
 }
 
@@ -572,37 +578,38 @@ int b200_fp8_terms_plan(int T, int N, int K, int* tok, long long* partial_floats
   return 0;
 }
 
-static bool terms_out(f8t::TermsOut* o, int T, int K, int tok, void* xq, float* sx) {
-  if (T <= 0 || T > 65535 || K <= 0 || (K % 128) != 0 || tok != f8t::tile_tokens(T)) return false;
+static bool terms_out(f8t::TermsOut* o, int T, int K, int tok, void* xq, float* sx, void* rest) {
+  if (!xq || !sx || !rest || T <= 0 || T > 65535 || K <= 0 || (K % 128) != 0 || tok != f8t::tile_tokens(T)) return false;
   o->xq = reinterpret_cast<uint8_t*>(xq);
   o->sx = sx;
+  o->rest = reinterpret_cast<__nv_bfloat16*>(rest);
   o->tok = tok;
   o->cap = tok == f8t::PAIR_TOK ? tok / 2 : tok;
   o->kb = K / 128;
   return true;
 }
 
-// x [T, K] bf16 -> xq: ceil(T / tok) * (K / 128) blocks of 256 tok bytes, sx: as many blocks of tok floats.
-int b200_split_terms(const void* x_bf16, int T, int K, int tok, void* xq, float* sx, cudaStream_t stream) {
+// x [T, K] bf16 -> xq: ceil(T / tok) * (K / 128) blocks of 256 tok bytes, sx: as many blocks of tok floats, rest: [T, K] bf16.
+int b200_split_terms(const void* x_bf16, int T, int K, int tok, void* xq, float* sx, void* rest, cudaStream_t stream) {
   f8t::TermsOut o;
-  if (!terms_out(&o, T, K, tok, xq, sx)) return -ERR_BAD_ARG;
+  if (!terms_out(&o, T, K, tok, xq, sx, rest)) return -ERR_BAD_ARG;
   return (int)launch_pdl(f8t::split_terms_kernel, dim3((K / 8 + 255) / 256, T), dim3(256), 0, stream,
                          reinterpret_cast<const __nv_bfloat16*>(x_bf16), K, o);
 }
 
 // gu [T, 2 I] (gate | up) -> terms of bf16(silu(gate) up).
-int b200_silu_mul_terms(const void* gu, int T, int I, int tok, void* xq, float* sx, cudaStream_t stream) {
+int b200_silu_mul_terms(const void* gu, int T, int I, int tok, void* xq, float* sx, void* rest, cudaStream_t stream) {
   f8t::TermsOut o;
-  if (!terms_out(&o, T, I, tok, xq, sx)) return -ERR_BAD_ARG;
+  if (!terms_out(&o, T, I, tok, xq, sx, rest)) return -ERR_BAD_ARG;
   return (int)launch_pdl(f8t::silu_mul_terms_kernel, dim3((I / 8 + 255) / 256, T), dim3(256), 0, stream,
                          reinterpret_cast<const __nv_bfloat16*>(gu), I, o);
 }
 
 // x [T, cols] (+= delta, written back when delta is given) -> out = rmsnorm(x) gamma (bf16, optional) and its terms.
 int b200_rmsnorm_terms(void* x, const void* delta, const void* gamma, void* out, int T, int cols, float eps, int unit_offset, int tok,
-                       void* xq, float* sx, cudaStream_t stream) {
+                       void* xq, float* sx, void* rest, cudaStream_t stream) {
   f8t::TermsOut o;
-  if (cols > 4 * 8192 || !terms_out(&o, T, cols, tok, xq, sx)) return -ERR_BAD_ARG;
+  if (cols > 4 * 8192 || !terms_out(&o, T, cols, tok, xq, sx, rest)) return -ERR_BAD_ARG;
   auto* xp = reinterpret_cast<__nv_bfloat16*>(x);
   auto* dp = reinterpret_cast<const __nv_bfloat16*>(delta);
   auto* gp = reinterpret_cast<const __nv_bfloat16*>(gamma);
@@ -616,11 +623,11 @@ int b200_rmsnorm_terms(void* x, const void* delta, const void* gamma, void* out,
 }
 
 // Y = X W^T (+ residual) from the terms of X.  W: packed FP8 tiles (b200_gemm_wdec, wfmt 1), scales [ceil(N/128), K/128].
-int b200_gemm_fp8_terms(const void* W, const float* scales, const void* xq, const float* sx, void* out_bf16, const void* residual,
-                        int T, int N, int K, float* partial, int* counters, int* status, cudaStream_t stream) {
+int b200_gemm_fp8_terms(const void* W, const float* scales, const void* xq, const float* sx, const void* rest, void* out_bf16,
+                        const void* residual, int T, int N, int K, float* partial, int* counters, int* status, cudaStream_t stream) {
   int tok = 0, n_cnt = 0;
   long long n_part = 0;
-  if (!W || !scales || !xq || !sx || !out_bf16 || !partial || !counters || b200_fp8_terms_plan(T, N, K, &tok, &n_part, &n_cnt)) return -ERR_BAD_ARG;
+  if (!W || !scales || !xq || !sx || !rest || !out_bf16 || !partial || !counters || b200_fp8_terms_plan(T, N, K, &tok, &n_part, &n_cnt)) return -ERR_BAD_ARG;
   const int cg = tok == f8t::PAIR_TOK ? 2 : 1;
   f8t::Params p;
   memset(&p, 0, sizeof(p));
@@ -635,6 +642,7 @@ int b200_gemm_fp8_terms(const void* W, const float* scales, const void* xq, cons
   p.scales = scales;
   p.xq = reinterpret_cast<const uint8_t*>(xq);
   p.sx = sx;
+  p.rest = reinterpret_cast<const __nv_bfloat16*>(rest);
   p.out = reinterpret_cast<__nv_bfloat16*>(out_bf16);
   p.residual = reinterpret_cast<const __nv_bfloat16*>(residual);
   p.partial = partial;

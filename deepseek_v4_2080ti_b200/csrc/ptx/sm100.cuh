@@ -213,10 +213,11 @@ __host__ __device__ constexpr uint32_t umma_idesc_bf16(int M, int N) {
 __host__ __device__ constexpr uint32_t umma_idesc_f16(int M, int N) {
   return (1u << 4) | (0u << 7) | (0u << 10) | (uint32_t(N >> 3) << 17) | (uint32_t(M >> 4) << 24);
 }
-// kind::f8f6f4 with e4m3 A/B, fp32 D.
-__host__ __device__ constexpr uint32_t umma_idesc_e4m3(int M, int N) {
-  return (1u << 4) | (0u << 7) | (0u << 10) | (uint32_t(N >> 3) << 17) | (uint32_t(M >> 4) << 24);
+// kind::f8f6f4 with e4m3 A/B (e5m2 for an operand that is asked for), fp32 D.
+__host__ __device__ constexpr uint32_t umma_idesc_f8(int M, int N, bool a_e5m2 = false, bool b_e5m2 = false) {
+  return (1u << 4) | (uint32_t(a_e5m2) << 7) | (uint32_t(b_e5m2) << 10) | (uint32_t(N >> 3) << 17) | (uint32_t(M >> 4) << 24);
 }
+__host__ __device__ constexpr uint32_t umma_idesc_e4m3(int M, int N) { return umma_idesc_f8(M, N); }
 // D[tmem] (+)= A[smem] * B[smem]; issued by exactly one thread.
 __device__ __forceinline__ void umma_bf16_ss(uint32_t tmem_d, uint64_t desc_a, uint64_t desc_b,
                                              uint32_t idesc, uint32_t accumulate) {

@@ -577,7 +577,7 @@ class QwenHybridRuntime(PagedSequences):
         self._expand_ahead(x, w)
         return self.comm.all_reduce(gemm.linear(x, w))
 
-    # Projections of a decode step.  On one rank an activation goes to its matrix as the exact E4M3 terms the matrix is
+    # Projections of a decode step.  On one rank an activation goes to its matrix as the FP8 terms the matrix is
     # multiplied with (``gemm.Terms``); under tensor parallelism as E4M3 terms of the weight-streaming GEMM whose epilogue
     # carries the all-reduce.
     def _decode_norm(self, h: torch.Tensor, delta: torch.Tensor | None, gamma: torch.Tensor, want_bf16: bool):
@@ -610,7 +610,7 @@ class QwenHybridRuntime(PagedSequences):
         return self.comm.all_reduce(gemm.linear_stream(x, w, xsplit=xsplit))
 
     def _terms_rows(self, t: int, lw: LayerWeights) -> bool:
-        """Do the FP8 products of a ``t``-row batch through layer ``lw`` take their activations as E4M3 terms, straight from
+        """Do the FP8 products of a ``t``-row batch through layer ``lw`` take their activations as FP8 terms, straight from
         the kernels that make them?"""
         return self.comm.world == 1 and self.fused_decode and \
             not any(gemm.expands(t, m) or not gemm.terms_fit(t, m) for m in (lw.proj, lw.out, lw.gate_up, lw.down))
@@ -783,7 +783,7 @@ class QwenHybridRuntime(PagedSequences):
             proj = self._decode_linear(a, lw.proj)
             if lw.kind == "linear":
                 idx = self.lin_layers.index(i)
-                terms = gemm.empty_terms(t, self.vd, self.device) if self.comm.world == 1 else None
+                terms = gemm.Terms(t, self.vd, self.device) if self.comm.world == 1 else None
                 y = gdn.decode_fused(proj, x, lw.ab.weight, lw.a_log, lw.dt_bias, lw.conv_w, self.tails[:, idx],
                                      self.states[:, idx], slots_t, lw.gdn_norm, self.hv_lin, self.hk_lin, eps, terms=terms)
             else:

@@ -70,9 +70,9 @@ def rmsnorm_terms(resid: torch.Tensor, delta: torch.Tensor | None, gamma: torch.
     rows, cols = resid.shape
     assert resid.is_contiguous() and (delta is None or delta.is_contiguous())
     out = torch.empty_like(resid) if want_bf16 else None
-    xt = gemm.empty_terms(rows, cols, resid.device)
+    xt = gemm.Terms(rows, cols, resid.device)
     rc = _lib.lib().b200_rmsnorm_terms(_lib.ptr(resid), _lib.ptr(delta), _lib.ptr(gamma), _lib.ptr(out), rows, cols, _f(eps),
-                                       int(unit_offset), xt.sx.shape[2], _lib.ptr(xt.xq), _lib.ptr(xt.sx), _lib.stream())
+                                       int(unit_offset), xt.tok, *xt.ptrs, _lib.stream())
     _lib.check(rc, "rmsnorm_terms")
     return out, xt
 
@@ -81,8 +81,8 @@ def silu_mul_terms(gu: torch.Tensor):
     """gu [T, 2I] (gate | up) -> ``gemm.Terms`` of bf16(silu(gate) * up)."""
     from . import gemm
     assert gu.is_contiguous()
-    xt = gemm.empty_terms(gu.shape[0], gu.shape[1] // 2, gu.device)
-    rc = _lib.lib().b200_silu_mul_terms(_lib.ptr(gu), xt.t, xt.k, xt.sx.shape[2], _lib.ptr(xt.xq), _lib.ptr(xt.sx), _lib.stream())
+    xt = gemm.Terms(gu.shape[0], gu.shape[1] // 2, gu.device)
+    rc = _lib.lib().b200_silu_mul_terms(_lib.ptr(gu), xt.t, xt.k, xt.tok, *xt.ptrs, _lib.stream())
     _lib.check(rc, "silu_mul_terms")
     return xt
 

@@ -58,16 +58,16 @@ def decode_fused(proj, x, w_ab, a_log, dt_bias, conv_w, tails, states, slot_ids,
     proj [B, 2kd+2vd] bf16 = q|k|v|z projection output; x [B, hidden] bf16 normed layer input; w_ab [2Hv, hidden]
     bf16 (a rows, then b rows); conv_w [2kd+vd, 4] bf16; tails [slots, 3, 2kd+vd] bf16 and states
     [slots, Hv, 128, 128] fp32 are updated in place for ``slot_ids`` (int32 [B]).  Returns [B, Hv*128] bf16
-    (gated-RMSNorm output, the input of the output projection), or ``terms`` (``gemm.empty_terms(B, Hv*128)``) filled with it."""
+    (gated-RMSNorm output, the input of the output projection), or ``terms`` (a ``gemm.Terms`` of [B, Hv*128]) filled with it."""
     b = proj.shape[0]
     _lib.check_indices(slot_ids, 0, states.shape[0], 4)
     out = torch.empty(b, hv * 128, dtype=torch.bfloat16, device=proj.device) if terms is None else None
-    xq, sx, tok = (terms.xq, terms.sx, terms.sx.shape[2]) if terms is not None else (None, None, 0)
+    xq, sx, rest = terms.ptrs if terms is not None else (None, None, None)
     rc = _lib.lib().b200_gdn_decode_fused(
         _lib.ptr(proj), proj.stride(0), _lib.ptr(x), x.shape[1], _lib.ptr(w_ab), _lib.ptr(a_log), _lib.ptr(dt_bias),
         _lib.ptr(conv_w), conv_w.shape[1], _lib.ptr(tails), _ll(tails.stride(0)), _lib.ptr(states),
         _ll(states.stride(0)), _lib.ptr(slot_ids), _lib.ptr(gamma), _lib.ptr(out), b, hv, hk, ctypes.c_float(eps),
-        _lib.ptr(xq), _lib.ptr(sx), tok, _lib.stream())
+        xq, sx, rest, terms.tok if terms is not None else 0, _lib.stream())
     _lib.check(rc, "gdn_decode_fused")
     return out if terms is None else terms
 

@@ -368,14 +368,33 @@ def linear_stream(x: torch.Tensor, w: PackedLinear, residual: torch.Tensor | Non
     return out
 
 
-@dataclass
 class Terms:
-    """bf16 activations as two E4M3 terms per value, in the order ``linear_terms`` streams them
-    (csrc/kernels/gemm_fp8_terms.cu): blocks of 256 x ``tok`` bytes per (token tile, 128 inputs), and their scales."""
-    xq: torch.Tensor              # uint8 [ceil(t / tok), k / 128, 2 tok, 128]
-    sx: torch.Tensor              # fp32 [ceil(t / tok), k / 128, tok], powers of two
-    t: int
-    k: int
+    """bf16 activations [t, k] as two FP8 terms per value, in the order ``linear_terms`` streams them
+    (csrc/kernels/gemm_fp8_terms.cu): ``xq`` in blocks of 256 x ``tok`` bytes per (token tile, 128 inputs), ``sx`` their scales,
+    ``rest`` the values that a block's terms leave out; one allocation."""
+
+    def __init__(self, t: int, k: int, device):
+        self.t, self.k, self.device = t, k, device
+        self.tok = tok = _terms_plan(t, 128, k)[0]
+        self._blocks = blocks = (t + tok - 1) // tok * (k // 128)
+        self.buf = torch.empty(blocks * tok * 260 + t * k * 2, dtype=torch.uint8, device=device)
+        base = self.buf.data_ptr()
+        self.ptrs = tuple(ctypes.c_void_p(base + o) for o in (0, blocks * tok * 256, blocks * tok * 260))      # xq, sx, rest
+
+    @property
+    def xq(self) -> torch.Tensor:
+        """uint8 [ceil(t / tok), k / 128, 2 tok, 128]"""
+        return self.buf[:self._blocks * self.tok * 256].view(-1, self.k // 128, 2 * self.tok, 128)
+
+    @property
+    def sx(self) -> torch.Tensor:
+        """fp32 [ceil(t / tok), k / 128, tok]: powers of two, negative where ``rest`` has values of the block"""
+        return self.buf[self._blocks * self.tok * 256:self._blocks * self.tok * 260].view(torch.float32).view(-1, self.k // 128, self.tok)
+
+    @property
+    def rest(self) -> torch.Tensor:
+        """bf16 [t, k], defined in the blocks whose scale is negative"""
+        return self.buf[self._blocks * self.tok * 260:].view(torch.bfloat16).view(self.t, self.k)
 
 
 def _terms_plan(t: int, n: int, k: int) -> tuple[int, int, int]:
@@ -385,18 +404,11 @@ def _terms_plan(t: int, n: int, k: int) -> tuple[int, int, int]:
     return tok.value, part.value, cnt.value
 
 
-def empty_terms(t: int, k: int, device) -> Terms:
-    tok = _terms_plan(t, 128, k)[0]
-    blocks = ((t + tok - 1) // tok, k // 128)
-    return Terms(torch.empty(*blocks, 2 * tok, 128, dtype=torch.uint8, device=device),
-                 torch.empty(*blocks, tok, dtype=torch.float32, device=device), t, k)
-
-
 def split_terms(x: torch.Tensor) -> Terms:
-    """bf16 [T, K] (K % 128 == 0) as exact E4M3 terms."""
+    """bf16 [T, K] (K % 128 == 0) as terms."""
     assert x.dtype == torch.bfloat16 and x.is_contiguous()
-    xt = empty_terms(*x.shape, x.device)
-    rc = _lib.lib().b200_split_terms(_lib.ptr(x), xt.t, xt.k, xt.sx.shape[2], _lib.ptr(xt.xq), _lib.ptr(xt.sx), _lib.stream())
+    xt = Terms(*x.shape, x.device)
+    rc = _lib.lib().b200_split_terms(_lib.ptr(x), xt.t, xt.k, xt.tok, *xt.ptrs, _lib.stream())
     _lib.check(rc, "split_terms")
     return xt
 
@@ -410,14 +422,14 @@ def terms_fit(t: int, w: "PackedLinear") -> bool:
 def linear_terms(xt: Terms, w: PackedLinear, residual: torch.Tensor | None = None, out: torch.Tensor | None = None) -> torch.Tensor:
     """``x @ w^T`` (+ residual) for FP8 block-128 weights: bf16 [T, N]."""
     assert w.wfmt == WF_FP8_B128 and xt.k == w.k
-    dev = xt.xq.device
+    dev = xt.device
     if out is None:
         out = torch.empty(xt.t, w.n, dtype=torch.bfloat16, device=dev)
     _, part, cnt = _terms_plan(xt.t, w.n, w.k)
     assert cnt <= MAX_TILE_COUNTERS
     ws, counters = _workspace(part, dev)
-    rc = _lib.lib().b200_gemm_fp8_terms(_lib.ptr(w.weight), _lib.ptr(w.scales), _lib.ptr(xt.xq), _lib.ptr(xt.sx), _lib.ptr(out),
-                                        _lib.ptr(residual), xt.t, w.n, w.k, _lib.ptr(ws), _lib.ptr(counters),
+    rc = _lib.lib().b200_gemm_fp8_terms(_lib.ptr(w.weight), _lib.ptr(w.scales), *xt.ptrs, _lib.ptr(out), _lib.ptr(residual),
+                                        xt.t, w.n, w.k, _lib.ptr(ws), _lib.ptr(counters),
                                         _lib.ptr(_lib.status_word(dev)), _lib.stream())
     _lib.check(rc, "gemm_fp8_terms")
     return out
@@ -427,7 +439,7 @@ def linear(x: torch.Tensor, w: PackedLinear, residual: torch.Tensor | None = Non
            out: torch.Tensor | None = None, splits: int | None = None,
            out_f32: bool = False, stream: bool | None = None) -> torch.Tensor:
     """``x [T, K] bf16`` -> ``[T, N]`` bf16 (or fp32 when ``out_f32``).  FP8 weights go to the FP8 tensor pipe with the
-    activations as exact E4M3 terms, or, in prefill-sized batches that the CTA-pair kernel tiles evenly, are expanded to
+    activations as pairs of FP8 terms (``Terms``), or, in prefill-sized batches that the CTA-pair kernel tiles evenly, are expanded to
     bf16 first; ``stream=False``, or a number of ``splits``, asks for the decode-warp kernel (up to 32 tokens and not
     ``stream=False``: the weight-streaming kernel), whose split-K partials are reduced by the last-arriving CTA of each
     output tile."""

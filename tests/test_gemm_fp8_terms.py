@@ -1,4 +1,4 @@
-"""FP8 block-128 products from exact E4M3 terms (csrc/kernels/gemm_fp8_terms.cu, gemm_fp8_pair.cu)."""
+"""FP8 block-128 products from pairs of FP8 terms (csrc/kernels/gemm_fp8_terms.cu, gemm_fp8_pair.cu)."""
 import pytest
 import torch
 
@@ -12,17 +12,38 @@ SHAPES = [(1, 128, 128), (1, 5120, 4096), (16, 384, 512), (17, 1000, 1280), (32,
 
 
 def _terms(xt, t, k):
-    """hi + mid of every activation, times its block's scale, from the stored layout."""
-    tok = xt.sx.shape[2]
+    """What the stored layout says of every activation: (hi + mid) times its block's scale, plus what lies outside."""
+    tok = xt.tok
     cap = tok // 2 if tok == 256 else tok
     n, kb = xt.sx.shape[:2]
     b = xt.xq.reshape(n, kb, tok // cap, 2, cap, 8, 16)
     rows = torch.arange(cap, device=b.device)[:, None]
     src = torch.arange(8, device=b.device)[None] ^ (rows & 7)
     b = torch.gather(b, 5, src[None, None, None, None, :, :, None].expand_as(b))
-    v = b.reshape(n, kb, tok // cap, 2, cap, 32, 4)[..., [0, 2, 1, 3]].contiguous().view(torch.float8_e4m3fn).float()
-    v = v.sum(3).reshape(n, kb, tok, 128) * xt.sx[..., None]
-    return v.permute(0, 2, 1, 3).reshape(n * tok, k)[:t]
+    b = b.reshape(n, kb, tok // cap, 2, cap, 32, 4)[..., [0, 2, 1, 3]]
+    hi, mid = (b[:, :, :, i].contiguous().view(f).float() for i, f in ((0, torch.float8_e5m2), (1, torch.float8_e4m3fn)))
+    v = (hi + mid).reshape(n, kb, tok, 128) * xt.sx.abs()[..., None]
+    v = v.permute(0, 2, 1, 3).reshape(n * tok, k)[:t]
+    outside = (xt.sx < 0).permute(0, 2, 1).reshape(n * tok, kb)[:t].repeat_interleave(128, 1)
+    return torch.where(outside, v + xt.rest.float(), v)
+
+
+def _bound(x):
+    """How far a block's terms may be off: 2^-9 of a value in its smallest quarter (2^-10 of the units in which that value is at
+    least 2^-2), and 2^-21 of its largest where that is less."""
+    b = x.float().view(x.shape[0], -1, 128).abs()
+    quarter = torch.where(b > 0, b, float("inf")).sort(-1).values
+    at = ((b > 0).sum(-1, keepdim=True) // 4).clamp_max(127)
+    q = torch.gather(quarter, -1, at) * 2.0 ** -8
+    return torch.minimum(q, b.amax(-1, keepdim=True) * 2.0 ** -21).expand_as(b).reshape(x.shape)
+
+
+def _outliers(t, k, exponent, device="cuda"):
+    """Normal rows with two values of size 2^exponent in every block of 128."""
+    x = torch.randn(t, k, device=device)
+    x.view(t, -1, 128)[:, :, 5] = 2.0 ** exponent
+    x.view(t, -1, 128)[:, :, 77] = -1.5 * 2.0 ** exponent
+    return x.bfloat16()
 
 
 @pytest.mark.gpu
@@ -34,9 +55,65 @@ def test_terms_are_exact(t):
     x[0, :128] = 0
     got, xf = _terms(gemm.split_terms(x), t, 384), x.float()
     top = xf.view(t, 3, 128).abs().amax(-1, keepdim=True).expand(t, 3, 128).reshape(t, 384)
-    small = xf.abs() < top * 2.0 ** -9
+    small = xf.abs() < top * 2.0 ** -13
     assert torch.equal(got[~small], xf[~small])
-    assert ((got - xf).abs() <= top * 2.0 ** -17).all()
+    assert ((got - xf).abs() <= _bound(x)).all()
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("t", [1, 40, 90])
+@pytest.mark.parametrize("make", [
+    lambda t: _outliers(t, 384, 11), lambda t: _outliers(t, 384, 14), lambda t: _outliers(t, 384, 40),
+    lambda t: (torch.randn(t, 384, device="cuda") * torch.exp2(torch.randint(-120, 120, (t, 384), device="cuda").float())).bfloat16(),
+    lambda t: torch.where(torch.rand(t, 384, device="cuda") < 0.95, torch.zeros((), device="cuda"),      # sparse rows
+                          torch.exp2(torch.randint(-60, 60, (t, 384), device="cuda").float())).bfloat16()])
+def test_wide_blocks_keep_their_small_values(t, make):
+    from deepseek_v4_2080ti_b200.ops import gemm
+    torch.manual_seed(t)
+    x = make(t)
+    assert ((_terms(gemm.split_terms(x), t, 384) - x.float()).abs() <= _bound(x)).all()
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("t", [1, 6, 32, 33, 64, 65, 100, 300])
+@pytest.mark.parametrize("exponent", [8, 10, 11, 12, 14, 18, 30])
+def test_large_values_whose_weights_are_zero_hide_nothing(t, exponent):
+    """The large values of every block meet weights of zero: what is left is the product of the others."""
+    from deepseek_v4_2080ti_b200.ops import _lib, gemm
+    torch.manual_seed(t + exponent)
+    n, k = 320, 640
+    wf = torch.randn(n, k, device="cuda") * 0.05
+    wf.view(n, -1, 128)[:, :, 5] = wf.view(n, -1, 128)[:, :, 77] = 0
+    q, s = fp8fmt.quantize_block128(wf)
+    x = _outliers(t, k, exponent)
+    y = gemm.linear(x, gemm.PackedLinear.from_fp8(q, s))
+    torch.cuda.synchronize()
+    _lib.check_status()
+    ref = x.double() @ fp8fmt.dequantize_block128(q, s).double().t()
+    # 2^-9 of the result: its rounding to bf16 (2^-9 at most, 2^-9 / sqrt 3 in the mean) and the terms (a quarter of the values
+    # off by up to 2^-8 of the value at the quarter, a third of the mean size)
+    assert ((y.double() - ref).norm() / ref.norm()).item() < 2.0 ** -9
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("t,n,k", [(3, 200, 256), (30, 1000, 1280), (64, 384, 2560), (70, 33, 384), (257, 640, 2560), (300, 5120, 1024)])
+def test_values_outside_the_terms_are_multiplied(t, n, k):
+    """Outliers with weights like any other, in some blocks of some rows, runs cut and whole, with a residual."""
+    from deepseek_v4_2080ti_b200.ops import gemm
+    torch.manual_seed(t + n + k)
+    q, s = fp8fmt.quantize_block128(torch.randn(n, k, device="cuda") * 0.05)
+    w, wd = gemm.PackedLinear.from_fp8(q, s), fp8fmt.dequantize_block128(q, s).double()
+    x = torch.randn(t, k, device="cuda").bfloat16()
+    blocks = torch.rand(t, k // 128, 1, device="cuda") < 0.2
+    x = torch.where(blocks, _outliers(t, k, 16).view(t, -1, 128), x.view(t, -1, 128)).view(t, k)
+    r = torch.randn(t, n, device="cuda").bfloat16()
+    xt = gemm.split_terms(x)
+    assert (xt.sx[..., :].lt(0).any())
+    y, again, z = gemm.linear_terms(xt, w), gemm.linear_terms(xt, w), gemm.linear_terms(xt, w, residual=r)
+    ref = x.double() @ wd.t()
+    rel = lambda a, b: ((a.double() - b).norm(dim=1) / b.norm(dim=1)).max().item()
+    assert rel(y, ref) < 2.0 ** -8 and rel(z, ref + r.double()) < 2.0 ** -8          # every row: at most the rounding to bf16
+    assert torch.equal(y, again)
 
 
 @pytest.mark.gpu
@@ -64,7 +141,7 @@ def test_product_matches_64_bit(t, n, k):
 
 
 @pytest.mark.gpu
-@pytest.mark.parametrize("t", [3, 80])
+@pytest.mark.parametrize("t", [5, 40, 80])
 def test_infinities_and_nans_stay_in_their_row(t):
     from deepseek_v4_2080ti_b200.ops import gemm
     torch.manual_seed(t)
@@ -72,11 +149,17 @@ def test_infinities_and_nans_stay_in_their_row(t):
     w, wd = gemm.PackedLinear.from_fp8(q, s), fp8fmt.dequantize_block128(q, s)
     x = torch.randn(t, 256, device="cuda").bfloat16()
     clean = gemm.linear_terms(gemm.split_terms(x), w)
-    x[0, 5], x[1, 200] = float("inf"), float("nan")
-    y = gemm.linear_terms(gemm.split_terms(x), w)
-    ref = x[:1].float() @ wd.t()
-    assert torch.equal(y[2:], clean[2:]) and y[1].isnan().all()
-    assert torch.equal(y[0].float().isinf(), ref[0].isinf()) and torch.equal(y[0].float()[ref[0].isinf()], ref[0][ref[0].isinf()])
+    inf = float("inf")
+    x[0, 5], x[1, 200] = inf, float("nan")
+    x[2, 5], x[2, 77] = inf, -inf                 # two of a block
+    x[3, 5], x[3, 200] = inf, inf                 # two blocks
+    x[4, 200], x[4, 201], x[4, 202] = -inf, -inf, 2.0 ** 100
+    y = gemm.linear_terms(gemm.split_terms(x), w).double()
+    ref = x.double() @ wd.double().t()
+    assert torch.equal(y[5:], clean[5:].double())
+    for kind in (torch.isnan, torch.isposinf, torch.isneginf):
+        assert torch.equal(kind(y[:5]), kind(ref[:5]))
+    assert ref[2].isnan().any() and ref[2].isinf().any() and not ref[:5].isfinite().any()
 
 
 @pytest.mark.gpu
@@ -92,7 +175,7 @@ def test_norm_leaves_its_result_as_terms(t, cols):
     ref = basic.rmsnorm_ref(stream, g, 1e-6, True)
     assert ((out.float() - ref).abs() <= ref.abs() * 2.0 ** -8 + 1e-6).all()        # bf16 rounding, fp32 sums in any order
     got = _terms(xt, t, cols)
-    assert ((got - out.float()).abs() <= out.float().view(t, -1, 128).abs().amax(-1).repeat_interleave(128, 1) * 2.0 ** -17).all()
+    assert ((got - out.float()).abs() <= _bound(out)).all()
     none, alone = basic.rmsnorm_terms(stream, None, g, 1e-6, True, want_bf16=False)
     assert none is None and torch.equal(_terms(alone, t, cols), got)
 
@@ -104,8 +187,7 @@ def test_activation_leaves_its_result_as_terms(t, inter):
     torch.manual_seed(t + inter)
     gu = (torch.randn(t, 2 * inter, device="cuda") * 2).bfloat16()
     ref, got = basic.silu_mul_ref(gu), _terms(basic.silu_mul_terms(gu), t, inter)
-    top = ref.view(t, -1, 128).abs().amax(-1).repeat_interleave(128, 1)
-    assert ((got - ref).abs() <= ref.abs() * 2.0 ** -8 + top * 2.0 ** -17).all()
+    assert ((got - ref).abs() <= ref.abs() * 2.0 ** -8 + _bound(ref)).all()
 
 
 @pytest.mark.gpu
@@ -121,8 +203,8 @@ def test_decode_mixer_leaves_its_result_as_terms(b, hv, hk):
     slots = torch.randperm(b, device="cuda").int()
     args = lambda: (proj, x, w_ab, a_log, dt, conv, tails.clone(), states.clone(), slots, gamma, hv, hk)
     y = gdn.decode_fused(*args()).float()
-    got = _terms(gdn.decode_fused(*args(), terms=gemm.empty_terms(b, vd, "cuda")), b, vd)
-    assert ((got - y).abs() <= y.view(b, hv, 128).abs().amax(-1).repeat_interleave(128, 1) * 2.0 ** -17).all()
+    got = _terms(gdn.decode_fused(*args(), terms=gemm.Terms(b, vd, torch.device("cuda"))), b, vd)
+    assert ((got - y).abs() <= _bound(y)).all()
 
 
 @pytest.mark.gpu
