@@ -58,12 +58,13 @@ int pick_splits(int t, int n, int k) {
 
 // bf16 activations as FP8 terms (kernels/gemm_fp8_terms.cu)
 struct QwenNativeEngine::TermsBuffer {
-  DeviceBuffer xq, sx, rest;
+  DeviceBuffer xq, sx, rest, counters;
   void reset(size_t rows, size_t width) {
     const size_t tiled = (rows + 255) / 256 * 256;
     xq.reset(tiled * width * 2);
     sx.reset(tiled * (width / 128 + 1) * 4);
     rest.reset(rows * width * 2);
+    counters.reset(size_t(kSMs) * 4);
   }
 };
 
@@ -439,8 +440,8 @@ void QwenNativeEngine::linear(const void* x, const PackedMatrix& w, void* out, i
     return;
   }
   if (const int tok = terms_tile(T, w)) {
-    rc(b200_split_terms(x, T, w.k, tok, s.act_terms.xq.get(), s.act_terms.sx.as<float>(), s.act_terms.rest.get(), stream_),
-       "split_terms");
+    rc(b200_split_terms(x, T, w.k, tok, s.act_terms.xq.get(), s.act_terms.sx.as<float>(), s.act_terms.rest.get(),
+                        s.act_terms.counters.as<int>(), stream_), "split_terms");
     linear_terms(s.act_terms, w, out, T);
     return;
   }
@@ -455,14 +456,14 @@ void QwenNativeEngine::linear(const void* x, const PackedMatrix& w, void* out, i
 int QwenNativeEngine::terms_tile(int T, const PackedMatrix& w) {
   int tok = 0, counters = 0;
   long long floats = 0;
-  if (w.wfmt != 1 || w.k % 128 || T > kTermsMaxT || b200_fp8_terms_plan(T, w.n, w.k, &tok, &floats, &counters)) return 0;
-  return size_t(floats) <= s_->splitk_floats && counters <= (1 << 16) ? tok : 0;
+  if (w.wfmt != 1 || w.k % 128 || T > kTermsMaxT || b200_fp8_terms_plan(T, &tok, &floats, &counters)) return 0;
+  return size_t(floats) <= s_->splitk_floats && counters <= kSMs ? tok : 0;
 }
 
 void QwenNativeEngine::linear_terms(const TermsBuffer& x, const PackedMatrix& w, void* out, int T) {
   Scratch& s = *s_;
   rc(b200_gemm_fp8_terms(w.weight.get(), w.scales.as<float>(), x.xq.get(), x.sx.as<float>(), x.rest.get(), out, nullptr, T, w.n, w.k,
-                         s.splitk_ws.as<float>(), s.counters.as<int>(), s.status.as<int>(), stream_), "gemm_fp8_terms");
+                         s.splitk_ws.as<float>(), x.counters.as<int>(), s.status.as<int>(), stream_), "gemm_fp8_terms");
 }
 
 // ------------------------------------------------------------------------------------------------ prefill
@@ -601,7 +602,8 @@ void QwenNativeEngine::forward_decode(const std::vector<int>& slots, const std::
     uint8_t* vc = v_cache_.as<uint8_t>() + kv_layer_stride_ * L.cache_index * 2;
     if (fused) {
       rc(b200_rmsnorm_terms(s.h.get(), delta, L.in_ln.get(), L.linear ? s.x.get() : nullptr, B, H, eps, 1, tok,
-                            s.norm_terms.xq.get(), s.norm_terms.sx.as<float>(), s.norm_terms.rest.get(), stream_), "rmsnorm_terms");
+                            s.norm_terms.xq.get(), s.norm_terms.sx.as<float>(), s.norm_terms.rest.get(),
+                            s.norm_terms.counters.as<int>(), stream_), "rmsnorm_terms");
       linear_terms(s.norm_terms, L.proj, s.proj.get(), B);
     } else {
       rc(b200_rmsnorm(s.h.get(), delta, nullptr, 0, L.in_ln.get(), s.x.get(), B, H, eps, 1, delta ? 1 : 0, stream_), "rmsnorm");
@@ -613,8 +615,8 @@ void QwenNativeEngine::forward_decode(const std::vector<int>& slots, const std::
         rc(b200_gdn_decode_fused(s.proj.get(), ldp, s.x.get(), H, L.ab.weight.get(), L.a_log.as<float>(),
                                  L.dt_bias.as<float>(), L.conv_w.get(), kw, tails, (long long)tail_slot_stride_, states,
                                  (long long)state_slot_stride_, s.slot_ids.as<int>(), L.gdn_norm.get(), nullptr, B, hv_,
-                                 hk_, eps, s.act_terms.xq.get(), s.act_terms.sx.as<float>(), s.act_terms.rest.get(), tok,
-                                 stream_), "gdn_decode_fused");
+                                 hk_, eps, s.act_terms.xq.get(), s.act_terms.sx.as<float>(), s.act_terms.rest.get(),
+                                 s.act_terms.counters.as<int>(), tok, stream_), "gdn_decode_fused");
       } else {
         linear(s.x.get(), L.ab, s.ab.get(), B);
         rc(b200_gdn_gates(s.ab.get(), 2 * hv_, 0, hv_, L.a_log.as<float>(), L.dt_bias.as<float>(), s.g.as<float>(),
@@ -641,14 +643,15 @@ void QwenNativeEngine::forward_decode(const std::vector<int>& slots, const std::
     if (fused) {
       if (!L.linear)
         rc(b200_split_terms(mix_out, B, L.out.k, tok, s.act_terms.xq.get(), s.act_terms.sx.as<float>(), s.act_terms.rest.get(),
-                            stream_), "split_terms");
+                            s.act_terms.counters.as<int>(), stream_), "split_terms");
       linear_terms(s.act_terms, L.out, s.d_attn.get(), B);
       reduce_rows(s.d_attn.get(), B);
       rc(b200_rmsnorm_terms(s.h.get(), s.d_attn.get(), L.post_ln.get(), nullptr, B, H, eps, 1, tok, s.norm_terms.xq.get(),
-                            s.norm_terms.sx.as<float>(), s.norm_terms.rest.get(), stream_), "rmsnorm_terms");
+                            s.norm_terms.sx.as<float>(), s.norm_terms.rest.get(), s.norm_terms.counters.as<int>(), stream_),
+         "rmsnorm_terms");
       linear_terms(s.norm_terms, L.gate_up, s.gu.get(), B);
       rc(b200_silu_mul_terms(s.gu.get(), B, I, tok, s.act_terms.xq.get(), s.act_terms.sx.as<float>(), s.act_terms.rest.get(),
-                             stream_), "silu_mul_terms");
+                             s.act_terms.counters.as<int>(), stream_), "silu_mul_terms");
       linear_terms(s.act_terms, L.down, s.d_mlp.get(), B);
     } else {
       linear(mix_out, L.out, s.d_attn.get(), B);

@@ -17,6 +17,7 @@
 #include "fp8_terms.cuh"
 #include "ops.h"
 #include "launch.h"
+#include "tma_host.h"
 
 namespace {
 
@@ -103,6 +104,7 @@ gdn_decode_fused_kernel(GdnDecodeParams p) {
   __shared__ float s_gate[2];
   b200::pdl_grid_trigger();
   b200::pdl_grid_wait();
+  p.terms.zero_counters(blockIdx.x == 0 && blockIdx.y == 0);
   const int h = blockIdx.x, b = blockIdx.y, kh = h / R;
   const int j = threadIdx.x & 127, rg = threadIdx.x >> 7;
   const int kd = p.Hk * DK, vd = p.Hv * DV, C = 2 * kd + vd;
@@ -434,14 +436,14 @@ extern "C" {
 // proj: [B, ldp] bf16 holding q | k | v | z at offsets 0, kd, 2kd, 2kd+vd (kd = Hk*128, vd = Hv*128);
 // x: [B, hidden] bf16; w_ab: [2*Hv, hidden] bf16; conv_w: [2kd+vd, kw] bf16; tails: [slots, kw-1, 2kd+vd] bf16
 // (tail_stride elements per slot); states: fp32 [slots, Hv, 128, 128] (state_stride floats per slot);
-// out: [B, Hv*128] bf16, or null with terms_xq / terms_sx / terms_rest: the result as FP8 terms (gemm_fp8_terms.cu,
+// out: [B, Hv*128] bf16, or null with the terms_ pointers (gemm.Terms): the result as FP8 terms (gemm_fp8_terms.cu,
 // tok tokens per tile, no pair).  Hv / Hk must be 1, 2 or 4 and kw == 4.
 int b200_gdn_decode_fused(const void* proj, int ldp, const void* x, int hidden, const void* w_ab, const float* a_log,
                           const float* dt_bias, const void* conv_w, int kw, void* tails, long long tail_stride,
                           float* states, long long state_stride, const int* slot_ids, const void* gamma, void* out,
-                          int B, int Hv, int Hk, float eps, void* terms_xq, float* terms_sx, void* terms_rest, int tok,
-                          cudaStream_t stream) {
-  if ((!out && (!terms_xq || !terms_sx || !terms_rest || tok < B || tok > b200::f8t::MAX_SINGLE)) || B <= 0 || Hv <= 0 || Hk <= 0 || Hv % Hk != 0 || kw != 4 || hidden % 8 != 0) return -6;
+                          int B, int Hv, int Hk, float eps, void* terms_xq, float* terms_sx, void* terms_rest,
+                          int* terms_counters, int tok, cudaStream_t stream) {
+  if ((!out && (!terms_xq || !terms_sx || !terms_rest || !terms_counters || tok < B || tok > b200::f8t::MAX_SINGLE)) || B <= 0 || Hv <= 0 || Hk <= 0 || Hv % Hk != 0 || kw != 4 || hidden % 8 != 0) return -6;
   GdnDecodeParams p;
   p.proj = reinterpret_cast<const __nv_bfloat16*>(proj);
   p.ldp = ldp;
@@ -465,6 +467,8 @@ int b200_gdn_decode_fused(const void* proj, int ldp, const void* x, int hidden, 
   p.terms.xq = out ? nullptr : reinterpret_cast<uint8_t*>(terms_xq);
   p.terms.sx = terms_sx;
   p.terms.rest = reinterpret_cast<__nv_bfloat16*>(terms_rest);
+  p.terms.counters = terms_counters;
+  p.terms.n_counters = out ? 0 : b200::sm_count();
   p.terms.tok = p.terms.cap = tok;
   p.terms.kb = Hv;
   switch (Hv / Hk) {

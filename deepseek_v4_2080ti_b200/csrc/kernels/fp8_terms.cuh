@@ -26,7 +26,7 @@ struct Params {
   __nv_bfloat16* out;               // [T, N]
   const __nv_bfloat16* residual;
   float* partial;                   // [workers][2][CTAs][tokens of a CTA's tile x its features]
-  int* counters;                    // [tiles x CTAs], zero, left zero
+  int* counters;                    // [workers x CTAs], zero, left zero; a cut tile uses those of its first contributor
   int* status;
   int vec;                          // rows of `out` (and `residual`) are whole, aligned 16-byte groups
   // first unit of a worker
@@ -42,7 +42,12 @@ struct TermsOut {
   uint8_t* xq;
   float* sx;
   __nv_bfloat16* rest;                // [T, K]; written only in blocks that have values outside their terms
-  int tok, cap, kb;
+  int* counters;                      // [n_counters], zeroed by the kernel that makes the terms for the products that take them
+  int tok, cap, kb, n_counters;
+  __device__ __forceinline__ void zero_counters(bool first_block) const {
+    if (first_block)
+      for (int i = threadIdx.x; i < n_counters; i += blockDim.x) counters[i] = 0;
+  }
   // first byte of token t's hi row in block c; its mid row is `cap` rows further
   __device__ __forceinline__ uint8_t* hi_row(int t, int c, int& row) const {
     const int n = t / tok, tt = t - n * tok, r = tt / cap;

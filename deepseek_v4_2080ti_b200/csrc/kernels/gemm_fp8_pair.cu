@@ -302,7 +302,7 @@ gemm_fp8_pair_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_const
         }
         epi_sync();
         if (threadIdx.x == 0) {
-          int* cnt = p.counters + tile * 2 + rank;
+          int* cnt = p.counters + i0 * 2 + rank;
           const int prev = atomicAdd(cnt, 1);
           *fix_last = prev == i1 - i0;
           if (prev == i1 - i0) *cnt = 0;

@@ -366,7 +366,7 @@ gemm_fp8_terms_kernel(Params p) {
         }
         epi_sync();
         if (threadIdx.x == 0) {
-          int* cnt = p.counters + tile;
+          int* cnt = p.counters + i0;
           const int prev = atomicAdd(cnt, 1);
           *fix_last = prev == i1 - i0;
           if (prev == i1 - i0) *cnt = 0;
@@ -465,6 +465,7 @@ struct Eight {
 __global__ void __launch_bounds__(256) split_terms_kernel(const __nv_bfloat16* __restrict__ x, int K, TermsOut o) {
   pdl_launch_dependents();
   pdl_wait();
+  o.zero_counters(blockIdx.x == 0 && blockIdx.y == 0);
   const int i = (blockIdx.x * 256 + threadIdx.x) * 8, t = blockIdx.y;
   Eight e = {};
   if (i < K) e.load(x + (size_t)t * K + i);
@@ -475,6 +476,7 @@ __global__ void __launch_bounds__(256) split_terms_kernel(const __nv_bfloat16* _
 __global__ void __launch_bounds__(256) silu_mul_terms_kernel(const __nv_bfloat16* __restrict__ gu, int I, TermsOut o) {
   pdl_launch_dependents();
   pdl_wait();
+  o.zero_counters(blockIdx.x == 0 && blockIdx.y == 0);
   const int i = (blockIdx.x * 256 + threadIdx.x) * 8, t = blockIdx.y;
   Eight g = {}, u = {};
   if (i < I) {
@@ -502,6 +504,7 @@ __global__ void __launch_bounds__(1024) rmsnorm_terms_kernel(__nv_bfloat16* __re
     if (i < cols) g[j].load(gamma + i);
   }
   pdl_wait();
+  o.zero_counters(blockIdx.x == 0);
   const int t = blockIdx.x;
   Eight e[V];
   float ss = 0.f;
@@ -567,49 +570,51 @@ using namespace b200;
 
 extern "C" {
 
-// Tokens per tile, floats of partial sums and counters that b200_gemm_fp8_terms needs for a T-token product.
-int b200_fp8_terms_plan(int T, int N, int K, int* tok, long long* partial_floats, int* counters) {
-  if (T <= 0 || N <= 0 || K <= 0 || (K % 128) != 0) return -ERR_BAD_ARG;
+// Tokens per tile of T-token terms, the counters that go with them, and the floats of partial sums of a product that takes them.
+int b200_fp8_terms_plan(int T, int* tok, long long* partial_floats, int* counters) {
+  if (T <= 0) return -ERR_BAD_ARG;
   const int tk = f8t::tile_tokens(T), cg = tk == f8t::PAIR_TOK ? 2 : 1;
-  const int m_tiles = (N + 127) / 128, n_tiles = (T + tk - 1) / tk;
   *tok = tk;
   *partial_floats = (long long)(sm_count() / cg) * 2 * tk * 128 * cg;
-  *counters = (m_tiles + cg - 1) / cg * cg * n_tiles;
+  *counters = sm_count();
   return 0;
 }
 
-static bool terms_out(f8t::TermsOut* o, int T, int K, int tok, void* xq, float* sx, void* rest) {
-  if (!xq || !sx || !rest || T <= 0 || T > 65535 || K <= 0 || (K % 128) != 0 || tok != f8t::tile_tokens(T)) return false;
+static bool terms_out(f8t::TermsOut* o, int T, int K, int tok, void* xq, float* sx, void* rest, int* counters) {
+  if (!xq || !sx || !rest || !counters || T <= 0 || T > 65535 || K <= 0 || (K % 128) != 0 || tok != f8t::tile_tokens(T)) return false;
   o->xq = reinterpret_cast<uint8_t*>(xq);
   o->sx = sx;
   o->rest = reinterpret_cast<__nv_bfloat16*>(rest);
+  o->counters = counters;
+  o->n_counters = sm_count();
   o->tok = tok;
   o->cap = tok == f8t::PAIR_TOK ? tok / 2 : tok;
   o->kb = K / 128;
   return true;
 }
 
-// x [T, K] bf16 -> xq: ceil(T / tok) * (K / 128) blocks of 256 tok bytes, sx: as many blocks of tok floats, rest: [T, K] bf16.
-int b200_split_terms(const void* x_bf16, int T, int K, int tok, void* xq, float* sx, void* rest, cudaStream_t stream) {
+// x [T, K] bf16 -> xq: ceil(T / tok) * (K / 128) blocks of 256 tok bytes, sx: as many blocks of tok floats, rest: [T, K] bf16,
+// counters: as many as b200_fp8_terms_plan says (zeroed).
+int b200_split_terms(const void* x_bf16, int T, int K, int tok, void* xq, float* sx, void* rest, int* counters, cudaStream_t stream) {
   f8t::TermsOut o;
-  if (!terms_out(&o, T, K, tok, xq, sx, rest)) return -ERR_BAD_ARG;
+  if (!terms_out(&o, T, K, tok, xq, sx, rest, counters)) return -ERR_BAD_ARG;
   return (int)launch_pdl(f8t::split_terms_kernel, dim3((K / 8 + 255) / 256, T), dim3(256), 0, stream,
                          reinterpret_cast<const __nv_bfloat16*>(x_bf16), K, o);
 }
 
 // gu [T, 2 I] (gate | up) -> terms of bf16(silu(gate) up).
-int b200_silu_mul_terms(const void* gu, int T, int I, int tok, void* xq, float* sx, void* rest, cudaStream_t stream) {
+int b200_silu_mul_terms(const void* gu, int T, int I, int tok, void* xq, float* sx, void* rest, int* counters, cudaStream_t stream) {
   f8t::TermsOut o;
-  if (!terms_out(&o, T, I, tok, xq, sx, rest)) return -ERR_BAD_ARG;
+  if (!terms_out(&o, T, I, tok, xq, sx, rest, counters)) return -ERR_BAD_ARG;
   return (int)launch_pdl(f8t::silu_mul_terms_kernel, dim3((I / 8 + 255) / 256, T), dim3(256), 0, stream,
                          reinterpret_cast<const __nv_bfloat16*>(gu), I, o);
 }
 
 // x [T, cols] (+= delta, written back when delta is given) -> out = rmsnorm(x) gamma (bf16, optional) and its terms.
 int b200_rmsnorm_terms(void* x, const void* delta, const void* gamma, void* out, int T, int cols, float eps, int unit_offset, int tok,
-                       void* xq, float* sx, void* rest, cudaStream_t stream) {
+                       void* xq, float* sx, void* rest, int* counters, cudaStream_t stream) {
   f8t::TermsOut o;
-  if (cols > 4 * 8192 || !terms_out(&o, T, cols, tok, xq, sx, rest)) return -ERR_BAD_ARG;
+  if (cols > 4 * 8192 || !terms_out(&o, T, cols, tok, xq, sx, rest, counters)) return -ERR_BAD_ARG;
   auto* xp = reinterpret_cast<__nv_bfloat16*>(x);
   auto* dp = reinterpret_cast<const __nv_bfloat16*>(delta);
   auto* gp = reinterpret_cast<const __nv_bfloat16*>(gamma);
@@ -625,10 +630,8 @@ int b200_rmsnorm_terms(void* x, const void* delta, const void* gamma, void* out,
 // Y = X W^T (+ residual) from the terms of X.  W: packed FP8 tiles (b200_gemm_wdec, wfmt 1), scales [ceil(N/128), K/128].
 int b200_gemm_fp8_terms(const void* W, const float* scales, const void* xq, const float* sx, const void* rest, void* out_bf16,
                         const void* residual, int T, int N, int K, float* partial, int* counters, int* status, cudaStream_t stream) {
-  int tok = 0, n_cnt = 0;
-  long long n_part = 0;
-  if (!W || !scales || !xq || !sx || !rest || !out_bf16 || !partial || !counters || b200_fp8_terms_plan(T, N, K, &tok, &n_part, &n_cnt)) return -ERR_BAD_ARG;
-  const int cg = tok == f8t::PAIR_TOK ? 2 : 1;
+  if (!W || !scales || !xq || !sx || !rest || !out_bf16 || !partial || !counters || T <= 0 || N <= 0 || K <= 0 || K % 128) return -ERR_BAD_ARG;
+  const int tok = f8t::tile_tokens(T), cg = tok == f8t::PAIR_TOK ? 2 : 1;
   f8t::Params p;
   memset(&p, 0, sizeof(p));
   p.T = T; p.N = N; p.kb = K / 128;

@@ -24,11 +24,11 @@ int b200_splitk_reduce(const float* part, int splits, long long n, const void* r
                        void* out_bf16, cudaStream_t stream);
 
 // ---- FP8 block-128 weights times activations as pairs of FP8 terms (gemm_fp8_terms.cu, gemm_fp8_pair.cu)
-int b200_fp8_terms_plan(int T, int N, int K, int* tok, long long* partial_floats, int* counters);
-int b200_split_terms(const void* x_bf16, int T, int K, int tok, void* xq, float* sx, void* rest, cudaStream_t stream);
-int b200_silu_mul_terms(const void* gu, int T, int I, int tok, void* xq, float* sx, void* rest, cudaStream_t stream);
+int b200_fp8_terms_plan(int T, int* tok, long long* partial_floats, int* counters);
+int b200_split_terms(const void* x_bf16, int T, int K, int tok, void* xq, float* sx, void* rest, int* counters, cudaStream_t stream);
+int b200_silu_mul_terms(const void* gu, int T, int I, int tok, void* xq, float* sx, void* rest, int* counters, cudaStream_t stream);
 int b200_rmsnorm_terms(void* x, const void* delta, const void* gamma, void* out, int T, int cols, float eps, int unit_offset,
-                       int tok, void* xq, float* sx, void* rest, cudaStream_t stream);
+                       int tok, void* xq, float* sx, void* rest, int* counters, cudaStream_t stream);
 int b200_gemm_fp8_terms(const void* W, const float* scales, const void* xq, const float* sx, const void* rest, void* out_bf16,
                         const void* residual, int T, int N, int K, float* partial, int* counters, int* status, cudaStream_t stream);
 
@@ -45,8 +45,8 @@ int b200_gemm_w8a8s(const void* W, const float* scales, const void* xq, const fl
 int b200_gdn_decode_fused(const void* proj, int ldp, const void* x, int hidden, const void* w_ab, const float* a_log,
                           const float* dt_bias, const void* conv_w, int kw, void* tails, long long tail_stride,
                           float* states, long long state_stride, const int* slot_ids, const void* gamma, void* out,
-                          int B, int Hv, int Hk, float eps, void* terms_xq, float* terms_sx, void* terms_rest, int tok,
-                          cudaStream_t stream);
+                          int B, int Hv, int Hk, float eps, void* terms_xq, float* terms_sx, void* terms_rest,
+                          int* terms_counters, int tok, cudaStream_t stream);
 int b200_rmsnorm_split(void* x, const void* delta, const void* gamma, void* out, void* xq, float* inv_c, int T,
                        int cols, float eps, int unit_offset, int terms, cudaStream_t stream);
 int b200_silu_mul_split(const void* gu, void* xq, float* inv_c, int T, int inter, int terms, cudaStream_t stream);

@@ -72,7 +72,7 @@ def rmsnorm_terms(resid: torch.Tensor, delta: torch.Tensor | None, gamma: torch.
     out = torch.empty_like(resid) if want_bf16 else None
     xt = gemm.Terms(rows, cols, resid.device)
     rc = _lib.lib().b200_rmsnorm_terms(_lib.ptr(resid), _lib.ptr(delta), _lib.ptr(gamma), _lib.ptr(out), rows, cols, _f(eps),
-                                       int(unit_offset), xt.tok, *xt.ptrs, _lib.stream())
+                                       int(unit_offset), xt.tok, *xt.ptrs, xt.counters_ptr, _lib.stream())
     _lib.check(rc, "rmsnorm_terms")
     return out, xt
 
@@ -82,7 +82,7 @@ def silu_mul_terms(gu: torch.Tensor):
     from . import gemm
     assert gu.is_contiguous()
     xt = gemm.Terms(gu.shape[0], gu.shape[1] // 2, gu.device)
-    rc = _lib.lib().b200_silu_mul_terms(_lib.ptr(gu), xt.t, xt.k, xt.tok, *xt.ptrs, _lib.stream())
+    rc = _lib.lib().b200_silu_mul_terms(_lib.ptr(gu), xt.t, xt.k, xt.tok, *xt.ptrs, xt.counters_ptr, _lib.stream())
     _lib.check(rc, "silu_mul_terms")
     return xt
 

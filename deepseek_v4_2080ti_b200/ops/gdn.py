@@ -62,12 +62,12 @@ def decode_fused(proj, x, w_ab, a_log, dt_bias, conv_w, tails, states, slot_ids,
     b = proj.shape[0]
     _lib.check_indices(slot_ids, 0, states.shape[0], 4)
     out = torch.empty(b, hv * 128, dtype=torch.bfloat16, device=proj.device) if terms is None else None
-    xq, sx, rest = terms.ptrs if terms is not None else (None, None, None)
+    xq, sx, rest, counters = (*terms.ptrs, terms.counters_ptr) if terms is not None else (None,) * 4
     rc = _lib.lib().b200_gdn_decode_fused(
         _lib.ptr(proj), proj.stride(0), _lib.ptr(x), x.shape[1], _lib.ptr(w_ab), _lib.ptr(a_log), _lib.ptr(dt_bias),
         _lib.ptr(conv_w), conv_w.shape[1], _lib.ptr(tails), _ll(tails.stride(0)), _lib.ptr(states),
         _ll(states.stride(0)), _lib.ptr(slot_ids), _lib.ptr(gamma), _lib.ptr(out), b, hv, hk, ctypes.c_float(eps),
-        xq, sx, rest, terms.tok if terms is not None else 0, _lib.stream())
+        xq, sx, rest, counters, terms.tok if terms is not None else 0, _lib.stream())
     _lib.check(rc, "gdn_decode_fused")
     return out if terms is None else terms
 

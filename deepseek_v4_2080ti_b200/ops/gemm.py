@@ -371,15 +371,22 @@ def linear_stream(x: torch.Tensor, w: PackedLinear, residual: torch.Tensor | Non
 class Terms:
     """bf16 activations [t, k] as two FP8 terms per value, in the order ``linear_terms`` streams them
     (csrc/kernels/gemm_fp8_terms.cu): ``xq`` in blocks of 256 x ``tok`` bytes per (token tile, 128 inputs), ``sx`` their scales,
-    ``rest`` the values that a block's terms leave out; one allocation."""
+    ``rest`` the values that a block's terms leave out, and the tile counters of the products that take them, which the kernel
+    that makes the terms clears; one allocation.  Products of the same terms share the counters: they run one after the other,
+    on the stream of that kernel."""
 
     def __init__(self, t: int, k: int, device):
         self.t, self.k, self.device = t, k, device
-        self.tok = tok = _terms_plan(t, 128, k)[0]
+        tok, part, counters = ctypes.c_int(), ctypes.c_longlong(), ctypes.c_int()
+        _lib.check(_lib.lib().b200_fp8_terms_plan(t, ctypes.byref(tok), ctypes.byref(part), ctypes.byref(counters)), "fp8_terms_plan", 0)
+        tok = self.tok = tok.value
+        self.partial_floats = part.value
         self._blocks = blocks = (t + tok - 1) // tok * (k // 128)
-        self.buf = torch.empty(blocks * tok * 260 + t * k * 2, dtype=torch.uint8, device=device)
+        at = (0, blocks * tok * 256, blocks * tok * 260, blocks * tok * 260 + t * k * 2)
+        self.buf = torch.empty(at[3] + counters.value * 4, dtype=torch.uint8, device=device)
         base = self.buf.data_ptr()
-        self.ptrs = tuple(ctypes.c_void_p(base + o) for o in (0, blocks * tok * 256, blocks * tok * 260))      # xq, sx, rest
+        self.ptrs = tuple(ctypes.c_void_p(base + o) for o in at[:3])       # xq, sx, rest
+        self.counters_ptr = ctypes.c_void_p(base + at[3])
 
     @property
     def xq(self) -> torch.Tensor:
@@ -394,43 +401,36 @@ class Terms:
     @property
     def rest(self) -> torch.Tensor:
         """bf16 [t, k], defined in the blocks whose scale is negative"""
-        return self.buf[self._blocks * self.tok * 260:].view(torch.bfloat16).view(self.t, self.k)
-
-
-def _terms_plan(t: int, n: int, k: int) -> tuple[int, int, int]:
-    """(tokens per tile, floats of partial sums, tile counters) of a ``linear_terms`` product."""
-    tok, part, cnt = ctypes.c_int(), ctypes.c_longlong(), ctypes.c_int()
-    _lib.check(_lib.lib().b200_fp8_terms_plan(t, n, k, ctypes.byref(tok), ctypes.byref(part), ctypes.byref(cnt)), "fp8_terms_plan", 0)
-    return tok.value, part.value, cnt.value
+        at = self._blocks * self.tok * 260
+        return self.buf[at:at + self.t * self.k * 2].view(torch.bfloat16).view(self.t, self.k)
 
 
 def split_terms(x: torch.Tensor) -> Terms:
     """bf16 [T, K] (K % 128 == 0) as terms."""
     assert x.dtype == torch.bfloat16 and x.is_contiguous()
     xt = Terms(*x.shape, x.device)
-    rc = _lib.lib().b200_split_terms(_lib.ptr(x), xt.t, xt.k, xt.tok, *xt.ptrs, _lib.stream())
+    rc = _lib.lib().b200_split_terms(_lib.ptr(x), xt.t, xt.k, xt.tok, *xt.ptrs, xt.counters_ptr, _lib.stream())
     _lib.check(rc, "split_terms")
     return xt
 
 
 def terms_fit(t: int, w: "PackedLinear") -> bool:
     """Can ``linear_terms`` take FP8 matrix ``w`` for ``t`` tokens?"""
-    tiles = ((w.n + 255) // 256 * 2) * ((t + 255) // 256)
-    return w.wfmt == WF_FP8_B128 and w.k % 128 == 0 and t <= 65535 and tiles <= MAX_TILE_COUNTERS
+    blocks = ((w.n + 255) // 256 * 2) * ((t + 255) // 256) * (w.k // 128)
+    return w.wfmt == WF_FP8_B128 and w.k % 128 == 0 and t <= 65535 and blocks < 1 << 31
 
 
 def linear_terms(xt: Terms, w: PackedLinear, residual: torch.Tensor | None = None, out: torch.Tensor | None = None) -> torch.Tensor:
-    """``x @ w^T`` (+ residual) for FP8 block-128 weights: bf16 [T, N]."""
+    """``x @ w^T`` (+ residual) for FP8 block-128 weights: bf16 [T, N].  The scratch of a product is its own, so products of
+    different terms may run beside each other on several streams."""
     assert w.wfmt == WF_FP8_B128 and xt.k == w.k
     dev = xt.device
     if out is None:
         out = torch.empty(xt.t, w.n, dtype=torch.bfloat16, device=dev)
-    _, part, cnt = _terms_plan(xt.t, w.n, w.k)
-    assert cnt <= MAX_TILE_COUNTERS
-    ws, counters = _workspace(part, dev)
+    partial = torch.empty(xt.partial_floats, dtype=torch.float32, device=dev)
     rc = _lib.lib().b200_gemm_fp8_terms(_lib.ptr(w.weight), _lib.ptr(w.scales), *xt.ptrs, _lib.ptr(out), _lib.ptr(residual),
-                                        xt.t, w.n, w.k, _lib.ptr(ws), _lib.ptr(counters),
-                                        _lib.ptr(_lib.status_word(dev)), _lib.stream())
+                                        xt.t, w.n, w.k, _lib.ptr(partial), xt.counters_ptr, _lib.ptr(_lib.status_word(dev)),
+                                        _lib.stream())
     _lib.check(rc, "gemm_fp8_terms")
     return out
 

@@ -141,6 +141,55 @@ def test_product_matches_64_bit(t, n, k):
 
 
 @pytest.mark.gpu
+@pytest.mark.parametrize("t", [7, 40, 300])
+def test_products_on_two_streams_share_no_scratch(t):
+    from deepseek_v4_2080ti_b200.ops import _lib, gemm
+    torch.manual_seed(t)
+    q, s = fp8fmt.quantize_block128(torch.randn(2560, 2560, device="cuda") * 0.05)
+    w = gemm.PackedLinear.from_fp8(q, s)
+    xs = [torch.randn(t, 2560, device="cuda").bfloat16() for _ in range(2)]
+    before = dict(gemm._workspaces)
+    want = [gemm.linear(x, w) for x in xs]
+    assert gemm._workspaces == before              # nothing kept per device, which the streams would meet in
+    streams = [torch.cuda.Stream() for _ in xs]
+    torch.cuda.synchronize()
+    got = [[], []]
+    for _ in range(20):
+        for x, st, ys in zip(xs, streams, got):
+            with torch.cuda.stream(st):
+                ys.append(gemm.linear(x, w))
+    torch.cuda.synchronize()
+    _lib.check_status()
+    assert all(torch.equal(y, z) for ys, z in zip(got, want) for y in ys)
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("t,n,k", [(1, 5120, 1280), (20, 1000, 640), (64, 201, 384), (65, 640, 2560), (300, 5120, 1024), (300, 33, 256)])
+def test_products_stay_inside_their_buffers(t, n, k):
+    from deepseek_v4_2080ti_b200.ops import _lib, gemm
+    from deepseek_v4_2080ti_b200.utils import canary
+    torch.manual_seed(t + n)
+    q, s = fp8fmt.quantize_block128(torch.randn(n, k, device="cuda") * 0.05)
+    w = gemm.PackedLinear.from_fp8(q, s)
+    x = _outliers(t, k, 16)
+    plain = gemm.split_terms(x)
+    want = gemm.linear_terms(plain, w)
+    with canary.enabled():
+        buf = lambda n, dtype, name: canary.empty(n, dtype=dtype, device="cuda", name=name)
+        xq, sx, rest = (buf(v.numel(), v.dtype, n) for v, n in ((plain.xq, "terms"), (plain.sx, "scales"), (plain.rest, "rest")))
+        partial, out = buf(plain.partial_floats, torch.float32, "partial sums"), buf(t * n, torch.bfloat16, "product")
+        counters = buf(plain.buf.numel() - plain.xq.numel() - 4 * plain.sx.numel() - 2 * plain.rest.numel() >> 2, torch.int32, "counters")
+        L, p, st = _lib.lib(), _lib.ptr, _lib.stream()
+        _lib.check(L.b200_split_terms(p(x), t, k, plain.tok, p(xq), p(sx), p(rest), p(counters), st), "split")
+        _lib.check(L.b200_gemm_fp8_terms(p(w.weight), p(w.scales), p(xq), p(sx), p(rest), p(out), None, t, n, k, p(partial), p(counters),
+                                         p(_lib.status_word(x.device)), st), "product")
+        torch.cuda.synchronize()
+        _lib.check_status()
+        assert not canary.verify_all() and not counters.any()
+    assert torch.equal(out.view(t, n), want)
+
+
+@pytest.mark.gpu
 @pytest.mark.parametrize("t", [5, 40, 80])
 def test_infinities_and_nans_stay_in_their_row(t):
     from deepseek_v4_2080ti_b200.ops import gemm
