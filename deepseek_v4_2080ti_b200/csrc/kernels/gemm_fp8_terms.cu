@@ -560,6 +560,20 @@ static int launch(const Params& p, cudaStream_t stream) {
   return (int)launch_pdl(gemm_fp8_terms_kernel<TOK>, dim3(p.workers), dim3(THREADS), L::TOTAL, stream, p);
 }
 
+// CTAs (pairs) that share `tiles` tiles of `kb` blocks.  Enough tiles: all of them, in equal runs.  Where every tile is cut more
+// than once, each contributor costs the last one a read of its partial sums, about as long as two blocks of one CTA or four of a
+// pair, so a tile takes some sqrt(kb / 2) (kb / 4) contributors at most; and a whole number of them, so that none works on two cut
+// tiles.  us with its split, against all SMs: 576 x 7168 11 for 20 at 1 token, 17 for 37 at 64, 33 for 80 on pairs at 65;
+// 2048 x 5120 10 for 14, 16 for 22, 29 for 46; 5120 x 4096 10.5 for 12.8, 16 for 20, 28 for 37.
+static int workers(int tiles, int kb, int cg) {
+  const int all = sm_count() / cg;
+  if (2 * tiles > all) return all < tiles * kb ? all : tiles * kb;
+  int most = 1;
+  while ((most + 1) * (most + 1) * 2 * cg <= kb) ++most;
+  const int each = all / tiles < most + 1 ? all / tiles : most + 1;
+  return tiles * (each < kb ? each : kb);
+}
+
 // Tokens of a tile for T tokens.
 static int tile_tokens(int T) { return T <= 16 ? 16 : T <= 32 ? 32 : T <= MAX_SINGLE ? 64 : PAIR_TOK; }
 
@@ -640,7 +654,7 @@ int b200_gemm_fp8_terms(const void* W, const float* scales, const void* xq, cons
   const long long units = (long long)((p.m_tiles + cg - 1) / cg) * p.n_tiles * p.kb;
   if (units > 0x7fffffff) return -ERR_BAD_ARG;
   p.units = (int)units;
-  p.workers = sm_count() / cg < p.units ? sm_count() / cg : p.units;
+  p.workers = f8t::workers(p.units / p.kb, p.kb, cg);
   p.w = reinterpret_cast<const uint8_t*>(W);
   p.scales = scales;
   p.xq = reinterpret_cast<const uint8_t*>(xq);

@@ -5,10 +5,12 @@ import torch
 from deepseek_v4_2080ti_b200.formats import fp8 as fp8fmt
 
 # (tokens, features, inputs): both sides of every tile width (16, 32, 64 tokens; 256 on pairs), ragged feature counts, an odd
-# number of weight tiles, one K block, runs that cut tiles several times, more runs than one per tile
+# number of weight tiles, one K block, runs that cut tiles several times, more runs than one per tile, narrow matrices whose tiles
+# are shared by a few contributors each (one CTA and pairs, one and several token tiles), and ones with a CTA per tile
 SHAPES = [(1, 128, 128), (1, 5120, 4096), (16, 384, 512), (17, 1000, 1280), (32, 1536, 4096), (33, 201, 640), (64, 12288, 512),
           (65, 128, 128), (100, 384, 1024), (128, 200, 384), (129, 640, 2560), (256, 1024, 4096), (257, 5120, 1024),
-          (300, 33, 256), (700, 3072, 1152)]
+          (300, 33, 256), (700, 3072, 1152), (2, 576, 7168), (40, 576, 7168), (65, 576, 7168), (300, 576, 7168), (8, 2048, 5120),
+          (129, 2048, 5120), (500, 2048, 5120), (64, 5120, 4096), (200, 5120, 4096), (1, 128, 6144), (10, 18944, 256), (70, 18944, 384)]
 
 
 def _terms(xt, t, k):
