@@ -54,6 +54,18 @@ int pick_splits(int t, int n, int k) {
   return best;
 }
 
+// Whether splitting T bf16 rows into terms is the fastest way to an [n, k] FP8 product (rule and figures: terms_pay in ops/gemm.py).
+bool terms_pay(int t, int n, int k) {
+  const int m = (n + 127) / 128, kb = k / 128;
+  if (t <= kFusedMaxT) return true;
+  if (t <= 128) return pick_splits(t, n, k) > 1 || 2 * m < kSMs;
+  const long long tokens = (t + 255) / 256, tiles = (m + 1) / 2 * tokens;
+  const int pairs = kSMs / 2;
+  const double share = 2 * tiles > pairs ? double(tiles) * kb / pairs
+                                         : double(kb) / std::min<double>(double(pairs / tiles), std::floor(std::sqrt(kb / 4)) + 1);
+  return (tiles % pairs == 0 ? 5 : 23) + share + 1.3e-6 * t * k <= 9.5 + 1.03 * kb * ((m * tokens + kSMs - 1) / kSMs);
+}
+
 }  // namespace
 
 // bf16 activations as FP8 terms (kernels/gemm_fp8_terms.cu)
@@ -439,7 +451,7 @@ void QwenNativeEngine::linear(const void* x, const PackedMatrix& w, void* out, i
                          nullptr, s.status.as<int>(), stream_), "gemm(f32)");
     return;
   }
-  if (const int tok = terms_tile(T, w)) {
+  if (const int tok = terms_pay(T, w.n, w.k) ? terms_tile(T, w) : 0) {
     rc(b200_split_terms(x, T, w.k, tok, s.act_terms.xq.get(), s.act_terms.sx.as<float>(), s.act_terms.rest.get(),
                         s.act_terms.counters.as<int>(), stream_), "split_terms");
     linear_terms(s.act_terms, w, out, T);

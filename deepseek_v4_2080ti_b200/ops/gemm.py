@@ -9,6 +9,7 @@ from __future__ import annotations
 
 import contextlib
 import ctypes
+import math
 import os
 from dataclasses import dataclass
 
@@ -420,6 +421,31 @@ def terms_fit(t: int, w: "PackedLinear") -> bool:
     return w.wfmt == WF_FP8_B128 and w.k % 128 == 0 and t <= 65535 and blocks < 1 << 31
 
 
+def terms_pay(t: int, n: int, k: int) -> bool:
+    """Is splitting ``t`` bf16 rows and ``linear_terms`` the fastest product with an [n, k] FP8 matrix?  us with the split, against
+    the kernel that is taken otherwise, in graphs of 16 products:
+
+    * up to 64 tokens: yes (5120 x 4096 10.3 for 14.4 of the decode-warp kernel at 1 token, 16 for 41 at 64; 34816 x 5120 33 for
+      62, 46 for 193; 576 x 7168 11 for 12, 17 for 37).
+    * up to 128: yes where the decode-warp kernel must split K to fill the SMs (12288 x 5120 47 for 55 at 128, 5120 x 17408 58 for
+      67), no where its 128-token tiles fill them (14336 x 5120 50 for 34, 34816 x 5120 87 for 62): half of a pair's 256 tokens is
+      padding then.
+    * above, the decode-warp kernel walks a 256-token tile of 128 features in 1.03 us per 128 inputs, wave after wave; the pairs share
+      the tiles evenly, about 1 us per 128 inputs of two, but pay 18 us for tiles that are cut, and for the split.  By that: 7168 x
+      2048 at 257 tokens 34 for 27, 5120 x 4096 at 700 50 for 41, 12288 x 5120 at 700 101 for 92 go to the decode warps, 5120 x
+      17408 (129: 59 for 131; 1901: 391 for 468), 12288 x 5120 at 333 (70 for 82) and 34816 x 5120 at 1901 (741 for 790) do not."""
+    m, kb = (n + 127) // 128, k // 128
+    if t <= TERMS_SINGLE_T:
+        return True
+    if t <= 128:
+        return pick_splits(t, n, k) > 1 or 2 * m < NUM_SMS
+    tokens = (t + 255) // 256
+    tiles, pairs = (m + 1) // 2 * tokens, NUM_SMS // 2
+    share = tiles * kb / pairs if 2 * tiles > pairs else kb / min(pairs // tiles, math.isqrt(kb // 4) + 1)
+    terms_us = (5 if tiles % pairs == 0 else 23) + share + 1.3e-6 * t * k
+    return terms_us <= 9.5 + 1.03 * kb * ((m * tokens + NUM_SMS - 1) // NUM_SMS)
+
+
 def linear_terms(xt: Terms, w: PackedLinear, residual: torch.Tensor | None = None, out: torch.Tensor | None = None) -> torch.Tensor:
     """``x @ w^T`` (+ residual) for FP8 block-128 weights: bf16 [T, N].  The scratch of a product is its own, so products of
     different terms may run beside each other on several streams."""
@@ -439,10 +465,10 @@ def linear(x: torch.Tensor, w: PackedLinear, residual: torch.Tensor | None = Non
            out: torch.Tensor | None = None, splits: int | None = None,
            out_f32: bool = False, stream: bool | None = None) -> torch.Tensor:
     """``x [T, K] bf16`` -> ``[T, N]`` bf16 (or fp32 when ``out_f32``).  FP8 weights go to the FP8 tensor pipe with the
-    activations as pairs of FP8 terms (``Terms``), or, in prefill-sized batches that the CTA-pair kernel tiles evenly, are expanded to
-    bf16 first; ``stream=False``, or a number of ``splits``, asks for the decode-warp kernel (up to 32 tokens and not
-    ``stream=False``: the weight-streaming kernel), whose split-K partials are reduced by the last-arriving CTA of each
-    output tile."""
+    activations as pairs of FP8 terms (``Terms``) where that is the fastest (``terms_pay``), are expanded to bf16 first in
+    prefill-sized batches, and take the decode-warp kernel otherwise.  ``stream=False``, or a number of ``splits``, asks for the
+    decode-warp kernel (up to 32 tokens and not ``stream=False``: the weight-streaming kernel), whose split-K partials are
+    reduced by the last-arriving CTA of each output tile."""
     assert x.dtype == torch.bfloat16 and x.is_cuda and x.dim() == 2 and x.is_contiguous()
     t, k = x.shape
     assert k == w.k, (k, w.k)
@@ -450,7 +476,7 @@ def linear(x: torch.Tensor, w: PackedLinear, residual: torch.Tensor | None = Non
     if w.wfmt == WF_FP8_B128 and not out_f32:
         if splits is not None and t <= STREAM_MAX_T and k % 128 == 0 and stream is not False:
             return linear_stream(x, w, residual, out, splits)
-        if splits is None and stream is not False and terms_fit(t, w) and not expands(t, w):
+        if splits is None and stream is not False and terms_fit(t, w) and not expands(t, w) and terms_pay(t, n, k):
             return linear_terms(split_terms(x), w, residual, out)
         if t >= PREDECODE_MIN_T and n % 128 == 0 and k % 64 == 0:
             # every weight tile would be decoded once per 256-token tile of the batch, so the matrix is expanded to bf16

@@ -88,13 +88,15 @@ def test_large_values_whose_weights_are_zero_hide_nothing(t, exponent):
     wf.view(n, -1, 128)[:, :, 5] = wf.view(n, -1, 128)[:, :, 77] = 0
     q, s = fp8fmt.quantize_block128(wf)
     x = _outliers(t, k, exponent)
-    y = gemm.linear(x, gemm.PackedLinear.from_fp8(q, s))
+    w = gemm.PackedLinear.from_fp8(q, s)
+    y, z = gemm.linear_terms(gemm.split_terms(x), w), gemm.linear(x, w)
     torch.cuda.synchronize()
     _lib.check_status()
     ref = x.double() @ fp8fmt.dequantize_block128(q, s).double().t()
     # 2^-9 of the result: its rounding to bf16 (2^-9 at most, 2^-9 / sqrt 3 in the mean) and the terms (a quarter of the values
-    # off by up to 2^-8 of the value at the quarter, a third of the mean size)
+    # off by up to 2^-8 of the value at the quarter, a third of the mean size); 2^-9 more where the decode warps round the weights
     assert ((y.double() - ref).norm() / ref.norm()).item() < 2.0 ** -9
+    assert ((z.double() - ref).norm() / ref.norm()).item() < 2.0 ** -8
 
 
 @pytest.mark.gpu
@@ -284,3 +286,37 @@ def test_expert_rows_are_combined(t, k, h):
     _lib.check(_lib.lib().b200_moe_combine(_lib.ptr(y), _lib.ptr(rows), _lib.ptr(w), _lib.ptr(base), _lib.ptr(out), t, k, h, _lib.stream()), "moe_combine")
     ref = base.double() + torch.where(rows[..., None] >= 0, w.double()[..., None] * y.double()[rows.clamp_min(0).long()], 0.0).sum(1)
     assert ((out.double() - ref).abs() <= ref.abs() * 2.0 ** -8 + 1e-5).all()
+
+
+# (tokens, features, inputs, us with the split, us of the kernel that takes its place): the two sides of the rule
+ROUTES = [(1, 576, 7168, 11.2, 11.8), (1, 5120, 4096, 10.3, 14.4), (32, 576, 7168, 12.8, 21.9), (64, 34816, 5120, 46, 193), (65, 34816, 5120, 80, 59), (100, 14336, 5120, 47, 34),
+          (128, 34816, 5120, 88, 62), (128, 12288, 5120, 47, 55), (128, 5120, 17408, 58, 67), (65, 576, 7168, 31, 32),
+          (128, 1536, 7168, 34, 48), (129, 5120, 17408, 59, 131), (257, 7168, 2048, 34, 27), (256, 5120, 4096, 31, 40),
+          (700, 5120, 4096, 50, 41), (700, 12288, 5120, 101, 92), (333, 12288, 5120, 70, 82), (1500, 2048, 5120, 58, 46),
+          (1901, 1536, 7168, 78, 59), (1901, 7168, 2048, 76, 68), (1000, 5120, 17408, 178, 268), (1901, 34816, 5120, 741, 790),
+          (1901, 4096, 4096, 81, 67), (1000, 2048, 5120, 41, 45), (1500, 7168, 2048, 66, 55)]
+
+
+@pytest.mark.parametrize("t,n,k,terms_us,other_us", ROUTES)
+def test_terms_are_chosen_where_they_are_faster(t, n, k, terms_us, other_us):
+    from deepseek_v4_2080ti_b200.ops import gemm
+    assert gemm.terms_pay(t, n, k) == (terms_us <= other_us)
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("t,n,k", [(1, 576, 7168), (2, 200, 256), (65, 14336, 256), (128, 19072, 384), (257, 7168, 2048), (513, 12288, 256),
+                                   (701, 5120, 512), (1501, 2048, 512), (2047, 1536, 640), (2049, 640, 384), (3001, 200, 256), (2048, 300, 384)])
+def test_every_route_of_linear_gives_the_same_product(t, n, k):
+    """Both sides of each line that ``linear`` draws, and the prefill-sized batches past the last, against 64 bits."""
+    from deepseek_v4_2080ti_b200.ops import _lib, gemm
+    torch.manual_seed(t + n)
+    q, s = fp8fmt.quantize_block128(torch.randn(n, k, device="cuda") * 0.05)
+    w = gemm.PackedLinear.from_fp8(q, s)
+    x, r = torch.randn(t, k, device="cuda").bfloat16(), torch.randn(t, n, device="cuda").bfloat16()
+    y, z, other = gemm.linear(x, w), gemm.linear(x, w, residual=r), gemm.linear_terms(gemm.split_terms(x), w)
+    torch.cuda.synchronize()
+    _lib.check_status()
+    ref = x.double() @ fp8fmt.dequantize_block128(q, s).double().t()
+    rel = lambda a, b: ((a.double() - b).norm() / b.norm()).item()
+    # the result rounded to bf16, and where the decode warps or the expansion take it every scaled weight too: 2^-9 at most each
+    assert rel(y, ref) < 2.0 ** -8 and rel(z, ref + r.double()) < 2.0 ** -8 and rel(other, ref) < 2.0 ** -9
