@@ -549,9 +549,8 @@ class QwenHybridRuntime(PagedSequences):
         return gemm.linear(x, w)
 
     def _expand_ahead(self, x: torch.Tensor, w: PackedLinear) -> None:
-        nxt = self._next_w.get(id(w))
-        # a sequence-parallel product expands whatever its size
-        if x.shape[0] >= gemm.PREDECODE_MIN_T and nxt is not None and (self._sp or gemm.expands(x.shape[0], nxt)):
+        if x.shape[0] >= gemm.PREDECODE_MIN_T:
+            nxt = self._next_w.get(id(w))
             fused = nxt is not None and id(nxt) in self._gate_up_ids and self._swiglu_fused(x.shape[0], nxt)
             gemm.prefetch_bf16(nxt, x.device, w, gate_up=fused)
 

@@ -303,6 +303,12 @@ def test_terms_are_chosen_where_they_are_faster(t, n, k, terms_us, other_us):
     assert gemm.terms_pay(t, n, k) == (terms_us <= other_us)
 
 
+def test_prefill_sized_batches_are_expanded_ragged_or_not():
+    from deepseek_v4_2080ti_b200.ops import gemm
+    w = gemm.PackedLinear(gemm.WF_FP8_B128, torch.empty(0), None, 5120, 4096)
+    assert [gemm.expands(t, w) for t in (64, 2047, 2048, 2049, 3001, 8191, 8192)] == [False] * 2 + [True] * 5
+
+
 @pytest.mark.gpu
 @pytest.mark.parametrize("t,n,k", [(1, 576, 7168), (2, 200, 256), (65, 14336, 256), (128, 19072, 384), (257, 7168, 2048), (513, 12288, 256),
                                    (701, 5120, 512), (1501, 2048, 512), (2047, 1536, 640), (2049, 640, 384), (3001, 200, 256), (2048, 300, 384)])
