@@ -35,6 +35,7 @@
 #include <cuda_bf16.h>
 #include <cuda_fp8.h>
 #include <string.h>
+#include <initializer_list>
 #include "../ptx/sm100.cuh"
 #include "fp8_terms.cuh"
 #include "launch.h"
@@ -445,8 +446,16 @@ gemm_fp8_terms_kernel(Params p) {
 // Row kernels that leave their result as terms.  Eight neighbouring values per thread, sixteen threads per K block.
 struct Eight {
   float v[8];
+  // HALVES: `p` is aligned to 8 bytes only
+  template <bool HALVES = false>
   __device__ __forceinline__ void load(const __nv_bfloat16* p) {
-    const uint4 u = *reinterpret_cast<const uint4*>(p);
+    uint4 u;
+    if constexpr (HALVES) {
+      const uint2 a = *reinterpret_cast<const uint2*>(p), b = *reinterpret_cast<const uint2*>(p + 4);
+      u = make_uint4(a.x, a.y, b.x, b.y);
+    } else {
+      u = *reinterpret_cast<const uint4*>(p);
+    }
     const __nv_bfloat162* h = reinterpret_cast<const __nv_bfloat162*>(&u);
 #pragma unroll
     for (int i = 0; i < 4; ++i) {
@@ -470,13 +479,14 @@ struct Eight {
   }
 };
 
+template <bool HALVES>
 __global__ void __launch_bounds__(256) split_terms_kernel(const __nv_bfloat16* __restrict__ x, int K, TermsOut o) {
   pdl_launch_dependents();
   pdl_wait();
   o.zero_counters(blockIdx.x == 0 && blockIdx.y == 0);
   const int i = (blockIdx.x * 256 + threadIdx.x) * 8, t = blockIdx.y;
   Eight e = {};
-  if (i < K) e.load(x + (size_t)t * K + i);
+  if (i < K) e.load<HALVES>(x + (size_t)t * K + i);
   put_terms(o, t, i, e.v, i < K);
 }
 
@@ -602,8 +612,14 @@ int b200_fp8_terms_plan(int T, int* tok, long long* partial_floats, int* counter
   return 0;
 }
 
+static bool aligned(std::initializer_list<const void*> ptrs, int bytes) {
+  uintptr_t all = 0;
+  for (const void* p : ptrs) all |= reinterpret_cast<uintptr_t>(p);
+  return all % bytes == 0;
+}
+
 static bool terms_out(f8t::TermsOut* o, int T, int K, int tok, void* xq, float* sx, void* rest, int* counters) {
-  if (!xq || !sx || !rest || !counters || T <= 0 || T > 65535 || K <= 0 || (K % 128) != 0 || tok != f8t::tile_tokens(T)) return false;
+  if (!xq || !sx || !rest || !counters || !aligned({xq, sx, rest}, 16) || T <= 0 || T > 65535 || K <= 0 || (K % 128) != 0 || tok != f8t::tile_tokens(T)) return false;
   o->xq = reinterpret_cast<uint8_t*>(xq);
   o->sx = sx;
   o->rest = reinterpret_cast<__nv_bfloat16*>(rest);
@@ -619,15 +635,17 @@ static bool terms_out(f8t::TermsOut* o, int T, int K, int tok, void* xq, float* 
 // counters: as many as b200_fp8_terms_plan says (zeroed).
 int b200_split_terms(const void* x_bf16, int T, int K, int tok, void* xq, float* sx, void* rest, int* counters, cudaStream_t stream) {
   f8t::TermsOut o;
-  if (!terms_out(&o, T, K, tok, xq, sx, rest, counters)) return -ERR_BAD_ARG;
-  return (int)launch_pdl(f8t::split_terms_kernel, dim3((K / 8 + 255) / 256, T), dim3(256), 0, stream,
-                         reinterpret_cast<const __nv_bfloat16*>(x_bf16), K, o);
+  // up to 32 rows need to be aligned to 8 bytes only, as they do for the weight-streaming kernel
+  const bool halves = !aligned({x_bf16}, 16);
+  if (!x_bf16 || (halves && (T > 32 || !aligned({x_bf16}, 8))) || !terms_out(&o, T, K, tok, xq, sx, rest, counters)) return -ERR_BAD_ARG;
+  return (int)launch_pdl(halves ? f8t::split_terms_kernel<true> : f8t::split_terms_kernel<false>, dim3((K / 8 + 255) / 256, T), dim3(256), 0,
+                         stream, reinterpret_cast<const __nv_bfloat16*>(x_bf16), K, o);
 }
 
 // gu [T, 2 I] (gate | up) -> terms of bf16(silu(gate) up).
 int b200_silu_mul_terms(const void* gu, int T, int I, int tok, void* xq, float* sx, void* rest, int* counters, cudaStream_t stream) {
   f8t::TermsOut o;
-  if (!terms_out(&o, T, I, tok, xq, sx, rest, counters)) return -ERR_BAD_ARG;
+  if (!gu || !aligned({gu}, 16) || !terms_out(&o, T, I, tok, xq, sx, rest, counters)) return -ERR_BAD_ARG;
   return (int)launch_pdl(f8t::silu_mul_terms_kernel, dim3((I / 8 + 255) / 256, T), dim3(256), 0, stream,
                          reinterpret_cast<const __nv_bfloat16*>(gu), I, o);
 }
@@ -636,7 +654,7 @@ int b200_silu_mul_terms(const void* gu, int T, int I, int tok, void* xq, float* 
 int b200_rmsnorm_terms(void* x, const void* delta, const void* gamma, void* out, int T, int cols, float eps, int unit_offset, int tok,
                        void* xq, float* sx, void* rest, int* counters, cudaStream_t stream) {
   f8t::TermsOut o;
-  if (cols > 4 * 8192 || !terms_out(&o, T, cols, tok, xq, sx, rest, counters)) return -ERR_BAD_ARG;
+  if (!x || !gamma || !aligned({x, delta, gamma, out}, 16) || cols > 4 * 8192 || !terms_out(&o, T, cols, tok, xq, sx, rest, counters)) return -ERR_BAD_ARG;
   auto* xp = reinterpret_cast<__nv_bfloat16*>(x);
   auto* dp = reinterpret_cast<const __nv_bfloat16*>(delta);
   auto* gp = reinterpret_cast<const __nv_bfloat16*>(gamma);
@@ -652,7 +670,9 @@ int b200_rmsnorm_terms(void* x, const void* delta, const void* gamma, void* out,
 // Y = X W^T (+ residual) from the terms of X.  W: packed FP8 tiles (b200_gemm_wdec, wfmt 1), scales [ceil(N/128), K/128].
 int b200_gemm_fp8_terms(const void* W, const float* scales, const void* xq, const float* sx, const void* rest, void* out_bf16,
                         const void* residual, int T, int N, int K, float* partial, int* counters, int* status, cudaStream_t stream) {
-  if (!W || !scales || !xq || !sx || !rest || !out_bf16 || !partial || !counters || T <= 0 || N <= 0 || K <= 0 || K % 128) return -ERR_BAD_ARG;
+  if (!W || !scales || !xq || !sx || !rest || !out_bf16 || !partial || !counters || !aligned({W, xq, sx, rest, partial}, 16) ||
+      T <= 0 || N <= 0 || K <= 0 || K % 128)
+    return -ERR_BAD_ARG;
   const int tok = f8t::tile_tokens(T), cg = tok == f8t::PAIR_TOK ? 2 : 1;
   f8t::Params p;
   memset(&p, 0, sizeof(p));

@@ -193,6 +193,40 @@ def test_products_stay_inside_their_buffers(t, n, k):
     assert torch.equal(out.view(t, n), want)
 
 
+@pytest.mark.parametrize("off", [2, 4, 8])
+def test_rows_that_no_load_fits_are_refused(off):
+    """The pointers are looked at before anything is launched: these are addresses of nothing."""
+    import ctypes
+    from deepseek_v4_2080ti_b200.ops import _lib
+    lib, v, f = _lib.lib(), ctypes.c_void_p, ctypes.c_float(1e-6)
+    good, bad = v(1 << 20), v((1 << 20) + off)
+    terms = (v(2 << 20), v(3 << 20), v(4 << 20), v(5 << 20), None)
+    assert lib.b200_split_terms(bad, 33, 256, 64, *terms) == -6
+    if off < 8:
+        assert lib.b200_split_terms(bad, 32, 256, 32, *terms) == -6
+    assert lib.b200_silu_mul_terms(bad, 4, 256, 16, *terms) == -6
+    for x, delta, gamma, out in ((bad, None, good, good), (good, bad, good, good), (good, None, bad, good), (good, None, good, bad)):
+        assert lib.b200_rmsnorm_terms(x, delta, gamma, out, 4, 256, f, 1, 16, *terms) == -6
+    for at in (0, 2, 3, 4):                        # weights, terms, their scales, what lies outside
+        args = [good, good, good, good, good]
+        args[at] = bad
+        assert lib.b200_gemm_fp8_terms(*args, good, None, 4, 256, 256, good, good, good, None) == -6
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("t", [1, 5, 32])
+def test_rows_aligned_to_eight_bytes(t):
+    from deepseek_v4_2080ti_b200.ops import _lib, gemm
+    torch.manual_seed(t)
+    q, s = fp8fmt.quantize_block128(torch.randn(384, 1280, device="cuda") * 0.05)
+    w = gemm.PackedLinear.from_fp8(q, s)
+    wide = torch.randn(40 * 1280 + 4, device="cuda").bfloat16()
+    x = wide[4:4 + t * 1280].view(t, 1280)
+    assert torch.equal(gemm.linear(x, w), gemm.linear(x.clone(), w))
+    with pytest.raises(_lib.KernelError):
+        gemm.linear(wide[4:].view(40, 1280), w)    # past 32 rows they are refused, as they were
+
+
 @pytest.mark.gpu
 @pytest.mark.parametrize("t", [5, 40, 80])
 def test_infinities_and_nans_stay_in_their_row(t):
