@@ -1,5 +1,5 @@
-"""4-bit and GGUF expert matrices in the weight-decoding GEMM (csrc/kernels/gemm_wdec_kernel.cuh): k-blocks are given back in
-pairs, so an odd number of them makes pairs that span two tiles; every token-tile width has its own number of decoded slots."""
+"""4-bit and GGUF expert matrices in the weight-decoding GEMM (csrc/kernels/gemm_wdec_kernel.cuh): every token-tile width has its
+own number of decoded slots and raw stages, and a CTA carries their phases from one tile to the next."""
 import pytest
 import torch
 
@@ -32,6 +32,61 @@ def test_fp4_experts_with_odd_k_blocks(rows, hidden, inter):
     # three roundings to bf16 on the way (2^-9 each at most, here of equal size on both sides) and one at the end
     assert ((y.double() - ref).norm() / ref.norm()).item() < 4 * 2.0 ** -9
     assert torch.equal(y, again)
+
+
+# (tokens, hidden, expert width): 24 experts, six for each token, so 2, 24, 50, 100 and 250 rows an expert - token tiles of 16, 32,
+# 64, 128 and 256.  The long side of a product is three times as many k-blocks as the deepest ring has stages (16), and the other
+# product more work items than there are SMs, so that CTAs go from tile to tile with every phase of both rings; odd counts of
+# k-blocks where the format has them.
+LONG = [(8, 3136, 448), (8, 448, 3136), (96, 3136, 448), (96, 448, 3136), (200, 3136, 448), (400, 3136, 320), (1000, 3136, 192)]
+
+
+def _through_experts(t, hidden, inter, w13, w2, values13, values2):
+    from deepseek_v4_2080ti_b200.ops import _lib, moe
+    e, k = w13.experts, 6
+    torch.manual_seed(t)
+    x = torch.randn(t, hidden, device="cuda").bfloat16()
+    idx = torch.rand(t, e, device="cuda").topk(k).indices.int().contiguous()
+    wts = torch.rand(t, k, device="cuda")
+    ys = [moe.experts_forward(x, idx, wts, w13, w2, 0) for _ in range(4)]
+    torch.cuda.synchronize()
+    _lib.check_status()
+    ref = torch.zeros(t, hidden, dtype=torch.float64, device="cuda")
+    for i in range(e):
+        at, slot = (idx == i).nonzero(as_tuple=True)
+        if at.numel() == 0:
+            continue
+        gu = (x[at].double() @ values13(i).t()).bfloat16().double()
+        act = (torch.nn.functional.silu(gu[:, :inter]) * gu[:, inter:]).bfloat16().double()
+        ref.index_add_(0, at, wts[at, slot, None].double() * (act @ values2(i).t()).bfloat16().double())
+    # three roundings to bf16 on the way (2^-9 each at most, here of equal size on both sides) and one at the end
+    assert ((ys[0].double() - ref).norm() / ref.norm()).item() < 4 * 2.0 ** -9
+    assert all(torch.equal(y, ys[0]) for y in ys[1:])
+
+
+@pytest.mark.parametrize("t,hidden,inter", LONG)
+def test_fp4_experts_over_many_stages_and_tiles(t, hidden, inter):
+    from deepseek_v4_2080ti_b200.ops import moe
+    torch.manual_seed(hidden)
+    mats = lambda n, k: [fp4fmt.quantize(torch.randn(n, k, device="cuda") * 0.1) for _ in range(24)]
+    w13, w2 = mats(2 * inter, hidden), mats(hidden, inter)
+    _through_experts(t, hidden, inter, moe.ExpertWeights.from_fp4(*map(list, zip(*w13))), moe.ExpertWeights.from_fp4(*map(list, zip(*w2))),
+                     lambda i: fp4fmt.dequantize(*w13[i]).double(), lambda i: fp4fmt.dequantize(*w2[i]).double())
+
+
+@pytest.mark.parametrize("types", [("Q4_K", "Q2_K"), ("Q2_K", "Q4_K"), ("Q5_K", "Q6_K"), ("Q8_0", "Q3_K")])
+@pytest.mark.parametrize("t,hidden,inter", [(8, 3328, 512), (96, 512, 3328), (200, 3328, 512), (400, 3328, 256)])
+def test_gguf_experts_over_many_stages_and_tiles(types, t, hidden, inter):
+    from deepseek_v4_2080ti_b200.formats import gguf as G
+    from deepseek_v4_2080ti_b200.ops import moe
+    torch.manual_seed(hidden)
+    ty = [G.GGMLType[n] for n in types]
+    raw = [[G.quantize(torch.randn(n, k, device="cuda") * 0.1, q) for _ in range(4)] for q, n, k in ((ty[0], 2 * inter, hidden), (ty[1], hidden, inter))]
+    w13, w2 = (moe.ExpertWeights.from_gguf(r * 6, q, n, k) for r, q, n, k in ((raw[0], ty[0], 2 * inter, hidden), (raw[1], ty[1], hidden, inter)))
+    # the kernel rounds decoded weights to bf16
+    value = lambda j, k: [G.dequantize(r, ty[j], k).bfloat16().double() for r in raw[j]]
+    v13, v2 = value(0, hidden), value(1, inter)
+    _through_experts(t, hidden, inter, w13, w2, lambda i: v13[i % 4], lambda i: v2[i % 4])
 
 
 def test_fp4_codes_and_scales_over_their_range():

@@ -73,6 +73,34 @@ def test_batched_decode_equals_serial():
         assert out[1:] == [step[i] for step in batched], (i, out, batched)
 
 
+@pytest.mark.parametrize("b", [33, 48, 64, 65])
+def test_wide_decode_batches_follow_narrow_ones(b):
+    """Batches past 32 rows, on both sides of the last fused one, against the same slots decoded eight at a time."""
+    from deepseek_v4_2080ti_b200.ops import _lib
+    cfg, state, rt = _build(max_slots=b)
+    _, _, few = _build(max_slots=b)
+    assert rt.fused_decode and rt.fused_rows == 64
+    torch.manual_seed(b)
+    prompts = [torch.randint(0, cfg.vocab_size, (3 + (5 * i) % 23,), device="cuda", dtype=torch.int32) for i in range(b)]
+    slots, others = [rt.allocate() for _ in prompts], [few.allocate() for _ in prompts]
+    for p, s, o in zip(prompts, slots, others):
+        rt.prefill(s, p)
+        few.prefill(o, p)
+    for _ in range(3):
+        ids = torch.randint(0, cfg.vocab_size, (b,), device="cuda", dtype=torch.int32)
+        rt.decode(slots, ids)
+        wide = rt.last_logits.double().clone()
+        narrow = torch.cat([(few.decode(others[i:i + 8], ids[i:i + 8]), few.last_logits.double().clone())[1] for i in range(0, b, 8)])
+        torch.cuda.synchronize()
+        _lib.check_status()
+        # the kernels sum in another order, so single bf16 values round the other way: 0.9 % of a row's logits at most as
+        # measured, which a wrong row, state or scale exceeds by far
+        err = (wide - narrow).norm(dim=1) / narrow.norm(dim=1)
+        assert err.max().item() < 0.03, err
+    state_err = (rt.states[slots] - few.states[others]).flatten(1).norm(dim=1) / few.states[others].flatten(1).norm(dim=1)
+    assert state_err.max().item() < 0.03, state_err
+
+
 @pytest.mark.parametrize("kv", ["fp8", "int8_per_token_head", "turboquant_k8v4"])
 def test_quantised_kv_cache_tracks_the_bf16_cache(kv):
     """Chunked prefill + graph decode with an 8-bit KV cache: logits stay close to the bf16-cache runtime's and the
