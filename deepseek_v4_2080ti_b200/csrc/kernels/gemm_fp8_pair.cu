@@ -69,6 +69,33 @@ __device__ __forceinline__ void tma_load_pair(void* smem_dst, const CUtensorMap*
 }
 __device__ __forceinline__ void epi_sync() { asm volatile("bar.sync 1, %0;" ::"n"(EPI_THREADS) : "memory"); }
 
+// Adds to a thread's partial sums ([4 features][token]) what its token has outside its terms in K blocks c0 .. c0 + len - 1.  The
+// warp calls it together; `rows`: how many of its tokens there are.  It works on memory because the sums' registers are few enough
+// as it is (in registers: up to 1 % more for products that have no such values).
+__device__ __forceinline__ void add_outside(const Params& p, float* sums, int m, int n, int c0, int len, int t0, int rows) {
+  const int lane = threadIdx.x & 31;
+#pragma unroll 1
+  for (int c = c0; c < c0 + len; ++c) {
+    const float* sx = p.sx + ((size_t)n * p.kb + c) * PAIR_TOK + t0;
+    uint32_t tokens = __ballot_sync(0xffffffffu, lane < rows && __ldcg(sx + lane) < 0.f);
+    const uint8_t* wb = p.w + ((size_t)m * p.kb + c) * W_BYTES;
+    const float sw = __ldg(p.scales + (size_t)m * p.kb + c);
+#pragma unroll 1
+    for (; tokens; tokens &= tokens - 1) {
+      const int src = __ffs(tokens) - 1;
+      for_each_outside(p.rest, p.kb, n * PAIR_TOK + t0 + src, c, [&](int k, float x) {
+        // the token's sums, four features a lane
+        float* at = sums + (src - lane) * 4 + lane * (ROWS * 4);
+        float4 v = *reinterpret_cast<float4*>(at);
+        const float2 a = e4m3x2_to_float2(wb[w_offset(4 * lane, k)] | wb[w_offset(4 * lane + 1, k)] << 8);
+        const float2 b = e4m3x2_to_float2(wb[w_offset(4 * lane + 2, k)] | wb[w_offset(4 * lane + 3, k)] << 8);
+        v.x += x * (a.x * sw); v.y += x * (a.y * sw); v.z += x * (b.x * sw); v.w += x * (b.y * sw);
+        *reinterpret_cast<float4*>(at) = v;
+      });
+    }
+  }
+}
+
 __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(PAIR_THREADS, 1)
 gemm_fp8_pair_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constant__ CUtensorMap tmX, Params p) {
   extern __shared__ uint8_t smem_raw_base[];
@@ -87,6 +114,7 @@ gemm_fp8_pair_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_const
   volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_slot + 1);
   volatile int* epi_abort = abort_flag + 1;     // written by epilogue threads only, always before a barrier
   int* fix_last = const_cast<int*>(abort_flag) + 2;
+  volatile int* last_outside = abort_flag + 3;  // the last block so far in which a token of this CTA has values outside its terms
 
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int rank = (int)ctarank();
@@ -100,6 +128,7 @@ gemm_fp8_pair_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_const
     for (int a = 0; a < A; ++a) mbar_init(&acc_free[a], 2 * EPI_WARPS);
     *abort_flag = 0;
     *epi_abort = 0;
+    *last_outside = -1;
     mbar_fence_init();
   }
   if (warp == WARP_MMA) {
@@ -221,7 +250,8 @@ gemm_fp8_pair_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_const
       f2 acc[BM / 2];
 #pragma unroll
       for (int i = 0; i < BM / 2; ++i) acc[i] = 0;
-      bool ok = true, outside = false;
+      bool ok = true;
+      const float lim = row < rows ? 0.f : -INFINITY;      // scales of tokens past the last one are undefined
       for (int c = 0; c < len; ++c) {
         const int blk = u - u0 + c, b = blk % S, a = blk % A;
         const float sw = c < RUN ? sc_run[c] : __ldg(srow + c);
@@ -241,7 +271,7 @@ gemm_fp8_pair_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_const
         };
         if (busy) {
           const float sr = sSx[b * ROWS + row], sv = fabsf(sr) * sw;
-          outside |= sr < 0.f;
+          if (sr < lim) *last_outside = blk;
           const f2 s = pack2f(sv, sv);
           const uint32_t taddr = tmem_base + (uint32_t((warp & 3) * 32) << 16) + a * 2 * BM + group * BM;
 #pragma unroll
@@ -263,30 +293,13 @@ gemm_fp8_pair_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_const
         if (lane == 0) atomicExch(p.status, ERR_WAIT_ACC);
         *abort_flag = 1;
         *epi_abort = 1;
-      } else if (__any_sync(0xffffffffu, outside && row < rows)) {
-        // values outside the terms, on the CUDA cores: as a rule there are none, and in a block that has them a few
-        for (int c = 0; c < len; ++c) {
-          const float* sx = p.sx + ((size_t)n * p.kb + c0 + c) * PAIR_TOK + rank * ROWS;
-          uint32_t tokens = __ballot_sync(0xffffffffu, row < rows && __ldcg(sx + row) < 0.f);
-          const uint8_t* wb = p.w + ((size_t)m * p.kb + c0 + c) * W_BYTES;
-          const float sw = __ldg(srow + c);
-          for (; tokens; tokens &= tokens - 1) {
-            const int src = __ffs(tokens) - 1;
-            for_each_outside(p.rest, p.kb, n * PAIR_TOK + rank * ROWS + (warp & 3) * 32 + src, c0 + c, [&](int k, float x) {
-              const float mine = lane == src ? x : 0.f;
-#pragma unroll
-              for (int i = 0; i < BM / 2; ++i) {
-                const float2 w = e4m3x2_to_float2(wb[w_offset(2 * i, k)] | wb[w_offset(2 * i + 1, k)] << 8);
-                acc[i] = fma2(pack2f(w.x * sw, w.y * sw), pack2f(mine, mine), acc[i]);
-              }
-            });
-          }
-        }
       }
       epi_sync();
       if (*epi_abort) break;
       const bool mine = busy && row < rows;
-      bool store = len == p.kb;
+      // values outside the terms are added to the partial sums, so a tile that has some goes that way even if it is whole
+      const bool outside = *last_outside >= u - u0;
+      bool store = len == p.kb && !outside;
       if (!store) {
         // ---- a cut tile: leave the partial sums; the last contributor adds them in K order
         const int i0 = p.owner(tile * p.kb), i1 = p.owner(tile * p.kb + p.kb - 1);
@@ -298,14 +311,19 @@ gemm_fp8_pair_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_const
 #pragma unroll
           for (int j = 0; j < BM / 4; ++j)
             *reinterpret_cast<float4*>(dst + j * (ROWS * 4)) = make_float4(at(acc, 4 * j), at(acc, 4 * j + 1), at(acc, 4 * j + 2), at(acc, 4 * j + 3));
-          __threadfence();
         }
+        if (outside && busy) {
+          __syncwarp();
+          add_outside(p, part(worker), m, n, c0, len, rank * ROWS + (warp & 3) * 32, rows - (warp & 3) * 32);
+        }
+        if (busy) __threadfence();
         epi_sync();
         if (threadIdx.x == 0) {
+          // (a whole tile has no counter: that of this worker counts for its last tile, if that is cut)
           int* cnt = p.counters + i0 * 2 + rank;
-          const int prev = atomicAdd(cnt, 1);
+          const int prev = len == p.kb ? 0 : atomicAdd(cnt, 1);
           *fix_last = prev == i1 - i0;
-          if (prev == i1 - i0) *cnt = 0;
+          if (len != p.kb && prev == i1 - i0) *cnt = 0;
         }
         epi_sync();
         store = *fix_last != 0;

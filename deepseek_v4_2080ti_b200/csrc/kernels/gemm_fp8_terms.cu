@@ -357,7 +357,9 @@ gemm_fp8_terms_kernel(Params p) {
       } else {
         // ---- a cut tile: leave the partial sums; the last contributor adds them in K order
         const int i0 = p.owner(tile * p.kb), i1 = p.owner(tile * p.kb + p.kb - 1);
-        auto part = [&](int i) { return p.partial + ((size_t)i * 2 + p.place(i, tile)) * (TOK * BM); };
+        // (a tile is the first of all its contributors but the first of them, and place() divides)
+        const int first_place = p.place(i0, tile);
+        auto part = [&](int i) { return p.partial + ((size_t)i * 2 + (i == i0 ? first_place : 0)) * (TOK * BM); };
         if (holds) {
           float* mine = part(worker) + w0 * BM + row;
 #pragma unroll
@@ -376,28 +378,42 @@ gemm_fp8_terms_kernel(Params p) {
         if (*fix_last) {
           __threadfence();
           constexpr int U = TOK >= 64 ? 8 : TOK / 8;   // tokens of a thread in flight; warps take every eighth
-          constexpr int B = TOK >= 64 ? 1 : 16 / U;    // contributors in flight: one after the other, each is a round trip to L2
           const int fc = tile * BM + lane * 4;
           for (int tb = warp; tb < p.T; tb += EPI_WARPS * U) {
             float4 s[U];
 #pragma unroll
             for (int j = 0; j < U; ++j) s[j] = make_float4(0.f, 0.f, 0.f, 0.f);
-#pragma unroll (B == 1 ? 2 : 1)
-            for (int i = i0; i <= i1; i += B) {
-              float4 v[B][U];
+            if constexpr (TOK < 64) {
+              // eight values of a thread in flight, from several contributors: one after the other, each is a round trip to L2
+              constexpr int B = 8 / U;
+              for (int i = i0; i <= i1; i += B) {
+                float4 v[B][U];
 #pragma unroll
-              for (int e = 0; e < B; ++e)
+                for (int e = 0; e < B; ++e) {
+                  const float* src = part(i + e) + tb * BM + lane * 4;
+#pragma unroll
+                  for (int j = 0; j < U; ++j)
+                    if (i + e <= i1 && tb + EPI_WARPS * j < p.T) v[e][j] = __ldcg(reinterpret_cast<const float4*>(src + EPI_WARPS * j * BM));
+                }
+#pragma unroll
+                for (int e = 0; e < B; ++e)
+#pragma unroll
+                  for (int j = 0; j < U; ++j)
+                    if (i + e <= i1 && tb + EPI_WARPS * j < p.T) {
+                      s[j].x += v[e][j].x; s[j].y += v[e][j].y; s[j].z += v[e][j].z; s[j].w += v[e][j].w;
+                    }
+              }
+            } else {
+#pragma unroll 2
+              for (int i = i0; i <= i1; ++i) {
+                const float* src = part(i) + lane * 4;
 #pragma unroll
                 for (int j = 0; j < U; ++j)
-                  v[e][j] = i + e <= i1 && tb + EPI_WARPS * j < p.T
-                                ? __ldcg(reinterpret_cast<const float4*>(part(i + e) + (tb + EPI_WARPS * j) * BM + lane * 4))
-                                : make_float4(0.f, 0.f, 0.f, 0.f);
-#pragma unroll
-              for (int e = 0; e < B; ++e)
-#pragma unroll
-                for (int j = 0; j < U; ++j) {
-                  s[j].x += v[e][j].x; s[j].y += v[e][j].y; s[j].z += v[e][j].z; s[j].w += v[e][j].w;
-                }
+                  if (tb + EPI_WARPS * j < p.T) {
+                    const float4 v = __ldcg(reinterpret_cast<const float4*>(src + (tb + EPI_WARPS * j) * BM));
+                    s[j].x += v.x; s[j].y += v.y; s[j].z += v.z; s[j].w += v.w;
+                  }
+              }
             }
 #pragma unroll
             for (int j = 0; j < U; ++j) {
