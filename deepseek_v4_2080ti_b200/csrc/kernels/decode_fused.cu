@@ -85,8 +85,9 @@ struct ConvStep {
 // thread, their partial dot products meet in shared memory.
 //
 // The state, 64 KB in and out per head, is asked for first and arrives while the projections, the convolution and the gates are
-// computed; a block holds one head and two blocks fit an SM.  At 32 rows of 32 heads that takes 41 to 42 us, where the bytes take 20;
-// what the rest goes on has not been measured.  (All heads of a key head in one block of 1024 threads, one block per
+// computed; a block holds one head and two blocks fit an SM, which leaves 64 registers a thread: 52 bytes of the state's 32 values
+// and the convolution's are spilled.  At 32 rows of 32 heads that takes 41 to 42 us, where the bytes take 20; what the rest goes
+// on has not been measured.  (All heads of a key head in one block of 1024 threads, one block per
 // SM, the state loaded last: 45.6.  Four columns per thread, 16 bytes per load: 46.6.  Weights fetched before the wait for the
 // previous kernel: 48.4.  One row takes 14 us in every form.)
 // Every block convolves the q and k channels of its key head itself; the first of the cluster moves their tail on when all of

@@ -312,9 +312,9 @@ int b200_moe_route(const float* logits, int ld, const float* bias, int T, int E,
   const int wpb = 4;
   const dim3 grid((T + wpb - 1) / wpb), block(wpb * 32);
 #define B200_ROUTE(J)                                                                                                 \
-  if (E <= 32 * J) {                                                                                                  \
-    return (int)b200::launch_pdl(moe_route_kernel<J>, grid, block, 0, stream, logits, ld, bias, T, E, K, score_fn, norm_topk, route_scale, idx, wts);                                                                                   \
-  }
+  if (E <= 32 * J)                                                                                                    \
+    return (int)b200::launch_pdl(moe_route_kernel<J>, grid, block, 0, stream, logits, ld, bias, T, E, K, score_fn,    \
+                                 norm_topk, route_scale, idx, wts);
   B200_ROUTE(1) B200_ROUTE(2) B200_ROUTE(4) B200_ROUTE(8) B200_ROUTE(16) B200_ROUTE(32)
 #undef B200_ROUTE
   return -6;

@@ -9,6 +9,7 @@ from __future__ import annotations
 
 import contextlib
 import ctypes
+import functools
 import math
 import os
 from dataclasses import dataclass
@@ -369,6 +370,14 @@ def linear_stream(x: torch.Tensor, w: PackedLinear, residual: torch.Tensor | Non
     return out
 
 
+@functools.lru_cache(maxsize=4096)
+def _terms_plan(t: int) -> tuple[int, int, int]:
+    """(tokens of a tile, floats of a product's partial sums, tile counters) for ``t`` tokens"""
+    tok, part, counters = ctypes.c_int(), ctypes.c_longlong(), ctypes.c_int()
+    _lib.check(_lib.lib().b200_fp8_terms_plan(t, ctypes.byref(tok), ctypes.byref(part), ctypes.byref(counters)), "fp8_terms_plan", 0)
+    return tok.value, part.value, counters.value
+
+
 class Terms:
     """bf16 activations [t, k] as two FP8 terms per value, in the order ``linear_terms`` streams them
     (csrc/kernels/gemm_fp8_terms.cu): ``xq`` in blocks of 256 x ``tok`` bytes per (token tile, 128 inputs), ``sx`` their scales,
@@ -378,13 +387,11 @@ class Terms:
 
     def __init__(self, t: int, k: int, device):
         self.t, self.k, self.device = t, k, device
-        tok, part, counters = ctypes.c_int(), ctypes.c_longlong(), ctypes.c_int()
-        _lib.check(_lib.lib().b200_fp8_terms_plan(t, ctypes.byref(tok), ctypes.byref(part), ctypes.byref(counters)), "fp8_terms_plan", 0)
-        tok = self.tok = tok.value
-        self.partial_floats = part.value
+        self.tok, self.partial_floats, counters = _terms_plan(t)
+        tok = self.tok
         self._blocks = blocks = (t + tok - 1) // tok * (k // 128)
         at = (0, blocks * tok * 256, blocks * tok * 260, blocks * tok * 260 + t * k * 2)
-        self.buf = torch.empty(at[3] + counters.value * 4, dtype=torch.uint8, device=device)
+        self.buf = torch.empty(at[3] + counters * 4, dtype=torch.uint8, device=device)
         base = self.buf.data_ptr()
         self.ptrs = tuple(ctypes.c_void_p(base + o) for o in at[:3])       # xq, sx, rest
         self.counters_ptr = ctypes.c_void_p(base + at[3])
@@ -466,15 +473,15 @@ def linear(x: torch.Tensor, w: PackedLinear, residual: torch.Tensor | None = Non
            out_f32: bool = False, stream: bool | None = None) -> torch.Tensor:
     """``x [T, K] bf16`` -> ``[T, N]`` bf16 (or fp32 when ``out_f32``).  FP8 weights go to the FP8 tensor pipe with the
     activations as pairs of FP8 terms (``Terms``) where that is the fastest (``terms_pay``), are expanded to bf16 first in
-    prefill-sized batches, and take the decode-warp kernel otherwise.  ``stream=False``, or a number of ``splits``, asks for the
-    decode-warp kernel (up to 32 tokens and not ``stream=False``: the weight-streaming kernel), whose split-K partials are
-    reduced by the last-arriving CTA of each output tile."""
+    prefill-sized batches, and take the decode-warp kernel otherwise.  ``stream=True`` asks for the weight-streaming kernel (up to
+    32 tokens), ``stream=False`` for the decode-warp kernel, a number of ``splits`` for the former where it takes that many
+    tokens, else the latter; split-K partials are reduced by the last-arriving CTA of each output tile."""
     assert x.dtype == torch.bfloat16 and x.is_cuda and x.dim() == 2 and x.is_contiguous()
     t, k = x.shape
     assert k == w.k, (k, w.k)
     n = w.n
     if w.wfmt == WF_FP8_B128 and not out_f32:
-        if splits is not None and t <= STREAM_MAX_T and k % 128 == 0 and stream is not False:
+        if (stream or (splits is not None and stream is None)) and t <= STREAM_MAX_T and k % 128 == 0:
             return linear_stream(x, w, residual, out, splits)
         if splits is None and stream is not False and terms_fit(t, w) and not expands(t, w) and terms_pay(t, n, k):
             return linear_terms(split_terms(x), w, residual, out)

@@ -123,6 +123,27 @@ def test_stream_kernel_matches_fp32(t, n, k):
     assert torch.equal(y3, y3b)
 
 
+@pytest.mark.parametrize("t", [1, 7, 32])
+def test_linear_asked_for_the_stream_kernel_takes_it(t):
+    from deepseek_v4_2080ti_b200.ops import _lib, gemm
+    torch.manual_seed(t)
+    q, s = fp8fmt.quantize_block128(torch.randn(640, 1280, device="cuda") * 0.05)
+    pl = gemm.PackedLinear.from_fp8(q, s)
+    x = torch.randn(t, 1280, device="cuda").to(torch.bfloat16)
+    calls, take = [], gemm.linear_stream
+    try:
+        gemm.linear_stream = lambda *a, **kw: (calls.append(1), take(*a, **kw))[1]
+        y, z = gemm.linear(x, pl, stream=True), gemm.linear(x, pl, splits=2)
+        gemm.linear(x, pl)
+        gemm.linear(x, pl, stream=False)
+        gemm.linear(x, pl, splits=2, stream=False)
+    finally:
+        gemm.linear_stream = take
+    torch.cuda.synchronize()
+    _lib.check_status()
+    assert len(calls) == 2 and torch.equal(y, take(x, pl)) and torch.equal(z, take(x, pl, splits=2))
+
+
 def test_activation_split_reconstructs_rows():
     from deepseek_v4_2080ti_b200.ops import gemm
     torch.manual_seed(5)
