@@ -7,11 +7,15 @@
 // 32 shared-memory reads of 16 bytes per block and thread, beside operand traffic that already fills shared memory (112 KB
 // per 1024 tensor cycles), doubled the time (978 against 670 us for 1920 x 34816 x 5120).
 //
-// Measured, us per product (12288 x 5120, 5120 x 4096, 34816 x 5120, 5120 x 17408): 128 tokens 46, 36, 88, 60; 333 tokens 67, 37,
-// 153, 82; 1901 tokens 216, 84, 616, 320.  The decode-warp kernel before: 128 tokens 121, 103, 84, 135; 333 tokens 91, 43, 182,
-// 146; 1901 tokens 256, 102, 681, 409.  The split of the activations into terms, which that kernel had no need of, is not
-// counted: 3 to 5 us at 128 tokens, 11 to 36 at 1901, once for all products of the same input.  At 128 tokens the 34816 x 5120
-// product alone is slower than before; the other three outweigh it.
+// Measured, us per product in a graph of 16 (12288 x 5120, 5120 x 4096, 34816 x 5120, 5120 x 17408): 128 tokens 43, 28, 85, 52; 333
+// tokens 64, 37, 159, 81; 1901 tokens 237, 83, 650 to 730, 340 to 355 (the larger ones go with the power limit).  The split of the
+// activations, 3 to 5 us at 128 tokens and 13 to 55 at 1901, is not counted.  The decode-warp kernel, which needs none, as it is
+// now: 128 tokens 55, 44, 62, 67; 333 tokens 82, 40, 188, 138; 1901 tokens 266, 96, 790, 468.  Where it is the faster one with the
+// split counted - half of a pair's tokens are padding up to 128 - `linear` takes it (terms_pay in ops/gemm.py).
+//
+// What bounds it: with two accumulators of 256 columns (all of tensor memory) the products of a block wait for the epilogue to have
+// read the block before last; the tensor pipe is busy for 65 % of the cycles at 1901 tokens.  The epilogue's 216 registers are all
+// in use and 52 bytes are spilled.
 //
 // Same work list and treatment of cut tiles as the one-CTA kernel; the tokens past the last one of a tile are not staged when
 // they fill a CTA, and not read back.  Roles: warps 0-7 epilogue (group of four: one weight tile of the pair), warp 8 weight

@@ -12,8 +12,8 @@
 // into the block's activation scales, and the epilogue warps add scale x block into fp32 registers, two tokens per instruction,
 // while the tensor core is on the next blocks.
 //
-// This file: up to 64 tokens, one CTA per worker, weights as the MMA's M operand; bound by the weight stream, up to 190 KB in
-// flight per SM.  More tokens: gemm_fp8_pair.cu.
+// This file: up to 64 tokens, one CTA per worker, weights as the MMA's M operand; bound by the weight stream, 160 KB of it in flight
+// per SM at 16 tokens, 144 at 32, 96 at 64.  More tokens: gemm_fp8_pair.cu.
 //
 // Work: the (tile, K block) pairs are one list, cut into equal contiguous runs, one per worker, so no wave is partly empty
 // whatever N and K are.  A tile that is cut is finished by whichever contributor arrives last, which adds the fp32 partial
@@ -23,12 +23,11 @@
 // are bounded.  The two epilogue groups of four share the work of a block by tokens (32 tokens and more) or take every other
 // block.
 //
-// Measured, us per product in a chain (weights 63, 21, 178, 89 MB: 12288 x 5120, 5120 x 4096, 34816 x 5120, 5120 x 17408;
-// a plain read of as many bytes takes 9.7, 3.7, 25.3, 13.2):
-//   1 token 17.3, 11.6, 34.5, 22.5;  32 tokens 20.0, 13.1, 39.7, 25.7;  64 tokens 23.3, 16.8, 46.8, 30.2
-//   (the 32-token figures are those of an earlier build, whose 64-token ones were 22.5, 15.3, 45.4, 28.7)
-// The kernels this one took over from: gemm_w8a8s.cu at 1 token 20.6, 12.0, 38.7, 29.8, at 32 tokens 47.6, 52.6, 45.9, 71.8;
-// the decode-warp kernel at 64 tokens 77.9, 83.1, 188, 111.
+// Measured, us per product in a graph of 16, the split not counted (weights 63, 21, 178, 89 MB: 12288 x 5120, 5120 x 4096,
+// 34816 x 5120, 5120 x 17408; a plain read of as many bytes takes 9.7, 3.7, 25.3, 13.2):
+//   1 token 14.8, 9.4, 31, 19.4;  32 tokens 16.6, 10.6, 33.9, 20.5;  64 tokens 20.8, 13.5, 42.2, 26.0
+// The kernels this one took over from, in a chain: gemm_w8a8s.cu at 1 token 20.6, 12.0, 38.7, 29.8, at 32 tokens 47.6, 52.6,
+// 45.9, 71.8; the decode-warp kernel at 64 tokens 77.9, 83.1, 188, 111 (with the converged issue it has now 38, 41, 193, 57).
 //
 // Reference behaviour covered: the FP8 block-128 projections of the Qwen path
 // (cpp_engine/backends/cuda/kernels/qwen_half_ops.cu:130-535, 988-1199).
