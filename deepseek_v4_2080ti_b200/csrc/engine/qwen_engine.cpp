@@ -57,7 +57,7 @@ int pick_splits(int t, int n, int k) {
 // Whether splitting T bf16 rows into terms is the fastest way to an [n, k] FP8 product (rule and figures: terms_pay in ops/gemm.py).
 bool terms_pay(int t, int n, int k) {
   const int m = (n + 127) / 128, kb = k / 128;
-  if (t <= kFusedMaxT) return true;
+  if (t <= kFusedMaxT || kb > 254) return true;      // the decode warps keep the scales of 254 blocks
   if (t <= 128) return pick_splits(t, n, k) > 1 || 2 * m < kSMs;
   const long long tokens = (t + 255) / 256, tiles = (m + 1) / 2 * tokens;
   const int pairs = kSMs / 2;

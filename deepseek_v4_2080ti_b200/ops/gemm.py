@@ -442,7 +442,7 @@ def terms_pay(t: int, n: int, k: int) -> bool:
       2048 at 257 tokens 34 for 27, 5120 x 4096 at 700 50 for 41, 12288 x 5120 at 700 101 for 92 go to the decode warps, 5120 x
       17408 (129: 59 for 131; 1901: 391 for 468), 12288 x 5120 at 333 (70 for 82) and 34816 x 5120 at 1901 (741 for 790) do not."""
     m, kb = (n + 127) // 128, k // 128
-    if t <= TERMS_SINGLE_T:
+    if t <= TERMS_SINGLE_T or kb > 254:            # the decode warps keep the scales of 254 blocks
         return True
     if t <= 128:
         return pick_splits(t, n, k) > 1 or 2 * m < NUM_SMS
@@ -483,9 +483,10 @@ def linear(x: torch.Tensor, w: PackedLinear, residual: torch.Tensor | None = Non
     if w.wfmt == WF_FP8_B128 and not out_f32:
         if (stream or (splits is not None and stream is None)) and t <= STREAM_MAX_T and k % 128 == 0:
             return linear_stream(x, w, residual, out, splits)
-        if splits is None and stream is not False and terms_fit(t, w) and not expands(t, w) and terms_pay(t, n, k):
+        expand = expands(t, w) and n % 128 == 0 and k % 64 == 0
+        if splits is None and stream is not False and terms_fit(t, w) and not expand and terms_pay(t, n, k):
             return linear_terms(split_terms(x), w, residual, out)
-        if t >= PREDECODE_MIN_T and n % 128 == 0 and k % 64 == 0:
+        if expand:
             # every weight tile would be decoded once per 256-token tile of the batch, so the matrix is expanded to bf16
             # once (one pass over the weights, ~3 % of the GEMM) and multiplied by the bf16 path, which has no decode
             # traffic through shared memory (1.17 / 1.38 PFLOP/s against 1.09 / 1.16 at 8192 x 17408 x 5120 and

@@ -335,6 +335,7 @@ ROUTES = [(1, 576, 7168, 11.2, 11.8), (1, 5120, 4096, 10.3, 14.4), (32, 576, 716
 def test_terms_are_chosen_where_they_are_faster(t, n, k, terms_us, other_us):
     from deepseek_v4_2080ti_b200.ops import gemm
     assert gemm.terms_pay(t, n, k) == (terms_us <= other_us)
+    assert gemm.terms_pay(t, n, 255 * 128)         # more inputs than the decode warps take
 
 
 def test_prefill_sized_batches_are_expanded_ragged_or_not():
@@ -345,7 +346,8 @@ def test_prefill_sized_batches_are_expanded_ragged_or_not():
 
 @pytest.mark.gpu
 @pytest.mark.parametrize("t,n,k", [(1, 576, 7168), (2, 200, 256), (65, 14336, 256), (128, 19072, 384), (257, 7168, 2048), (513, 12288, 256),
-                                   (701, 5120, 512), (1501, 2048, 512), (2047, 1536, 640), (2049, 640, 384), (3001, 200, 256), (2048, 300, 384)])
+                                   (701, 5120, 512), (1501, 2048, 512), (2047, 1536, 640), (2049, 640, 384), (3001, 200, 256), (2048, 300, 384),
+                                   (128, 384, 32768), (700, 128, 32640), (2100, 72, 32640)])
 def test_every_route_of_linear_gives_the_same_product(t, n, k):
     """Both sides of each line that ``linear`` draws, and the prefill-sized batches past the last, against 64 bits."""
     from deepseek_v4_2080ti_b200.ops import _lib, gemm
