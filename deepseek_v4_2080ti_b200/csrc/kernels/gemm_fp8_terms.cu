@@ -392,7 +392,8 @@ gemm_fp8_terms_kernel(Params p) {
                   const float* src = part(i + e) + tb * BM + lane * 4;
 #pragma unroll
                   for (int j = 0; j < U; ++j)
-                    if (i + e <= i1 && tb + EPI_WARPS * j < p.T) v[e][j] = __ldcg(reinterpret_cast<const float4*>(src + EPI_WARPS * j * BM));
+                    if (i + e <= i1 && tb + EPI_WARPS * j < p.T)
+                      v[e][j] = __ldcg(reinterpret_cast<const float4*>(src + EPI_WARPS * j * BM));
                 }
 #pragma unroll
                 for (int e = 0; e < B; ++e)
@@ -596,8 +597,8 @@ static int launch(const Params& p, cudaStream_t stream) {
 // CTAs (pairs) that share `tiles` tiles of `kb` blocks.  Enough tiles: all of them, in equal runs.  Where every tile is cut more
 // than once, each contributor costs the last one a read of its partial sums, about as long as two blocks of one CTA or four of a
 // pair, so a tile takes some sqrt(kb / 2) (kb / 4) contributors at most; and a whole number of them, so that none works on two cut
-// tiles.  us with its split, against all SMs: 576 x 7168 11 for 20 at 1 token, 17 for 37 at 64, 33 for 80 on pairs at 65;
-// 2048 x 5120 10 for 14, 16 for 22, 29 for 46; 5120 x 4096 10.5 for 12.8, 16 for 20, 28 for 37.
+// tiles.  us with its split, against all SMs: 576 x 7168 9.4 for 20 at 1 token, 15 for 37 at 64, 31 for 80 on pairs at 65;
+// 2048 x 5120 8.9 for 13, 15 for 23, 29 for 46; 5120 x 4096 9.6 for 12.6, 15 for 21, 28 for 37.
 static int workers(int tiles, int kb, int cg) {
   const int all = sm_count() / cg;
   if (2 * tiles > all) return all < tiles * kb ? all : tiles * kb;
@@ -634,7 +635,8 @@ static bool aligned(std::initializer_list<const void*> ptrs, int bytes) {
 }
 
 static bool terms_out(f8t::TermsOut* o, int T, int K, int tok, void* xq, float* sx, void* rest, int* counters) {
-  if (!xq || !sx || !rest || !counters || !aligned({xq, sx, rest}, 16) || T <= 0 || T > 65535 || K <= 0 || (K % 128) != 0 || tok != f8t::tile_tokens(T)) return false;
+  if (!xq || !sx || !rest || !counters || !aligned({xq, sx, rest}, 16)) return false;
+  if (T <= 0 || T > 65535 || K <= 0 || (K % 128) != 0 || tok != f8t::tile_tokens(T)) return false;
   o->xq = reinterpret_cast<uint8_t*>(xq);
   o->sx = sx;
   o->rest = reinterpret_cast<__nv_bfloat16*>(rest);
@@ -652,9 +654,10 @@ int b200_split_terms(const void* x_bf16, int T, int K, int tok, void* xq, float*
   f8t::TermsOut o;
   // up to 32 rows need to be aligned to 8 bytes only, as they do for the weight-streaming kernel
   const bool halves = !aligned({x_bf16}, 16);
-  if (!x_bf16 || (halves && (T > 32 || !aligned({x_bf16}, 8))) || !terms_out(&o, T, K, tok, xq, sx, rest, counters)) return -ERR_BAD_ARG;
-  return (int)launch_pdl(halves ? f8t::split_terms_kernel<true> : f8t::split_terms_kernel<false>, dim3((K / 8 + 255) / 256, T), dim3(256), 0,
-                         stream, reinterpret_cast<const __nv_bfloat16*>(x_bf16), K, o);
+  if (!x_bf16 || (halves && (T > 32 || !aligned({x_bf16}, 8)))) return -ERR_BAD_ARG;
+  if (!terms_out(&o, T, K, tok, xq, sx, rest, counters)) return -ERR_BAD_ARG;
+  return (int)launch_pdl(halves ? f8t::split_terms_kernel<true> : f8t::split_terms_kernel<false>, dim3((K / 8 + 255) / 256, T), dim3(256),
+                         0, stream, reinterpret_cast<const __nv_bfloat16*>(x_bf16), K, o);
 }
 
 // gu [T, 2 I] (gate | up) -> terms of bf16(silu(gate) up).
@@ -669,7 +672,8 @@ int b200_silu_mul_terms(const void* gu, int T, int I, int tok, void* xq, float* 
 int b200_rmsnorm_terms(void* x, const void* delta, const void* gamma, void* out, int T, int cols, float eps, int unit_offset, int tok,
                        void* xq, float* sx, void* rest, int* counters, cudaStream_t stream) {
   f8t::TermsOut o;
-  if (!x || !gamma || !aligned({x, delta, gamma, out}, 16) || cols > 4 * 8192 || !terms_out(&o, T, cols, tok, xq, sx, rest, counters)) return -ERR_BAD_ARG;
+  if (!x || !gamma || !aligned({x, delta, gamma, out}, 16) || cols > 4 * 8192) return -ERR_BAD_ARG;
+  if (!terms_out(&o, T, cols, tok, xq, sx, rest, counters)) return -ERR_BAD_ARG;
   auto* xp = reinterpret_cast<__nv_bfloat16*>(x);
   auto* dp = reinterpret_cast<const __nv_bfloat16*>(delta);
   auto* gp = reinterpret_cast<const __nv_bfloat16*>(gamma);

@@ -432,8 +432,8 @@ def terms_pay(t: int, n: int, k: int) -> bool:
     """Is splitting ``t`` bf16 rows and ``linear_terms`` the fastest product with an [n, k] FP8 matrix?  us with the split, against
     the kernel that is taken otherwise, in graphs of 16 products:
 
-    * up to 64 tokens: yes (5120 x 4096 10.3 for 14.4 of the decode-warp kernel at 1 token, 16 for 41 at 64; 34816 x 5120 33 for
-      62, 46 for 193; 576 x 7168 11 for 12, 17 for 37).
+    * up to 64 tokens: yes (5120 x 4096 9.6 for 14.4 of the decode-warp kernel at 1 token, 15 for 41 at 64; 34816 x 5120 33 for
+      62, 45 for 193; 576 x 7168 9.4 for 12, 15 for 37).
     * up to 128: yes where the decode-warp kernel must split K to fill the SMs (12288 x 5120 47 for 55 at 128, 5120 x 17408 58 for
       67), no where its 128-token tiles fill them (14336 x 5120 50 for 34, 34816 x 5120 87 for 62): half of a pair's 256 tokens is
       padding then.
