@@ -89,21 +89,21 @@ __device__ __forceinline__ uint32_t block_sum(uint32_t v) {
   for (int d = LANES / 2; d > 0; d >>= 1) v += __shfl_xor_sync(0xffffffffu, v, d);
   return v;
 }
-// The scale of a block of V values on each of 128 / V neighbouring lanes; the whole warp takes part.
-template <int V>
+// The scale of a block of V values on each of LANES neighbouring lanes; the whole warp takes part.  It puts the top at 2^TOP;
+// values are exact terms down to DEPTH exponents below it.
+template <int V, int LANES = 128 / V, int DEPTH = 13, int TOP = 11>
 __device__ __forceinline__ TermScale term_scale(const float (&x)[V]) {
-  constexpr int LANES = 128 / V;
   uint32_t m = 0;
 #pragma unroll
   for (int i = 0; i < V; ++i) m = max(m, bf16_magnitude(x[i]));
   m = block_max<LANES>(m);
-  // values below 2^-2 under a top exponent e, and nonzero ones, in the halves of a word
+  // values more than DEPTH below a top exponent e, and nonzero ones, in the halves of a word
   auto counts = [&](int e) {
     uint32_t n = 0;
 #pragma unroll
     for (int i = 0; i < V; ++i) {
       const uint32_t b = bf16_magnitude(x[i]);
-      n += b ? (b >> 7 < (uint32_t)(e - 13) ? 0x10001u : 1u) : 0u;
+      n += b ? (b >> 7 < (uint32_t)(e - DEPTH) ? 0x10001u : 1u) : 0u;
     }
     return block_sum<LANES>(n);
   };
@@ -129,8 +129,8 @@ __device__ __forceinline__ TermScale term_scale(const float (&x)[V]) {
     r.outside |= lo < last;
   }
   r.top = (uint32_t)(e + 1) << 7;
-  r.scale = __uint_as_float((uint32_t)(127 + 138 - e) << 23);       // x < 2^(e - 126) -> x scale < 2^12
-  r.inv = __uint_as_float((uint32_t)(127 + e - 138) << 23);
+  r.scale = __uint_as_float((uint32_t)(254 + TOP - e) << 23);       // x < 2^(e - 126) -> x scale < 2^(TOP + 1)
+  r.inv = __uint_as_float((uint32_t)(e - TOP) << 23);
   return r;
 }
 // Two values (as fp32) -> their terms, a byte each.

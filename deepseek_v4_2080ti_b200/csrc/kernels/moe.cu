@@ -5,6 +5,7 @@
 //                      GEMMs, all on the device (nothing is read back by the host);
 //   moe_gather       - token rows -> expert-sorted rows;
 //   moe_glu          - gated unit on the sorted rows: silu(gate) * up (with the DeepSeek clamp) or the one-plus form;
+//   moe_gather_terms, moe_glu_terms - the same with the result as FP8 terms for gemm_fp4_terms.cu;
 //   moe_combine      - out[t] = (shared[t]) + sum_k w[t,k] * y[row(t,k)], k ascending (deterministic).
 // Routes whose expert lives on another rank are dropped locally (expert-range sharding) or carried by the
 // dispatch kernels of csrc/comm.
@@ -15,6 +16,7 @@
 #include <stdint.h>
 #include "glu.cuh"
 #include "launch.h"
+#include "mx_terms.cuh"
 #include "ops.h"
 #include "vec8.cuh"
 
@@ -126,7 +128,7 @@ __global__ void __launch_bounds__(1024)
 moe_plan_kernel(const int* __restrict__ idx, int R, int K, int lo, int hi, int* __restrict__ offsets,
                 int* __restrict__ route_row, int* __restrict__ row_token, int4* __restrict__ work13, int* __restrict__ n13,
                 int m_tiles13, int bn13, int4* __restrict__ work2, int* __restrict__ n2, int m_tiles2, int bn2,
-                int max_work) {
+                int max_work, int rows_first) {
   __shared__ int cnt[MAX_EXPERTS], ws[32], mine[4];
   b200::pdl_grid_trigger();
   b200::pdl_grid_wait();
@@ -193,16 +195,17 @@ moe_plan_kernel(const int* __restrict__ idx, int R, int K, int lo, int hi, int* 
       }
     placed += n;
   }
-  // work tables: m-tile fastest inside a token tile so one expert's weight tiles are swept once per token tile
-  auto emit = [&](int4* work, int base, int m_tiles, int bn) {
-    const int n = m_tiles * ((c + bn - 1) / bn);
+  // work tables: m-tile fastest inside a token tile so one expert's weight tiles are swept once per token tile, or
+  // (rows_first) the token tiles that share a weight tile one after the other
+  auto emit = [&](int4* work, int base, int m_tiles, int bn, int rows_first) {
+    const int n_tiles = (c + bn - 1) / bn, n = m_tiles * n_tiles;
     for (int i = tid; i < n; i += 1024) {
-      const int nt = i / m_tiles;
-      if (base + i < max_work) work[base + i] = make_int4(e, i - nt * m_tiles, off + nt * bn, min(bn, c - nt * bn));
+      const int nt = rows_first ? i % n_tiles : i / m_tiles, mt = rows_first ? i / n_tiles : i - nt * m_tiles;
+      if (base + i < max_work) work[base + i] = make_int4(e, mt, off + nt * bn, min(bn, c - nt * bn));
     }
   };
-  emit(work13, mine[2], m_tiles13, bn13);
-  emit(work2, mine[3], m_tiles2, bn2);
+  emit(work13, mine[2], m_tiles13, bn13, rows_first & 1);
+  emit(work2, mine[3], m_tiles2, bn2, rows_first & 2);
 }
 
 // xs[row, :] = x[row_token[row], :]; one block per sorted row; H % 8 == 0.
@@ -217,6 +220,23 @@ __global__ void moe_gather_kernel(const __nv_bfloat16* __restrict__ x, const int
   for (int i = threadIdx.x; i < H / 8; i += blockDim.x) dst[i] = src[i];
 }
 
+// Gated unit of eight columns in fp32; slope 0: silu(min(g, limit)) clamp(u), the limit optional.
+template <bool FAST>
+__device__ __forceinline__ void glu8(float (&gv)[8], float (&uv)[8], const b200::GluShape& s) {
+#pragma unroll
+  for (int j = 0; j < 8; ++j) {
+    if (s.slope > 0.f) {
+      gv[j] = b200::glu<FAST>(gv[j], uv[j], s);
+      continue;
+    }
+    if (s.limit > 0.f) {
+      uv[j] = fminf(fmaxf(uv[j], -s.limit), s.limit);
+      gv[j] = fminf(gv[j], s.limit);
+    }
+    gv[j] = __fdividef(gv[j], 1.f + __expf(-gv[j])) * uv[j];
+  }
+}
+
 // rows [gate | up] of 2 I columns -> gated unit (glu.cuh); slope 0: silu(min(g, limit)) clamp(u), the limit optional.
 template <typename T>
 __global__ void moe_glu_kernel(const T* __restrict__ gu, const int* __restrict__ offsets, int EL, T* __restrict__ act, int I,
@@ -226,25 +246,48 @@ __global__ void moe_glu_kernel(const T* __restrict__ gu, const int* __restrict__
   const int row = blockIdx.x;
   if (row >= offsets[EL]) return;
   const T* g = gu + (size_t)row * 2 * I;
-  const b200::GluShape shape = {limit, slope};
   for (int i = threadIdx.x * 8; i < I; i += blockDim.x * 8) {
     float gv[8], uv[8];
     b200::load8(g + i, gv);
     b200::load8(g + I + i, uv);
-#pragma unroll
-    for (int j = 0; j < 8; ++j) {
-      if (slope > 0.f) {
-        gv[j] = b200::glu<sizeof(T) == 2>(gv[j], uv[j], shape);
-        continue;
-      }
-      if (limit > 0.f) {
-        uv[j] = fminf(fmaxf(uv[j], -limit), limit);
-        gv[j] = fminf(gv[j], limit);
-      }
-      gv[j] = __fdividef(gv[j], 1.f + __expf(-gv[j])) * uv[j];
-    }
+    glu8<sizeof(T) == 2>(gv, uv, {limit, slope});
     b200::store8(act + (size_t)row * I + i, gv);
   }
+}
+
+// Gathered rows and gated units as FP8 terms; one block per sorted row.  The tile counters of the product that takes them are
+// cleared here.
+__global__ void __launch_bounds__(512) moe_gather_terms_kernel(const __nv_bfloat16* __restrict__ x, const int* __restrict__ row_token,
+                                                               const int* __restrict__ offsets, int EL, b200::mx::Rows o,
+                                                               int* __restrict__ counters, int n_counters) {
+  b200::pdl_grid_trigger();
+  b200::pdl_grid_wait();
+  const int row = blockIdx.x;
+  if (row == 0)
+    for (int i = threadIdx.x; i < n_counters; i += blockDim.x) counters[i] = 0;
+  if (row >= offsets[EL]) return;
+  const __nv_bfloat16* src = x + (size_t)row_token[row] * o.K;
+  o.put_row(row, [&](int i, float (&v)[8]) { b200::load8(src + i, v); });
+}
+
+__global__ void __launch_bounds__(512) moe_glu_terms_kernel(const __nv_bfloat16* __restrict__ gu, const int* __restrict__ offsets, int EL,
+                                                            b200::GluShape shape, b200::mx::Rows o, int* __restrict__ counters,
+                                                            int n_counters) {
+  b200::pdl_grid_trigger();
+  b200::pdl_grid_wait();
+  const int row = blockIdx.x;
+  if (row == 0)
+    for (int i = threadIdx.x; i < n_counters; i += blockDim.x) counters[i] = 0;
+  if (row >= offsets[EL]) return;
+  const __nv_bfloat16* g = gu + (size_t)row * 2 * o.K;
+  o.put_row(row, [&](int i, float (&v)[8]) {
+    float u[8];
+    b200::load8(g + i, v);
+    b200::load8(g + o.K + i, u);
+    glu8<true>(v, u, shape);
+#pragma unroll
+    for (int j = 0; j < 8; ++j) v[j] = __bfloat162float(__float2bfloat16(v[j]));
+  });
 }
 
 // out[t, :] = base[t, :] (optional) + sum_k wts[t,k] * y[route_row[t,k], :]
@@ -322,14 +365,21 @@ int b200_moe_route(const float* logits, int ld, const float* bias, int T, int E,
 
 // Plans the grouped GEMMs of this rank's experts [expert_lo, expert_hi).  All outputs are device buffers:
 // offsets int32 [EL+1]; route_row int32 [T*K]; row_token int32 [T*K]; work13 / work2: int4 [max_work]; n13 / n2: int32 [1].
-int b200_moe_plan(const int* idx, int T, int K, int expert_lo, int expert_hi, int* offsets, int* route_row,
-                  int* row_token, void* work13, int* n13, int m_tiles13, int bn13, void* work2, int* n2, int m_tiles2,
-                  int bn2, int max_work, cudaStream_t stream) {
+// rows_first, bit 0 for the first table, bit 1 for the second: token tiles that share weights follow each other.
+int b200_moe_plan_ordered(const int* idx, int T, int K, int expert_lo, int expert_hi, int* offsets, int* route_row, int* row_token,
+                          void* work13, int* n13, int m_tiles13, int bn13, void* work2, int* n2, int m_tiles2, int bn2, int max_work,
+                          int rows_first, cudaStream_t stream) {
   const int EL = expert_hi - expert_lo;
   if (T <= 0 || K <= 0 || EL <= 0 || EL > MAX_EXPERTS || max_work <= 0) return -6;
   return (int)b200::launch_pdl(moe_plan_kernel, dim3(EL), dim3(1024), 0, stream, idx, T * K, K, expert_lo, expert_hi, offsets, route_row,
                                row_token, reinterpret_cast<int4*>(work13), n13, m_tiles13, bn13, reinterpret_cast<int4*>(work2), n2,
-                               m_tiles2, bn2, max_work);
+                               m_tiles2, bn2, max_work, rows_first);
+}
+int b200_moe_plan(const int* idx, int T, int K, int expert_lo, int expert_hi, int* offsets, int* route_row,
+                  int* row_token, void* work13, int* n13, int m_tiles13, int bn13, void* work2, int* n2, int m_tiles2,
+                  int bn2, int max_work, cudaStream_t stream) {
+  return b200_moe_plan_ordered(idx, T, K, expert_lo, expert_hi, offsets, route_row, row_token, work13, n13, m_tiles13, bn13, work2, n2,
+                               m_tiles2, bn2, max_work, 0, stream);
 }
 
 int b200_moe_gather(const void* x, const int* row_token, const int* offsets, int EL, void* xs, int max_rows, int H,
@@ -337,6 +387,38 @@ int b200_moe_gather(const void* x, const int* row_token, const int* offsets, int
   if (max_rows <= 0 || H % 8) return -6;
   return (int)b200::launch_pdl(moe_gather_kernel, dim3(max_rows), dim3(128), 0, stream, reinterpret_cast<const __nv_bfloat16*>(x), row_token,
                                offsets, EL, reinterpret_cast<__nv_bfloat16*>(xs), H);
+}
+
+static bool rows_out(b200::mx::Rows* o, int R, int K, void* xq, void* sf, int* outside, void* rest) {
+  if (!xq || !sf || !outside || !rest || R <= 0 || K <= 0 || K % 128 ||
+      (reinterpret_cast<uintptr_t>(xq) | reinterpret_cast<uintptr_t>(rest)) % 16)
+    return false;
+  *o = {reinterpret_cast<uint8_t*>(xq), reinterpret_cast<uint8_t*>(sf), outside, reinterpret_cast<__nv_bfloat16*>(rest), R, K};
+  return true;
+}
+// A few rows: as many threads as a row has groups of eight, up to 512.  Many: small blocks, of which an SM holds more than the
+// latency of a row needs (12000 rows of 4096: 59 us for 80 with 512 threads).
+static dim3 row_threads(int rows, int K) {
+  const int most = rows > 1024 ? 128 : 512;
+  return dim3(K / 8 >= most ? most : (K / 8 + 31) / 32 * 32);
+}
+
+// x [tokens, K] -> terms of the sorted rows: xq [2][max_rows][K], sf [K/128][max_rows][4], outside [max_rows], rest [max_rows][K].
+// counters [n_counters]: cleared.
+int b200_moe_gather_terms(const void* x, const int* row_token, const int* offsets, int EL, void* xq, void* sf, int* outside, void* rest,
+                          int max_rows, int K, int* counters, int n_counters, cudaStream_t stream) {
+  b200::mx::Rows o;
+  if (!x || reinterpret_cast<uintptr_t>(x) % 16 || !rows_out(&o, max_rows, K, xq, sf, outside, rest)) return -6;
+  return (int)b200::launch_pdl(moe_gather_terms_kernel, dim3(max_rows), row_threads(max_rows, K), 0, stream, reinterpret_cast<const __nv_bfloat16*>(x),
+                               row_token, offsets, EL, o, counters, n_counters);
+}
+// gu [max_rows, 2 I] (gate | up) -> terms of the gated unit in bf16.
+int b200_moe_glu_terms(const void* gu, const int* offsets, int EL, void* xq, void* sf, int* outside, void* rest, int max_rows, int I,
+                       float limit, float slope, int* counters, int n_counters, cudaStream_t stream) {
+  b200::mx::Rows o;
+  if (!gu || reinterpret_cast<uintptr_t>(gu) % 16 || !rows_out(&o, max_rows, I, xq, sf, outside, rest)) return -6;
+  return (int)b200::launch_pdl(moe_glu_terms_kernel, dim3(max_rows), row_threads(max_rows, I), 0, stream, reinterpret_cast<const __nv_bfloat16*>(gu),
+                               offsets, EL, b200::GluShape{limit, slope}, o, counters, n_counters);
 }
 
 // slope > 0: the clamped one-plus unit of glu.cuh, else SwiGLU with the optional clamp.  I % 8 == 0.

@@ -64,6 +64,16 @@ int b200_moe_gather(const void* x, const int* row_token, const int* offsets, int
                     cudaStream_t stream);
 int b200_moe_glu(const void* gu, const int* offsets, int EL, void* act, int max_rows, int I, float limit, float slope, int f32,
                  cudaStream_t stream);
+int b200_moe_plan_ordered(const int* idx, int T, int K, int expert_lo, int expert_hi, int* offsets, int* route_row, int* row_token,
+                          void* work13, int* n13, int m_tiles13, int bn13, void* work2, int* n2, int m_tiles2, int bn2, int max_work,
+                          int rows_first, cudaStream_t stream);
+int b200_moe_gather_terms(const void* x, const int* row_token, const int* offsets, int EL, void* xq, void* sf, int* outside, void* rest,
+                          int max_rows, int K, int* counters, int n_counters, cudaStream_t stream);
+int b200_moe_glu_terms(const void* gu, const int* offsets, int EL, void* xq, void* sf, int* outside, void* rest, int max_rows, int I,
+                       float limit, float slope, int* counters, int n_counters, cudaStream_t stream);
+int b200_fp4_terms_plan(int* tok, long long* partial_floats, int* counters);
+int b200_gemm_fp4_terms(const void* W, const void* xq, const void* sf, const int* outside, const void* rest, void* out_bf16, int R, int N,
+                        int K, int groups, const void* work, const int* num_work, int max_work, float* partial, int* counters, int* status, cudaStream_t stream);
 int b200_moe_combine(const void* y, const int* route_row, const float* wts, const void* base, void* out, int T, int K,
                      int H, cudaStream_t stream);
 

@@ -4,6 +4,7 @@ number of rows per expert only exists on the device."""
 from __future__ import annotations
 
 import ctypes
+import functools
 from dataclasses import dataclass
 
 import torch
@@ -18,8 +19,10 @@ SCORE_FN = {"softmax": 0, "sigmoid": 1, "sqrtsoftplus": 2, "softmax_chosen": 3}
 
 
 def prepack_fp4(packed: torch.Tensor, scale_e8m0: torch.Tensor) -> torch.Tensor:
-    """FP4 weight (uint8 [N, K/2] two codes per byte, low nibble first; E8M0 uint8 [N, K/32]) -> the GEMM's
-    tile-major layout uint8 [ceil(N/128), K/64, 4352]: per stage 128 rows x 32 code bytes, then 128 x 2 scale bytes."""
+    """FP4 weight (uint8 [N, K/2] two codes per byte, low nibble first; E8M0 uint8 [N, K/32]) -> the tile-major layout of the
+    product that takes it.  Whole blocks of 128 inputs (``gemm_fp4_terms.cu``): uint8 [ceil(N/128), K/128, 8704], 16 code bytes (32
+    inputs) of each of 128 rows four times, then their 128 x 4 scales with row r at 16 (r % 32) + 4 (r / 32), 255 (NaN to the tensor
+    core) as 254.  Else (``gemm_wdec.cu``): uint8 [ceil(N/128), K/64, 4352], 128 rows x 32 code bytes, then 128 x 2 scales."""
     n, kh = packed.shape
     k = kh * 2
     assert k % 64 == 0 and scale_e8m0.shape == (n, k // 32)
@@ -27,8 +30,13 @@ def prepack_fp4(packed: torch.Tensor, scale_e8m0: torch.Tensor) -> torch.Tensor:
     if npad != n:
         packed = torch.cat([packed, packed.new_zeros(npad - n, kh)])
         scale_e8m0 = torch.cat([scale_e8m0, scale_e8m0.new_zeros(npad - n, k // 32)])
-    codes = packed.view(npad // 128, 128, k // 64, 32).permute(0, 2, 1, 3).reshape(npad // 128, k // 64, 128 * 32)
-    sc = scale_e8m0.view(npad // 128, 128, k // 64, 2).permute(0, 2, 1, 3).reshape(npad // 128, k // 64, 128 * 2)
+    mt, bk = npad // 128, 128 if k % 128 == 0 else 64
+    if bk == 128:
+        codes = packed.view(mt, 128, k // 128, 4, 16).permute(0, 2, 3, 1, 4).reshape(mt, k // 128, -1)
+        sc = scale_e8m0.clamp(max=254).view(mt, 4, 32, k // 128, 4).permute(0, 3, 2, 1, 4).reshape(mt, k // 128, -1)
+    else:
+        codes = packed.view(mt, 128, k // 64, 32).permute(0, 2, 1, 3).reshape(mt, k // 64, -1)
+        sc = scale_e8m0.view(mt, 128, k // 64, 2).permute(0, 2, 1, 3).reshape(mt, k // 64, -1)
     return torch.cat([codes, sc], -1).contiguous()
 
 
@@ -41,6 +49,11 @@ class ExpertWeights:
     n: int
     k: int
     experts: int
+
+    @property
+    def block_scaled(self) -> bool:
+        """FP4 matrices in the layout of csrc/kernels/gemm_fp4_terms.cu (``prepack_fp4``)"""
+        return self.wfmt == WF_FP4 and self.k % 128 == 0
 
     @staticmethod
     def from_fp4(packed: list[torch.Tensor], scales: list[torch.Tensor]) -> "ExpertWeights":
@@ -122,6 +135,31 @@ def pack_experts(gate: list[torch.Tensor], up: list[torch.Tensor], down: list[to
     return pack(w13), pack(w2)
 
 
+@functools.lru_cache(maxsize=1)
+def _fp4_terms_plan() -> tuple[int, int, int]:
+    """(rows of a tile, floats of partial sums, tile counters) of the block-scaled products"""
+    tok, part, counters = ctypes.c_int(), ctypes.c_longlong(), ctypes.c_int()
+    _lib.check(_lib.lib().b200_fp4_terms_plan(ctypes.byref(tok), ctypes.byref(part), ctypes.byref(counters)), "fp4_terms_plan", 0)
+    return tok.value, part.value, counters.value
+
+
+class _RowTerms:
+    """``r`` rows of ``k`` values as pairs of E4M3 terms (csrc/kernels/mx_terms.cuh), and the scratch of the product that takes them, in
+    one allocation."""
+
+    def __init__(self, r: int, k: int, device):
+        _, part, self.n_counters = _fp4_terms_plan()
+        # terms, scales, flags, values outside the terms, partial sums, counters
+        sizes = (2 * r * k, r * k // 32, 4 * r, 2 * r * k, 4 * part, 4 * self.n_counters)
+        at = [0]
+        for n in sizes:
+            at.append(at[-1] + (n + 127) // 128 * 128)
+        self.buf = torch.empty(at[-1], dtype=torch.uint8, device=device)
+        base = self.buf.data_ptr()
+        *ptrs, self.partial, self.counters = (ctypes.c_void_p(base + o) for o in at[:-1])
+        self.ptrs = tuple(ptrs)
+
+
 F32_TILE = 64                   # rows and features of a tile of the fp32 grouped GEMM
 
 
@@ -140,43 +178,58 @@ def experts_rows(x: torch.Tensor, idx: torch.Tensor, w13: ExpertWeights, w2: Exp
     dev = x.device
     f32 = w13.wfmt == WF_F32
     assert x.dtype == (torch.float32 if f32 else torch.bfloat16) and x.is_contiguous() and h == w13.k
+    terms = [w.block_scaled for w in (w13, w2)]           # products that take their rows as pairs of E4M3 terms
     bn = F32_TILE if f32 else gemm._bn(min(256, max(16, (r + el - 1) // el)))      # token tile sized for the average rows per expert
     if 3 <= w13.wfmt < WF_F32:
         bn = min(bn, int(L.b200_gguf_max_bn(w13.wfmt)), int(L.b200_gguf_max_bn(w2.wfmt)))
+    bn13, bn2 = (_fp4_terms_plan()[0] if m else bn for m in terms)
     bm = F32_TILE if f32 else 128
-    mt13, mt2 = (w13.n + bm - 1) // bm, (w2.n + bm - 1) // bm
-    max_work = (mt13 + mt2) * ((r + bn - 1) // bn + el)
-    i32 = lambda *s: torch.empty(*s, dtype=torch.int32, device=dev)
-    offsets, route_row, row_token = i32(el + 1), i32(t, k), i32(r)
-    work13, work2 = i32(max_work, 4), i32(max_work, 4)
-    n13, n2 = i32(1), i32(1)
+    mt13, mt2 = ((w.n + f - 1) // f for w, f in ((w13, 256 if terms[0] else bm), (w2, 256 if terms[1] else bm)))
+    max_work = (mt13 + mt2) * ((r + min(bn13, bn2) - 1) // min(bn13, bn2) + el)
+    # the plan, in one allocation: work tables, counts, expert offsets, source token of every row
+    plan = torch.empty(8 * max_work + 4 + el + 1 + r, dtype=torch.int32, device=dev)
+    at = plan.data_ptr()
+    work13, work2, n13, n2, offsets, row_token = (ctypes.c_void_p(at + 4 * o) for o in (
+        0, 4 * max_work, 8 * max_work, 8 * max_work + 1, 8 * max_work + 4, 8 * max_work + 5 + el))
+    route_row = torch.empty(t, k, dtype=torch.int32, device=dev)
     s = _lib.stream()
-    rc = L.b200_moe_plan(_lib.ptr(idx), t, k, expert_lo, expert_lo + el, _lib.ptr(offsets), _lib.ptr(route_row),
-                         _lib.ptr(row_token), _lib.ptr(work13), _lib.ptr(n13), mt13, bn, _lib.ptr(work2), _lib.ptr(n2),
-                         mt2, bn, max_work, s)
+    rc = L.b200_moe_plan_ordered(_lib.ptr(idx), t, k, expert_lo, expert_lo + el, offsets, _lib.ptr(route_row),
+                                 row_token, work13, n13, mt13, bn13, work2, n2, mt2, bn2, max_work, int(terms[0]) | int(terms[1]) << 1, s)
     _lib.check(rc, "moe_plan")
-    # rows past the real count are never read: sized for the worst case (every route local)
-    xs = torch.empty(r, h, dtype=x.dtype, device=dev)
-    # 16-bit columns: an fp32 row counts twice
-    rc = L.b200_moe_gather(_lib.ptr(x), _lib.ptr(row_token), _lib.ptr(offsets), el, _lib.ptr(xs), r, 2 * h if f32 else h, s)
-    _lib.check(rc, "moe_gather")
 
-    def product(w: ExpertWeights, a: torch.Tensor, work, num, what: str) -> torch.Tensor:
+    def product(w: ExpertWeights, a, work, num, what: str) -> torch.Tensor:
         out = torch.empty(r, w.n, dtype=x.dtype, device=dev)
-        if f32:
-            rc = L.b200_gemm_f32_grouped(_lib.ptr(a), _lib.ptr(w.weight), _lib.ptr(out), w.n, w.k, _lib.ptr(work), _lib.ptr(num),
-                                         max_work, s)
+        if isinstance(a, _RowTerms):
+            rc = L.b200_gemm_fp4_terms(_lib.ptr(w.weight), *a.ptrs, _lib.ptr(out), r, w.n, w.k, el, work, num, max_work,
+                                       a.partial, a.counters, _lib.ptr(_lib.status_word(dev)), s)
+        elif f32:
+            rc = L.b200_gemm_f32_grouped(_lib.ptr(a), _lib.ptr(w.weight), _lib.ptr(out), w.n, w.k, work, num, max_work, s)
         else:
             grouped = L.b200_gemm_wdec_grouped if w.wfmt < 3 else L.b200_gemm_wdec_gguf_grouped
             rc = grouped(w.wfmt, _lib.ptr(w.weight), _lib.ptr(w.scales), _lib.ptr(a), _lib.ptr(out), r, w.n, w.k, el,
-                         _lib.ptr(work), _lib.ptr(num), bn, _lib.ptr(_lib.status_word(dev)), s)
+                         work, num, bn, _lib.ptr(_lib.status_word(dev)), s)
         _lib.check(rc, what)
         return out
 
+    # rows past the real count are never read: sized for the worst case (every route local)
+    if terms[0]:
+        xs = _RowTerms(r, h, dev)
+        rc = L.b200_moe_gather_terms(_lib.ptr(x), row_token, offsets, el, *xs.ptrs, r, h, xs.counters,
+                                     xs.n_counters, s)
+    else:
+        xs = torch.empty(r, h, dtype=x.dtype, device=dev)
+        # 16-bit columns: an fp32 row counts twice
+        rc = L.b200_moe_gather(_lib.ptr(x), row_token, offsets, el, _lib.ptr(xs), r, 2 * h if f32 else h, s)
+    _lib.check(rc, "moe_gather")
     gu = product(w13, xs, work13, n13, "grouped gemm w13")
-    act = torch.empty(r, inter, dtype=x.dtype, device=dev)
-    rc = L.b200_moe_glu(_lib.ptr(gu), _lib.ptr(offsets), el, _lib.ptr(act), r, inter, ctypes.c_float(limit), ctypes.c_float(slope),
-                        int(f32), s)
+    if terms[1]:
+        act = _RowTerms(r, inter, dev)
+        rc = L.b200_moe_glu_terms(_lib.ptr(gu), offsets, el, *act.ptrs, r, inter, ctypes.c_float(limit), ctypes.c_float(slope),
+                                  act.counters, act.n_counters, s)
+    else:
+        act = torch.empty(r, inter, dtype=x.dtype, device=dev)
+        rc = L.b200_moe_glu(_lib.ptr(gu), offsets, el, _lib.ptr(act), r, inter, ctypes.c_float(limit), ctypes.c_float(slope),
+                            int(f32), s)
     _lib.check(rc, "moe_glu")
     return product(w2, act, work2, n2, "grouped gemm w2"), route_row
 
