@@ -21,6 +21,7 @@
 #include "per_device.h"
 #include "../ptx/sm100.cuh"
 #include "tma_host.h"
+#include "launch.h"
 #include "ops.h"
 
 namespace b200 {
@@ -66,6 +67,8 @@ constexpr uint32_t idesc_pv = umma_idesc_bf16(128, 128) | (1u << 16);  // B is M
 __global__ void __launch_bounds__(NTHREADS, 1)
 gqa_prefill_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ CUtensorMap tmK,
                    const __grid_constant__ CUtensorMap tmV, Params p) {
+  pdl_launch_dependents();
+  pdl_wait();
   extern __shared__ uint8_t smem_base[];
   uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_base) + 1023) & ~uintptr_t(1023));
   uint8_t* sQ = smem;
@@ -423,8 +426,7 @@ extern "C" int b200_gqa_prefill(const void* q, const void* k_cache, const void* 
   p.window = g_window;
   p.sinks = g_sinks;
   dim3 grid((max_q_len + BQ - 1) / BQ, n_q_heads, batch);
-  gqa_prefill_kernel<<<grid, NTHREADS, SMEM_BYTES, stream>>>(tmQ, tmK, tmV, p);
-  return (int)cudaGetLastError();
+  return (int)launch_pdl(gqa_prefill_kernel, grid, dim3(NTHREADS), SMEM_BYTES, stream, tmQ, tmK, tmV, p);
 }
 
 // As b200_gqa_prefill, restricted to a sliding window with attention sinks: a query at position p attends to the keys

@@ -22,6 +22,7 @@
 #include "per_device.h"
 #include <cuda_fp16.h>
 #include <stdint.h>
+#include "launch.h"
 #include "ops.h"
 
 namespace {
@@ -323,6 +324,8 @@ __global__ void __launch_bounds__(256, 3)
 gdn_prepare_mma_kernel(const __nv_bfloat16* __restrict__ mixed, int ld, int q_off, int k_off, int v_off,
                        const float* __restrict__ g, const float* __restrict__ beta, PrepOut o, int T, int Hv, int Hk,
                        float q_scale) {
+  b200::pdl_grid_trigger();
+  b200::pdl_grid_wait();
   extern __shared__ __align__(16) unsigned char prep_raw[];
   __half* sKh = reinterpret_cast<__half*>(prep_raw);   // [64][LDH] k_hat
   __half* sQh = sKh + C * LDH;                         // [64][LDH] q_hat * scale
@@ -579,6 +582,8 @@ constexpr int SCAN_SMEM_BYTES = (2 * SCAN_WQ_HALVES + SCAN_KA_HALVES + SL * WS +
 // (key dims) [32w, 32w+32) for the state update.
 __global__ void __launch_bounds__(128, 2)
 gdn_scan_kernel(PrepOut w, float* __restrict__ state, __nv_bfloat16* __restrict__ out, int T, int nchunks, int Hv) {
+  b200::pdl_grid_trigger();
+  b200::pdl_grid_wait();
   extern __shared__ __align__(16) __half sh[];
   __half* const bK = sh + 2 * SCAN_WQ_HALVES;     // [128][TS] KgT of the current chunk
   __half* const bA = bK + DK * TS;                // [64][TS]  Aqk of the current chunk
@@ -802,15 +807,18 @@ int b200_gdn_chunked(const void* mixed, int ld, int q_off, int k_off, int v_off,
     if (e != cudaSuccess) return (int)e;
     configured = true;
   }
-  if (g_prepare_simt)
+  cudaError_t launched = cudaSuccess;
+  if (g_prepare_simt) {
     gdn_prepare_kernel<<<dim3(Hv, nch), 256, prep_smem, stream>>>(
         reinterpret_cast<const __nv_bfloat16*>(mixed), ld, q_off, k_off, v_off, g, beta, o, T, Hv, Hk, q_scale);
+    launched = cudaGetLastError();
+  }
   else
-    gdn_prepare_mma_kernel<<<dim3(Hv, nch), 256, PREP_MMA_SMEM, stream>>>(
-        reinterpret_cast<const __nv_bfloat16*>(mixed), ld, q_off, k_off, v_off, g, beta, o, T, Hv, Hk, q_scale);
-  gdn_scan_kernel<<<dim3(Hv, DV / SL), 128, scan_smem, stream>>>(o, state, reinterpret_cast<__nv_bfloat16*>(out), T,
-                                                                  nch, Hv);
-  return (int)cudaGetLastError();
+    launched = b200::launch_pdl(gdn_prepare_mma_kernel, dim3(Hv, nch), dim3(256), PREP_MMA_SMEM, stream,
+                                reinterpret_cast<const __nv_bfloat16*>(mixed), ld, q_off, k_off, v_off, g, beta, o, T, Hv, Hk, q_scale);
+  if (launched != cudaSuccess) return (int)launched;
+  return (int)b200::launch_pdl(gdn_scan_kernel, dim3(Hv, DV / SL), dim3(128), scan_smem, stream, o, state,
+                               reinterpret_cast<__nv_bfloat16*>(out), T, nch, Hv);
 }
 
 // One token per sequence: mixed [B, ld], g/beta [B, Hv], states [slots, Hv, 128, 128], out [B, Hv, 128].

@@ -41,6 +41,10 @@ int b200_gemm_w8a8s(const void* W, const float* scales, const void* xq, const fl
 // b200_gemm_w8a8s_allreduce (same arguments + the peer-memory communicator) is declared beside the communicator in
 // gemm_w8a8s.cu: this header stays free of the communicator's types.
 
+// ---- a / b projections and gates of a Gated DeltaNet prompt portion (gdn_ab_gates.cu)
+int b200_gdn_ab_gates(const void* x, int H, const void* w, const float* a_log, const float* dt_bias, float* g, float* beta, int T, int Hv,
+                      cudaStream_t stream);
+
 // ---- fused decode-step kernels (decode_fused.cu)
 int b200_gdn_decode_fused(const void* proj, int ldp, const void* x, int hidden, const void* w_ab, const float* a_log,
                           const float* dt_bias, const void* conv_w, int kw, void* tails, long long tail_stride,

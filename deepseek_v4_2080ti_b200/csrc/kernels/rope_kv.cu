@@ -8,6 +8,7 @@
 // cuda_ops.cu head_rmsnorm_rope :477-670, src/csrc/minimax_rope_kernel.cu:41-78.
 #include <cuda_bf16.h>
 #include <stdint.h>
+#include "launch.h"
 #include "ops.h"
 
 namespace {
@@ -88,6 +89,8 @@ __device__ __forceinline__ void norm_rope(float (&x)[4], const __nv_bfloat16* ga
 }
 
 __global__ void qk_norm_rope_append_kernel(RopeParams p) {
+  b200::pdl_grid_trigger();
+  b200::pdl_grid_wait();
   const int lane = threadIdx.x & 31;
   const size_t w = (size_t)blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
   const int heads = p.Hq + 2 * p.Hkv;
@@ -148,8 +151,7 @@ int launch_rope(RopeParams& p, cudaStream_t stream) {
   const int heads = p.Hq + 2 * p.Hkv;
   const size_t warps = (size_t)p.T * heads;
   const int wpb = 8;
-  qk_norm_rope_append_kernel<<<(unsigned)((warps + wpb - 1) / wpb), wpb * 32, 0, stream>>>(p);
-  return (int)cudaGetLastError();
+  return (int)b200::launch_pdl(qk_norm_rope_append_kernel, dim3((unsigned)((warps + wpb - 1) / wpb)), dim3(wpb * 32), 0, stream, p);
 }
 
 }  // namespace

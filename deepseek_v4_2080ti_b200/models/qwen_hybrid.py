@@ -640,10 +640,13 @@ class QwenHybridRuntime(PagedSequences):
         cfg = self.cfg
         with PROFILER.scope("lin.qkvz"):
             proj = self._col_parallel(x, lw.proj) if terms is None else gemm.linear_terms(terms, lw.proj)    # [T, 2kd + vd + vd]
-        ab = gemm.linear(x, lw.ab)                           # [T, 2 hv]
         cw = 2 * self.kd + self.vd
         idx = self.lin_layers.index(li)
-        g, beta = basic.gdn_gates(ab, 0, self.hv_lin, lw.a_log, lw.dt_bias, self.hv_lin)
+        if slot is not None and not self._sp and gdn.ab_gates_fit(t, cfg.hidden_size, self.hv_lin):
+            g, beta = gdn.ab_gates(x, lw.ab.weight, lw.a_log, lw.dt_bias, self.hv_lin)
+        else:
+            ab = gemm.linear(x, lw.ab)                       # [T, 2 hv]
+            g, beta = basic.gdn_gates(ab, 0, self.hv_lin, lw.a_log, lw.dt_bias, self.hv_lin)
         if slot is not None:   # one sequence, T consecutive tokens
             mixed = basic.conv_silu(proj[:, :cw], lw.conv_w, self.tails[slot, idx])
             with PROFILER.scope("gdn.chunked"):

@@ -34,6 +34,26 @@ def chunked(mixed, q_off, k_off, v_off, g, beta, state, hv, hk):
     return out
 
 
+AB_GATES_MAX_T = 2047           # longest portion whose gates ``ab_gates`` makes (csrc/kernels/gdn_ab_gates.cu)
+
+
+def ab_gates_fit(t: int, hidden: int, hv: int) -> bool:
+    return t <= AB_GATES_MAX_T and hidden % 32 == 0 and hv <= 32
+
+
+def ab_gates(x, w_ab, a_log, dt_bias, hv):
+    """a | b = x @ w_ab^T (rounded to bf16), g = -exp(A_log) * softplus(a + dt_bias), beta = sigmoid(b): fp32 [T, Hv] each.
+    x [T, hidden] bf16, w_ab [2 Hv, hidden] bf16 (a rows, then b rows)."""
+    t, h = x.shape
+    assert x.is_contiguous() and w_ab.is_contiguous() and w_ab.shape == (2 * hv, h)
+    g = torch.empty(t, hv, dtype=torch.float32, device=x.device)
+    beta = torch.empty_like(g)
+    rc = _lib.lib().b200_gdn_ab_gates(_lib.ptr(x), h, _lib.ptr(w_ab), _lib.ptr(a_log), _lib.ptr(dt_bias), _lib.ptr(g), _lib.ptr(beta), t, hv,
+                                      _lib.stream())
+    _lib.check(rc, "gdn_ab_gates")
+    return g, beta
+
+
 def use_simt_prepare(on: bool) -> bool:
     """Route the chunk preparation of ``chunked`` through the scalar fp32 kernel (the yardstick of the tensor-core
     one); returns the previous setting."""
