@@ -45,6 +45,10 @@ int b200_gemm_w8a8s(const void* W, const float* scales, const void* xq, const fl
 int b200_gdn_ab_gates(const void* x, int H, const void* w, const float* a_log, const float* dt_bias, float* g, float* beta, int T, int Hv,
                       cudaStream_t stream);
 
+// ---- prompt portions of the hybrid decoder (qwen_rows.cu, which declares the structures)
+int b200_portion_meta(const int* block_row, int past, int T, int block_size, int* pos, int* kv_slots, int* meta, long long* last_row,
+                      cudaStream_t stream);
+
 // ---- fused decode-step kernels (decode_fused.cu)
 int b200_gdn_decode_fused(const void* proj, int ldp, const void* x, int hidden, const void* w_ab, const float* a_log,
                           const float* dt_bias, const void* conv_w, int kw, void* tails, long long tail_stride,

@@ -9,6 +9,7 @@ package's sm_100a kernels; decode steps are replayed from CUDA graphs.
 """
 from __future__ import annotations
 
+import ctypes
 import json
 import math
 from dataclasses import dataclass, field
@@ -707,12 +708,60 @@ class QwenHybridRuntime(PagedSequences):
         h = basic.embedding(ids, self.w.embed, self.w.vocab_lo, self.w.vocab_hi)
         return h if self.w.embed_replicated else self.comm.all_reduce(h)
 
+    def _issues_natively(self, t: int, meta, slot: int | None) -> bool:
+        """Does a prompt portion of ``t`` tokens go through the layers in one native call (csrc/kernels/qwen_rows.cu)?  One rank, a
+        bf16 cache, FP8 products that all take terms; not while launches are looked at one by one."""
+        return slot is not None and meta["mode"] == "prefill" and self.kv8 is None and not self._sp and not PROFILER.enabled and \
+            not _lib.bounds_checks_on() and gdn.ab_gates_fit(t, self.cfg.hidden_size, self.hv_lin) and \
+            all(self._terms_rows(t, lw) for lw in self.w.layers)
+
+    def _layers_native(self, h: torch.Tensor, positions, kv_slots, meta, slot: int) -> torch.Tensor:
+        """The layers of ``_forward`` for one prompt portion: ``h`` [T, H] becomes the residual, returned is what is still to be
+        added to it.  The pointers are gathered for this call only."""
+        cfg, L, s = self.cfg, _lib.lib(), _lib.stream()
+        t, hidden = h.shape
+        full = {l: i for i, l in enumerate(self.full_layers)}
+        lin = {l: i for i, l in enumerate(self.lin_layers)}
+        at = lambda x: 0 if x is None else x.data_ptr()
+        tail0, state0 = self.tails[slot].data_ptr(), self.states[slot].data_ptr()
+        tail_step, state_step = self.tails.stride(1) * 2, self.states.stride(1) * 4
+        rows: list[int] = []
+        for i, lw in enumerate(self.w.layers):
+            j = lin.get(i, 0)
+            linear = lw.kind == "linear"
+            rows += [linear, at(lw.in_ln), at(lw.post_ln), at(lw.proj.weight), at(lw.proj.scales), lw.proj.n, at(lw.out.weight),
+                     at(lw.out.scales), lw.out.k, gemm.terms_pay(t, lw.out.n, lw.out.k), at(lw.gate_up.weight), at(lw.gate_up.scales),
+                     at(lw.down.weight), at(lw.down.scales)]
+            if linear:
+                rows += [at(lw.ab.weight), at(lw.a_log), at(lw.dt_bias), at(lw.conv_w), at(lw.gdn_norm), tail0 + j * tail_step,
+                         state0 + j * state_step, 0, 0, 0, 0]
+            else:
+                rows += [0] * 7 + [at(lw.q_norm), at(lw.k_norm), at(self.k_cache[full[i]]), at(self.v_cache[full[i]])]
+        table = (ctypes.c_longlong * len(rows))(*rows)
+        delta = torch.empty_like(h)
+        bt = meta["block_table"]
+        call = [t, hidden, cfg.intermediate_size, self.hq, self.hkv, self.hk_lin, self.hv_lin, bool(cfg.attn_output_gate), cfg.rotary_dim,
+                self.block_size, bt.shape[1], self.num_blocks, self.attention_window, self.attention_sinks, at(self.inv_freq), at(positions),
+                at(kv_slots), at(bt), at(meta["q_start"]), at(meta["q_len"]), at(meta["kv_len"]), at(h), at(delta), 0, 0,
+                at(_lib.status_word(h.device)), 0]
+        run = (ctypes.c_longlong * len(call))(*call)
+        args = (table, len(self.w.layers), run, ctypes.c_float(cfg.rms_norm_eps), ctypes.c_float(1.0 / math.sqrt(cfg.head_dim)), s)
+        _lib.check(L.b200_qwen_rows(*args), "qwen_rows plan", 0)
+        scratch = torch.empty(run[24], dtype=torch.uint8, device=h.device)
+        run[23] = scratch.data_ptr()
+        _lib.check(L.b200_qwen_rows(*args), "qwen_rows", 0)
+        _lib.LAUNCHES += run[26]
+        return delta
+
     def _forward(self, ids, positions, kv_slots, meta, slot, slots_t, logits_rows: torch.Tensor | None):
         cfg, w = self.cfg, self.w
         t = ids.numel()
         h = self._embed(ids)
         delta = None
-        for i, lw in enumerate(w.layers):
+        native = self._issues_natively(t, meta, slot)
+        if native:
+            delta = self._layers_native(h, positions, kv_slots, meta, slot)
+        for i, lw in enumerate(w.layers if not native else ()):
             a = None
             if self._terms_rows(t, lw):
                 x, a = basic.rmsnorm_terms(h, delta, lw.in_ln, cfg.rms_norm_eps, True, want_bf16=lw.kind == "linear")
@@ -832,13 +881,15 @@ class QwenHybridRuntime(PagedSequences):
             ids = token_ids[s:e]
             t = ids.numel()
             self._ensure_blocks(st, st.length + t)
-            pos = torch.arange(st.length, st.length + t, dtype=torch.int32, device=self.device)
-            bt_row = self.block_table[slot]
-            kv_slots = (bt_row[(pos // self.block_size).long()] * self.block_size + pos % self.block_size).to(torch.int32)
-            i32 = lambda v: torch.tensor([v], dtype=torch.int32, device=self.device)
-            meta = {"mode": "prefill", "block_table": self.block_table[slot:slot + 1], "q_start": i32(0),
-                    "q_len": i32(t), "kv_len": i32(st.length + t), "max_q_len": t, "past": st.length}
-            rows = torch.tensor([t - 1], dtype=torch.int64, device=self.device)
+            # written on the device: an upload each would wait for everything launched so far
+            buf = torch.empty(t + 3, dtype=torch.int64, device=self.device)
+            i32, rows = buf.view(torch.int32), buf[t + 2:]
+            pos, kv_slots, lens = i32[:t], i32[t:2 * t], i32[2 * t:2 * t + 3]
+            rc = _lib.lib().b200_portion_meta(_lib.ptr(self.block_table[slot]), st.length, t, self.block_size, _lib.ptr(pos),
+                                              _lib.ptr(kv_slots), _lib.ptr(lens), _lib.ptr(rows), _lib.stream())
+            _lib.check(rc, "portion_meta")
+            meta = {"mode": "prefill", "block_table": self.block_table[slot:slot + 1], "q_start": lens[:1],
+                    "q_len": lens[1:2], "kv_len": lens[2:], "max_q_len": t, "past": st.length}
             sp_rows = self.comm.sp_rows(t, self.cfg.hidden_size) if hasattr(self.comm, "sp_rows") else 0
             if sp_rows:
                 logits = self._forward_sp(ids, pos, kv_slots, meta, slot, rows, sp_rows)
