@@ -17,7 +17,9 @@ constexpr int PAIR_TOK = 256;       // tokens of a pair's tile
 
 struct Params {
   int T, N, m_tiles, n_tiles, kb;   // kb: 128-wide K blocks; m_tiles: 128-feature tiles; n_tiles: token tiles
-  int units, workers;               // units = tiles x kb (a pair's tile covers two m tiles)
+  int workers;                      // CTAs or pairs; a pair's tile covers two m tiles
+  int waves;                        // whole tiles that every worker takes, one of each run of `workers` tiles,
+  int units;                        // and (tile, K block) pairs of the tiles after those, shared in equal contiguous runs
   const uint8_t* w;                 // [m_tiles][kb][16 KB]
   const float* scales;              // [m_tiles][kb]
   const uint8_t* xq;                // [n_tiles][kb][CTA of the worker][hi, mid][tokens of a CTA][128 bytes]
@@ -31,10 +33,34 @@ struct Params {
   int vec;                          // rows of `out` (and `residual`) are whole, aligned 16-byte groups
   // first unit of a worker
   __device__ __forceinline__ int first(int worker) const { return (int)((long long)units * worker / workers); }
+  __device__ __forceinline__ int tail() const { return waves * workers; }
   // worker of a unit: the largest i with units * i / workers <= u
   __device__ __forceinline__ int owner(int u) const { return (int)((((long long)u + 1) * workers - 1) / units); }
-  // where worker i leaves its share of a cut tile: its first tile in place 0, its last in place 1
+  // where worker i leaves its share of a cut tile (counted from the tail): its first tile in place 0, its last in place 1
   __device__ __forceinline__ int place(int i, int tile) const { return first(i) / kb == tile ? 0 : 1; }
+};
+
+// The pieces of tiles that a worker computes, in order.
+struct Pieces {
+  const Params& p;
+  int worker, wave, u, u1;
+  int tile, c0, len;                // the piece: K blocks c0 .. c0 + len - 1 of a tile
+  __device__ __forceinline__ Pieces(const Params& p, int worker) : p(p), worker(worker), wave(0), u(p.first(worker)), u1(p.first(worker + 1)) {}
+  __device__ __forceinline__ bool next() {
+    if (wave < p.waves) {
+      tile = wave++ * p.workers + worker;
+      c0 = 0;
+      len = p.kb;
+      return true;
+    }
+    if (u >= u1) return false;
+    const int t = u / p.kb;
+    tile = p.tail() + t;
+    c0 = u - t * p.kb;
+    len = min(p.kb - c0, u1 - u);
+    u += len;
+    return true;
+  }
 };
 
 // ---- activations as terms.  Where the terms of a [T, K] matrix go: tiles of `tok` tokens, each CTA of a worker staging `cap`.

@@ -324,7 +324,6 @@ __global__ void __launch_bounds__(256, 3)
 gdn_prepare_mma_kernel(const __nv_bfloat16* __restrict__ mixed, int ld, int q_off, int k_off, int v_off,
                        const float* __restrict__ g, const float* __restrict__ beta, PrepOut o, int T, int Hv, int Hk,
                        float q_scale) {
-  b200::pdl_grid_trigger();
   b200::pdl_grid_wait();
   extern __shared__ __align__(16) unsigned char prep_raw[];
   __half* sKh = reinterpret_cast<__half*>(prep_raw);   // [64][LDH] k_hat

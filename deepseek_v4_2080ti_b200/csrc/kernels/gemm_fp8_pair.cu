@@ -17,7 +17,11 @@
 // read the block before last; the tensor pipe is busy for 65 % of the cycles at 1901 tokens.  The epilogue's 216 registers are all
 // in use and 52 bytes are spilled.
 //
-// Same work list and treatment of cut tiles as the one-CTA kernel; the tokens past the last one of a tile are not staged when
+// Work: as long as there are more tiles than workers, every worker takes a whole tile of each run of as many tiles, so that at any time the
+// chip works on neighbouring tiles, which share weights (all token tiles of a pair of weight tiles follow each other) and rows.  (With
+// contiguous runs 74 workers hold the weights of 74 places and all rows live, 116 MB at 1901 x 34816 x 5120: L2 gave back 59 % of the
+// operands, and without the products and the epilogue's reads of tensor memory it took 468 of 640 us.)  What is left, between one and
+// two tiles a worker, is cut as in the one-CTA kernel.  The tokens past the last one of a tile are not staged when
 // they fill a CTA, and not read back.  Roles: warps 0-7 epilogue (group of four: one weight tile of the pair), warp 8 weight
 // copies, warp 9 MMA issuer (first CTA), warp 10 activation copies.  All waits are bounded.
 #include <cuda_bf16.h>
@@ -151,7 +155,7 @@ gemm_fp8_pair_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_const
   asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
 
   const int worker = blockIdx.x >> 1;
-  const int u0 = p.first(worker), u1 = p.first(worker + 1);
+  Pieces piece(p, worker);
 
   // A thread of the epilogue holds 128 sums: its warps take registers from the others
   // (12 warps x 168 at launch; 8 x 32 x 216 + 4 x 32 x 64 = 63,488 of 64,512).
@@ -160,49 +164,57 @@ gemm_fp8_pair_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_const
     if (warp == WARP_W) {
       // ---------------------------------------------------------- weight copies, ahead of the previous kernel's end
       if (lane == 0) {
-        int tile = u0 / p.kb, c = u0 - tile * p.kb;
-        for (int blk = 0; blk < u1 - u0 && !*abort_flag; ++blk) {
-          const int b = blk % S;
-          if (blk >= S && !mbar_wait(&slot_free[b], ((blk / S) & 1) ^ 1)) {
-            atomicExch(p.status, ERR_WAIT_STAGE);
-            *abort_flag = 1;
-            break;
-          }
-          if (rank == 0) mbar_expect_tx(&full[b], 2 * W_BYTES);
+        bool ok = true;
+        for (int blk = 0; ok && piece.next();) {
           // an odd last weight tile: its partner lies past the map and reads zeros
-          const int m = (tile / p.n_tiles) * 2 + rank;
-          tma_load_pair(sW + b * W_BYTES, &tmW, on_leader(&full[b]), 0, (m * p.kb + c) * (W_BYTES / 256));
-          if (++c == p.kb) { c = 0; ++tile; }
+          const int m = (piece.tile / p.n_tiles) * 2 + rank;
+          int row = (m * p.kb + piece.c0) * (W_BYTES / 256);
+          for (int c = 0; c < piece.len; ++c, ++blk, row += W_BYTES / 256) {
+            const int b = blk % S;
+            ok = blk < S || mbar_wait(&slot_free[b], ((blk / S) & 1) ^ 1);
+            if (!ok) atomicExch(p.status, ERR_WAIT_STAGE);
+            if (!ok || *abort_flag) {
+              ok = false;
+              *abort_flag = 1;
+              break;
+            }
+            if (rank == 0) mbar_expect_tx(&full[b], 2 * W_BYTES);
+            tma_load_pair(sW + b * W_BYTES, &tmW, on_leader(&full[b]), 0, row);
+          }
         }
       }
     } else if (warp == WARP_X) {
       // ---------------------------------------------------------- activation copies
       if (lane == 0) {
         pdl_wait();
-        int tile = u0 / p.kb, c = u0 - tile * p.kb;
-        for (int blk = 0; blk < u1 - u0 && !*abort_flag; ++blk) {
-          const int b = blk % S;
-          if (blk >= S && !mbar_wait(&slot_free[b], ((blk / S) & 1) ^ 1)) {
-            atomicExch(p.status, ERR_WAIT_STAGE);
-            *abort_flag = 1;
-            break;
-          }
-          const int n = tile % p.n_tiles;
+        bool ok = true;
+        for (int blk = 0; ok && piece.next();) {
+          const int n = piece.tile % p.n_tiles;
           const bool both = p.T - n * PAIR_TOK > ROWS;       // else the second CTA has no tokens
-          const size_t xb = (size_t)n * p.kb + c;
-          if (rank == 0) mbar_expect_tx(&full[b], both ? 2 * X_BYTES : X_BYTES);
-          if (rank == 0 || both)
-            tma_load_pair(sX + b * X_BYTES, &tmX, on_leader(&full[b]), 0, (int)(xb * 2 + rank) * (X_BYTES / 256));
-          mbar_expect_tx(&sx_full[b], SX_BYTES);
-          bulk_load(sSx + b * ROWS, p.sx + xb * PAIR_TOK + rank * ROWS, SX_BYTES, &sx_full[b]);
-          if (++c == p.kb) { c = 0; ++tile; }
+          size_t xb = (size_t)n * p.kb + piece.c0;
+          for (int c = 0; c < piece.len; ++c, ++blk, ++xb) {
+            const int b = blk % S;
+            ok = blk < S || mbar_wait(&slot_free[b], ((blk / S) & 1) ^ 1);
+            if (!ok) atomicExch(p.status, ERR_WAIT_STAGE);
+            if (!ok || *abort_flag) {
+              ok = false;
+              *abort_flag = 1;
+              break;
+            }
+            if (rank == 0) mbar_expect_tx(&full[b], both ? 2 * X_BYTES : X_BYTES);
+            if (rank == 0 || both)
+              tma_load_pair(sX + b * X_BYTES, &tmX, on_leader(&full[b]), 0, (int)(xb * 2 + rank) * (X_BYTES / 256));
+            mbar_expect_tx(&sx_full[b], SX_BYTES);
+            bulk_load(sSx + b * ROWS, p.sx + xb * PAIR_TOK + rank * ROWS, SX_BYTES, &sx_full[b]);
+          }
         }
       }
     } else if (warp == WARP_MMA && rank == 0) {
       // ---------------------------------------------------------- MMA issuer
       const uint32_t on = elect_one();
       constexpr uint32_t idesc_hi = umma_idesc_f8(2 * ROWS, 2 * BM, true), idesc_mid = umma_idesc_f8(2 * ROWS, 2 * BM);
-      for (int blk = 0; blk < u1 - u0; ++blk) {
+      const int blocks = p.waves * p.kb + piece.u1 - piece.u;
+      for (int blk = 0; blk < blocks; ++blk) {
         const int b = blk % S, a = blk % A;
         int err = 0;
         if (!mbar_wait(&acc_free[a], ((blk / A) & 1) ^ 1)) err = ERR_WAIT_ACC;
@@ -228,20 +240,19 @@ gemm_fp8_pair_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_const
     // ------------------------------------------------------------ epilogue: one token, the 128 features of one weight tile
     const int group = warp >> 2, row = (warp & 3) * 32 + lane;
     float sc_a = 0.f, sc_b = 0.f;
-    auto fetch_scales = [&](int u) {       // of the next run of blocks, a run ahead
-      if (u >= u1) return;
-      const int tile = u / p.kb, c0 = u - tile * p.kb, len = min(p.kb - c0, u1 - u);
-      const int m = min((tile / p.n_tiles) * 2 + group, p.m_tiles - 1);
-      const float* srow = p.scales + (size_t)m * p.kb + c0;
-      if (row < len) sc_a = __ldg(srow + row);
-      if (128 + row < len) sc_b = __ldg(srow + 128 + row);
+    bool more = piece.next();
+    auto fetch_scales = [&] {              // of the next piece, a piece ahead
+      if (!more) return;
+      const int m = min((piece.tile / p.n_tiles) * 2 + group, p.m_tiles - 1);
+      const float* srow = p.scales + (size_t)m * p.kb + piece.c0;
+      if (row < piece.len) sc_a = __ldg(srow + row);
+      if (128 + row < piece.len) sc_b = __ldg(srow + 128 + row);
     };
-    fetch_scales(u0);
+    fetch_scales();
     pdl_wait();   // everything else this role reads, or writes, belongs after the previous kernel
-    int run = 0;
-    for (int u = u0; u < u1; ++run) {
-      const int tile = u / p.kb, c0 = u - tile * p.kb;
-      const int len = min(p.kb - c0, u1 - u);
+    int run = 0, blk0 = 0;
+    for (; more; ++run) {
+      const int tile = piece.tile, c0 = piece.c0, len = piece.len;
       const int m = (tile / p.n_tiles) * 2 + group, n = tile % p.n_tiles;
       const int rows = min(PAIR_TOK, p.T - n * PAIR_TOK) - rank * ROWS;       // tokens of this CTA (0 and less: none)
       const bool busy = (warp & 3) * 32 < rows && m < p.m_tiles;
@@ -250,14 +261,15 @@ gemm_fp8_pair_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_const
       sc_run[row] = sc_a;
       sc_run[128 + row] = sc_b;
       epi_sync();
-      fetch_scales(u + len);
+      more = piece.next();
+      fetch_scales();
       f2 acc[BM / 2];
 #pragma unroll
       for (int i = 0; i < BM / 2; ++i) acc[i] = 0;
       bool ok = true;
       const float lim = row < rows ? 0.f : -INFINITY;      // scales of tokens past the last one are undefined
       for (int c = 0; c < len; ++c) {
-        const int blk = u - u0 + c, b = blk % S, a = blk % A;
+        const int blk = blk0 + c, b = blk % S, a = blk % A;
         const float sw = c < RUN ? sc_run[c] : __ldg(srow + c);
         ok = mbar_wait(&sx_full[b], (blk / S) & 1) && mbar_wait(&done[b], (blk / S) & 1);
         ok = __all_sync(0xffffffffu, ok);
@@ -302,13 +314,15 @@ gemm_fp8_pair_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_const
       if (*epi_abort) break;
       const bool mine = busy && row < rows;
       // values outside the terms are added to the partial sums, so a tile that has some goes that way even if it is whole
-      const bool outside = *last_outside >= u - u0;
+      const bool outside = *last_outside >= blk0;
       bool store = len == p.kb && !outside;
       if (!store) {
         // ---- a cut tile: leave the partial sums; the last contributor adds them in K order
-        const int i0 = p.owner(tile * p.kb), i1 = p.owner(tile * p.kb + p.kb - 1);
+        const int tt = tile - p.tail();
+        const bool cut = len != p.kb;
+        const int i0 = cut ? p.owner(tt * p.kb) : worker, i1 = cut ? p.owner(tt * p.kb + p.kb - 1) : worker;
         auto part = [&](int i) {     // [4 features][token]
-          return p.partial + (((size_t)i * 2 + p.place(i, tile)) * 2 + rank) * PART + (size_t)group * (ROWS * BM) + row * 4;
+          return p.partial + (((size_t)i * 2 + p.place(i, tt)) * 2 + rank) * PART + (size_t)group * (ROWS * BM) + row * 4;
         };
         if (mine) {
           float* dst = part(worker);
@@ -323,11 +337,10 @@ gemm_fp8_pair_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_const
         if (busy) __threadfence();
         epi_sync();
         if (threadIdx.x == 0) {
-          // (a whole tile has no counter: that of this worker counts for its last tile, if that is cut)
           int* cnt = p.counters + i0 * 2 + rank;
-          const int prev = len == p.kb ? 0 : atomicAdd(cnt, 1);
+          const int prev = cut ? atomicAdd(cnt, 1) : 0;
           *fix_last = prev == i1 - i0;
-          if (len != p.kb && prev == i1 - i0) *cnt = 0;
+          if (cut && prev == i1 - i0) *cnt = 0;
         }
         epi_sync();
         store = *fix_last != 0;
@@ -387,7 +400,7 @@ gemm_fp8_pair_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_const
             if (j < left) p.out[off + j] = __float2bfloat16(at(acc, j) + (p.residual ? __bfloat162float(p.residual[off + j]) : 0.f));
         }
       }
-      u += len;
+      blk0 += len;
     }
   }
 

@@ -700,8 +700,11 @@ int b200_gemm_fp8_terms(const void* W, const float* scales, const void* xq, cons
   p.n_tiles = (T + tok - 1) / tok;
   const long long units = (long long)((p.m_tiles + cg - 1) / cg) * p.n_tiles * p.kb;
   if (units > 0x7fffffff) return -ERR_BAD_ARG;
-  p.units = (int)units;
-  p.workers = f8t::workers(p.units / p.kb, p.kb, cg);
+  const int tiles = (int)(units / p.kb);
+  p.workers = f8t::workers(tiles, p.kb, cg);
+  // one CTA: one token tile, so tiles share nothing but the rows
+  p.waves = cg == 1 || tiles <= p.workers ? 0 : tiles % p.workers ? tiles / p.workers - 1 : tiles / p.workers;
+  p.units = (tiles - p.waves * p.workers) * p.kb;
   p.w = reinterpret_cast<const uint8_t*>(W);
   p.scales = scales;
   p.xq = reinterpret_cast<const uint8_t*>(xq);
