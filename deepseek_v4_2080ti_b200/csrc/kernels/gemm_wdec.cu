@@ -352,6 +352,35 @@ extern "C" int b200_gemm_bf16_glu(const void* W, const void* X, void* out_bf16, 
   return b200_gemm_bf16_2cta_glu(W, X, out_bf16, T, N, K, GluShape{limit, slope}, status, stream);
 }
 
+// out = sum of the splits in order, fp32; four values a thread.
+static __global__ void splitk_sum_kernel(const float* __restrict__ part, int splits, size_t n, float* __restrict__ out) {
+  b200::pdl_grid_trigger();
+  b200::pdl_grid_wait();
+  const size_t i = ((size_t)blockIdx.x * blockDim.x + threadIdx.x) * 4;
+  if (i + 4 <= n) {
+    float4 a = make_float4(0.f, 0.f, 0.f, 0.f);
+    for (int s = 0; s < splits; ++s) {
+      const float* p = part + (size_t)s * n + i;
+      float4 v;
+      if (n % 4 == 0) v = *reinterpret_cast<const float4*>(p);
+      else v = make_float4(p[0], p[1], p[2], p[3]);
+      a.x += v.x; a.y += v.y; a.z += v.z; a.w += v.w;
+    }
+    out[i] = a.x; out[i + 1] = a.y; out[i + 2] = a.z; out[i + 3] = a.w;
+  } else {
+    for (size_t j = i; j < n; ++j) {
+      float a = 0.f;
+      for (int s = 0; s < splits; ++s) a += part[(size_t)s * n + j];
+      out[j] = a;
+    }
+  }
+}
+extern "C" int b200_splitk_sum(const float* part, int splits, long long n, float* out, cudaStream_t stream) {
+  if (!part || !out || splits <= 0 || n <= 0 || reinterpret_cast<uintptr_t>(part) % 16) return -ERR_BAD_ARG;
+  const size_t blocks = ((size_t)n + 1023) / 1024;
+  return (int)launch_pdl(splitk_sum_kernel, dim3((unsigned)blocks), dim3(256), 0, stream, part, splits, (size_t)n, out);
+}
+
 extern "C" int b200_splitk_reduce(const float* part, int splits, long long n, const void* residual,
                                   void* out_bf16, cudaStream_t stream) {
   const int threads = 256;

@@ -20,6 +20,7 @@ int b200_gemm_wdec(int wfmt, const void* W, const float* scales, const void* X, 
 int b200_gemm_wdec_ex(int wfmt, const void* W, const float* scales, const void* X, void* out_bf16,
                       float* out_f32, const void* residual, int T, int N, int K, int splits,
                       int* tile_counters, int* status, cudaStream_t stream);
+int b200_splitk_sum(const float* part, int splits, long long n, float* out, cudaStream_t stream);
 int b200_splitk_reduce(const float* part, int splits, long long n, const void* residual,
                        void* out_bf16, cudaStream_t stream);
 
@@ -48,6 +49,8 @@ int b200_gdn_ab_gates(const void* x, int H, const void* w, const float* a_log, c
 // ---- prompt portions of the hybrid decoder (qwen_rows.cu, which declares the structures)
 int b200_portion_meta(const int* block_row, int past, int T, int block_size, int* pos, int* kv_slots, int* meta, long long* last_row,
                       cudaStream_t stream);
+int b200_step_meta(const int* rows, int B, const int* ids, const int* tables, int max_blocks, int* o_ids, int* pos, int* kv_len, int* slots,
+                   int* kv_slots, int* bt, cudaStream_t stream);
 
 // ---- fused decode-step kernels (decode_fused.cu)
 int b200_gdn_decode_fused(const void* proj, int ldp, const void* x, int hidden, const void* w_ab, const float* a_log,

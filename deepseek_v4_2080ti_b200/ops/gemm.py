@@ -22,6 +22,7 @@ from . import _lib
 WF_BF16 = 0
 WF_FP8_B128 = 1
 NUM_SMS = 148
+_ll = ctypes.c_longlong
 
 
 def prepack_fp8(w: torch.Tensor) -> torch.Tensor:
@@ -286,6 +287,25 @@ def pick_splits(t: int, n: int, k: int) -> int:
     return best
 
 
+def pick_splits_f32(t: int, n: int, k: int) -> int:
+    """Splits of K for an fp32 product of bf16 weights (output heads): where the feature tiles leave a wave of SMs nearly empty.  Walking
+    64 inputs of a tile takes an SM 0.26 us in a decode batch, adding up the splits 3 us, about 16 such steps, and the partial sums must
+    be few beside the weights.  18992 x 5120 is 149 tiles for 148 SMs: eight splits 31 + 3 us for 41 (1 row); 151936 x 5120, 1187 tiles,
+    takes eight, 9 waves of 80 steps for 65 of 10."""
+    tiles, kb = (n + 127) // 128, (k + 63) // 64
+    if t > 64 or tiles <= NUM_SMS:
+        return 1
+    best, best_steps = 1, (tiles + NUM_SMS - 1) // NUM_SMS * kb - 16
+    for s in range(2, min(kb // 8, k // (16 * t), 16) + 1):
+        per = (kb + s - 1) // s
+        if (kb + per - 1) // per != s:
+            continue
+        steps = (tiles * s + NUM_SMS - 1) // NUM_SMS * per
+        if steps < best_steps:
+            best, best_steps = s, steps
+    return best
+
+
 STREAM_MAX_T = 32   # token counts served by the weight-streaming FP8 kernel (csrc/kernels/gemm_w8a8s.cu)
 TERMS_SINGLE_T = 64  # token counts the one-CTA form of ``linear_terms`` serves
 
@@ -494,10 +514,18 @@ def linear(x: torch.Tensor, w: PackedLinear, residual: torch.Tensor | None = Non
             w = _expanded_bf16(w, x.device)
     if splits is None:
         splits = 1 if out_f32 else pick_splits(t, n, k)
+    f32_splits = pick_splits_f32(t, n, k) if out_f32 and w.wfmt == WF_BF16 else 1
     L = _lib.lib()
     st = _lib.status_word(x.device)
     if out_f32:
         o32 = out if out is not None else torch.empty(t, n, dtype=torch.float32, device=x.device)
+        if f32_splits > 1 and o32.is_contiguous():
+            part = torch.empty(f32_splits, t, n, dtype=torch.float32, device=x.device)
+            rc = L.b200_gemm_wdec(w.wfmt, _lib.ptr(w.weight), None, _lib.ptr(x), None, _lib.ptr(part), None, t, n, k, f32_splits, _lib.ptr(st),
+                                  _lib.stream())
+            _lib.check(rc, "gemm_wdec")
+            _lib.check(L.b200_splitk_sum(_lib.ptr(part), f32_splits, _ll(t * n), _lib.ptr(o32), _lib.stream()), "splitk_sum")
+            return o32
         rc = L.b200_gemm_wdec(w.wfmt, _lib.ptr(w.weight), _lib.ptr(w.scales), _lib.ptr(x), None,
                               _lib.ptr(o32), None, t, n, k, 1, _lib.ptr(st), _lib.stream())
         _lib.check(rc, "gemm_wdec")

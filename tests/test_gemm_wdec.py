@@ -187,3 +187,18 @@ def test_prefill_sized_batch_takes_the_expanded_path_and_matches():
     _lib.check_status()
     ref = gemm.linear_ref(x, fp8fmt.dequantize_block128(q, s)) + r.float()
     assert _rel_err(y, ref) < 1e-2 and _rel_err(y, y_small) < 5e-3
+
+
+# one tile past the SMs, and an odd number of features past that; rows to the last that is split
+@pytest.mark.gpu
+@pytest.mark.parametrize("t,n,k", [(1, 18992, 1024), (7, 18950, 2048), (33, 18947, 1600), (64, 19100, 5120), (64, 18992, 1024)])
+def test_fp32_heads_in_splits(t, n, k):
+    from deepseek_v4_2080ti_b200.ops import _lib, gemm
+    torch.manual_seed(t)
+    x, w = torch.randn(t, k, device="cuda").bfloat16(), (torch.randn(n, k, device="cuda") * 0.02).bfloat16()
+    got = gemm.linear(x, gemm.PackedLinear.from_bf16(w), out_f32=True)
+    torch.cuda.synchronize()
+    _lib.check_status()
+    assert gemm.pick_splits_f32(1, 18992, 5120) > 1 and gemm.pick_splits_f32(64, 18992, 1024) == 1
+    ref = x.double() @ w.double().t()
+    assert ((got.double() - ref).abs() <= (x.double().abs() @ w.double().abs().t()) * k * 2.0 ** -24).all()
