@@ -944,16 +944,16 @@ class QwenHybridRuntime(PagedSequences):
             entry = {"buf": self._decode_buffers(b), "graph": None, "out": None}
             self._graphs[key] = entry
         buf = entry["buf"]
-        host = torch.tensor([[st.length, st.length + 1, st.slot,
-                              st.blocks[st.length // self.block_size] * self.block_size + st.length % self.block_size]
-                             for st in sts], dtype=torch.int32)
-        dev = host.to(self.device, non_blocking=True)
-        buf["ids"].copy_(token_ids)
-        buf["pos"].copy_(dev[:, 0])
-        buf["kv_len"].copy_(dev[:, 1])
-        buf["slots"].copy_(dev[:, 2])
-        buf["kv_slots"].copy_(dev[:, 3])
-        buf["bt"].copy_(self.block_table[buf["slots"].long()])
+        rows = [v for st in sts for v in (
+            st.length, st.length + 1, st.slot,
+            st.blocks[st.length // self.block_size] * self.block_size + st.length % self.block_size)]
+        if token_ids.numel() != b:
+            token_ids = token_ids.expand(b)
+        token_ids = token_ids.to(self.device, torch.int32).contiguous()
+        rc = _lib.lib().b200_step_meta((ctypes.c_int * (4 * b))(*rows), b, _lib.ptr(token_ids), _lib.ptr(self.block_table),
+                                       self.max_blocks_per_seq, *(_lib.ptr(buf[n]) for n in ("ids", "pos", "kv_len", "slots", "kv_slots", "bt")),
+                                       _lib.stream())
+        _lib.check(rc, "step_meta", 0)
         if not use_graph:
             l0 = _lib.LAUNCHES
             out = self._decode_body(buf, bucket)

@@ -52,3 +52,21 @@ def test_portions_do_not_wait_for_the_device():
     rt.prefill(slot, ids[:33])
     assert not done.query()
     torch.cuda.synchronize()
+
+
+# rows around what one launch carries; slots in any order, contexts around page edges
+@pytest.mark.parametrize("b", [1, 3, 127, 128, 129, 300])
+def test_step_rows_reach_the_device(b):
+    import ctypes
+    from deepseek_v4_2080ti_b200.ops import _lib
+    torch.manual_seed(b)
+    rows = torch.randint(0, 5000, (b, 4), dtype=torch.int32)
+    rows[:, 2] = torch.randperm(b).int()
+    tables = torch.randint(0, 9000, (b, 37), device="cuda", dtype=torch.int32)
+    ids = torch.randint(0, 9000, (b,), device="cuda", dtype=torch.int32)
+    o = [torch.full((b,), -1, dtype=torch.int32, device="cuda") for _ in range(5)]
+    bt = torch.full((b, 37), -1, dtype=torch.int32, device="cuda")
+    host = (ctypes.c_int * (4 * b))(*rows.flatten().tolist())
+    _lib.check(_lib.lib().b200_step_meta(host, b, _lib.ptr(ids), _lib.ptr(tables), 37, *map(_lib.ptr, o), _lib.ptr(bt), _lib.stream()), "meta")
+    want = [ids.cpu(), rows[:, 0], rows[:, 1], rows[:, 2], rows[:, 3]]
+    assert all(torch.equal(a.cpu(), w) for a, w in zip(o, want)) and torch.equal(bt.cpu(), tables.cpu()[rows[:, 2].long()])
