@@ -12,7 +12,7 @@ namespace f8t {
 constexpr int BM = 128;             // features of a weight block
 constexpr int W_BYTES = BM * 128;   // one 128 x 128 block: two 64-byte-swizzled halves of 8 KB
 constexpr int RUN = 256;            // weight scales of a run of K blocks kept in shared memory
-constexpr int MAX_SINGLE = 64;      // tokens up to which one CTA per worker is used
+constexpr int MAX_SINGLE = 128;      // tokens up to which one CTA per worker is used
 constexpr int PAIR_TOK = 256;       // tokens of a pair's tile
 
 struct Params {

@@ -1,4 +1,4 @@
-// The products of gemm_fp8_terms.cu for more than 64 tokens, on CTA pairs (tcgen05.mma.cta_group::2):
+// The products of gemm_fp8_terms.cu for more than 128 tokens, on CTA pairs (tcgen05.mma.cta_group::2):
 //   Y[T, N] = X[T, K] * W[N, K]^T,  W = E4M3 with one scale per 128 x 128 block, X as two FP8 terms.
 //
 // Here the tokens are the MMA's M dimension: a pair computes 256 tokens x 256 features, each CTA its own 128 tokens, and a
@@ -7,11 +7,11 @@
 // 32 shared-memory reads of 16 bytes per block and thread, beside operand traffic that already fills shared memory (112 KB
 // per 1024 tensor cycles), doubled the time (978 against 670 us for 1920 x 34816 x 5120).
 //
-// Measured, us per product in a graph of 16 (12288 x 5120, 5120 x 4096, 34816 x 5120, 5120 x 17408): 128 tokens 43, 28, 85, 52; 333
-// tokens 64, 37, 159, 81; 1901 tokens 237, 83, 650 to 730, 340 to 355 (the larger ones go with the power limit).  The split of the
-// activations, 3 to 5 us at 128 tokens and 13 to 55 at 1901, is not counted.  The decode-warp kernel, which needs none, as it is
-// now: 128 tokens 55, 44, 62, 67; 333 tokens 82, 40, 188, 138; 1901 tokens 266, 96, 790, 468.  Where it is the faster one with the
-// split counted - half of a pair's tokens are padding up to 128 - `linear` takes it (terms_pay in ops/gemm.py).
+// Measured, us per product in a graph of 16 (12288 x 5120, 5120 x 4096, 34816 x 5120, 5120 x 17408): 333
+// tokens 64, 37, 155, 81; 1901 tokens 220 to 260, 83 to 100, 575 to 605, 300 to 310 (the larger ones go with the power limit).  The split of
+// the activations, 5 us at 333 tokens and 13 to 55 at 1901, is not counted.  The decode-warp kernel, which needs none, as it is
+// now: 333 tokens 82, 40, 188, 138; 1901 tokens 266, 96, 790, 468.  Where it is the faster one with the split counted, `linear` takes it
+// (terms_pay in ops/gemm.py).
 //
 // What bounds it: with two accumulators of 256 columns (all of tensor memory) the products of a block wait for the epilogue to have
 // read the block before last; the tensor pipe is busy for 65 % of the cycles at 1901 tokens.  The epilogue's 216 registers are all

@@ -12,8 +12,8 @@
 // into the block's activation scales, and the epilogue warps add scale x block into fp32 registers, two tokens per instruction,
 // while the tensor core is on the next blocks.
 //
-// This file: up to 64 tokens, one CTA per worker, weights as the MMA's M operand; bound by the weight stream, 160 KB of it in flight
-// per SM at 16 tokens, 144 at 32, 96 at 64.  More tokens: gemm_fp8_pair.cu.
+// This file: up to 128 tokens, one CTA per worker, weights as the MMA's M operand; bound by the weight stream, 160 KB of it in flight
+// per SM at 16 tokens, 144 at 32, 96 at 64, 64 at 128.  More tokens: gemm_fp8_pair.cu.
 //
 // Work: the (tile, K block) pairs are one list, cut into equal contiguous runs, one per worker, so no wave is partly empty
 // whatever N and K are.  A tile that is cut is finished by whichever contributor arrives last, which adds the fp32 partial
@@ -25,7 +25,13 @@
 //
 // Measured, us per product in a graph of 16, the split not counted (weights 63, 21, 178, 89 MB: 12288 x 5120, 5120 x 4096,
 // 34816 x 5120, 5120 x 17408; a plain read of as many bytes takes 9.7, 3.7, 25.3, 13.2):
-//   1 token 14.8, 9.4, 31, 19.4;  32 tokens 16.6, 10.6, 33.9, 20.5;  64 tokens 20.8, 13.5, 42.2, 26.0
+//   1 token 14.8, 9.4, 31, 19.4;  32 tokens 16.6, 10.6, 33.9, 20.5;  64 tokens 20.8, 13.5, 42.2, 26.0;
+// with the split: 65 tokens 31.5, 19.6, 63, 42;  100 tokens 35, 21.8, 70.5, 48;  128 tokens 37, 22.8, 74, 50.7.  (On pairs, half of whose 256
+// tokens are padding then: 65 tokens 44, 28.5, 81.6, 57;  128 tokens 47.6, 31, 88, 60.)
+// Of these, about 6.5 us a product are fixed at 1 token and 8 at 64: filling the pipeline and the sums of cut tiles; above them a
+// block takes 0.354 us at 1 token, 6.85 TB/s, and 0.467 at 64.  Tried at 64 tokens and slower: more weight slots beside fewer activation
+// slots (47.8 to 50 for 45.8), slots given back by the commit and accumulators read a block ahead (54.5), two feature blocks per
+// activation block (47.0, and 21.5 for 15.3 where every tile is cut), the next blocks prefetched to L2 (1 to 8 % more).
 // The kernels this one took over from, in a chain: gemm_w8a8s.cu at 1 token 20.6, 12.0, 38.7, 29.8, at 32 tokens 47.6, 52.6,
 // 45.9, 71.8; the decode-warp kernel at 64 tokens 77.9, 83.1, 188, 111 (with the converged issue it has now 38, 41, 193, 57).
 //
@@ -290,18 +296,20 @@ gemm_fp8_terms_kernel(Params p) {
       } else if (*last_outside >= u - u0) {
         // values outside the terms, on the CUDA cores: as a rule there are none, and in a block that has them a few
         for (int c = L::BY_TOKENS ? 0 : (group ^ ((u - u0) & 1)); c < len; c += L::BY_TOKENS ? 1 : 2) {
-          const float* sx = p.sx + (size_t)(c0 + c) * TOK + w0;
-          uint32_t tokens = __ballot_sync(0xffffffffu, lane < WT && w0 + lane < w1 && __ldcg(sx + lane) < 0.f);
-          if (!tokens) continue;
           const uint8_t* wb = p.w + (size_t)(u + c) * W_BYTES;
           const float sc = __ldg(p.scales + u + c);
-          for (; tokens; tokens &= tokens - 1) {
-            const int t = __ffs(tokens) - 1;
-            float sum = 0.f;
-            for_each_outside(p.rest, p.kb, w0 + t, c0 + c,
-                             [&](int k, float x) { sum += x * (e4m3x2_to_float2(wb[w_offset(row, k)]).x * sc); });
+#pragma unroll 1
+          for (int t0 = 0; t0 < WT; t0 += 32) {
+            const float* sx = p.sx + (size_t)(c0 + c) * TOK + w0 + t0;
+            uint32_t tokens = __ballot_sync(0xffffffffu, t0 + lane < WT && w0 + t0 + lane < w1 && __ldcg(sx + lane) < 0.f);
+            for (; tokens; tokens &= tokens - 1) {
+              const int t = t0 + __ffs(tokens) - 1;
+              float sum = 0.f;
+              for_each_outside(p.rest, p.kb, w0 + t, c0 + c,
+                               [&](int k, float x) { sum += x * (e4m3x2_to_float2(wb[w_offset(row, k)]).x * sc); });
 #pragma unroll
-            for (int i = 0; i < WT / 2; ++i) acc[i] = add2(acc[i], pack2f(t == 2 * i ? sum : 0.f, t == 2 * i + 1 ? sum : 0.f));
+              for (int i = 0; i < WT / 2; ++i) acc[i] = add2(acc[i], pack2f(t == 2 * i ? sum : 0.f, t == 2 * i + 1 ? sum : 0.f));
+            }
           }
         }
       }
@@ -609,7 +617,7 @@ static int workers(int tiles, int kb, int cg) {
 }
 
 // Tokens of a tile for T tokens.
-static int tile_tokens(int T) { return T <= 16 ? 16 : T <= 32 ? 32 : T <= MAX_SINGLE ? 64 : PAIR_TOK; }
+static int tile_tokens(int T) { return T <= 16 ? 16 : T <= 32 ? 32 : T <= 64 ? 64 : T <= MAX_SINGLE ? MAX_SINGLE : PAIR_TOK; }
 
 }  // namespace f8t
 }  // namespace b200
@@ -719,7 +727,8 @@ int b200_gemm_fp8_terms(const void* W, const float* scales, const void* xq, cons
   if (cg == 2) return gemm_fp8_pair_launch(p, stream);
   if (tok == 16) return f8t::launch<16>(p, stream);
   if (tok == 32) return f8t::launch<32>(p, stream);
-  return f8t::launch<64>(p, stream);
+  if (tok == 64) return f8t::launch<64>(p, stream);
+  return f8t::launch<f8t::MAX_SINGLE>(p, stream);
 }
 
 }  // extern "C"

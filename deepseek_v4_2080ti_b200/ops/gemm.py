@@ -454,9 +454,8 @@ def terms_pay(t: int, n: int, k: int) -> bool:
 
     * up to 64 tokens: yes (5120 x 4096 9.6 for 14.4 of the decode-warp kernel at 1 token, 15 for 41 at 64; 34816 x 5120 33 for
       62, 45 for 193; 576 x 7168 9.4 for 12, 15 for 37).
-    * up to 128: yes where the decode-warp kernel must split K to fill the SMs (12288 x 5120 47 for 55 at 128, 5120 x 17408 58 for
-      67), no where its 128-token tiles fill them (14336 x 5120 50 for 34, 34816 x 5120 87 for 62): half of a pair's 256 tokens is
-      padding then.
+    * up to 128: yes where the decode-warp kernel must split K to fill the SMs (12288 x 5120 37 for 55 at 128, 5120 x 17408 51 for
+      67), no where its 128-token tiles fill them (34816 x 5120 63 for 59 at 65, 74 for 62 at 128).
     * above, the decode-warp kernel walks a 256-token tile of 128 features in 1.03 us per 128 inputs, wave after wave; the pairs share
       the tiles evenly, about 1 us per 128 inputs of two, but pay 18 us for tiles that are cut, and for the split.  By that: 7168 x
       2048 at 257 tokens 34 for 27, 5120 x 4096 at 700 50 for 41, 12288 x 5120 at 700 101 for 92 go to the decode warps, 5120 x
