@@ -55,86 +55,83 @@ struct GdnDecodeParams {
   __nv_bfloat16* out;          // [B, Hv*128]
   int Hv, Hk;
   float eps, q_scale;
+  bool vec;                    // rows, tails and the small weights lie on 16-byte boundaries
   b200::f8t::TermsOut terms;   // where the result goes as FP8 terms (xq set) instead of `out`: a head is one block of 128
 };
 
-// One channel of the causal convolution: the tail's values and the new one.
-template <int KW>
-struct ConvStep {
-  float v[KW];
-  __device__ __forceinline__ void load(const __nv_bfloat16* tail, int C, int c, __nv_bfloat16 cur) {
+// 128 bf16 values on their way to shared memory, 8 a thread; `vec`: 16 bytes at a time (cp.async), else one by one.
+__device__ __forceinline__ void copy8(__nv_bfloat16* dst, const __nv_bfloat16* src, bool vec) {
+  if (vec) {
+    asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"((uint32_t)__cvta_generic_to_shared(dst)), "l"(src) : "memory");
+  } else {
 #pragma unroll
-    for (int k = 0; k < KW - 1; ++k) v[k] = __bfloat162float(tail[(size_t)k * C + c]);
-    v[KW - 1] = __bfloat162float(cur);
+    for (int i = 0; i < 8; ++i) dst[i] = src[i];
   }
-  // y = silu(sum_k w[c][k] * v[k]), rounded as the unfused path stores it
-  __device__ __forceinline__ float result(const __nv_bfloat16* w, int c) const {
-    float acc = v[KW - 1] * __bfloat162float(w[(size_t)c * KW + KW - 1]);
-#pragma unroll
-    for (int k = 0; k < KW - 1; ++k) acc += v[k] * __bfloat162float(w[(size_t)c * KW + k]);
-    return bf16_round(silu_f(acc));
-  }
-  __device__ __forceinline__ void store(__nv_bfloat16* tail, int C, int c) const {
-#pragma unroll
-    for (int k = 0; k < KW - 1; ++k) tail[(size_t)k * C + c] = __float2bfloat16(v[k + 1]);
-  }
-};
+}
 
 // grid (Hv, B), clusters of the R = Hv / Hk value heads that share a key head; block = 128 * RG threads.  Thread (rg, j) owns
 // rows [rg*128/RG, (rg+1)*128/RG) of column j of the head's state; the row groups cut the serial length of the recurrence per
 // thread, their partial dot products meet in shared memory.
 //
-// The state, 64 KB in and out per head, is asked for first and arrives while the projections, the convolution and the gates are
-// computed; a block holds one head and two blocks fit an SM, which leaves 64 registers a thread: 52 bytes of the state's 32 values
-// and the convolution's are spilled.  At 32 rows of 32 heads that takes 41 to 42 us, where the bytes take 20; what the rest goes
-// on has not been measured.  (All heads of a key head in one block of 1024 threads, one block per
-// SM, the state loaded last: 45.6.  Four columns per thread, 16 bytes per load: 46.6.  Weights fetched before the wait for the
-// previous kernel: 48.4.  One row takes 14 us in every form.)
+// What a step costs beside the state's 64 KB in and out per head is a chain of loads and barriers, so everything small - the
+// projection's row, the convolution's tails and weights, the norm's weight - is asked for at once, straight to shared memory, and so is the
+// state, whose 32 values a thread then fit the 64 registers that two blocks per SM leave.  A few rows ask L2 for
+// the a / b weights even before the previous kernel has ended.  XXMEASURED
 // Every block convolves the q and k channels of its key head itself; the first of the cluster moves their tail on when all of
 // them have read it.
 template <int KW, int R, int RG>
 __global__ void __launch_bounds__(128 * RG, 2)
 gdn_decode_fused_kernel(GdnDecodeParams p) {
+  static_assert(KW == 4, "three rows of tail");
   constexpr int ROWS = DK / RG;
   constexpr int WARPS = 4 * RG;
   __shared__ float sq[DK], sk[DK], s_v[DV];
-  __shared__ __align__(16) float s_part[RG][DV];
+  __shared__ __align__(16) float s_part[2][RG][DV];
   __shared__ float red_ab[WARPS][2];
   __shared__ float red_qk[8];
   __shared__ float red_o[4];
   __shared__ float s_gate[2];
+  __shared__ __align__(16) __nv_bfloat16 s_row[4][128], s_tail[3][KW - 1][128], s_cw[3][128 * KW], s_gamma[128];   // q, k, v (, z)
+  const int h = blockIdx.x, b = blockIdx.y, kh = h / R, tid = threadIdx.x;
+  const int j = tid & 127, rg = tid >> 7;
+  const int kd = p.Hk * DK, vd = p.Hv * DV, C = 2 * kd + vd;
+  const int chan[3] = {kh * DK, kd + kh * DK, 2 * kd + h * DV};
   b200::pdl_grid_trigger();
+  // constants do not wait for the previous kernel
+  if (tid < 3 * 64) copy8(s_cw[tid >> 6] + (tid & 63) * 8, p.conv_w + (size_t)chan[tid >> 6] * KW + (tid & 63) * 8, p.vec);
+  else if (tid < 3 * 64 + 16) copy8(s_gamma + (tid - 3 * 64) * 8, p.gamma + (tid - 3 * 64) * 8, p.vec);
+  float a_log = 0.f, dt_bias = 0.f;
+  if (tid == 128) {
+    a_log = p.a_log[h];
+    dt_bias = p.dt_bias[h];
+  }
+  const __nv_bfloat16* wa = p.w_ab + (size_t)h * p.hidden;
+  const __nv_bfloat16* wb = p.w_ab + (size_t)(p.Hv + h) * p.hidden;
+  if (gridDim.y <= 4) {
+    for (int i = tid * 64; i < p.hidden; i += 128 * RG * 64) {
+      asm volatile("prefetch.global.L2 [%0];" ::"l"(wa + i));
+      asm volatile("prefetch.global.L2 [%0];" ::"l"(wb + i));
+    }
+  }
   b200::pdl_grid_wait();
   p.terms.zero_counters(blockIdx.x == 0 && blockIdx.y == 0);
-  const int h = blockIdx.x, b = blockIdx.y, kh = h / R;
-  const int j = threadIdx.x & 127, rg = threadIdx.x >> 7;
-  const int kd = p.Hk * DK, vd = p.Hv * DV, C = 2 * kd + vd;
   const int slot = p.slot_ids ? p.slot_ids[b] : b;
   __nv_bfloat16* tail = p.tails + (size_t)slot * p.tail_stride;
   const __nv_bfloat16* row = p.proj + (size_t)b * p.ldp;
-
   float* S = p.states + (size_t)slot * p.state_stride + (size_t)h * DK * DV + (size_t)rg * ROWS * DV;
   float col[ROWS];
 #pragma unroll
   for (int i = 0; i < ROWS; ++i) col[i] = S[(size_t)i * DV + j];
-
-  // ---- convolution (row group 0)
-  const int cq = kh * DK + j, ck = kd + kh * DK + j, cv = 2 * kd + h * DV + j;
-  ConvStep<KW> tq, tk, tv;
-  if (rg == 0) {
-    tq.load(tail, C, cq, row[cq]);
-    tk.load(tail, C, ck, row[ck]);
-    tv.load(tail, C, cv, row[cv]);
+  {
+    const int part = tid >> 4, i = (tid & 15) * 8;          // 13 pieces of 128 values: the row's four, the tails' nine
+    if (part < 4) copy8(s_row[part] + i, row + (part < 3 ? chan[part] : C + h * DV) + i, p.vec);
+    else if (part < 13) copy8(s_tail[(part - 4) / 3][(part - 4) % 3] + i, tail + (size_t)((part - 4) % 3) * C + chan[(part - 4) / 3] + i, p.vec);
   }
-  if constexpr (R > 1) asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory");
-
   // ---- a/b projections of this value head: two dot products of length hidden
   {
     const __nv_bfloat16* xr = p.x + (size_t)b * p.hidden;
-    const __nv_bfloat16* wa = p.w_ab + (size_t)h * p.hidden;
-    const __nv_bfloat16* wb = p.w_ab + (size_t)(p.Hv + h) * p.hidden;
     float da = 0.f, db = 0.f;
-    for (int i = (int)threadIdx.x * 8; i < p.hidden; i += 128 * RG * 8) {
+    for (int i = tid * 8; i < p.hidden; i += 128 * RG * 8) {
       const uint4 xv = *reinterpret_cast<const uint4*>(xr + i);
       const uint4 av = *reinterpret_cast<const uint4*>(wa + i);
       const uint4 bv = *reinterpret_cast<const uint4*>(wb + i);
@@ -151,24 +148,36 @@ gdn_decode_fused_kernel(GdnDecodeParams p) {
     da = warp_sum(da);
     db = warp_sum(db);
     if ((j & 31) == 0) {
-      red_ab[threadIdx.x >> 5][0] = da;
-      red_ab[threadIdx.x >> 5][1] = db;
+      red_ab[tid >> 5][0] = da;
+      red_ab[tid >> 5][1] = db;
     }
   }
+  if (p.vec) asm volatile("cp.async.wait_all;" ::: "memory");
+  __syncthreads();
+  if constexpr (R > 1) asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory");   // this block has read its tails
   float qv = 0.f, kv = 0.f;
   if (rg == 0) {
-    qv = tq.result(p.conv_w, cq);
-    kv = tk.result(p.conv_w, ck);
-    s_v[j] = tv.result(p.conv_w, cv);
-    tv.store(tail, C, cv);
+    // y = silu(sum_k w[c][k] * v[k]), rounded as the unfused path stores it
+    auto conv = [&](int c) {
+      float acc = __bfloat162float(s_row[c][j]) * __bfloat162float(s_cw[c][j * KW + KW - 1]);
+#pragma unroll
+      for (int k = 0; k < KW - 1; ++k) acc += __bfloat162float(s_tail[c][k][j]) * __bfloat162float(s_cw[c][j * KW + k]);
+      return bf16_round(silu_f(acc));
+    };
+    qv = conv(0);
+    kv = conv(1);
+    s_v[j] = conv(2);
     const float qs = warp_sum(qv * qv), ks = warp_sum(kv * kv);
     if ((j & 31) == 0) {
       red_qk[j >> 5] = qs;
       red_qk[4 + (j >> 5)] = ks;
     }
-  }
-  __syncthreads();
-  if (threadIdx.x == 0) {
+    asm volatile("bar.sync 1, 128;" ::: "memory");
+    const float qn = rsqrtf(red_qk[0] + red_qk[1] + red_qk[2] + red_qk[3] + 1e-6f);
+    const float kn = rsqrtf(red_qk[4] + red_qk[5] + red_qk[6] + red_qk[7] + 1e-6f);
+    sq[j] = qv * qn * p.q_scale;
+    sk[j] = kv * kn;
+  } else if (tid == 128) {
     float a = 0.f, bb = 0.f;
 #pragma unroll
     for (int w = 0; w < WARPS; ++w) {
@@ -178,16 +187,14 @@ gdn_decode_fused_kernel(GdnDecodeParams p) {
     // the unfused path rounds the a/b projection outputs to bf16 before the gate math
     a = bf16_round(a);
     bb = bf16_round(bb);
-    const float av = a + p.dt_bias[h];
+    const float av = a + dt_bias;
     const float sp = av > 20.f ? av : log1pf(expf(av));
-    s_gate[0] = __expf(-expf(p.a_log[h]) * sp);   // decay = exp(g)
+    s_gate[0] = __expf(-expf(a_log) * sp);   // decay = exp(g)
     s_gate[1] = sigmoid_f(bb);
-  }
-  if (rg == 0) {
-    const float qn = rsqrtf(red_qk[0] + red_qk[1] + red_qk[2] + red_qk[3] + 1e-6f);
-    const float kn = rsqrtf(red_qk[4] + red_qk[5] + red_qk[6] + red_qk[7] + 1e-6f);
-    sq[j] = qv * qn * p.q_scale;
-    sk[j] = kv * kn;
+  } else if (rg == RG - 1) {
+    // the value channels' tail, this block's own, moves on
+#pragma unroll
+    for (int k = 0; k < KW - 1; ++k) tail[(size_t)k * C + chan[2] + j] = k + 1 < KW - 1 ? s_tail[2][k + 1][j] : s_row[2][j];
   }
   __syncthreads();
   // ---- gated delta rule on rows [rg*ROWS, (rg+1)*ROWS) of state column j
@@ -198,13 +205,12 @@ gdn_decode_fused_kernel(GdnDecodeParams p) {
     col[i] *= decay;
     part += col[i] * sk[rg * ROWS + i];
   }
-  s_part[rg][j] = part;
+  s_part[0][rg][j] = part;
   __syncthreads();
   float kv_mem = 0.f;
 #pragma unroll
-  for (int g2 = 0; g2 < RG; ++g2) kv_mem += s_part[g2][j];
+  for (int g2 = 0; g2 < RG; ++g2) kv_mem += s_part[0][g2][j];
   const float delta = (s_v[j] - kv_mem) * bt;
-  __syncthreads();   // s_part is reused for the read-out partials
   part = 0.f;
 #pragma unroll
   for (int i = 0; i < ROWS; ++i) {
@@ -212,33 +218,35 @@ gdn_decode_fused_kernel(GdnDecodeParams p) {
     S[(size_t)i * DV + j] = col[i];
     part += col[i] * sq[rg * ROWS + i];
   }
-  s_part[rg][j] = part;
+  s_part[1][rg][j] = part;
   if constexpr (R > 1) asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");   // every head has read the q and k tails
-  if (rg == 0 && h % R == 0) {
-    tq.store(tail, C, cq);
-    tk.store(tail, C, ck);
+  if (rg == RG - 1 && h % R == 0) {
+#pragma unroll
+    for (int c = 0; c < 2; ++c)
+#pragma unroll
+      for (int k = 0; k < KW - 1; ++k) tail[(size_t)k * C + chan[c] + j] = k + 1 < KW - 1 ? s_tail[c][k + 1][j] : s_row[c][j];
   }
   __syncthreads();
   if (rg != 0) return;
   // ---- per-head gated RMSNorm by row group 0 (the unfused path stores o as bf16 first)
   float o = 0.f;
 #pragma unroll
-  for (int g2 = 0; g2 < RG; ++g2) o += s_part[g2][j];
+  for (int g2 = 0; g2 < RG; ++g2) o += s_part[1][g2][j];
   o = bf16_round(o);
   const float ss = warp_sum(o * o);
   if ((j & 31) == 0) red_o[j >> 5] = ss;
   asm volatile("bar.sync 1, 128;" ::: "memory");
   const float inv = rsqrtf((red_o[0] + red_o[1] + red_o[2] + red_o[3]) / (float)DV + p.eps);
-  const float z = __bfloat162float(row[2 * kd + vd + h * DV + j]);
-  const float y = bf16_round(o * inv * __bfloat162float(p.gamma[j]) * silu_f(z));
+  const float z = __bfloat162float(s_row[3][j]);
+  const float y = bf16_round(o * inv * __bfloat162float(s_gamma[j]) * silu_f(z));
   if (!p.terms.xq) {
     p.out[((size_t)b * p.Hv + h) * DV + j] = __float2bfloat16(y);
     return;
   }
-  s_part[0][j] = y;
+  s_part[0][0][j] = y;
   asm volatile("bar.sync 1, 128;" ::: "memory");
   if (j < 32) {
-    const float4 f = *reinterpret_cast<const float4*>(&s_part[0][j * 4]);
+    const float4 f = *reinterpret_cast<const float4*>(&s_part[0][0][j * 4]);
     const float v[4] = {f.x, f.y, f.z, f.w};
     b200::f8t::put_terms(p.terms, b, h * DV + j * 4, v, true);
   }
@@ -465,6 +473,9 @@ int b200_gdn_decode_fused(const void* proj, int ldp, const void* x, int hidden, 
   p.Hk = Hk;
   p.eps = eps;
   p.q_scale = rsqrtf((float)DK);
+  const uintptr_t all = reinterpret_cast<uintptr_t>(proj) | reinterpret_cast<uintptr_t>(conv_w) | reinterpret_cast<uintptr_t>(tails) |
+                        reinterpret_cast<uintptr_t>(gamma);
+  p.vec = all % 16 == 0 && ldp % 8 == 0 && tail_stride % 8 == 0;
   p.terms.xq = out ? nullptr : reinterpret_cast<uint8_t*>(terms_xq);
   p.terms.sx = terms_sx;
   p.terms.rest = reinterpret_cast<__nv_bfloat16*>(terms_rest);
