@@ -17,6 +17,7 @@
 #include "fp8_terms.cuh"
 #include "ops.h"
 #include "launch.h"
+#include "per_device.h"
 #include "tma_host.h"
 
 namespace {
@@ -56,6 +57,9 @@ struct GdnDecodeParams {
   int Hv, Hk;
   float eps, q_scale;
   bool vec;                    // rows, tails and the small weights lie on 16-byte boundaries
+  int B;
+  bool ahead;                  // several rows a block: dynamic shared memory for the next state, and for the a / b weights if `keep_w`
+  bool keep_w;
   b200::f8t::TermsOut terms;   // where the result goes as FP8 terms (xq set) instead of `out`: a head is one block of 128
 };
 
@@ -69,14 +73,16 @@ __device__ __forceinline__ void copy8(__nv_bfloat16* dst, const __nv_bfloat16* s
   }
 }
 
-// grid (Hv, B), clusters of the R = Hv / Hk value heads that share a key head; block = 128 * RG threads.  Thread (rg, j) owns
+// grid (Hv, row groups), clusters of the R = Hv / Hk value heads that share a key head; block = 128 * RG threads.  Thread (rg, j) owns
 // rows [rg*128/RG, (rg+1)*128/RG) of column j of the head's state; the row groups cut the serial length of the recurrence per
 // thread, their partial dot products meet in shared memory.
 //
 // What a step costs beside the state's 64 KB in and out per head is a chain of loads and barriers, so everything small - the
-// projection's row, the convolution's tails and weights, the norm's weight - is asked for at once, straight to shared memory, and so is the
-// state, whose 32 values a thread then fit the 64 registers that two blocks per SM leave.  A few rows ask L2 for
-// the a / b weights even before the previous kernel has ended.  XXMEASURED
+// projection's row, the convolution's tails and weights, the norm's weight - is asked for at once, straight to shared memory.  Two blocks
+// fit an SM; with more rows than these hold a block walks several rows of its head, the constants stay, and the next row's state
+// and small inputs are on their way while one is computed.  A few rows ask L2 for the a / b weights even before the previous kernel has
+// ended.  us a layer of 32 heads: 1 row 11.4, 16 rows 19, 32 rows 34.5, 64 rows 68 (the state's bytes take 0.7, 10, 21, 42); with each input
+// loaded where it is used and a row per block 13.7, 25, 43, 85.
 // Every block convolves the q and k channels of its key head itself; the first of the cluster moves their tail on when all of
 // them have read it.
 template <int KW, int R, int RG>
@@ -85,20 +91,24 @@ gdn_decode_fused_kernel(GdnDecodeParams p) {
   static_assert(KW == 4, "three rows of tail");
   constexpr int ROWS = DK / RG;
   constexpr int WARPS = 4 * RG;
-  __shared__ float sq[DK], sk[DK], s_v[DV];
+  __shared__ __align__(16) float sq[DK], sk[DK], s_v[DV];
   __shared__ __align__(16) float s_part[2][RG][DV];
   __shared__ float red_ab[WARPS][2];
   __shared__ float red_qk[8];
   __shared__ float red_o[4];
   __shared__ float s_gate[2];
-  __shared__ __align__(16) __nv_bfloat16 s_row[4][128], s_tail[3][KW - 1][128], s_cw[3][128 * KW], s_gamma[128];   // q, k, v (, z)
-  const int h = blockIdx.x, b = blockIdx.y, kh = h / R, tid = threadIdx.x;
+  __shared__ __align__(16) __nv_bfloat16 s_rows[2][4][128], s_tails[2][3][KW - 1][128], s_cw[3][128 * KW], s_gamma[128];   // q, k, v (, z)
+  __shared__ uint64_t s_bar;
+  extern __shared__ __align__(128) uint8_t dyn[];
+  float* s_state = reinterpret_cast<float*>(dyn);
+  __nv_bfloat16* s_w = reinterpret_cast<__nv_bfloat16*>(dyn + DK * DV * 4);
+  const int h = blockIdx.x, kh = h / R, tid = threadIdx.x;
   const int j = tid & 127, rg = tid >> 7;
   const int kd = p.Hk * DK, vd = p.Hv * DV, C = 2 * kd + vd;
-  const int chan[3] = {kh * DK, kd + kh * DK, 2 * kd + h * DV};
+  auto chan = [&](int c) { return c == 0 ? kh * DK : c == 1 ? kd + kh * DK : 2 * kd + h * DV; };
   b200::pdl_grid_trigger();
   // constants do not wait for the previous kernel
-  if (tid < 3 * 64) copy8(s_cw[tid >> 6] + (tid & 63) * 8, p.conv_w + (size_t)chan[tid >> 6] * KW + (tid & 63) * 8, p.vec);
+  if (tid < 3 * 64) copy8(s_cw[tid >> 6] + (tid & 63) * 8, p.conv_w + (size_t)chan(tid >> 6) * KW + (tid & 63) * 8, p.vec);
   else if (tid < 3 * 64 + 16) copy8(s_gamma + (tid - 3 * 64) * 8, p.gamma + (tid - 3 * 64) * 8, p.vec);
   float a_log = 0.f, dt_bias = 0.f;
   if (tid == 128) {
@@ -107,32 +117,68 @@ gdn_decode_fused_kernel(GdnDecodeParams p) {
   }
   const __nv_bfloat16* wa = p.w_ab + (size_t)h * p.hidden;
   const __nv_bfloat16* wb = p.w_ab + (size_t)(p.Hv + h) * p.hidden;
-  if (gridDim.y <= 4) {
+  if (p.keep_w) {
+    for (int i = tid * 8; i < p.hidden; i += 128 * RG * 8) {
+      copy8(s_w + i, wa + i, true);
+      copy8(s_w + p.hidden + i, wb + i, true);
+    }
+    wa = s_w;
+    wb = s_w + p.hidden;
+  } else if (gridDim.y <= 4) {
     for (int i = tid * 64; i < p.hidden; i += 128 * RG * 64) {
       asm volatile("prefetch.global.L2 [%0];" ::"l"(wa + i));
       asm volatile("prefetch.global.L2 [%0];" ::"l"(wb + i));
     }
   }
+  if (p.ahead && tid == 0) {
+    b200::mbar_init(&s_bar, 1);
+    b200::mbar_fence_init();
+  }
   b200::pdl_grid_wait();
   p.terms.zero_counters(blockIdx.x == 0 && blockIdx.y == 0);
-  const int slot = p.slot_ids ? p.slot_ids[b] : b;
+  auto slot_of = [&](int b) { return p.slot_ids ? p.slot_ids[b] : b; };
+  auto ask = [&](int b, int slot, int buf) {                // 13 pieces of 128 values: the row's four, the tails' nine
+    const __nv_bfloat16* row = p.proj + (size_t)b * p.ldp;
+    const __nv_bfloat16* tail = p.tails + (size_t)slot * p.tail_stride;
+    const int part = tid >> 4, i = (tid & 15) * 8;
+    if (part < 4) {
+      copy8(s_rows[buf][part] + i, row + (part < 3 ? chan(part) : C + h * DV) + i, p.vec);
+    } else if (part < 13) {
+      const int c = (part - 4) / 3, k = (part - 4) % 3;
+      copy8(s_tails[buf][c][k] + i, tail + (size_t)k * C + chan(c) + i, p.vec);
+    }
+  };
+  int slot = slot_of(blockIdx.y);
+  ask(blockIdx.y, slot, 0);
+  for (int b = blockIdx.y, round = 0; b < p.B; b += gridDim.y, ++round) {
+  const int buf = round & 1, nb = b + gridDim.y;
+  const int next_slot = nb < p.B ? slot_of(nb) : 0;
   __nv_bfloat16* tail = p.tails + (size_t)slot * p.tail_stride;
-  const __nv_bfloat16* row = p.proj + (size_t)b * p.ldp;
+  const auto& s_row = s_rows[buf];
+  const auto& s_tail = s_tails[buf];
   float* S = p.states + (size_t)slot * p.state_stride + (size_t)h * DK * DV + (size_t)rg * ROWS * DV;
+  const __nv_bfloat16* xr = p.x + (size_t)b * p.hidden;
+  uint4 xv = make_uint4(0, 0, 0, 0), xw = xv;              // the first two pieces of the row, asked for before the state is waited for
+  if (tid * 8 < p.hidden) xv = *reinterpret_cast<const uint4*>(xr + tid * 8);
+  if (tid * 8 + 128 * RG * 8 < p.hidden) xw = *reinterpret_cast<const uint4*>(xr + tid * 8 + 128 * RG * 8);
   float col[ROWS];
+  if (round > 0 && b200::mbar_wait(&s_bar, (round - 1) & 1)) {
 #pragma unroll
-  for (int i = 0; i < ROWS; ++i) col[i] = S[(size_t)i * DV + j];
-  {
-    const int part = tid >> 4, i = (tid & 15) * 8;          // 13 pieces of 128 values: the row's four, the tails' nine
-    if (part < 4) copy8(s_row[part] + i, row + (part < 3 ? chan[part] : C + h * DV) + i, p.vec);
-    else if (part < 13) copy8(s_tail[(part - 4) / 3][(part - 4) % 3] + i, tail + (size_t)((part - 4) % 3) * C + chan[(part - 4) / 3] + i, p.vec);
+    for (int i = 0; i < ROWS; ++i) col[i] = s_state[(rg * ROWS + i) * DV + j];
+  } else {
+#pragma unroll
+    for (int i = 0; i < ROWS; ++i) col[i] = S[(size_t)i * DV + j];
   }
+  if (round == 0 && p.keep_w) {          // the a / b weights are read before the first barrier below
+    asm volatile("cp.async.wait_all;" ::: "memory");
+    __syncthreads();
+  }
+
   // ---- a/b projections of this value head: two dot products of length hidden
   {
-    const __nv_bfloat16* xr = p.x + (size_t)b * p.hidden;
     float da = 0.f, db = 0.f;
     for (int i = tid * 8; i < p.hidden; i += 128 * RG * 8) {
-      const uint4 xv = *reinterpret_cast<const uint4*>(xr + i);
+      if (i >= 2 * 128 * RG * 8) xv = *reinterpret_cast<const uint4*>(xr + i);
       const uint4 av = *reinterpret_cast<const uint4*>(wa + i);
       const uint4 bv = *reinterpret_cast<const uint4*>(wb + i);
       const __nv_bfloat162* xh = reinterpret_cast<const __nv_bfloat162*>(&xv);
@@ -144,6 +190,7 @@ gdn_decode_fused_kernel(GdnDecodeParams p) {
         da += xf.x * af.x + xf.y * af.y;
         db += xf.x * bf.x + xf.y * bf.y;
       }
+      xv = xw;
     }
     da = warp_sum(da);
     db = warp_sum(db);
@@ -154,6 +201,14 @@ gdn_decode_fused_kernel(GdnDecodeParams p) {
   }
   if (p.vec) asm volatile("cp.async.wait_all;" ::: "memory");
   __syncthreads();
+  if (nb < p.B) {
+    if (tid == 0) {
+      b200::fence_proxy_async_smem();    // every thread has its share of this state
+      b200::mbar_expect_tx(&s_bar, DK * DV * 4);
+      b200::bulk_load(s_state, p.states + (size_t)next_slot * p.state_stride + (size_t)h * DK * DV, DK * DV * 4, &s_bar);
+    }
+    ask(nb, next_slot, buf ^ 1);
+  }
   if constexpr (R > 1) asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory");   // this block has read its tails
   float qv = 0.f, kv = 0.f;
   if (rg == 0) {
@@ -194,16 +249,21 @@ gdn_decode_fused_kernel(GdnDecodeParams p) {
   } else if (rg == RG - 1) {
     // the value channels' tail, this block's own, moves on
 #pragma unroll
-    for (int k = 0; k < KW - 1; ++k) tail[(size_t)k * C + chan[2] + j] = k + 1 < KW - 1 ? s_tail[2][k + 1][j] : s_row[2][j];
+    for (int k = 0; k < KW - 1; ++k) tail[(size_t)k * C + chan(2) + j] = k + 1 < KW - 1 ? s_tail[2][k + 1][j] : s_row[2][j];
   }
   __syncthreads();
   // ---- gated delta rule on rows [rg*ROWS, (rg+1)*ROWS) of state column j
   const float decay = s_gate[0], bt = s_gate[1];
   float part = 0.f;
 #pragma unroll
-  for (int i = 0; i < ROWS; ++i) {
-    col[i] *= decay;
-    part += col[i] * sk[rg * ROWS + i];
+  for (int i = 0; i < ROWS; i += 4) {      // four keys a read: one at a time, the reads are half of what shared memory has to do
+    const float4 k4 = *reinterpret_cast<const float4*>(sk + rg * ROWS + i);
+    const float kk[4] = {k4.x, k4.y, k4.z, k4.w};
+#pragma unroll
+    for (int e = 0; e < 4; ++e) {
+      col[i + e] *= decay;
+      part += col[i + e] * kk[e];
+    }
   }
   s_part[0][rg][j] = part;
   __syncthreads();
@@ -213,10 +273,15 @@ gdn_decode_fused_kernel(GdnDecodeParams p) {
   const float delta = (s_v[j] - kv_mem) * bt;
   part = 0.f;
 #pragma unroll
-  for (int i = 0; i < ROWS; ++i) {
-    col[i] += sk[rg * ROWS + i] * delta;
-    S[(size_t)i * DV + j] = col[i];
-    part += col[i] * sq[rg * ROWS + i];
+  for (int i = 0; i < ROWS; i += 4) {
+    const float4 k4 = *reinterpret_cast<const float4*>(sk + rg * ROWS + i), q4 = *reinterpret_cast<const float4*>(sq + rg * ROWS + i);
+    const float kk[4] = {k4.x, k4.y, k4.z, k4.w}, qq[4] = {q4.x, q4.y, q4.z, q4.w};
+#pragma unroll
+    for (int e = 0; e < 4; ++e) {
+      col[i + e] += kk[e] * delta;
+      S[(size_t)(i + e) * DV + j] = col[i + e];
+      part += col[i + e] * qq[e];
+    }
   }
   s_part[1][rg][j] = part;
   if constexpr (R > 1) asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");   // every head has read the q and k tails
@@ -224,10 +289,11 @@ gdn_decode_fused_kernel(GdnDecodeParams p) {
 #pragma unroll
     for (int c = 0; c < 2; ++c)
 #pragma unroll
-      for (int k = 0; k < KW - 1; ++k) tail[(size_t)k * C + chan[c] + j] = k + 1 < KW - 1 ? s_tail[c][k + 1][j] : s_row[c][j];
+      for (int k = 0; k < KW - 1; ++k) tail[(size_t)k * C + chan(c) + j] = k + 1 < KW - 1 ? s_tail[c][k + 1][j] : s_row[c][j];
   }
   __syncthreads();
-  if (rg != 0) return;
+  slot = next_slot;
+  if (rg != 0) continue;
   // ---- per-head gated RMSNorm by row group 0 (the unfused path stores o as bf16 first)
   float o = 0.f;
 #pragma unroll
@@ -241,7 +307,7 @@ gdn_decode_fused_kernel(GdnDecodeParams p) {
   const float y = bf16_round(o * inv * __bfloat162float(s_gamma[j]) * silu_f(z));
   if (!p.terms.xq) {
     p.out[((size_t)b * p.Hv + h) * DV + j] = __float2bfloat16(y);
-    return;
+    continue;
   }
   s_part[0][0][j] = y;
   asm volatile("bar.sync 1, 128;" ::: "memory");
@@ -250,12 +316,31 @@ gdn_decode_fused_kernel(GdnDecodeParams p) {
     const float v[4] = {f.x, f.y, f.z, f.w};
     b200::f8t::put_terms(p.terms, b, h * DV + j * 4, v, true);
   }
+  }
 }
 
 template <int R>
-static int launch_gdn(const GdnDecodeParams& p, int B, cudaStream_t stream) {
+static int launch_gdn(GdnDecodeParams p, int B, cudaStream_t stream) {
+  // rows a block walks: as few as two blocks per SM allow, shared evenly
+  const bool walk = (reinterpret_cast<uintptr_t>(p.states) & 15) == 0 && p.state_stride % 4 == 0;
+  const int groups = 2 * b200::sm_count() / p.Hv, rounds = !walk || groups < 1 ? 1 : (B + groups - 1) / groups;
+  p.B = B;
+  p.ahead = rounds > 1;
+  p.keep_w = p.ahead && p.vec && p.hidden <= 6144;         // 2 x 12 KB beside the state, twice an SM
+  const int smem = p.ahead ? DK * DV * 4 + (p.keep_w ? p.hidden * 4 : 0) : 0;
+  if (p.ahead) {
+    static b200::PerDeviceOnce once_;
+    bool& configured = once_.slot();
+    if (!configured) {
+      const cudaError_t e = cudaFuncSetAttribute(gdn_decode_fused_kernel<4, R, 4>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                                 DK * DV * 4 + 6144 * 4);
+      if (e != cudaSuccess) return (int)e;
+      configured = true;
+    }
+  }
   cudaLaunchConfig_t cfg = {};
-  cfg.gridDim = dim3(p.Hv, B);
+  cfg.gridDim = dim3(p.Hv, (B + rounds - 1) / rounds);
+  cfg.dynamicSmemBytes = smem;
   cfg.blockDim = dim3(512);
   cfg.stream = stream;
   cudaLaunchAttribute attr[2];

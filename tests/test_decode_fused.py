@@ -89,3 +89,34 @@ def test_fused_decode_path_follows_unfused_tokens():
         outs.append(rt.generate(ids, 12))
     agree = sum(a == b for a, b in zip(*outs))
     assert outs[0][0] == outs[1][0] and agree >= 10, outs
+
+
+# rows a block walks: one (9 at 32 heads), two with an uneven last group, many; inputs whose weights stay in shared memory (up to 6144)
+# or not; projections and tails that lie on 16-byte boundaries or not; heads that share a key head by one, two and four
+@pytest.mark.parametrize("b,hv,hk,hidden,pad", [(9, 32, 16, 256, 0), (10, 32, 16, 512, 0), (19, 32, 16, 6152, 0), (64, 32, 16, 256, 4),
+                                                (37, 48, 12, 6144, 0), (33, 40, 40, 128, 8), (64, 32, 32, 1024, 1)])
+def test_rows_walked_by_one_block(b, hv, hk, hidden, pad):
+    from deepseek_v4_2080ti_b200.ops import basic, gdn
+    torch.manual_seed(b + hv)
+    kd, vd = hk * 128, hv * 128
+    c = 2 * kd + vd
+    wide = (torch.randn(b, c + vd + pad, device="cuda") * 0.5).bfloat16()
+    proj = wide[:, :c + vd]
+    x = (torch.randn(b, hidden, device="cuda") * 0.5).bfloat16()
+    w_ab = (torch.randn(2 * hv, hidden, device="cuda") * hidden ** -0.5).bfloat16()
+    a_log, dt = torch.randn(hv, device="cuda") * 0.3, torch.randn(hv, device="cuda") * 0.3
+    conv_w = (torch.randn(c, 4, device="cuda") * 0.3).bfloat16()
+    gamma = (torch.randn(128, device="cuda") * 0.1 + 1).bfloat16()
+    slots = torch.randperm(b + 3, device="cuda")[:b].int()
+    tails = (torch.randn(b + 3, 3, c, device="cuda") * 0.5).bfloat16()
+    states = torch.randn(b + 3, hv, 128, 128, device="cuda") * 0.1
+    t0, s0 = tails.clone(), states.clone()
+    runs = []
+    for lo in (None, 0):                               # all rows at once, and one by one
+        tails.copy_(t0)
+        states.copy_(s0)
+        call = lambda r: gdn.decode_fused(proj[r], x[r], w_ab, a_log, dt, conv_w, tails, states, slots[r], gamma, hv, hk)
+        y = call(slice(0, b)) if lo is None else torch.cat([call(slice(i, i + 1)) for i in range(b)])
+        torch.cuda.synchronize()
+        runs.append((y, tails.clone(), states.clone()))
+    assert all(torch.equal(a, e) for a, e in zip(*runs))
