@@ -81,14 +81,15 @@ __device__ __forceinline__ void copy8(__nv_bfloat16* dst, const __nv_bfloat16* s
 // projection's row, the convolution's tails and weights, the norm's weight - is asked for at once, straight to shared memory.  Two blocks
 // fit an SM; with more rows than these hold a block walks several rows of its head, the constants stay, and the next row's state
 // and small inputs are on their way while one is computed.  A few rows ask L2 for the a / b weights even before the previous kernel has
-// ended.  us a layer of 32 heads: 1 row 11.4, 16 rows 19, 32 rows 34.5, 64 rows 68 (the state's bytes take 0.7, 10, 21, 42); with each input
-// loaded where it is used and a row per block 13.7, 25, 43, 85.
+// ended.  us a layer of 32 heads: 1 row 10.7, 16 rows 17, 32 rows 29, 64 rows 53.5 (the state's bytes take 0.7, 10, 21, 42); with each
+// input loaded where it is used and a row per block 1 row took 13.7, 32 rows 43, 64 rows 85.  (A cluster arrival with release, which waits
+// for the row before's state to reach memory: 34.5 and 68 for 32 and 64 rows.)
 // Every block convolves the q and k channels of its key head itself; the first of the cluster moves their tail on when all of
 // them have read it.
 template <int KW, int R, int RG>
 __global__ void __launch_bounds__(128 * RG, 2)
 gdn_decode_fused_kernel(GdnDecodeParams p) {
-  static_assert(KW == 4, "three rows of tail");
+  static_assert(KW == 4 && RG == 4, "three rows of tail; row groups for q, k, v and the gates");
   constexpr int ROWS = DK / RG;
   constexpr int WARPS = 4 * RG;
   __shared__ __align__(16) float sq[DK], sk[DK], s_v[DV];
@@ -111,7 +112,7 @@ gdn_decode_fused_kernel(GdnDecodeParams p) {
   if (tid < 3 * 64) copy8(s_cw[tid >> 6] + (tid & 63) * 8, p.conv_w + (size_t)chan(tid >> 6) * KW + (tid & 63) * 8, p.vec);
   else if (tid < 3 * 64 + 16) copy8(s_gamma + (tid - 3 * 64) * 8, p.gamma + (tid - 3 * 64) * 8, p.vec);
   float a_log = 0.f, dt_bias = 0.f;
-  if (tid == 128) {
+  if (tid == 3 * 128) {
     a_log = p.a_log[h];
     dt_bias = p.dt_bias[h];
   }
@@ -209,9 +210,10 @@ gdn_decode_fused_kernel(GdnDecodeParams p) {
     }
     ask(nb, next_slot, buf ^ 1);
   }
-  if constexpr (R > 1) asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory");   // this block has read its tails
-  float qv = 0.f, kv = 0.f;
-  if (rg == 0) {
+  // This block has read its tails: they are in shared memory.  Nothing else is published, and a release would wait for the previous row's
+  // state to reach memory.
+  if constexpr (R > 1) asm volatile("barrier.cluster.arrive.relaxed.aligned;" ::: "memory");
+  if (rg < 3) {                            // a row group each for q, k and v
     // y = silu(sum_k w[c][k] * v[k]), rounded as the unfused path stores it
     auto conv = [&](int c) {
       float acc = __bfloat162float(s_row[c][j]) * __bfloat162float(s_cw[c][j * KW + KW - 1]);
@@ -219,20 +221,19 @@ gdn_decode_fused_kernel(GdnDecodeParams p) {
       for (int k = 0; k < KW - 1; ++k) acc += __bfloat162float(s_tail[c][k][j]) * __bfloat162float(s_cw[c][j * KW + k]);
       return bf16_round(silu_f(acc));
     };
-    qv = conv(0);
-    kv = conv(1);
-    s_v[j] = conv(2);
-    const float qs = warp_sum(qv * qv), ks = warp_sum(kv * kv);
-    if ((j & 31) == 0) {
-      red_qk[j >> 5] = qs;
-      red_qk[4 + (j >> 5)] = ks;
+    const float y = conv(rg);
+    if (rg == 2) {
+      s_v[j] = y;
+    } else {
+      const float ss = warp_sum(y * y);
+      if ((j & 31) == 0) red_qk[tid >> 5] = ss;
+      asm volatile("bar.sync %0, 128;" ::"r"(1 + rg) : "memory");
+      const float* red = red_qk + 4 * rg;
+      const float n = rsqrtf(red[0] + red[1] + red[2] + red[3] + 1e-6f);
+      if (rg == 0) sq[j] = y * n * p.q_scale;
+      else sk[j] = y * n;
     }
-    asm volatile("bar.sync 1, 128;" ::: "memory");
-    const float qn = rsqrtf(red_qk[0] + red_qk[1] + red_qk[2] + red_qk[3] + 1e-6f);
-    const float kn = rsqrtf(red_qk[4] + red_qk[5] + red_qk[6] + red_qk[7] + 1e-6f);
-    sq[j] = qv * qn * p.q_scale;
-    sk[j] = kv * kn;
-  } else if (tid == 128) {
+  } else if (tid == 3 * 128) {
     float a = 0.f, bb = 0.f;
 #pragma unroll
     for (int w = 0; w < WARPS; ++w) {
@@ -246,10 +247,12 @@ gdn_decode_fused_kernel(GdnDecodeParams p) {
     const float sp = av > 20.f ? av : log1pf(expf(av));
     s_gate[0] = __expf(-expf(a_log) * sp);   // decay = exp(g)
     s_gate[1] = sigmoid_f(bb);
-  } else if (rg == RG - 1) {
+  }
+  if (rg == 3 && tid >= 3 * 128 + 32) {
     // the value channels' tail, this block's own, moves on
+    for (int c = j - 32; c < DV; c += 96)
 #pragma unroll
-    for (int k = 0; k < KW - 1; ++k) tail[(size_t)k * C + chan(2) + j] = k + 1 < KW - 1 ? s_tail[2][k + 1][j] : s_row[2][j];
+      for (int k = 0; k < KW - 1; ++k) tail[(size_t)k * C + chan(2) + c] = k + 1 < KW - 1 ? s_tail[2][k + 1][c] : s_row[2][c];
   }
   __syncthreads();
   // ---- gated delta rule on rows [rg*ROWS, (rg+1)*ROWS) of state column j
