@@ -9,7 +9,8 @@
 //     (cp.async.bulk.tensor, destination = this CTA only, never multicast);
 //   * warps 7.. decode the raw weight tile (FP8 E4M3 with one scale per
 //     128x128 block) into bf16, written in the 128-byte-swizzled K-major layout
-//     the tensor core reads; the quantised matrix is never expanded in HBM;
+//     the tensor core reads (GGUF formats: into tensor memory, for up to 128
+//     tokens); the quantised matrix is never expanded in HBM;
 //   * warp 5 issues tcgen05.mma (kind::f16, fp32 accumulate in TMEM, two
 //     accumulator buffers) and commits stage/accumulator barriers;
 //   * warps 0..3 drain TMEM with tcgen05.ld and store bf16 (+residual) or fp32
@@ -180,19 +181,29 @@ struct SmemLayout {
   static constexpr int BUDGET = 232448 - 1024 /*align slack*/ - 512 /*barriers*/ - EPI_BYTES;
   static constexpr int W_STAGE_BYTES = (WFMT == WF_BF16) ? A_BYTES : RAW_BYTES;
   static constexpr int STAGE_BYTES = W_STAGE_BYTES + X_BYTES;
-  static constexpr int fit(int sa) { return (BUDGET - sa * A_BYTES) / STAGE_BYTES; }
+  // GGUF weights are decoded into tensor memory, a row by the thread that owns its lane, beside accumulators of up to 128 tokens.
+  // Through shared memory a 64-input tile costs 128 cycles to write and 128 to read, and a product of 16 tokens 39 cycles for the
+  // 9 it takes with its weights in tensor memory.  Blocks of 256 experts of 3072 x 1536, Q4_K gate / up and Q2_K down, eight for each
+  // of 1 / 8 / 24 / 400 / 2000 tokens, us: 94 / 279 / 518 / 1448 / 1908 through shared memory, 84 / 223 / 405 / 1120 / 1476 so, and
+  // 85 / 216 / 390 / 1068 / 1409 with the shorter unpacking of both formats below and each group stepping from one of its k-blocks
+  // to the next.  A 9216 x 4096 matrix of any format takes 4 to 15 % less at 1 to 100 tokens.  A k-block takes 400 cycles: 64 % of
+  // the issue slots, with 200 of them left when nothing is unpacked, stored or multiplied.  Twice the slots: 412 at 24 tokens, a
+  // commit for every two k-blocks besides: 427, a fifth group: 395.  Beside two accumulators of 256 tokens there is no room.
+  static constexpr bool A_TMEM = gguf_qb(WFMT) != 0 && BN <= 128;
+  static constexpr int A_SLOT_BYTES = A_TMEM ? 0 : A_BYTES;     // shared memory of a decoded slot
+  static constexpr int fit(int sa) { return (BUDGET - sa * A_SLOT_BYTES) / STAGE_BYTES; }
   // Decode warps work in GROUPS independent groups; group g owns decoded slot g and every
   // GROUPS-th k-block, so barrier/fence latency of one stage overlaps another's ALU work.  A slot's round - decode, product,
   // commit, free - is some 2500 cycles for the formats with a long unpacking, so those take as many slots as shared memory
   // holds beside a raw ring of as many stages, and more warps; FP8, a shift and a mask, keeps four slots and eight warps.
   static constexpr bool LONG_UNPACK = WFMT != WF_BF16 && WFMT != WF_FP8_B128;
-  static constexpr int GROUPS = !LONG_UNPACK ? 4 : fit(8) >= 8 ? 8 : fit(6) >= 6 ? 6 : 4;
-  static constexpr int WARPS_PER_GROUP = LONG_UNPACK && GROUPS == 4 ? 4 : 2;
+  static constexpr int GROUPS = !LONG_UNPACK || A_TMEM ? 4 : fit(8) >= 8 ? 8 : fit(6) >= 6 ? 6 : 4;
+  static constexpr int WARPS_PER_GROUP = A_TMEM || (LONG_UNPACK && GROUPS == 4) ? 4 : 2;
   static constexpr int DEC_WARPS = WFMT == WF_BF16 ? 0 : GROUPS * WARPS_PER_GROUP;
   static constexpr int THREADS = (DEC_WARP0 + DEC_WARPS) * 32;
   static constexpr int SA = (WFMT == WF_BF16) ? 0 : GROUPS;
   static constexpr int SR = fit(SA) > 16 ? 16 : fit(SA);
-  static constexpr int TOTAL = SR * STAGE_BYTES + SA * A_BYTES + EPI_BYTES + 1024 + 512;
+  static constexpr int TOTAL = SR * STAGE_BYTES + SA * A_SLOT_BYTES + EPI_BYTES + 1024 + 512;
   static_assert(SR >= 2, "pipeline needs at least two raw stages");
 };
 
@@ -214,9 +225,20 @@ __device__ __forceinline__ void e2m1x4_to_bf16x4(uint32_t q, uint32_t& w01, uint
   w01 = __byte_perm(lo, hi, 0x5140);
   w23 = __byte_perm(lo, hi, 0x7362);
 }
-// Byte i of four small integers -> float, without the conversion unit (a quarter of the rate): 2^23 + v has v in its low bits.
-__device__ __forceinline__ float byte_to_float(uint32_t four, int i) {
-  return __uint_as_float(__byte_perm(four, 0x4B000000u, 0x7440 | i)) - 8388608.f;
+// Bytes I and I + 1 of four codes of four bits, each standing at the top of seven bits below a set one -> 16 + code as floats (the
+// byte goes below the exponent), times sc, plus k, which holds the offset: 2.5
+// instructions a weight, 3.5 with the offset taken off first.
+template <int I>
+__device__ __forceinline__ void codes_to_floats(uint32_t four, uint64_t sc, uint64_t k, float& a, float& b) {
+  const uint32_t lo = __byte_perm(four, 0x41000000u, 0x7044 | I << 8), hi = __byte_perm(four, 0x41000000u, 0x7044 | (I + 1) << 8);
+  uint64_t d;
+  asm("{\n.reg .b64 c;\nmov.b64 c, {%1, %2};\nfma.rn.f32x2 %0, c, %3, %4;\n}" : "=l"(d) : "r"(lo), "r"(hi), "l"(sc), "l"(k));
+  asm("mov.b64 {%0, %1}, %2;" : "=f"(a), "=f"(b) : "l"(d));
+}
+__device__ __forceinline__ uint64_t both(float x) {
+  uint64_t d;
+  asm("mov.b64 %0, {%1, %1};" : "=l"(d) : "f"(x));
+  return d;
 }
 __device__ __forceinline__ uint32_t bf16x2_mul(uint32_t a, uint32_t b) {
   uint32_t d;
@@ -232,13 +254,14 @@ gemm_wdec_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constant_
   constexpr int S = L::SR;                       // raw ring depth
   constexpr int SA = L::SA;                      // decoded ring depth (0 for bf16 weights)
   constexpr int SAB = SA > 0 ? SA : 1;
-  constexpr uint32_t TMEM_COLS = (2 * BN < 32) ? 32 : 2 * BN;
+  constexpr uint32_t COLS = 2 * BN + (L::A_TMEM ? SA * (BK / 2) : 0);      // two accumulators, decoded slots
+  constexpr uint32_t TMEM_COLS = COLS <= 32 ? 32 : COLS <= 64 ? 64 : COLS <= 128 ? 128 : COLS <= 256 ? 256 : 512;
   extern __shared__ uint8_t smem_raw_base[];
   uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw_base) + 1023) &
                                              ~uintptr_t(1023));
   // bf16 weights: sA is the raw ring itself (S stages); FP8: sA is the decoded ring (SA stages)
   uint8_t* sA = smem;
-  uint8_t* sX = sA + (WFMT == WF_BF16 ? S : SA) * L::A_BYTES;
+  uint8_t* sX = sA + (WFMT == WF_BF16 ? S : SA) * L::A_SLOT_BYTES;
   uint8_t* sRaw = sX + S * L::X_BYTES;
   uint64_t* bars = reinterpret_cast<uint64_t*>(sRaw + (WFMT == WF_BF16 ? 0 : S * L::RAW_BYTES));
   uint64_t* tma_full = bars;                  // [S]   raw stage landed
@@ -406,7 +429,10 @@ gemm_wdec_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constant_
 #pragma unroll
         for (int k = 0; k < BK / 16; ++k) {
           // advance 16 bf16 = 32 bytes inside the swizzle row: +2 in 16-byte units
-          umma_bf16_ss_warp(on, tmem_d, da + 2 * k, db + 2 * k, idesc, (kb > kb0 || k > 0) ? 1u : 0u);
+          if constexpr (L::A_TMEM)
+            umma_bf16_ts_warp(on, tmem_d, tmem_base + 2 * BN + sa * (BK / 2) + 8 * k, db + 2 * k, idesc, (kb > kb0 || k > 0) ? 1u : 0u);
+          else
+            umma_bf16_ss_warp(on, tmem_d, da + 2 * k, db + 2 * k, idesc, (kb > kb0 || k > 0) ? 1u : 0u);
         }
         // One commit per k-block frees the raw stage for the producer and, SA k-blocks later, the
         // decoded slot for the decode warps (they wait on the same barrier): tcgen05.commit occupies
@@ -458,8 +484,9 @@ gemm_wdec_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constant_
           }
         }
         bool failed = false;
-        for (int kb = kb0; kb < kb1; ++kb, ++it) {
-          if ((int)(it % G) != grp) continue;
+        const uint32_t it0 = it;
+        it += (grp + G - it % G) % G;            // this group's k-blocks: every G-th
+        for (int kb = kb0 + (int)(it - it0); kb < kb1; kb += G, it += G) {
           const int s = it % S;
           const uint32_t ph = (it / S) & 1;
           uint32_t scw = 0;
@@ -546,12 +573,14 @@ gemm_wdec_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constant_
             // one unit = (row, half of the 64-wide K tile) = 32 inputs -> 32 bf16 = four 16-byte chunks
             constexpr int QB = gguf_qb(WFMT), SB = gguf_sb(WFMT);
             const uint8_t* sreg = raw + BM * QB;
-#pragma unroll 1
-            for (int i = d; i < BM * 2; i += GT) {
-              const int r = i >> 1, hh = i & 1;
+            [[maybe_unused]] uint32_t packed[BK / 2];
+#pragma unroll(L::A_TMEM ? 2 : 1)
+            for (int i = L::A_TMEM ? 0 : d; i < (L::A_TMEM ? 2 : BM * 2); i += L::A_TMEM ? 1 : GT) {
+              const int r = L::A_TMEM ? (warp & 3) * 32 + lane : i >> 1, hh = i & 1;
               const uint8_t* qrow = raw + r * QB;
               const uint8_t* srow = sreg + r * SB;
-              float v[32];
+              float v[32];                           // the unit's values, or their bf16 pairs straight away
+              uint32_t out[16];
               if constexpr (WFMT == WF_Q8_0) {
                 const float dd = __half2float(*reinterpret_cast<const __half*>(srow + 2 * hh));
                 const int4 a = *reinterpret_cast<const int4*>(qrow + hh * 32), b = *reinterpret_cast<const int4*>(qrow + hh * 32 + 16);
@@ -562,10 +591,15 @@ gemm_wdec_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constant_
                 const float dd = __half2float(*reinterpret_cast<const __half*>(srow));
                 const float dm = __half2float(*reinterpret_cast<const __half*>(srow + 2));
                 const float sc = dd * (float)srow[4 + 2 * hh], mn = dm * (float)srow[5 + 2 * hh];
+                const uint64_t sc2 = both(sc), k2 = both(-fmaf(16.f, sc, mn));
                 const int4 a = *reinterpret_cast<const int4*>(qrow), b = *reinterpret_cast<const int4*>(qrow + 16);
                 const int w8[8] = {a.x, a.y, a.z, a.w, b.x, b.y, b.z, b.w};
 #pragma unroll
-                for (int e = 0; e < 32; ++e) v[e] = sc * byte_to_float((w8[e >> 2] >> (4 * hh)) & 0x0F0F0F0Fu, e & 3) - mn;
+                for (int e = 0; e < 32; e += 4) {
+                  const uint32_t four = ((hh ? (uint32_t)w8[e >> 2] >> 1 : (uint32_t)w8[e >> 2] << 3) & 0x78787878u) | 0x80808080u;
+                  codes_to_floats<0>(four, sc2, k2, v[e], v[e + 1]);
+                  codes_to_floats<2>(four, sc2, k2, v[e + 2], v[e + 3]);
+                }
               } else if constexpr (WFMT == WF_Q2_K) {
                 const float dd = __half2float(*reinterpret_cast<const __half*>(srow));
                 const float dm = __half2float(*reinterpret_cast<const __half*>(srow + 2));
@@ -575,8 +609,16 @@ gemm_wdec_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constant_
                 for (int g = 0; g < 2; ++g) {           // 16 inputs of one scale: the low, then the high nibbles
                   const int sb = srow[4 + 2 * hh + g];
                   const float sc = dd * (float)(sb & 15), mn = dm * (float)(sb >> 4);
+                  // Four values there are: their bf16 stand in a pair of registers, and one byte permutation fetches two weights
+                  // (code c: bytes 2c and 2c + 1, so c * 0x22 + 0x10 selects them).  135 -> 122 us for the down blocks above.
+                  const __nv_bfloat162 t01 = __floats2bfloat162_rn(-mn, sc - mn), t23 = __floats2bfloat162_rn(2.f * sc - mn, 3.f * sc - mn);
+                  const uint32_t t0 = *reinterpret_cast<const uint32_t*>(&t01), t1 = *reinterpret_cast<const uint32_t*>(&t23);
 #pragma unroll
-                  for (int e = 0; e < 16; ++e) v[16 * g + e] = sc * byte_to_float((w4[e >> 2] >> (4 * g + 2 * hh)) & 0x03030303u, e & 3) - mn;
+                  for (int e = 0; e < 4; ++e) {
+                    const uint32_t sel = ((w4[e] >> (4 * g + 2 * hh)) & 0x03030303u) * 0x22u + 0x10101010u;
+                    out[8 * g + 2 * e] = __byte_perm(t0, t1, sel);
+                    out[8 * g + 2 * e + 1] = __byte_perm(t0, t1, sel >> 16);
+                  }
                 }
               } else if constexpr (WFMT == WF_Q5_K) {
                 const float dd = __half2float(*reinterpret_cast<const __half*>(srow));
@@ -693,22 +735,36 @@ gemm_wdec_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constant_
                   }
                 }
               }
-              uint8_t* rowp = A + (r >> 3) * 1024 + (r & 7) * 128;
-              const int sw = r & 7;
+              if constexpr (WFMT != WF_Q2_K) {
 #pragma unroll
-              for (int wd = 0; wd < 4; ++wd) {
-                uint4 o;
-                __nv_bfloat162* oh = reinterpret_cast<__nv_bfloat162*>(&o);
+                for (int e = 0; e < 16; ++e) {
+                  const __nv_bfloat162 o = __floats2bfloat162_rn(v[2 * e], v[2 * e + 1]);
+                  out[e] = *reinterpret_cast<const uint32_t*>(&o);
+                }
+              }
+              if constexpr (L::A_TMEM) {
 #pragma unroll
-                for (int e = 0; e < 4; ++e) oh[e] = __floats2bfloat162_rn(v[wd * 8 + 2 * e], v[wd * 8 + 2 * e + 1]);
-                *reinterpret_cast<uint4*>(rowp + (((hh * 4 + wd) ^ sw) << 4)) = o;
+                for (int e = 0; e < 16; ++e) packed[hh * 16 + e] = out[e];
+              } else {
+                uint8_t* rowp = A + (r >> 3) * 1024 + (r & 7) * 128;
+                const int sw = r & 7;
+#pragma unroll
+                for (int wd = 0; wd < 4; ++wd)
+                  *reinterpret_cast<uint4*>(rowp + (((hh * 4 + wd) ^ sw) << 4)) =
+                      make_uint4(out[4 * wd], out[4 * wd + 1], out[4 * wd + 2], out[4 * wd + 3]);
               }
             }
+            if constexpr (L::A_TMEM) {
+              tmem_st_32x32(tmem_base + (uint32_t(warp & 3) << 21) + 2 * BN + grp * (BK / 2), packed);
+              tmem_st_wait();
+              tc_fence_before();
+            }
           }
-          fence_proxy_async_smem();
+          if constexpr (!L::A_TMEM) fence_proxy_async_smem();
           __syncwarp();
           if (lane == 0) mbar_arrive(&a_full[grp]);
         }
+        it = it0 + max(kb1 - kb0, 0);
         if (failed) {
           *abort_flag = 1;
           break;
