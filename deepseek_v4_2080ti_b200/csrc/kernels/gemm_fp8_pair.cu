@@ -14,7 +14,7 @@
 // (terms_pay in ops/gemm.py).
 //
 // What bounds it: with two accumulators of 256 columns (all of tensor memory) the products of a block wait for the epilogue to have
-// read the block before last; the tensor pipe is busy for 65 % of the cycles at 1901 tokens.  The epilogue's 216 registers are all
+// read the block before last; the tensor pipe is busy for 66 % of the cycles at 1901 tokens.  The epilogue's 216 registers are all
 // in use and 52 bytes are spilled.
 //
 // Work: as long as there are more tiles than workers, every worker takes a whole tile of each run of as many tiles, so that at any time the

@@ -185,7 +185,7 @@ struct SmemLayout {
   // Through shared memory a 64-input tile costs 128 cycles to write and 128 to read, and a product of 16 tokens 39 cycles for the
   // 9 it takes with its weights in tensor memory.  Blocks of 256 experts of 3072 x 1536, Q4_K gate / up and Q2_K down, eight for each
   // of 1 / 8 / 24 / 400 / 2000 tokens, us: 94 / 279 / 518 / 1448 / 1908 through shared memory, 84 / 223 / 405 / 1120 / 1476 so, and
-  // 85 / 216 / 390 / 1068 / 1409 with the shorter unpacking of both formats below and each group stepping from one of its k-blocks
+  // 87 / 217 / 390 / 1074 / 1436 with the shorter unpacking of both formats below and each group stepping from one of its k-blocks
   // to the next.  A 9216 x 4096 matrix of any format takes 4 to 15 % less at 1 to 100 tokens.  A k-block takes 400 cycles: 64 % of
   // the issue slots, with 200 of them left when nothing is unpacked, stored or multiplied.  Twice the slots: 412 at 24 tokens, a
   // commit for every two k-blocks besides: 427, a fifth group: 395.  Beside two accumulators of 256 tokens there is no room.
@@ -485,8 +485,8 @@ gemm_wdec_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constant_
         }
         bool failed = false;
         const uint32_t it0 = it;
-        it += (grp + G - it % G) % G;            // this group's k-blocks: every G-th
-        for (int kb = kb0 + (int)(it - it0); kb < kb1; kb += G, it += G) {
+        for (int kb = kb0; kb < kb1; ++kb, ++it) {
+          if ((int)(it % G) != grp) continue;
           const int s = it % S;
           const uint32_t ph = (it / S) & 1;
           uint32_t scw = 0;
@@ -763,6 +763,8 @@ gemm_wdec_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constant_
           if constexpr (!L::A_TMEM) fence_proxy_async_smem();
           __syncwarp();
           if (lane == 0) mbar_arrive(&a_full[grp]);
+          kb += G - 1;                           // the next ones are the other groups'
+          it += G - 1;
         }
         it = it0 + max(kb1 - kb0, 0);
         if (failed) {
