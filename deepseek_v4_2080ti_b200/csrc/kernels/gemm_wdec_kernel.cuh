@@ -185,8 +185,8 @@ struct SmemLayout {
   // Through shared memory a 64-input tile costs 128 cycles to write and 128 to read, and a product of 16 tokens 39 cycles for the
   // 9 it takes with its weights in tensor memory.  Blocks of 256 experts of 3072 x 1536, Q4_K gate / up and Q2_K down, eight for each
   // of 1 / 8 / 24 / 400 / 2000 tokens, us: 94 / 279 / 518 / 1448 / 1908 through shared memory, 84 / 223 / 405 / 1120 / 1476 so, and
-  // 87 / 217 / 390 / 1074 / 1436 with the shorter unpacking of both formats below and each group stepping from one of its k-blocks
-  // to the next.  A 9216 x 4096 matrix of any format takes 4 to 15 % less at 1 to 100 tokens.  A k-block takes 400 cycles: 64 % of
+  // 84 / 225 / 409 / 1131 / 1506 with the shorter unpacking of both formats below and each group stepping from one of its k-blocks
+  // to the next (5 % of it for infinite block scales, which need the offset taken off first).  A 9216 x 4096 matrix of any format takes 4 to 15 % less at 1 to 100 tokens.  A k-block takes 400 cycles: 64 % of
   // the issue slots, with 200 of them left when nothing is unpacked, stored or multiplied.  Twice the slots: 412 at 24 tokens, a
   // commit for every two k-blocks besides: 427, a fifth group: 395.  Beside two accumulators of 256 tokens there is no room.
   static constexpr bool A_TMEM = gguf_qb(WFMT) != 0 && BN <= 128;
@@ -600,6 +600,10 @@ gemm_wdec_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constant_
                   codes_to_floats<0>(four, sc2, k2, v[e], v[e + 1]);
                   codes_to_floats<2>(four, sc2, k2, v[e + 2], v[e + 3]);
                 }
+                if (fabsf(sc) == INFINITY) {            // the offset would meet its own infinity
+#pragma unroll
+                  for (int e = 0; e < 32; ++e) v[e] = __fmaf_rn(sc, (float)(((uint32_t)w8[e >> 2] >> (8 * (e & 3) + 4 * hh)) & 15u), -mn);
+                }
               } else if constexpr (WFMT == WF_Q2_K) {
                 const float dd = __half2float(*reinterpret_cast<const __half*>(srow));
                 const float dm = __half2float(*reinterpret_cast<const __half*>(srow + 2));
@@ -611,7 +615,8 @@ gemm_wdec_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constant_
                   const float sc = dd * (float)(sb & 15), mn = dm * (float)(sb >> 4);
                   // Four values there are: their bf16 stand in a pair of registers, and one byte permutation fetches two weights
                   // (code c: bytes 2c and 2c + 1, so c * 0x22 + 0x10 selects them).  135 -> 122 us for the down blocks above.
-                  const __nv_bfloat162 t01 = __floats2bfloat162_rn(-mn, sc - mn), t23 = __floats2bfloat162_rn(2.f * sc - mn, 3.f * sc - mn);
+                  const __nv_bfloat162 t01 = __floats2bfloat162_rn(__fmaf_rn(sc, 0.f, -mn), sc - mn);
+                  const __nv_bfloat162 t23 = __floats2bfloat162_rn(2.f * sc - mn, 3.f * sc - mn);
                   const uint32_t t0 = *reinterpret_cast<const uint32_t*>(&t01), t1 = *reinterpret_cast<const uint32_t*>(&t23);
 #pragma unroll
                   for (int e = 0; e < 4; ++e) {
