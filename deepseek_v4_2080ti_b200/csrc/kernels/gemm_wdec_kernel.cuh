@@ -186,7 +186,8 @@ struct SmemLayout {
   // 9 it takes with its weights in tensor memory.  Blocks of 256 experts of 3072 x 1536, Q4_K gate / up and Q2_K down, eight for each
   // of 1 / 8 / 24 / 400 / 2000 tokens, us: 94 / 279 / 518 / 1448 / 1908 through shared memory, 84 / 223 / 405 / 1120 / 1476 so, and
   // 84 / 225 / 409 / 1131 / 1506 with the shorter unpacking of both formats below and each group stepping from one of its k-blocks
-  // to the next (5 % of it for infinite block scales, which need the offset taken off first).  A 9216 x 4096 matrix of any format takes 4 to 15 % less at 1 to 100 tokens.  A k-block takes 400 cycles: 64 % of
+  // to the next (5 % of it for infinite block scales, which need the offset taken off first).
+  // A 9216 x 4096 matrix of any format takes 4 to 15 % less at 1 to 100 tokens.  A k-block takes 400 cycles: 64 % of
   // the issue slots, with 200 of them left when nothing is unpacked, stored or multiplied.  Twice the slots: 412 at 24 tokens, a
   // commit for every two k-blocks besides: 427, a fifth group: 395.  Beside two accumulators of 256 tokens there is no room.
   static constexpr bool A_TMEM = gguf_qb(WFMT) != 0 && BN <= 128;
