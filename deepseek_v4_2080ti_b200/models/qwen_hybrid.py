@@ -947,9 +947,7 @@ class QwenHybridRuntime(PagedSequences):
         rows = [v for st in sts for v in (
             st.length, st.length + 1, st.slot,
             st.blocks[st.length // self.block_size] * self.block_size + st.length % self.block_size)]
-        if token_ids.numel() != b:
-            token_ids = token_ids.expand(b)
-        token_ids = token_ids.to(self.device, torch.int32).contiguous()
+        token_ids = _step_ids(token_ids, b, self.device)
         rc = _lib.lib().b200_step_meta((ctypes.c_int * (4 * b))(*rows), b, _lib.ptr(token_ids), _lib.ptr(self.block_table),
                                        self.max_blocks_per_seq, *(_lib.ptr(buf[n]) for n in ("ids", "pos", "kv_len", "slots", "kv_slots", "bt")),
                                        _lib.stream())
@@ -996,6 +994,11 @@ class QwenHybridRuntime(PagedSequences):
             return out
         finally:
             self.free(slot)
+
+
+def _step_ids(token_ids: torch.Tensor, b: int, device) -> torch.Tensor:
+    """Tokens of a decode step as int32 [b] on ``device``: one each, or one for all; other shapes are refused."""
+    return token_ids.to(device, torch.int32).expand(b).contiguous()
 
 
 def build_synthetic(cfg: QwenHybridConfig, device="cuda", seed: int = 0, tp_rank: int = 0, tp_world: int = 1,
