@@ -288,21 +288,26 @@ def pick_splits(t: int, n: int, k: int) -> int:
 
 
 def pick_splits_f32(t: int, n: int, k: int) -> int:
-    """Splits of K for an fp32 product of bf16 weights (output heads): where the feature tiles leave a wave of SMs nearly empty.  Walking
-    64 inputs of a tile takes an SM 0.26 us in a decode batch, adding up the splits 3 us, about 16 such steps, and the partial sums must
-    be few beside the weights.  18992 x 5120 is 149 tiles for 148 SMs: eight splits 31 + 3 us for 41 (1 row); 151936 x 5120, 1187 tiles,
-    takes eight, 9 waves of 80 steps for 65 of 10."""
+    """Splits of K for an fp32 product of bf16 weights (output heads), where the feature tiles leave a wave of SMs nearly empty.  us of a
+    product: walking 64 inputs of a tile takes an SM 0.26, but reading the weights bounds it too, 6.5 GB/ms; splits cost 3.5 for adding
+    them up, and their partial sums, written and read.  A prediction 4 us better is wanted, the error of this estimate.  5120 inputs, us
+    unsplit / in three at 1, 8, 32, 64 rows: 18992 features (149 tiles for 148 SMs) 40.9 / 35.8, 41.5 / 37.0, 43.0 / 40.8, 45.0 / 44.3;
+    25600 44.8 / 46.1, 45.8 / 47.4, 46.7 / 52.3, 47.9 / 56.4; 151936 230 / 237, 233 / 249, 240 / 270, 241 / 285; 248320 367 / 383,
+    376 / 404, 385 / 437, 386 / 460: heads of a few waves and more are bound by their weights, split or not."""
     tiles, kb = (n + 127) // 128, (k + 63) // 64
     if t > 64 or tiles <= NUM_SMS:
         return 1
-    best, best_steps = 1, (tiles + NUM_SMS - 1) // NUM_SMS * kb - 16
-    for s in range(2, min(kb // 8, k // (16 * t), 16) + 1):
+    read = 2 * n * k / 6.5e6
+
+    def us(s: int) -> float:
+        walk = 0.26 * ((tiles * s + NUM_SMS - 1) // NUM_SMS) * ((kb + s - 1) // s)
+        return max(walk, read) + (3.5 + 8 * s * t * n / 6.5e6 if s > 1 else 0.0)
+
+    best, best_us = 1, us(1) - 4.0
+    for s in range(2, min(kb // 8, 16) + 1):
         per = (kb + s - 1) // s
-        if (kb + per - 1) // per != s:
-            continue
-        steps = (tiles * s + NUM_SMS - 1) // NUM_SMS * per
-        if steps < best_steps:
-            best, best_steps = s, steps
+        if (kb + per - 1) // per == s and us(s) < best_us:
+            best, best_us = s, us(s)
     return best
 
 

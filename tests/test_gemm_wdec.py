@@ -202,3 +202,18 @@ def test_fp32_heads_in_splits(t, n, k):
     assert gemm.pick_splits_f32(1, 18992, 5120) > 1 and gemm.pick_splits_f32(64, 18992, 1024) == 1
     ref = x.double() @ w.double().t()
     assert ((got.double() - ref).abs() <= (x.double().abs() @ w.double().abs().t()) * k * 2.0 ** -24).all()
+
+
+# such shapes, whose reduction is long enough to be split, and one in more splits
+@pytest.mark.gpu
+@pytest.mark.parametrize("t,n,k", [(1, 18992, 5120), (7, 18951, 4096), (32, 18947, 5120), (3, 19000, 12288)])
+def test_fp32_heads_in_some_splits(t, n, k):
+    from deepseek_v4_2080ti_b200.ops import _lib, gemm
+    torch.manual_seed(t)
+    assert gemm.pick_splits_f32(t, n, k) > 1
+    x, w = torch.randn(t, k, device="cuda").bfloat16(), (torch.randn(n, k, device="cuda") * 0.02).bfloat16()
+    got = gemm.linear(x, gemm.PackedLinear.from_bf16(w), out_f32=True)
+    torch.cuda.synchronize()
+    _lib.check_status()
+    ref = x.double() @ w.double().t()
+    assert ((got.double() - ref).abs() <= (x.double().abs() @ w.double().abs().t()) * k * 2.0 ** -24).all()
