@@ -185,8 +185,8 @@ struct SmemLayout {
   // Through shared memory a 64-input tile costs 128 cycles to write and 128 to read, and a product of 16 tokens 39 cycles for the
   // 9 it takes with its weights in tensor memory.  Blocks of 256 experts of 3072 x 1536, Q4_K gate / up and Q2_K down, eight for each
   // of 1 / 8 / 24 / 400 / 2000 tokens, us: 94 / 279 / 518 / 1448 / 1908 through shared memory, 84 / 223 / 405 / 1120 / 1476 so, and
-  // 84 / 225 / 409 / 1131 / 1506 with the shorter unpacking of both formats below and each group stepping from one of its k-blocks
-  // to the next (5 % of it for infinite block scales, which need the offset taken off first).
+  // 84 / 227 / 410 / 1141 / 1447 with each group stepping from one of its k-blocks to the next, Q2_K weights from a table of four and
+  // Q4_K codes turned into floats in pairs (85 / 242 / 436 / 1213 / 1537 with them one by one).
   // A 9216 x 4096 matrix of any format takes 4 to 15 % less at 1 to 100 tokens.  A k-block takes 400 cycles: 64 % of
   // the issue slots, with 200 of them left when nothing is unpacked, stored or multiplied.  Twice the slots: 412 at 24 tokens, a
   // commit for every two k-blocks besides: 427, a fifth group: 395.  Beside two accumulators of 256 tokens there is no room.
@@ -226,14 +226,14 @@ __device__ __forceinline__ void e2m1x4_to_bf16x4(uint32_t q, uint32_t& w01, uint
   w01 = __byte_perm(lo, hi, 0x5140);
   w23 = __byte_perm(lo, hi, 0x7362);
 }
-// Bytes I and I + 1 of four codes of four bits, each standing at the top of seven bits below a set one -> 16 + code as floats (the
-// byte goes below the exponent), times sc, plus k, which holds the offset: 2.5
-// instructions a weight, 3.5 with the offset taken off first.
+// Bytes I and I + 1 of four codes of four bits, each standing at the top of seven bits below a set one (the byte goes below the
+// exponent of 16 + code), as floats: sc code - mn, rounded once.  No conversion unit, which runs at a quarter of the rate.
 template <int I>
-__device__ __forceinline__ void codes_to_floats(uint32_t four, uint64_t sc, uint64_t k, float& a, float& b) {
+__device__ __forceinline__ void codes_to_floats(uint32_t four, uint64_t sc, uint64_t minus_mn, float& a, float& b) {
   const uint32_t lo = __byte_perm(four, 0x41000000u, 0x7044 | I << 8), hi = __byte_perm(four, 0x41000000u, 0x7044 | (I + 1) << 8);
   uint64_t d;
-  asm("{\n.reg .b64 c;\nmov.b64 c, {%1, %2};\nfma.rn.f32x2 %0, c, %3, %4;\n}" : "=l"(d) : "r"(lo), "r"(hi), "l"(sc), "l"(k));
+  asm("{\n.reg .b64 c;\nmov.b64 c, {%1, %2};\nadd.rn.f32x2 c, c, %5;\nfma.rn.f32x2 %0, c, %3, %4;\n}"
+      : "=l"(d) : "r"(lo), "r"(hi), "l"(sc), "l"(minus_mn), "l"(0xC1800000C1800000ull));     // -16, -16
   asm("mov.b64 {%0, %1}, %2;" : "=f"(a), "=f"(b) : "l"(d));
 }
 __device__ __forceinline__ uint64_t both(float x) {
@@ -592,18 +592,14 @@ gemm_wdec_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constant_
                 const float dd = __half2float(*reinterpret_cast<const __half*>(srow));
                 const float dm = __half2float(*reinterpret_cast<const __half*>(srow + 2));
                 const float sc = dd * (float)srow[4 + 2 * hh], mn = dm * (float)srow[5 + 2 * hh];
-                const uint64_t sc2 = both(sc), k2 = both(-fmaf(16.f, sc, mn));
+                const uint64_t sc2 = both(sc), mn2 = both(-mn);
                 const int4 a = *reinterpret_cast<const int4*>(qrow), b = *reinterpret_cast<const int4*>(qrow + 16);
                 const int w8[8] = {a.x, a.y, a.z, a.w, b.x, b.y, b.z, b.w};
 #pragma unroll
                 for (int e = 0; e < 32; e += 4) {
                   const uint32_t four = ((hh ? (uint32_t)w8[e >> 2] >> 1 : (uint32_t)w8[e >> 2] << 3) & 0x78787878u) | 0x80808080u;
-                  codes_to_floats<0>(four, sc2, k2, v[e], v[e + 1]);
-                  codes_to_floats<2>(four, sc2, k2, v[e + 2], v[e + 3]);
-                }
-                if (fabsf(sc) == INFINITY) {            // the offset would meet its own infinity
-#pragma unroll
-                  for (int e = 0; e < 32; ++e) v[e] = __fmaf_rn(sc, (float)(((uint32_t)w8[e >> 2] >> (8 * (e & 3) + 4 * hh)) & 15u), -mn);
+                  codes_to_floats<0>(four, sc2, mn2, v[e], v[e + 1]);
+                  codes_to_floats<2>(four, sc2, mn2, v[e + 2], v[e + 3]);
                 }
               } else if constexpr (WFMT == WF_Q2_K) {
                 const float dd = __half2float(*reinterpret_cast<const __half*>(srow));
