@@ -231,7 +231,8 @@ template <int KW>
 __global__ void conv_silu_kernel(const __nv_bfloat16* __restrict__ x, int ldx, const __nv_bfloat16* __restrict__ w,
                                  __nv_bfloat16* __restrict__ tail, __nv_bfloat16* __restrict__ y, int ldy,
                                  int T, int C, int t_per_block, int update_tail) {
-  b200::pdl_grid_trigger();
+  // The next kernel is let go when this one ends: blocks of it that wait on an SM from the start, and those of the kernel after, leave
+  // uneven room for this kernel's (512 tokens 16.8 us for 11.3, 12.2 without any overlap).
   b200::pdl_grid_wait();
   const int c0 = (blockIdx.x * blockDim.x + threadIdx.x) * 8;
   if (c0 >= C) return;
@@ -536,9 +537,10 @@ int b200_conv_silu(const void* x, int ldx, const void* w, void* tail, void* y, i
   if (kw != 4 || C % 8) return -6;
   const int threads = 128;
   const int cblocks = (C / 8 + threads - 1) / threads;
-  // Short runs: a thread walks its tokens one after the other (64 at a time: 30 us at 333 tokens of 8192 channels).  Runs of 4 up to 512
-  // tokens: 40 tokens 5.0 us for 9.6 with runs of 16, 333 tokens 6.1 for 11.6.
-  const int t_per_block = T <= 4 ? T : T <= 512 ? 4 : 16;
+  // Short runs: a thread walks its tokens one after the other (64 at a time: 30 us at 333 tokens of 8192 channels).  us of a convolution and
+  // its tail, 8192 channels, in runs of 4 / 8 / 16: 64 tokens 5.4 / 7 / 10, 256 tokens 9.2 / 8.1 / 10, 512 tokens 16.5 / 11.3 / 11.3.  Up to
+  // six tokens one run, which moves the tail on itself (5 tokens 4.5 for 5.4).
+  const int t_per_block = T <= 6 ? T : T <= 192 ? 4 : T <= 512 ? 8 : 16;
   const int tblocks = (T + t_per_block - 1) / t_per_block;
   const auto* xp = reinterpret_cast<const __nv_bfloat16*>(x);
   auto* tp = reinterpret_cast<__nv_bfloat16*>(tail);
