@@ -30,6 +30,7 @@ struct DecodeParams {
   __nv_bfloat16* out;            // [B, Hq, D]
   const __nv_bfloat16* gate;     // optional [B, Hq, D]
   int max_blocks, bs, Hq, Hkv, splits;
+  uint32_t bs_mul, bs_shift;     // page of a key without a division (page())
   float scale_log2;
   int window, sinks;             // window > 0: only the first `sinks` and the last `window` keys are visible
   // KV 1 / 2: the caches hold E4M3 / INT8 bytes (same [num_blocks, Hkv, bs, D] layout) with one fp32 scale per
@@ -37,6 +38,8 @@ struct DecodeParams {
   const float* k_scale;
   const float* v_scale;
   const float* v_min;
+  // key / bs for keys below 2^31: bs_mul = 2^bs_shift / bs rounded up, bs_shift = 31 + ceil(log2 bs)
+  __device__ __forceinline__ int page(int key) const { return (int)((unsigned long long)(uint32_t)key * bs_mul >> bs_shift); }
 };
 
 __device__ __forceinline__ void e4m3x8_to_float(const uint2 u, float (&f)[8]) {
@@ -104,10 +107,15 @@ struct KvRow<0> {
   __device__ __forceinline__ void values(float (&f)[8]) const { get(v, f); }
 };
 
+template <int N>
+struct Int {
+  static constexpr int value = N;
+};
+
 template <int G, int KV>
 __global__ void __launch_bounds__(THREADS)
 gqa_decode_kernel(DecodeParams p) {
-  constexpr int U = G > 5 ? 2 : 4;
+  constexpr int U = G > 5 ? 2 : 3;
   __shared__ float s_m[NSTATE][G], s_l[NSTATE][G];
   __shared__ float s_o[NSTATE][G][D];
   b200::pdl_grid_trigger();
@@ -142,8 +150,10 @@ gqa_decode_kernel(DecodeParams p) {
   }
 
   // U keys of a half-warp at a time: their page numbers, then their rows, are asked for together, and the running maximum and the
-  // sums are rescaled once for all of them.  One after the other, a key is two trips to memory and a chain of shuffles and exponentials:
-  // 30 us for 32 rows of 5 x 8 heads over 70 to 90 keys, 17 so.
+  // sums are rescaled once for all of them; a rest of up to eight keys goes one key a half-warp.  One after the other, a key is two
+  // trips to memory and a chain of shuffles and exponentials.  us for 5 x 8 heads, rows x keys, one key at a time / U = 3: 1 x 24 4.9 /
+  // 4.5, 32 x 60 11 / 7, 64 x 1024 180 / 120, 32 x 4096 663 / 420.  U = 4 takes registers that four blocks an SM do not have (64 x 1024
+  // 207), as does U = 3 from six heads on.  A third of it was the division by the page size.
   const int mine = warp * 2 + half;
   auto key_at = [&](int kk) {                  // rows past the range contribute nothing: they repeat the first one
     const int kc = kk < k1 ? kk : k0;
@@ -151,21 +161,25 @@ gqa_decode_kernel(DecodeParams p) {
   };
   int page[U];
 #pragma unroll
-  for (int u = 0; u < U; ++u) page[u] = k0 < k1 ? bt[key_at(k0 + u * 8 + mine) / p.bs] : 0;
-  for (int base = k0; base < k1; base += 8 * U) {          // warp-uniform: every lane runs the shuffles
-    KvRow<KV> row[U];
-    bool valid[U];
+  for (int u = 0; u < U; ++u) page[u] = k0 < k1 ? bt[p.page(key_at(k0 + u * 8 + mine))] : 0;
+  // keys base + u * 8 + mine, u < N
+  auto chunk = [&](int base, auto count) {
+    constexpr int N = decltype(count)::value;
+    KvRow<KV> row[N];
+    bool valid[N];
 #pragma unroll
-    for (int u = 0; u < U; ++u) {
-      const int kk = base + u * 8 + mine;
+    for (int u = 0; u < N; ++u) {
+      const int kk = base + u * 8 + mine, key = key_at(kk);
       valid[u] = kk < k1;
-      row[u].load(p, ((size_t)(page[u] * p.Hkv + kvh) * p.bs + key_at(kk) % p.bs) * D + dl * 8);
+      row[u].load(p, ((size_t)(page[u] * p.Hkv + kvh) * p.bs + key - p.page(key) * p.bs) * D + dl * 8);
     }
+    if (N == U && base + 8 * U < k1) {
 #pragma unroll
-    for (int u = 0; u < U; ++u) page[u] = bt[key_at(base + 8 * U + u * 8 + mine) / p.bs];
-    float s[U][G];
+      for (int u = 0; u < U; ++u) page[u] = bt[p.page(key_at(base + 8 * U + u * 8 + mine))];
+    }
+    float s[N][G];
 #pragma unroll
-    for (int u = 0; u < U; ++u) {
+    for (int u = 0; u < N; ++u) {
       float kf[8];
       row[u].keys(kf);
 #pragma unroll
@@ -179,15 +193,15 @@ gqa_decode_kernel(DecodeParams p) {
 #pragma unroll
     for (int o = 8; o > 0; o >>= 1)
 #pragma unroll
-      for (int u = 0; u < U; ++u)
+      for (int u = 0; u < N; ++u)
 #pragma unroll
         for (int g = 0; g < G; ++g) s[u][g] += __shfl_xor_sync(0xffffffffu, s[u][g], o);
-    if (!valid[0]) continue;                   // the first key of a half-warp is past the range before the others are
+    if (!valid[0]) return;                     // the first key of a half-warp is past the range before the others are
 #pragma unroll
     for (int g = 0; g < G; ++g) {
       float mn = m[g];
 #pragma unroll
-      for (int u = 0; u < U; ++u) {
+      for (int u = 0; u < N; ++u) {
         if constexpr (KV != 0) s[u][g] *= row[u].ks;
         if (valid[u]) mn = fmaxf(mn, s[u][g]);
       }
@@ -196,14 +210,14 @@ gqa_decode_kernel(DecodeParams p) {
 #pragma unroll
       for (int i = 0; i < 8; ++i) acc[g][i] *= alpha;
 #pragma unroll
-      for (int u = 0; u < U; ++u) {
+      for (int u = 0; u < N; ++u) {
         s[u][g] = valid[u] ? exp2f(s[u][g] - mn) : 0.f;
         l[g] += s[u][g];
       }
       m[g] = mn;
     }
 #pragma unroll
-    for (int u = 0; u < U; ++u) {
+    for (int u = 0; u < N; ++u) {
       float vf[8];
       row[u].values(vf);
       if (!valid[u]) break;                    // (rows past the range repeat the first one's, which may hold anything)
@@ -212,6 +226,11 @@ gqa_decode_kernel(DecodeParams p) {
 #pragma unroll
         for (int i = 0; i < 8; ++i) acc[g][i] += s[u][g] * vf[i];
     }
+  };
+  // warp-uniform: every lane runs the shuffles
+  for (int base = k0; base < k1; base += 8 * U) {
+    if (k1 - base > 8) chunk(base, Int<U>());
+    else chunk(base, Int<1>());
   }
 
   const int st = warp * 2 + half;
@@ -282,7 +301,7 @@ static int decode_launch(int fmt, const void* q, const void* k_cache, const void
                          void* out, const void* gate, const int* block_table, const int* kv_len, float* workspace, int batch,
                          int max_blocks, int block_size, int n_q_heads, int n_kv_heads, int splits, float softmax_scale,
                          cudaStream_t stream) {
-  if (n_q_heads % n_kv_heads || splits < 1) return -6;
+  if (n_q_heads % n_kv_heads || splits < 1 || block_size < 1) return -6;
   const int G = n_q_heads / n_kv_heads;
   DecodeParams p;
   p.q = reinterpret_cast<const __nv_bfloat16*>(q);
@@ -295,6 +314,10 @@ static int decode_launch(int fmt, const void* q, const void* k_cache, const void
   p.gate = reinterpret_cast<const __nv_bfloat16*>(gate);
   p.max_blocks = max_blocks;
   p.bs = block_size;
+  int log2 = 0;
+  while ((1ll << log2) < block_size) ++log2;
+  p.bs_shift = 31 + log2;
+  p.bs_mul = (uint32_t)((1ull << p.bs_shift) / (unsigned)block_size + 1);
   p.Hq = n_q_heads;
   p.Hkv = n_kv_heads;
   p.splits = splits;

@@ -38,3 +38,48 @@ def test_key_counts_around_a_chunk(group, window, sinks):
         # half a unit of the result's bf16 is at most 2^-8 of it; fp32 scores of magnitude 40 are wrong by up to 2^-18 in the
         # exponent, and values of up to 5 weighted by their exponentials by 2^-15: 2^-12 leaves room for sums of 130 of them
         assert ((out.double() - want).abs() <= 2 ** -8 * want.abs() + 2 ** -12).all()
+
+
+# the 8-bit caches over the same key counts (1: E4M3, 2: INT8, 3: E4M3 keys and 4-bit values), and pages whose size is no power of two
+@pytest.mark.gpu
+@pytest.mark.parametrize("group", [1, 3, 5, 6])
+@pytest.mark.parametrize("fmt,bs", [(0, 1), (0, 5), (0, 48), (1, 16), (2, 48), (3, 7), (3, 64)])
+def test_every_cache_format_and_page_size(group, fmt, bs):
+    from deepseek_v4_2080ti_b200.ops import _lib, attention
+    g = torch.Generator(device="cuda").manual_seed(group * 8 + fmt)
+    hkv = 2
+    lens = [1, 2, 6, 7, 8, 9, 15, 16, 17, 23, 24, 25, 31, 32, 33, 47, 48, 49, 63, 65, 97, 130]
+    mb = (max(lens) + bs - 1) // bs + 1
+    b = len(lens)
+    bt = torch.randperm(b * mb, generator=g, device="cuda").to(torch.int32).view(b, mb).contiguous()
+    q = torch.randn(b, hkv * group, 128, generator=g, device="cuda").bfloat16()
+    kv_len = torch.tensor(lens, dtype=torch.int32, device="cuda")
+    shape = (b * mb, hkv, bs, 128)
+    byte = lambda *s: torch.randint(0, 256, s, generator=g, device="cuda", dtype=torch.uint8)
+    scale = lambda: torch.rand(*shape[:3], generator=g, device="cuda") * 0.01 + 0.002
+    if fmt == 0:
+        kc, vc = (torch.randn(shape, generator=g, device="cuda").bfloat16() for _ in range(2))
+        kd, vd = kc.double(), vc.double()
+        call = lambda n: attention.decode(q, kc, vc, bt, kv_len, splits=n, max_kv_len=max(lens))
+    else:
+        fp8 = lambda: torch.randn(shape, generator=g, device="cuda").mul(60).clamp(-400, 400).to(torch.float8_e4m3fn).view(torch.uint8)
+        ks, vs, vm = scale(), scale(), scale() - 0.007
+        k8 = byte(*shape) if fmt == 2 else fp8()
+        v8 = {1: fp8, 2: lambda: byte(*shape), 3: lambda: byte(*shape[:3], 64)}[fmt]()
+        value = lambda x: x.view(torch.int8).double() if fmt == 2 else x.view(torch.float8_e4m3fn).double()
+        kd = value(k8) * ks.double()[..., None]
+        if fmt == 3:
+            vd = torch.stack([v8 & 15, v8 >> 4], -1).flatten(-2).double() * vs.double()[..., None] + vm.double()[..., None]
+        else:
+            vd = value(v8) * vs.double()[..., None]
+        call = lambda n: attention.decode_kv8(fmt, q, k8, v8, ks, vs, bt, kv_len, splits=n, max_kv_len=max(lens), v_min=vm if fmt == 3 else None)
+    want = torch.empty(b, hkv * group, 128, dtype=torch.float64, device="cuda")
+    for i, n in enumerate(lens):
+        k, v = (c[bt[i].long()].permute(0, 2, 1, 3).reshape(-1, hkv, 128)[:n].repeat_interleave(group, 1) for c in (kd, vd))
+        w = torch.einsum("hd,nhd->hn", q[i].double(), k).mul(128 ** -0.5).softmax(-1)
+        want[i] = torch.einsum("hn,nhd->hd", w, v)
+    for splits in (1, 3):
+        out = call(splits)
+        torch.cuda.synchronize()
+        _lib.check_status()
+        assert ((out.double() - want).abs() <= 2 ** -8 * want.abs() + 2 ** -12).all()       # as above
