@@ -321,8 +321,8 @@ gemm_fp8_pair_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_const
         const int tt = tile - p.tail();
         const bool cut = len != p.kb;
         const int i0 = cut ? p.owner(tt * p.kb) : worker, i1 = cut ? p.owner(tt * p.kb + p.kb - 1) : worker;
-        auto part = [&](int i) {     // [4 features][token]
-          return p.partial + (((size_t)i * 2 + p.place(i, tt)) * 2 + rank) * PART + (size_t)group * (ROWS * BM) + row * 4;
+        auto part = [&](int i) {     // [4 features][token]; contributors after the first one begin within the tile
+          return p.partial + (((size_t)i * 2 + (i > i0 ? 0 : p.place(i, tt))) * 2 + rank) * PART + (size_t)group * (ROWS * BM) + row * 4;
         };
         if (mine) {
           float* dst = part(worker);
