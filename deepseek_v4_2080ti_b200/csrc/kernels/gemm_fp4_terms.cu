@@ -50,6 +50,7 @@ constexpr int A_COLS = 32;                   // tensor memory columns of a block
 
 struct Params {
   int R, N, kb, m_tiles, workers;
+  int most;                         // contributors of a tile that is cut, at most
   const int4* work;                 // {expert, pair of feature blocks, first row, rows}
   const int* num_work;
   const uint8_t* w;                 // [expert][m_tile][kb][BLOCK_BYTES]
@@ -57,7 +58,8 @@ struct Params {
   const int* row_outside;           // [R] the row has values that are not in its terms,
   const __nv_bfloat16* rest;        // [R][K] which are here among zeros (other rows undefined)
   __nv_bfloat16* out;               // [R, N]
-  float* partial;                   // [workers][2][MT][TOK][128]
+  float* partial;                   // [workers][2][MT][part_rows / 4][128][4]
+  int part_rows;                    // rows of a tile in `partial`: partial_rows(R)
   int* counters;                    // [workers], zero, left zero
   int* status;
   int vec;                          // even rows of `out`
@@ -72,7 +74,8 @@ constexpr int SR = (232448 - 2048 - SX * X_STAGE) / (MT * CODE_BYTES);     // st
 constexpr int A_COL = D_COLS, SF_COL = A_COL + SA * MT * A_COLS;
 constexpr uint32_t TMEM_COLS = 512;
 constexpr int SMEM = SX * X_STAGE + SR * MT * CODE_BYTES + 2048;
-constexpr int PART = MT * TOK * BM;
+// rows of a tile that partial sums are kept for: with fewer than TOK in all, none has more
+__host__ __device__ constexpr int partial_rows(int R) { return R < TOK ? (R + 3) / 4 * 4 : TOK; }
 static_assert(SF_COL + (MT + 1) * 4 <= 512 && SX > SA && SR >= 4 && SMEM <= 232448, "tensor and shared memory");
 
 __device__ __forceinline__ void epi_sync() { asm volatile("bar.sync 1, %0;" ::"n"(EPI_THREADS) : "memory"); }
@@ -181,7 +184,8 @@ gemm_fp4_terms_kernel(const __grid_constant__ CUtensorMap tmX, Params p) {
 
   const int tiles = *p.num_work, worker = blockIdx.x, waves = tiles / p.workers, tail = waves * p.workers;
   const int units = (tiles - tail) * p.kb;                    // of the tiles that are left, the first of them `tail`
-  const int workers = max(min(p.workers, units), 1);          // those that have some of them
+  const size_t part_size = (size_t)MT * BM * p.part_rows;
+  const int workers = max(min(p.workers, min(units, (tiles - tail) * p.most)), 1);          // those that have some of them
   auto first = [&](int i) { return (int)((long long)units * i / workers); };
   const int u0 = worker < workers ? first(worker) : 0, u1 = worker < workers ? first(worker + 1) : 0;
   // The pieces of tiles that this worker computes: f(tile, first K block, K blocks), until it returns false.
@@ -413,7 +417,7 @@ gemm_fp4_terms_kernel(const __grid_constant__ CUtensorMap tmX, Params p) {
       for (int t = lane; t < rows; t += 32) outside |= __ldg(p.row_outside + e.z + t);
       outside = __any_sync(0xffffffffu, outside != 0);
       const bool whole = len == p.kb && !outside;
-      float* mine = p.partial + ((size_t)worker * 2 + (u0 / p.kb == tile - tail ? 0 : 1)) * PART + m * TOK * BM + row;
+      float* mine = p.partial + ((size_t)worker * 2 + (u0 / p.kb == tile - tail ? 0 : 1)) * part_size + m * p.part_rows * BM + row * 4;
       const bool ok = __all_sync(0xffffffffu, mbar_wait(acc_full, piece & 1));
       tc_fence_after();
       if (!ok) {
@@ -433,9 +437,11 @@ gemm_fp4_terms_kernel(const __grid_constant__ CUtensorMap tmX, Params p) {
                 store2(q * 16 + t, __uint_as_float(hi[t]) + __uint_as_float(mid[t]),
                        __uint_as_float(hi[t + 1]) + __uint_as_float(mid[t + 1]));
             } else {
+              auto sum = [&](int t) { return __uint_as_float(hi[t]) + __uint_as_float(mid[t]); };
 #pragma unroll
-              for (int t = 0; t < 16; ++t)
-                if (q * 16 + t < rows) mine[(q * 16 + t) * BM] = __uint_as_float(hi[t]) + __uint_as_float(mid[t]);
+              for (int t = 0; t < 16; t += 4)
+                if (q * 16 + t < rows)
+                  *reinterpret_cast<float4*>(mine + (q * 16 + t) * BM) = make_float4(sum(t), sum(t + 1), sum(t + 2), sum(t + 3));
             }
           }
         tc_fence_before();
@@ -462,7 +468,7 @@ gemm_fp4_terms_kernel(const __grid_constant__ CUtensorMap tmX, Params p) {
                 if (x & 0x7fffffffu) sum += __uint_as_float(x) * weight_at(wb + (size_t)(k >> 7) * BLOCK_BYTES, row, (k & 127) + j);
               }
             }
-            mine[t * BM] += sum;
+            mine[(t & ~3) * BM + (t & 3)] += sum;
           }
         }
         // ---- the last contributor of a cut tile adds the partial sums in K order
@@ -480,18 +486,23 @@ gemm_fp4_terms_kernel(const __grid_constant__ CUtensorMap tmX, Params p) {
         epi_sync();
         if (*fix_last && busy) {
           __threadfence();
+          // contributors after the first one begin within the tile
+          const int place = first(i0) / p.kb == tile - tail ? 0 : 1;
+          const float* part = p.partial + m * p.part_rows * BM + row * 4;
           for (int t0 = 0; t0 < rows; t0 += 8) {
-            float v[8];
-#pragma unroll
-            for (int t = 0; t < 8; ++t) v[t] = 0.f;
+            float4 a = make_float4(0.f, 0.f, 0.f, 0.f), b = a;
+#pragma unroll 4
             for (int i = i0; i <= i1; ++i) {
-              const float* src = p.partial + ((size_t)i * 2 + (first(i) / p.kb == tile - tail ? 0 : 1)) * PART + m * TOK * BM + row;
-#pragma unroll
-              for (int t = 0; t < 8; ++t)
-                if (t0 + t < rows) v[t] += __ldcg(src + (t0 + t) * BM);
+              const float* src = part + ((size_t)i * 2 + (i == i0 ? place : 0)) * part_size;
+              const float4 c = __ldcg(reinterpret_cast<const float4*>(src + t0 * BM));
+              const float4 d = t0 + 4 < rows ? __ldcg(reinterpret_cast<const float4*>(src + (t0 + 4) * BM)) : make_float4(0.f, 0.f, 0.f, 0.f);
+              a.x += c.x; a.y += c.y; a.z += c.z; a.w += c.w;
+              b.x += d.x; b.y += d.y; b.z += d.z; b.w += d.w;
             }
-#pragma unroll
-            for (int t = 0; t < 8; t += 2) store2(t0 + t, v[t], v[t + 1]);
+            store2(t0, a.x, a.y);
+            store2(t0 + 2, a.z, a.w);
+            store2(t0 + 4, b.x, b.y);
+            store2(t0 + 6, b.z, b.w);
           }
         }
       }
@@ -521,10 +532,11 @@ using namespace b200;
 
 extern "C" {
 
-// Rows of a tile of a grouped product, floats of its partial sums, tile counters.
-int b200_fp4_terms_plan(int* tok, long long* partial_floats, int* counters) {
+// Rows of a tile of a grouped product, floats of the partial sums of one with R rows in all, tile counters.
+int b200_fp4_terms_plan(int R, int* tok, long long* partial_floats, int* counters) {
+  if (R <= 0) return -ERR_BAD_ARG;
   *tok = f4t::TOK;
-  *partial_floats = (long long)sm_count() * 2 * f4t::PART;
+  *partial_floats = (long long)sm_count() * 2 * f4t::MT * f4t::BM * f4t::partial_rows(R);
   *counters = sm_count();
   return 0;
 }
@@ -537,7 +549,7 @@ int b200_gemm_fp4_terms(const void* W, const void* xq, const void* sf, const int
                         int K, int groups, const void* work, const int* num_work, int max_work, float* partial, int* counters,
                         int* status, cudaStream_t stream) {
   const uintptr_t all = reinterpret_cast<uintptr_t>(W) | reinterpret_cast<uintptr_t>(xq) | reinterpret_cast<uintptr_t>(work) |
-                        reinterpret_cast<uintptr_t>(rest) | reinterpret_cast<uintptr_t>(out_bf16);
+                        reinterpret_cast<uintptr_t>(rest) | reinterpret_cast<uintptr_t>(out_bf16) | reinterpret_cast<uintptr_t>(partial);
   if (!W || !xq || !sf || !outside || !rest || !out_bf16 || !work || !num_work || !partial || !counters || all % 16 || R <= 0 || N <= 0 ||
       K <= 0 || K % 128 || groups <= 0 || max_work <= 0 || (long long)max_work * (K / 128) > 0x7fffffff ||
       (long long)groups * ((N + 127) / 128) > 0x7fffffff)
@@ -547,6 +559,11 @@ int b200_gemm_fp4_terms(const void* W, const void* xq, const void* sf, const int
   p.R = R; p.N = N; p.kb = K / 128;
   p.m_tiles = (N + 127) / 128;
   p.workers = sm_count();
+  // A K block takes some 0.45 us, a contributor's sums of 16 rows 0.35 us to read: of the tiles that are left after whole waves, too
+  // few for all SMs, each is shared by as many as make the sum of both least (8 experts of 4096 x 2048, 192 rows each: 170 us for 422
+  // with all SMs on the last four tiles, 32 contributors each).
+  const int rows = (R + groups - 1) / groups, sets = rows >= f4t::TOK ? f4t::TOK / 16 : (rows + 15) / 16;
+  for (p.most = 1; (p.most + 1) * (p.most + 1) * 7 * sets <= 9 * p.kb;) ++p.most;
   p.work = reinterpret_cast<const int4*>(work);
   p.num_work = num_work;
   p.w = reinterpret_cast<const uint8_t*>(W);
@@ -555,6 +572,7 @@ int b200_gemm_fp4_terms(const void* W, const void* xq, const void* sf, const int
   p.rest = reinterpret_cast<const __nv_bfloat16*>(rest);
   p.out = reinterpret_cast<__nv_bfloat16*>(out_bf16);
   p.partial = partial;
+  p.part_rows = f4t::partial_rows(R);
   p.counters = counters;
   p.status = status;
   p.vec = N % 2 == 0;

@@ -82,7 +82,7 @@ int b200_moe_gather_terms(const void* x, const int* row_token, const int* offset
                           int max_rows, int K, int* counters, int n_counters, cudaStream_t stream);
 int b200_moe_glu_terms(const void* gu, const int* offsets, int EL, void* xq, void* sf, int* outside, void* rest, int max_rows, int I,
                        float limit, float slope, int* counters, int n_counters, cudaStream_t stream);
-int b200_fp4_terms_plan(int* tok, long long* partial_floats, int* counters);
+int b200_fp4_terms_plan(int R, int* tok, long long* partial_floats, int* counters);
 int b200_gemm_fp4_terms(const void* W, const void* xq, const void* sf, const int* outside, const void* rest, void* out_bf16, int R, int N,
                         int K, int groups, const void* work, const int* num_work, int max_work, float* partial, int* counters, int* status, cudaStream_t stream);
 int b200_moe_combine(const void* y, const int* route_row, const float* wts, const void* base, void* out, int T, int K,

@@ -135,28 +135,28 @@ def pack_experts(gate: list[torch.Tensor], up: list[torch.Tensor], down: list[to
     return pack(w13), pack(w2)
 
 
-@functools.lru_cache(maxsize=1)
-def _fp4_terms_plan() -> tuple[int, int, int]:
-    """(rows of a tile, floats of partial sums, tile counters) of the block-scaled products"""
+@functools.lru_cache(maxsize=128)
+def _fp4_terms_plan(rows: int = 1 << 20) -> tuple[int, int, int]:
+    """(rows of a tile, floats of partial sums, tile counters) of the block-scaled products of ``rows`` rows in all"""
     tok, part, counters = ctypes.c_int(), ctypes.c_longlong(), ctypes.c_int()
-    _lib.check(_lib.lib().b200_fp4_terms_plan(ctypes.byref(tok), ctypes.byref(part), ctypes.byref(counters)), "fp4_terms_plan", 0)
+    _lib.check(_lib.lib().b200_fp4_terms_plan(min(rows, 1 << 20), ctypes.byref(tok), ctypes.byref(part), ctypes.byref(counters)), "fp4_terms_plan", 0)
     return tok.value, part.value, counters.value
 
 
 class _RowTerms:
-    """``r`` rows of ``k`` values as pairs of E4M3 terms (csrc/kernels/mx_terms.cuh), and the scratch of the product that takes them, in
-    one allocation."""
+    """``r`` rows of ``k`` values as pairs of E4M3 terms (csrc/kernels/mx_terms.cuh), and the tile counters of the product that takes
+    them, in one allocation."""
 
     def __init__(self, r: int, k: int, device):
-        _, part, self.n_counters = _fp4_terms_plan()
-        # terms, scales, flags, values outside the terms, partial sums, counters
-        sizes = (2 * r * k, r * k // 32, 4 * r, 2 * r * k, 4 * part, 4 * self.n_counters)
+        self.n_counters = _fp4_terms_plan()[2]
+        # terms, scales, flags, values outside the terms, counters
+        sizes = (2 * r * k, r * k // 32, 4 * r, 2 * r * k, 4 * self.n_counters)
         at = [0]
         for n in sizes:
             at.append(at[-1] + (n + 127) // 128 * 128)
         self.buf = torch.empty(at[-1], dtype=torch.uint8, device=device)
         base = self.buf.data_ptr()
-        *ptrs, self.partial, self.counters = (ctypes.c_void_p(base + o) for o in at[:-1])
+        *ptrs, self.counters = (ctypes.c_void_p(base + o) for o in at[:-1])
         self.ptrs = tuple(ptrs)
 
 
@@ -182,15 +182,18 @@ def experts_rows(x: torch.Tensor, idx: torch.Tensor, w13: ExpertWeights, w2: Exp
     bn = F32_TILE if f32 else gemm._bn(min(256, max(16, (r + el - 1) // el)))      # token tile sized for the average rows per expert
     if 3 <= w13.wfmt < WF_F32:
         bn = min(bn, int(L.b200_gguf_max_bn(w13.wfmt)), int(L.b200_gguf_max_bn(w2.wfmt)))
-    bn13, bn2 = (_fp4_terms_plan()[0] if m else bn for m in terms)
+    tile, floats, _ = _fp4_terms_plan(r) if any(terms) else (bn, 0, 0)
+    bn13, bn2 = (tile if m else bn for m in terms)
     bm = F32_TILE if f32 else 128
     mt13, mt2 = ((w.n + f - 1) // f for w, f in ((w13, 256 if terms[0] else bm), (w2, 256 if terms[1] else bm)))
     max_work = (mt13 + mt2) * ((r + min(bn13, bn2) - 1) // min(bn13, bn2) + el)
-    # the plan, in one allocation: work tables, counts, expert offsets, source token of every row
-    plan = torch.empty(8 * max_work + 4 + el + 1 + r, dtype=torch.int32, device=dev)
+    # the plan, in one allocation: work tables, counts, expert offsets, source token of every row; and room for the partial sums of the
+    # products that take terms, which run one after the other and share it
+    ints = (8 * max_work + 4 + el + 1 + r + 31) // 32 * 32
+    plan = torch.empty(ints + floats, dtype=torch.int32, device=dev)
     at = plan.data_ptr()
-    work13, work2, n13, n2, offsets, row_token = (ctypes.c_void_p(at + 4 * o) for o in (
-        0, 4 * max_work, 8 * max_work, 8 * max_work + 1, 8 * max_work + 4, 8 * max_work + 5 + el))
+    work13, work2, n13, n2, offsets, row_token, partial = (ctypes.c_void_p(at + 4 * o) for o in (
+        0, 4 * max_work, 8 * max_work, 8 * max_work + 1, 8 * max_work + 4, 8 * max_work + 5 + el, ints))
     route_row = torch.empty(t, k, dtype=torch.int32, device=dev)
     s = _lib.stream()
     rc = L.b200_moe_plan_ordered(_lib.ptr(idx), t, k, expert_lo, expert_lo + el, offsets, _lib.ptr(route_row),
@@ -201,13 +204,13 @@ def experts_rows(x: torch.Tensor, idx: torch.Tensor, w13: ExpertWeights, w2: Exp
         out = torch.empty(r, w.n, dtype=x.dtype, device=dev)
         if isinstance(a, _RowTerms):
             rc = L.b200_gemm_fp4_terms(_lib.ptr(w.weight), *a.ptrs, _lib.ptr(out), r, w.n, w.k, el, work, num, max_work,
-                                       a.partial, a.counters, _lib.ptr(_lib.status_word(dev)), s)
+                                       partial, a.counters, _lib.ptr(_lib.status_word(dev)), s)
         elif f32:
             rc = L.b200_gemm_f32_grouped(_lib.ptr(a), _lib.ptr(w.weight), _lib.ptr(out), w.n, w.k, work, num, max_work, s)
         else:
             grouped = L.b200_gemm_wdec_grouped if w.wfmt < 3 else L.b200_gemm_wdec_gguf_grouped
-            rc = grouped(w.wfmt, _lib.ptr(w.weight), _lib.ptr(w.scales), _lib.ptr(a), _lib.ptr(out), r, w.n, w.k, el,
-                         work, num, bn, _lib.ptr(_lib.status_word(dev)), s)
+            rc = grouped(w.wfmt, _lib.ptr(w.weight), _lib.ptr(w.scales), _lib.ptr(a), _lib.ptr(out), r,
+                         w.n, w.k, el, work, num, bn, _lib.ptr(_lib.status_word(dev)), s)
         _lib.check(rc, what)
         return out
 
@@ -222,6 +225,7 @@ def experts_rows(x: torch.Tensor, idx: torch.Tensor, w13: ExpertWeights, w2: Exp
         rc = L.b200_moe_gather(_lib.ptr(x), row_token, offsets, el, _lib.ptr(xs), r, 2 * h if f32 else h, s)
     _lib.check(rc, "moe_gather")
     gu = product(w13, xs, work13, n13, "grouped gemm w13")
+    del xs                                                # (given back in stream order: what follows may take its place)
     if terms[1]:
         act = _RowTerms(r, inter, dev)
         rc = L.b200_moe_glu_terms(_lib.ptr(gu), offsets, el, *act.ptrs, r, inter, ctypes.c_float(limit), ctypes.c_float(slope),
@@ -231,6 +235,7 @@ def experts_rows(x: torch.Tensor, idx: torch.Tensor, w13: ExpertWeights, w2: Exp
         rc = L.b200_moe_glu(_lib.ptr(gu), offsets, el, _lib.ptr(act), r, inter, ctypes.c_float(limit), ctypes.c_float(slope),
                             int(f32), s)
     _lib.check(rc, "moe_glu")
+    del gu
     return product(w2, act, work2, n2, "grouped gemm w2"), route_row
 
 

@@ -113,6 +113,27 @@ def test_values_outside_the_terms_reach_the_product():
     assert torch.equal(got[7].isnan(), ref[7].isnan()) and torch.equal(got[7].isinf(), ref[7].isinf()) and got[8].isfinite().all()
 
 
+# More tiles than SMs: whole waves of one tile a CTA, in which the rings wrap many times and phases pass from tile to tile, then a tail of
+# many tiles, of few (which have a bounded number of contributors each), of none.
+WAVES = [(300, 10240, 2048), (256, 9472, 640), (640, 9472, 1152), (64, 38400, 2304), (130, 25344, 384), (65, 18944, 4096)]
+
+
+@pytest.mark.parametrize("outliers", [False, True])
+@pytest.mark.parametrize("r,n,k", WAVES)
+def test_whole_waves_and_their_tail(r, n, k, outliers):
+    torch.manual_seed(r + n + k)
+    x = torch.randn(r, k, device="cuda")
+    if outliers:                                           # in rows of every token tile, whose feature tiles are in waves and in the tail
+        x[::9, ::37] *= 1e-4
+        x[::9, 5::64] = 3e8
+    x = x.bfloat16()
+    q, s, w = _weights(n, k)
+    got, again = _product(x, q, s), _product(x, q, s)
+    ref, size = x.double() @ w.t(), x.double().abs() @ w.abs().t()
+    assert torch.equal(got, again)
+    assert ((got.double() - ref).abs() <= ref.abs() * 2.0 ** -8 + size * k * 2.0 ** -24).all()
+
+
 def test_every_code_and_scale_comes_out():
     """A one-hot input of 1: the weight itself, under scales over the range that bf16 holds; 255 is taken as 254."""
     n, k = 256, 128
