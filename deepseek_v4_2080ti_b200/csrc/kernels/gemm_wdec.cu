@@ -187,7 +187,7 @@ extern "C" int b200_gemm_wdec_grouped(int wfmt, const void* W, const float* scal
     return -ERR_BAD_ARG;
   if (bn != 16 && bn != 32 && bn != 64 && bn != 128 && bn != 256) return -ERR_BAD_ARG;
   if (wfmt == WF_BF16 && (N % BM) != 0) return -ERR_BAD_ARG;
-  if (wfmt == WF_FP4 && (K % 64) != 0) return -ERR_BAD_ARG;
+  if ((wfmt == WF_FP4 && (K % 64) != 0) || (wfmt == WF_FP4_BLOCKS && (K % 128) != 0)) return -ERR_BAD_ARG;
   GemmParams p;
   memset(&p, 0, sizeof(p));
   p.T = rows_total; p.N = N; p.K = K;
@@ -202,7 +202,7 @@ extern "C" int b200_gemm_wdec_grouped(int wfmt, const void* W, const float* scal
   p.status = status;
   p.work_table = reinterpret_cast<const int4*>(work_table);
   p.num_work = num_work;
-  p.w_group_stride = (size_t)p.m_tiles * p.kb_total * raw_stage_bytes(wfmt);
+  p.w_group_stride = (size_t)p.m_tiles * p.kb_total * stored_stage_bytes(wfmt);
   p.scale_group_stride = (size_t)p.m_tiles * p.scale_ld;
   if (wfmt == WF_FP8_B128 && p.kb_total / 2 + 2 > 256) return -ERR_BAD_ARG;
   CUtensorMap tmW, tmX;
@@ -221,6 +221,7 @@ extern "C" int b200_gemm_wdec_grouped(int wfmt, const void* W, const float* scal
     return wfmt == WF_BF16       ? launch_one<BN_, WF_BF16>(tmW, tmX, p, stream)       \
            : wfmt == WF_FP8_B128 ? launch_one<BN_, WF_FP8_B128>(tmW, tmX, p, stream)   \
            : wfmt == WF_FP4      ? launch_one<BN_, WF_FP4>(tmW, tmX, p, stream)        \
+           : wfmt == WF_FP4_BLOCKS ? launch_one<BN_, WF_FP4_BLOCKS>(tmW, tmX, p, stream) \
                                  : -ERR_BAD_ARG;
   switch (bn) {
     B200_DISPATCH_G(16)

@@ -49,6 +49,8 @@ constexpr int DEC_WARP0 = 7;
 
 // WF_FP4: E2M1 nibbles (low nibble first) with one UE8M0 scale per 32 inputs, stored tile-major as
 // [m_tile][kb][128 rows x 32 code bytes | 128 rows x 2 scale bytes] (4352 bytes per stage).
+// WF_FP4_BLOCKS (grouped products): the same matrices as gemm_fp4_terms.cu has them, [m_tile][K / 128][4 x 128 rows x 16 code bytes |
+// 512 scale bytes, row r at 16 (r % 32) + 4 (r / 32)]; a stage takes half of a block's codes and its scales.
 // GGUF block formats keep their quantised bytes; they are only regrouped at load time so that one pipeline stage
 // (128 rows x 64 inputs) is a contiguous block [128 x QB quant bytes | 128 x SB scale bytes]:
 //   WF_Q8_0     QB 64 (int8), SB 4: two fp16 block scales
@@ -69,8 +71,9 @@ constexpr int DEC_WARP0 = 7;
 //               scale bytes (4 bits per 16 inputs); 512 x 8 magnitude grid + 128 sign bytes
 enum WFormat : int {
   WF_BF16 = 0, WF_FP8_B128 = 1, WF_FP4 = 2, WF_Q8_0 = 3, WF_Q4_K = 4, WF_Q2_K = 5, WF_IQ2_XXS = 6, WF_Q5_K = 7,
-  WF_IQ3_XXS = 8, WF_IQ1_M = 9, WF_Q6_K = 10, WF_Q3_K = 11, WF_IQ4_XS = 12, WF_IQ2_XS = 13
+  WF_IQ3_XXS = 8, WF_IQ1_M = 9, WF_Q6_K = 10, WF_Q3_K = 11, WF_IQ4_XS = 12, WF_IQ2_XS = 13, WF_FP4_BLOCKS = 14
 };
+constexpr int FP4_CODES = 128 * 64, FP4_SCALES = 128 * 4;      // bytes of a WF_FP4_BLOCKS block
 
 __host__ __device__ constexpr int gguf_qb(int wfmt) {
   return wfmt == WF_Q8_0 ? 64 : wfmt == WF_Q4_K ? 32 : wfmt == WF_Q2_K ? 16 : wfmt == WF_IQ2_XXS ? 16
@@ -85,8 +88,13 @@ __host__ __device__ constexpr int gguf_sb(int wfmt) {
 __host__ __device__ constexpr int raw_stage_bytes(int wfmt) {
   return wfmt == WF_FP8_B128 ? 128 * 64
          : wfmt == WF_FP4    ? 128 * 32 + 128 * 2
+         : wfmt == WF_FP4_BLOCKS ? FP4_CODES / 2 + FP4_SCALES
          : gguf_qb(wfmt)     ? 128 * (gguf_qb(wfmt) + gguf_sb(wfmt))
                              : 0;
+}
+
+__host__ __device__ constexpr int stored_stage_bytes(int wfmt) {      // what a stage takes of the stored matrix
+  return wfmt == WF_FP4_BLOCKS ? (FP4_CODES + FP4_SCALES) / 2 : raw_stage_bytes(wfmt);
 }
 
 struct GemmParams {
@@ -328,8 +336,8 @@ gemm_wdec_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constant_
       const Work wk = get_work<BN>(p, w);
       const int kb0 = wk.split * kb_per_split;
       const int kb1 = min(p.kb_total, kb0 + kb_per_split);
-      const uint8_t* wsrc = p.w_tiled + (size_t)wk.group * p.w_group_stride + ((size_t)wk.m_tile * p.kb_total + kb0) * L::RAW_BYTES;
-      for (int kb = kb0; kb < kb1; ++kb, ++it, wsrc += L::RAW_BYTES) {
+      const uint8_t* wsrc = p.w_tiled + (size_t)wk.group * p.w_group_stride + ((size_t)wk.m_tile * p.kb_total + kb0) * stored_stage_bytes(WFMT);
+      for (int kb = kb0; kb < kb1; ++kb, ++it) {
         const int s = it % S;
         const bool got = mbar_wait(&empty[s], ((it / S) & 1) ^ 1);
         stop = !__all_sync(0xffffffffu, got && *abort_flag == 0);
@@ -346,7 +354,15 @@ gemm_wdec_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constant_
         } else {
           // quantised weights are stored tile-major: one contiguous block per (m_tile, kb)
           mbar_expect_tx_warp(on, &tma_full[s], L::RAW_BYTES);
-          bulk_load_warp(on, sRaw + s * L::RAW_BYTES, wsrc, L::RAW_BYTES, &tma_full[s]);
+          if constexpr (WFMT == WF_FP4_BLOCKS) {
+            const int half = kb & 1;         // grouped products are not split: kb0 is 0
+            bulk_load_warp(on, sRaw + s * L::RAW_BYTES, wsrc + half * (FP4_CODES / 2), FP4_CODES / 2, &tma_full[s]);
+            bulk_load_warp(on, sRaw + s * L::RAW_BYTES + FP4_CODES / 2, wsrc + FP4_CODES, FP4_SCALES, &tma_full[s]);
+            wsrc += half * (FP4_CODES + FP4_SCALES);
+          } else {
+            bulk_load_warp(on, sRaw + s * L::RAW_BYTES, wsrc, L::RAW_BYTES, &tma_full[s]);
+            wsrc += L::RAW_BYTES;
+          }
         }
       }
     }
@@ -543,17 +559,18 @@ gemm_wdec_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constant_
               *reinterpret_cast<uint4*>(rowp + (((2 * c) ^ sw) << 4)) = o0;
               *reinterpret_cast<uint4*>(rowp + (((2 * c + 1) ^ sw) << 4)) = o1;
             }
-          } else if constexpr (WFMT == WF_FP4) {
-            // 128 rows x 32 code bytes, then 128 x 2 scale bytes; a 16-byte chunk = 32 values = one scale group.
+          } else if constexpr (WFMT == WF_FP4 || WFMT == WF_FP4_BLOCKS) {
+            // 128 rows x 32 code bytes, then their scale bytes; a 16-byte chunk = 32 values = one scale group.
             constexpr int REPS = (BM * 2) / GT;
-            const uint8_t* sc_bytes = raw + BM * 32;
+            constexpr bool BLOCKS = WFMT == WF_FP4_BLOCKS;
+            const uint8_t* sc_bytes = raw + BM * 32 + (BLOCKS ? 2 * (kb & 1) : 0);
 #pragma unroll
             for (int rep = 0; rep < REPS; ++rep) {
               const int i = d + rep * GT;
-              const int r = i >> 1, hh = i & 1;       // row, which half of the 64-wide K tile
-              const uint4 qv = *reinterpret_cast<const uint4*>(raw + r * 32 + hh * 16);
+              const int r = BLOCKS ? i & (BM - 1) : i >> 1, hh = BLOCKS ? i / BM : i & 1;       // row, which half of the 64-wide K tile
+              const uint4 qv = *reinterpret_cast<const uint4*>(raw + (BLOCKS ? hh * (BM * 16) + r * 16 : r * 32 + hh * 16));
               // 2^(e-127) is a bf16 with biased exponent e; 2^-127 is below the normal numbers
-              const uint32_t e = sc_bytes[r * 2 + hh];
+              const uint32_t e = sc_bytes[BLOCKS ? (r & 31) * 16 + (r >> 5) * 4 + hh : r * 2 + hh];
               const uint32_t s1 = e ? min(e, 254u) << 7 : 0x40u;
               const uint32_t sw2 = s1 | (s1 << 16);
               const uint32_t qq[4] = {qv.x, qv.y, qv.z, qv.w};

@@ -461,8 +461,8 @@ class MlaMoeGpuRuntime:
             return self.comm.all_reduce(lw.offload.forward(x, idx, wts, cfg.swiglu_limit, base))
         if getattr(self.comm, "world", 1) > 1 and hasattr(self.comm, "moe_combine"):
             # weighted combine + sum over the expert-parallel ranks in one peer-memory kernel
-            return moe.experts_forward(x, idx, wts, lw.w13, lw.w2, self.w.expert_lo, cfg.swiglu_limit, base, comm=self.comm)
-        y = moe.experts_forward(x, idx, wts, lw.w13, lw.w2, self.w.expert_lo, cfg.swiglu_limit, base)
+            return moe.experts_forward(x, idx, wts, lw.w13, lw.w2, self.w.expert_lo, cfg.swiglu_limit, base, comm=self.comm, total=cfg.num_experts)
+        y = moe.experts_forward(x, idx, wts, lw.w13, lw.w2, self.w.expert_lo, cfg.swiglu_limit, base, total=cfg.num_experts)
         return self.comm.all_reduce(y)
 
     @torch.no_grad()

@@ -13,6 +13,7 @@ from . import _lib, gemm
 from .gemm import WF_BF16, WF_FP8_B128
 
 WF_FP4 = 2
+WF_FP4_BLOCKS = 14              # FP4 as gemm_fp4_terms.cu stores it, to the decode-warp kernel
 WF_F32 = 100                   # not a GEMM format: plain fp32 matrices on the CUDA cores (gemm_f32.cu)
 # softmax_chosen: softmax over the chosen logits only, the bias belongs to the logits
 SCORE_FN = {"softmax": 0, "sigmoid": 1, "sqrtsoftplus": 2, "softmax_chosen": 3}
@@ -160,15 +161,31 @@ class _RowTerms:
         self.ptrs = tuple(ptrs)
 
 
+def fp4_terms_pay(rows: int, total: int, w13: ExpertWeights, w2: ExpertWeights) -> bool:
+    """Do block-scaled FP4 experts take ``rows`` rows, spread over ``total`` experts of which some are held here, as terms
+    (gemm_fp4_terms.cu), or are they unpacked to bf16 (gemm_wdec.cu)?  Times of a block unpacked over those of terms, even and skewed
+    routing, by rows of an expert:
+
+    * terms cost the same for tiles of 64 rows whatever is in them; unpacked weights serve tiles of up to 256.  256 experts of 4096 x
+      2048: 16 rows 2.6 and 2.8, 64 rows 1.7, 80 to 160 rows 1.0 to 1.3, 192 rows 0.84 and 1.2, 512 rows 0.92; 32 experts: 16 rows 2.2,
+      64 rows 1.4 and 1.5, 80 to 160 rows 0.96 to 1.2, 256 rows 0.96, 1024 rows 0.8.
+    * few experts leave the waves of terms short: 8 of 4096 x 2048, 24 to 64 rows 1.0 to 1.3, 80 to 160 rows 0.83 to 1.0; 16 of 3072 x
+      1536, 80 to 160 rows 0.92 to 1.0.
+    * with less than some ten blocks of 256 x 128 weights an SM, the fixed parts decide: 8 of 2048 x 768 0.82 to 1.1; 4 of 3072 x 1536 and
+      2 of 4096 x 2048, one row each, 1.04 and 1.25."""
+    blocks = (w13.n + 255) // 256 * (w13.k // 128) + (w2.n + 255) // 256 * (w2.k // 128)
+    return min(w13.experts, rows) * blocks >= 10 * gemm.NUM_SMS and rows <= (160 if w13.experts >= 32 else 64) * total
+
+
 F32_TILE = 64                   # rows and features of a tile of the fp32 grouped GEMM
 
 
 def experts_rows(x: torch.Tensor, idx: torch.Tensor, w13: ExpertWeights, w2: ExpertWeights, expert_lo: int = 0,
-                 limit: float = 0.0, slope: float = 0.0) -> tuple[torch.Tensor, torch.Tensor]:
+                 limit: float = 0.0, slope: float = 0.0, total: int | None = None) -> tuple[torch.Tensor, torch.Tensor]:
     """Outputs of the experts [expert_lo, expert_lo + E) held here for their tokens, in expert order (y [T k, w2.n]), and the
     row of every route (int32 [T, k], -1: not held here).  x [T, H] bf16 (fp32 for fp32 weights); w13: [E] x [2I, H] (gate
     rows then up rows); w2: [E] x [H', I].  The unit is SwiGLU with the optional clamp ``limit``, or with ``slope`` the
-    clamped one-plus form of csrc/kernels/glu.cuh."""
+    clamped one-plus form of csrc/kernels/glu.cuh.  ``total``: the experts that the ids range over, where more than those held here."""
     L = _lib.lib()
     t, h = x.shape
     k = idx.shape[1]
@@ -178,11 +195,12 @@ def experts_rows(x: torch.Tensor, idx: torch.Tensor, w13: ExpertWeights, w2: Exp
     dev = x.device
     f32 = w13.wfmt == WF_F32
     assert x.dtype == (torch.float32 if f32 else torch.bfloat16) and x.is_contiguous() and h == w13.k
-    terms = [w.block_scaled for w in (w13, w2)]           # products that take their rows as pairs of E4M3 terms
+    pay = (w13.block_scaled or w2.block_scaled) and fp4_terms_pay(r, max(total or el, el), w13, w2)
+    terms = [w.block_scaled and pay for w in (w13, w2)]   # products that take their rows as pairs of E4M3 terms
     bn = F32_TILE if f32 else gemm._bn(min(256, max(16, (r + el - 1) // el)))      # token tile sized for the average rows per expert
     if 3 <= w13.wfmt < WF_F32:
         bn = min(bn, int(L.b200_gguf_max_bn(w13.wfmt)), int(L.b200_gguf_max_bn(w2.wfmt)))
-    tile, floats, _ = _fp4_terms_plan(r) if any(terms) else (bn, 0, 0)
+    tile, floats, _ = _fp4_terms_plan(r) if pay else (bn, 0, 0)
     bn13, bn2 = (tile if m else bn for m in terms)
     bm = F32_TILE if f32 else 128
     mt13, mt2 = ((w.n + f - 1) // f for w, f in ((w13, 256 if terms[0] else bm), (w2, 256 if terms[1] else bm)))
@@ -209,7 +227,7 @@ def experts_rows(x: torch.Tensor, idx: torch.Tensor, w13: ExpertWeights, w2: Exp
             rc = L.b200_gemm_f32_grouped(_lib.ptr(a), _lib.ptr(w.weight), _lib.ptr(out), w.n, w.k, work, num, max_work, s)
         else:
             grouped = L.b200_gemm_wdec_grouped if w.wfmt < 3 else L.b200_gemm_wdec_gguf_grouped
-            rc = grouped(w.wfmt, _lib.ptr(w.weight), _lib.ptr(w.scales), _lib.ptr(a), _lib.ptr(out), r,
+            rc = grouped(WF_FP4_BLOCKS if w.block_scaled else w.wfmt, _lib.ptr(w.weight), _lib.ptr(w.scales), _lib.ptr(a), _lib.ptr(out), r,
                          w.n, w.k, el, work, num, bn, _lib.ptr(_lib.status_word(dev)), s)
         _lib.check(rc, what)
         return out
@@ -241,16 +259,16 @@ def experts_rows(x: torch.Tensor, idx: torch.Tensor, w13: ExpertWeights, w2: Exp
 
 def experts_forward(x: torch.Tensor, idx: torch.Tensor, wts: torch.Tensor, w13: ExpertWeights, w2: ExpertWeights,
                     expert_lo: int, swiglu_limit: float = 0.0, base: torch.Tensor | None = None, comm=None,
-                    residual: torch.Tensor | None = None, comm_mode: int = 0) -> torch.Tensor:
+                    residual: torch.Tensor | None = None, comm_mode: int = 0, total: int | None = None) -> torch.Tensor:
     """out[t] = base[t] + sum_k wts[t,k] * Expert_{idx[t,k]}(x[t]) over the experts [expert_lo, expert_lo + E) held here.
-    x [T, H] bf16; w13: [E] x [2I, H] (gate rows then up rows); w2: [E] x [H, I].
+    x [T, H] bf16; w13: [E] x [2I, H] (gate rows then up rows); w2: [E] x [H, I]; ``total`` as in ``experts_rows``.
 
     With ``comm`` (a peer-memory communicator of an expert-parallel group) the weighted combine, the sum over ranks
     and the residual add run as one kernel over NVLink (``PeerComm.moe_combine``): every rank gets
     ``residual + sum_ranks(base_r + local routes)``."""
     t, h = x.shape
     k = idx.shape[1]
-    y, route_row = experts_rows(x, idx, w13, w2, expert_lo, swiglu_limit)
+    y, route_row = experts_rows(x, idx, w13, w2, expert_lo, swiglu_limit, total=total)
     if comm is not None and getattr(comm, "world", 1) > 1:
         return comm.moe_combine(y, route_row, wts, base, residual, t, k, h, comm_mode)
     if residual is not None:

@@ -178,3 +178,85 @@ def test_experts_match_the_general_path(t, lo, monkeypatch):
     assert torch.equal(a, again)
     # sums in another order move a rounding to bf16 now and then, twice on the way and once at the end
     assert ((a.double() - b.double()).norm() / b.double().norm()).item() < 2.0 ** -8
+
+
+def _decode_layout(q, scales):
+    """One matrix of whole 128-blocks as the decode-warp kernel has matrices of other widths."""
+    n, kk = q.shape[0], q.shape[1] * 2
+    codes = q.view(n // 128, 128, kk // 64, 32).permute(0, 2, 1, 3).reshape(n // 128, kk // 64, -1)
+    sc = scales.view(n // 128, 128, kk // 64, 2).permute(0, 2, 1, 3).reshape(n // 128, kk // 64, -1)
+    return torch.cat([codes, sc], -1)
+
+
+# rows per expert around the token tiles of the decode-warp kernel (16 to 256)
+@pytest.mark.parametrize("t,h,inter", [(1, 128, 128), (20, 384, 256), (70, 640, 128), (150, 256, 384), (300, 384, 256), (900, 2048, 384)])
+def test_both_layouts_through_the_decode_warps(t, h, inter, monkeypatch):
+    """The same codes and scales, in the same order of sums: equal results."""
+    from deepseek_v4_2080ti_b200.ops import _lib, moe
+    torch.manual_seed(t)
+    el, k = 8, 3
+    m13, m2 = ([_weights(n, kk)[:2] for _ in range(el)] for n, kk in ((2 * inter, h), (h, inter)))
+    w13, w2 = (moe.ExpertWeights.from_fp4(*map(list, zip(*m))) for m in (m13, m2))
+    x = torch.randn(t, h, device="cuda").bfloat16()
+    idx = torch.rand(t, el, device="cuda").topk(k).indices.int().contiguous()
+    wts = torch.rand(t, k, device="cuda")
+    monkeypatch.setattr(moe, "fp4_terms_pay", lambda *a: False)
+    a = moe.experts_forward(x, idx, wts, w13, w2, 0, swiglu_limit=2.0)
+    monkeypatch.setattr(moe.ExpertWeights, "block_scaled", False)
+    w13.weight, w2.weight = (torch.stack([_decode_layout(*q) for q in m]) for m in (m13, m2))
+    b = moe.experts_forward(x, idx, wts, w13, w2, 0, swiglu_limit=2.0)
+    torch.cuda.synchronize()
+    _lib.check_status()
+    assert torch.equal(a, b)
+
+
+@pytest.mark.parametrize("terms", [True, False])
+@pytest.mark.parametrize("t", [1, 30, 400])
+@pytest.mark.parametrize("h,inter", [(256, 192), (192, 256)])
+def test_one_matrix_of_whole_blocks_beside_another(t, h, inter, terms, monkeypatch):
+    """Hidden or expert width of 64-blocks only: one product may take terms, the other unpacks."""
+    from deepseek_v4_2080ti_b200.ops import _lib, moe
+    monkeypatch.setattr(moe, "fp4_terms_pay", lambda *a: terms)
+    torch.manual_seed(t + h)
+    el, k = 4, 2
+    m13, m2 = ([_weights(n, kk, 1) for _ in range(el)] for n, kk in ((2 * inter, h), (h, inter)))
+    w13, w2 = (moe.ExpertWeights.from_fp4([q[0] for q in m], [q[1] for q in m]) for m in (m13, m2))
+    assert w13.block_scaled != w2.block_scaled
+    x = (torch.randn(t, h, device="cuda") * 0.02).bfloat16()
+    idx = torch.rand(t, el, device="cuda").topk(k).indices.int().contiguous()
+    wts = torch.rand(t, k, device="cuda")
+    got = moe.experts_forward(x, idx, wts, w13, w2, 0).double()
+    torch.cuda.synchronize()
+    _lib.check_status()
+    want = torch.zeros(t, h, dtype=torch.float64, device="cuda")
+    for e in range(el):
+        rows, col = (idx == e).nonzero(as_tuple=True)
+        gu = x[rows].double() @ m13[e][2].t()
+        act = torch.nn.functional.silu(gu[:, :inter]) * gu[:, inter:]
+        want.index_add_(0, rows, wts[rows, col].double()[:, None] * (act @ m2[e][2].t()))
+    # four roundings to bf16 on the way (gate, up, unit, expert) and one at the end
+    assert ((got - want).norm() / want.norm()).item() < 2.0 ** -7
+
+
+# the same shapes and ranges of held experts as above, one with as many tiles as SMs and more, and one whose rows are few for many SMs
+@pytest.mark.parametrize("t,lo,el,h,inter", [(1, 0, 8, 384, 256), (9, 0, 8, 384, 256), (40, 2, 8, 384, 256), (300, 2, 8, 384, 256),
+                                             (1100, 0, 8, 384, 256), (700, 0, 48, 1024, 512), (6, 0, 8, 2048, 768)])
+def test_experts_as_terms_match_the_unpacked(t, lo, el, h, inter, monkeypatch):
+    """Both routes of block-scaled experts: exact but for fp32 sums and the same roundings."""
+    from deepseek_v4_2080ti_b200.ops import _lib, moe
+    torch.manual_seed(t)
+    k = 3
+    m13, m2 = ([fp4fmt.quantize(torch.randn(n, kk, device="cuda") * 0.1) for _ in range(el)] for n, kk in ((2 * inter, h), (h, inter)))
+    w13, w2 = (moe.ExpertWeights.from_fp4(*map(list, zip(*m))) for m in (m13, m2))
+    x = torch.randn(t, h, device="cuda").bfloat16()
+    idx = torch.rand(t, el + 4, device="cuda").topk(k).indices.int().contiguous()
+    wts = torch.rand(t, k, device="cuda")
+    out = []
+    for terms in (True, True, False):
+        monkeypatch.setattr(moe, "fp4_terms_pay", lambda *a: terms)
+        out.append(moe.experts_forward(x, idx, wts, w13, w2, lo, swiglu_limit=2.0))
+    torch.cuda.synchronize()
+    _lib.check_status()
+    assert torch.equal(out[0], out[1])
+    # sums in another order move a rounding to bf16 now and then, twice on the way and once at the end
+    assert ((out[0].double() - out[2].double()).norm() / out[2].double().norm()).item() < 2.0 ** -8
