@@ -19,7 +19,7 @@ WF_F32 = 100                   # not a GEMM format: plain fp32 matrices on the C
 SCORE_FN = {"softmax": 0, "sigmoid": 1, "sqrtsoftplus": 2, "softmax_chosen": 3}
 
 
-def prepack_fp4(packed: torch.Tensor, scale_e8m0: torch.Tensor) -> torch.Tensor:
+def prepack_fp4(packed: torch.Tensor, scale_e8m0: torch.Tensor, out: torch.Tensor | None = None) -> torch.Tensor:
     """FP4 weight (uint8 [N, K/2] two codes per byte, low nibble first; E8M0 uint8 [N, K/32]) -> the tile-major layout of the
     product that takes it.  Whole blocks of 128 inputs (``gemm_fp4_terms.cu``): uint8 [ceil(N/128), K/128, 8704], 16 code bytes (32
     inputs) of each of 128 rows four times, then their 128 x 4 scales with row r at 16 (r % 32) + 4 (r / 32), 255 (NaN to the tensor
@@ -32,13 +32,17 @@ def prepack_fp4(packed: torch.Tensor, scale_e8m0: torch.Tensor) -> torch.Tensor:
         packed = torch.cat([packed, packed.new_zeros(npad - n, kh)])
         scale_e8m0 = torch.cat([scale_e8m0, scale_e8m0.new_zeros(npad - n, k // 32)])
     mt, bk = npad // 128, 128 if k % 128 == 0 else 64
+    codes = bk * 64
+    if out is None:
+        out = packed.new_empty(mt, k // bk, codes + bk * 4)
+    # one pass over the codes and one over the scales, straight to their places
     if bk == 128:
-        codes = packed.view(mt, 128, k // 128, 4, 16).permute(0, 2, 3, 1, 4).reshape(mt, k // 128, -1)
-        sc = scale_e8m0.clamp(max=254).view(mt, 4, 32, k // 128, 4).permute(0, 3, 2, 1, 4).reshape(mt, k // 128, -1)
+        out[..., :codes].unflatten(-1, (4, 128, 16)).copy_(packed.view(mt, 128, k // 128, 4, 16).permute(0, 2, 3, 1, 4))
+        torch.clamp(scale_e8m0.view(mt, 4, 32, k // 128, 4).permute(0, 3, 2, 1, 4), max=254, out=out[..., codes:].unflatten(-1, (32, 4, 4)))
     else:
-        codes = packed.view(mt, 128, k // 64, 32).permute(0, 2, 1, 3).reshape(mt, k // 64, -1)
-        sc = scale_e8m0.view(mt, 128, k // 64, 2).permute(0, 2, 1, 3).reshape(mt, k // 64, -1)
-    return torch.cat([codes, sc], -1).contiguous()
+        out[..., :codes].unflatten(-1, (128, 32)).copy_(packed.view(mt, 128, k // 64, 32).permute(0, 2, 1, 3))
+        out[..., codes:].unflatten(-1, (128, 2)).copy_(scale_e8m0.view(mt, 128, k // 64, 2).permute(0, 2, 1, 3))
+    return out
 
 
 @dataclass
@@ -59,7 +63,11 @@ class ExpertWeights:
     @staticmethod
     def from_fp4(packed: list[torch.Tensor], scales: list[torch.Tensor]) -> "ExpertWeights":
         n, kh = packed[0].shape
-        w = torch.stack([prepack_fp4(p, s) for p, s in zip(packed, scales)])
+        first = prepack_fp4(packed[0], scales[0])
+        w = first.new_empty(len(packed), *first.shape)
+        w[0] = first
+        for i in range(1, len(packed)):
+            prepack_fp4(packed[i], scales[i], w[i])
         return ExpertWeights(WF_FP4, w, None, n, kh * 2, len(packed))
 
     @staticmethod
