@@ -8,7 +8,7 @@
 // per 1024 tensor cycles), doubled the time (978 against 670 us for 1920 x 34816 x 5120).
 //
 // Measured, us per product in a graph of 16 (12288 x 5120, 5120 x 4096, 34816 x 5120, 5120 x 17408): 333
-// tokens 64, 37, 155, 81; 1901 tokens 220 to 260, 83 to 100, 575 to 605, 300 to 310 (the larger ones go with the power limit).  The split of
+// tokens 65, 35.5, 155, 79; 1901 tokens 205 to 260, 83 to 100, 553 to 643, 295 to 310 (the larger ones go with the power limit).  The split of
 // the activations, 5 us at 333 tokens and 13 to 55 at 1901, is not counted.  The decode-warp kernel, which needs none, as it is
 // now: 333 tokens 82, 40, 188, 138; 1901 tokens 266, 96, 790, 468.  Where it is the faster one with the split counted, `linear` takes it
 // (terms_pay in ops/gemm.py).

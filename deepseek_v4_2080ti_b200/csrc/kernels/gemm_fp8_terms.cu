@@ -605,8 +605,8 @@ static int launch(const Params& p, cudaStream_t stream) {
 // CTAs (pairs) that share `tiles` tiles of `kb` blocks.  Enough tiles: all of them, in equal runs.  Where every tile is cut more
 // than once, each contributor costs the last one a read of its partial sums, about as long as two blocks of one CTA or four of a
 // pair, so a tile takes some sqrt(kb / 2) (kb / 4) contributors at most; and a whole number of them, so that none works on two cut
-// tiles.  us with its split, against all SMs: 576 x 7168 9.4 for 20 at 1 token, 15 for 37 at 64, 31 for 80 on pairs at 65;
-// 2048 x 5120 8.9 for 13, 15 for 23, 29 for 46; 5120 x 4096 9.6 for 12.6, 15 for 21, 28 for 37.
+// tiles.  us with its split, against all SMs: 576 x 7168 9.4 for 11.2 at 1 token, 14.5 for 25 at 64, 20 for 43 at 65, 36 for 63 on pairs
+// at 129; 2048 x 5120 at 1, 64, 129 tokens 8.9 for 11, 14.8 for 18, 29 for 42; 5120 x 4096 9.7 for 11.9, 15.6 for 18, 30 for 36.
 static int workers(int tiles, int kb, int cg) {
   const int all = sm_count() / cg;
   if (2 * tiles > all) return all < tiles * kb ? all : tiles * kb;

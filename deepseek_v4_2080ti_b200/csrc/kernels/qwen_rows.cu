@@ -124,8 +124,11 @@ int b200_step_meta(const int* rows, int B, const int* ids, const int* tables, in
   return 0;
 }
 
-// scratch == null: scratch_bytes is set to what a call needs, and nothing runs.
-int b200_qwen_rows(const B200QwenRowsLayer* layers, int n_layers, B200QwenRows* r, float eps, float softmax_scale, cudaStream_t stream) {
+// scratch == null: scratch_bytes is set to what a call needs, and nothing runs.  layer_words, row_words: 64-bit words of a layer and of
+// `r` as the caller has them.
+int b200_qwen_rows(const B200QwenRowsLayer* layers, int n_layers, int layer_words, B200QwenRows* r, int row_words, float eps,
+                   float softmax_scale, cudaStream_t stream) {
+  if (!layers || !r || layer_words * 8 != (int)sizeof(B200QwenRowsLayer) || row_words * 8 != (int)sizeof(B200QwenRows)) return -6;
   const int T = (int)r->T, H = (int)r->H, I = (int)r->I, hq = (int)r->hq, hkv = (int)r->hkv, hk = (int)r->hk, hv = (int)r->hv;
   const int kd = hk * 128, vd = hv * 128, cw = 2 * kd + vd, qd = hq * 128;
   int tok, counters;

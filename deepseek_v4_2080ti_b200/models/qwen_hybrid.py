@@ -710,7 +710,9 @@ class QwenHybridRuntime(PagedSequences):
 
     def _issues_natively(self, t: int, meta, slot: int | None) -> bool:
         """Does a prompt portion of ``t`` tokens go through the layers in one native call (csrc/kernels/qwen_rows.cu)?  One rank, a
-        bf16 cache, FP8 products that all take terms; not while launches are looked at one by one."""
+        bf16 cache (an 8-bit one stages its rows around the attention, which that call has no steps for), FP8 products that all take
+        terms, heads that the one kernel for the gates takes (it has no other for them); not while launches are looked at one by
+        one.  Other portions are issued from here, layer by layer."""
         return slot is not None and meta["mode"] == "prefill" and self.kv8 is None and not self._sp and not PROFILER.enabled and \
             not _lib.bounds_checks_on() and gdn.ab_gates_fit(t, self.cfg.hidden_size, self.hv_lin) and \
             all(self._terms_rows(t, lw) for lw in self.w.layers)
@@ -745,7 +747,7 @@ class QwenHybridRuntime(PagedSequences):
                 at(kv_slots), at(bt), at(meta["q_start"]), at(meta["q_len"]), at(meta["kv_len"]), at(h), at(delta), 0, 0,
                 at(_lib.status_word(h.device)), 0]
         run = (ctypes.c_longlong * len(call))(*call)
-        args = (table, len(self.w.layers), run, ctypes.c_float(cfg.rms_norm_eps), ctypes.c_float(1.0 / math.sqrt(cfg.head_dim)), s)
+        args = (table, len(self.w.layers), len(rows) // len(self.w.layers), run, len(call), ctypes.c_float(cfg.rms_norm_eps), ctypes.c_float(1.0 / math.sqrt(cfg.head_dim)), s)
         _lib.check(L.b200_qwen_rows(*args), "qwen_rows plan", 0)
         scratch = torch.empty(run[24], dtype=torch.uint8, device=h.device)
         run[23] = scratch.data_ptr()

@@ -34,7 +34,9 @@ def chunked(mixed, q_off, k_off, v_off, g, beta, state, hv, hk):
     return out
 
 
-AB_GATES_MAX_T = 2047           # longest portion whose gates ``ab_gates`` makes (csrc/kernels/gdn_ab_gates.cu)
+# Longest portion whose gates ``ab_gates`` makes (csrc/kernels/gdn_ab_gates.cu).  us against projection and gates apart, 32 heads of 5120
+# inputs: 40 tokens 6.6 / 19, 1024 9.0 / 19, 1536 16.6 / 19, 2047 17.1 / 19.1, 3000 25 / 19.2, 8192 70 / 20.8.
+AB_GATES_MAX_T = 2047
 
 
 def ab_gates_fit(t: int, hidden: int, hv: int) -> bool:

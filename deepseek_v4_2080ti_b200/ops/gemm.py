@@ -312,7 +312,7 @@ def pick_splits_f32(t: int, n: int, k: int) -> int:
 
 
 STREAM_MAX_T = 32   # token counts served by the weight-streaming FP8 kernel (csrc/kernels/gemm_w8a8s.cu)
-TERMS_SINGLE_T = 64  # token counts the one-CTA form of ``linear_terms`` serves
+TERMS_SINGLE_T = 64  # token counts for which terms always pay, and whose decode steps hand them from kernel to kernel
 
 
 def stream_layout(t: int) -> tuple[int, int]:
@@ -457,14 +457,14 @@ def terms_pay(t: int, n: int, k: int) -> bool:
     """Is splitting ``t`` bf16 rows and ``linear_terms`` the fastest product with an [n, k] FP8 matrix?  us with the split, against
     the kernel that is taken otherwise, in graphs of 16 products:
 
-    * up to 64 tokens: yes (5120 x 4096 9.6 for 14.4 of the decode-warp kernel at 1 token, 15 for 41 at 64; 34816 x 5120 33 for
-      62, 45 for 193; 576 x 7168 9.4 for 12, 15 for 37).
-    * up to 128: yes where the decode-warp kernel must split K to fill the SMs (12288 x 5120 37 for 55 at 128, 5120 x 17408 51 for
-      67), no where its 128-token tiles fill them (34816 x 5120 63 for 59 at 65, 74 for 62 at 128).
+    * up to 64 tokens: yes (5120 x 4096 9.7 for 14.1 of the decode-warp kernel at 1 token, 15.6 for 40 at 64; 34816 x 5120 33 for
+      62, 45 for 179; 576 x 7168 9.4 for 12, 14.5 for 36).
+    * up to 128: yes where the decode-warp kernel must split K to fill the SMs (12288 x 5120 37.5 for 56 at 128, 5120 x 17408 50 for
+      67), no where its 128-token tiles fill them (34816 x 5120 62 for 59 at 65, 73 for 61 at 128).
     * above, the decode-warp kernel walks a 256-token tile of 128 features in 1.03 us per 128 inputs, wave after wave; the pairs share
       the tiles evenly, about 1 us per 128 inputs of two, but pay 18 us for tiles that are cut, and for the split.  By that: 7168 x
-      2048 at 257 tokens 34 for 27, 5120 x 4096 at 700 50 for 41, 12288 x 5120 at 700 101 for 92 go to the decode warps, 5120 x
-      17408 (129: 59 for 131; 1901: 391 for 468), 12288 x 5120 at 333 (70 for 82) and 34816 x 5120 at 1901 (741 for 790) do not."""
+      2048 at 257 tokens 33 for 27, 5120 x 4096 at 700 49 for 41, 12288 x 5120 at 700 95 for 89 go to the decode warps, 5120 x
+      17408 (129: 58 for 132; 1901: 344 for 519), 12288 x 5120 at 333 (76 for 87) and 34816 x 5120 at 1901 (642 for 770) do not."""
     m, kb = (n + 127) // 128, k // 128
     if t <= TERMS_SINGLE_T or kb > 254:            # the decode warps keep the scales of 254 blocks
         return True

@@ -1,6 +1,6 @@
 """Routed-expert MoE on the GPU: router top-k, device-side planning, grouped tcgen05 GEMMs over expert-sorted rows
-(csrc/kernels/moe.cu + the grouped mode of csrc/kernels/gemm_wdec.cu).  No host synchronisation anywhere: the
-number of rows per expert only exists on the device."""
+(csrc/kernels/moe.cu + the grouped mode of csrc/kernels/gemm_wdec.cu, and gemm_fp4_terms.cu for FP4 experts).  No host
+synchronisation anywhere: the number of rows per expert only exists on the device."""
 from __future__ import annotations
 
 import ctypes

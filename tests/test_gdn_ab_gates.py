@@ -41,3 +41,9 @@ def test_convolution_around_its_runs_of_tokens(t):
     got = basic.conv_silu(x[:, :c], w, tail)
     # one rounding to bf16 and a fast exponential
     assert ((got.float() - want).abs() <= want.abs() * 2.0 ** -8 + 1e-5).all() and torch.equal(tail, new_tail)
+
+
+# the lines between runs of all tokens, of 4, 8 and 16
+@pytest.mark.parametrize("t", [3, 6, 7, 191, 192, 193, 196, 200])
+def test_convolution_at_the_lines_between_its_runs(t):
+    test_convolution_around_its_runs_of_tokens(t)

@@ -144,6 +144,35 @@ def test_product_matches_64_bit(t, n, k):
     assert torch.equal(y, again) and torch.equal(y, u)
 
 
+# pairs with more tiles than there are pairs: whole waves of neighbouring tiles, then a tail of none (148 tiles), of one to two tiles a pair,
+# an odd last weight tile
+WAVES = [(257, 18944, 256), (513, 19072, 384), (300, 38144, 256), (129, 56832, 128), (700, 12800, 896)]
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("outliers", [False, True])
+@pytest.mark.parametrize("t,n,k", WAVES)
+def test_whole_waves_of_pair_tiles(t, n, k, outliers):
+    from deepseek_v4_2080ti_b200.ops import _lib, gemm
+    torch.manual_seed(t + n + k)
+    q, s = fp8fmt.quantize_block128(torch.randn(n, k, device="cuda") * 0.05)
+    w, wd = gemm.PackedLinear.from_fp8(q, s), fp8fmt.dequantize_block128(q, s).double()
+    x = torch.randn(t, k, device="cuda").bfloat16()
+    if outliers:                                           # in rows of every token tile, so in tiles of the waves and of the tail
+        blocks = torch.rand(t, k // 128, 1, device="cuda") < 0.05
+        x = torch.where(blocks, _outliers(t, k, 16).view(t, -1, 128), x.view(t, -1, 128)).view(t, k)
+    r = torch.randn(t, n, device="cuda").bfloat16()
+    xt = gemm.split_terms(x)
+    assert bool(xt.sx.permute(0, 2, 1).reshape(-1, k // 128)[:t].lt(0).any()) == outliers
+    y, again, z = gemm.linear_terms(xt, w), gemm.linear_terms(xt, w), gemm.linear_terms(xt, w, residual=r)
+    torch.cuda.synchronize()
+    _lib.check_status()
+    ref = x.double() @ wd.t()
+    rel = lambda a, b: ((a.double() - b).norm(dim=1) / b.norm(dim=1)).max().item()
+    assert rel(y, ref) < 2.0 ** -8 and rel(z, ref + r.double()) < 2.0 ** -8          # every row: at most the rounding to bf16
+    assert torch.equal(y, again)
+
+
 @pytest.mark.gpu
 @pytest.mark.parametrize("t", [7, 40, 300])
 def test_products_on_two_streams_share_no_scratch(t):
@@ -323,12 +352,12 @@ def test_expert_rows_are_combined(t, k, h):
 
 
 # (tokens, features, inputs, us with the split, us of the kernel that takes its place): the two sides of the rule
-ROUTES = [(1, 576, 7168, 11.2, 11.8), (1, 5120, 4096, 10.3, 14.4), (32, 576, 7168, 12.8, 21.9), (64, 34816, 5120, 46, 193), (65, 34816, 5120, 80, 59), (100, 14336, 5120, 47, 34),
-          (128, 34816, 5120, 88, 62), (128, 12288, 5120, 47, 55), (128, 5120, 17408, 58, 67), (65, 576, 7168, 31, 32),
-          (128, 1536, 7168, 34, 48), (129, 5120, 17408, 59, 131), (257, 7168, 2048, 34, 27), (256, 5120, 4096, 31, 40),
-          (700, 5120, 4096, 50, 41), (700, 12288, 5120, 101, 92), (333, 12288, 5120, 70, 82), (1500, 2048, 5120, 58, 46),
-          (1901, 1536, 7168, 78, 59), (1901, 7168, 2048, 76, 68), (1000, 5120, 17408, 178, 268), (1901, 34816, 5120, 741, 790),
-          (1901, 4096, 4096, 81, 67), (1000, 2048, 5120, 41, 45), (1500, 7168, 2048, 66, 55)]
+ROUTES = [(1, 576, 7168, 9.4, 11.7), (1, 5120, 4096, 9.7, 14.1), (32, 576, 7168, 11.1, 21.7), (64, 34816, 5120, 45, 179), (65, 34816, 5120, 62, 59),
+          (100, 14336, 5120, 38, 34), (128, 34816, 5120, 73, 61), (128, 12288, 5120, 37.5, 56), (128, 5120, 17408, 50, 67), (65, 576, 7168, 20, 32),
+          (128, 1536, 7168, 26, 47), (129, 5120, 17408, 58, 132), (257, 7168, 2048, 33, 27), (256, 5120, 4096, 31, 40),
+          (700, 5120, 4096, 49, 41), (700, 12288, 5120, 95, 89), (333, 12288, 5120, 76, 87), (1500, 2048, 5120, 58, 46),
+          (1901, 1536, 7168, 77, 58), (1901, 7168, 2048, 76, 70), (1000, 5120, 17408, 173, 301), (1901, 34816, 5120, 642, 770),
+          (1901, 4096, 4096, 101, 76), (1000, 2048, 5120, 43, 47), (1500, 7168, 2048, 69, 57)]
 
 
 @pytest.mark.parametrize("t,n,k,terms_us,other_us", ROUTES)

@@ -5,7 +5,7 @@ import torch
 pytestmark = pytest.mark.gpu
 
 
-# tokens around the tiles of the FP8 term products (16, 32, 64, 256) and of the attention and delta-rule chunks; two portions, so that
+# tokens around the tiles of the FP8 term products (16, 32, 64, 128, 256) and of the attention and delta-rule chunks; two portions, so that
 # the second starts from states, tails and a context
 @pytest.mark.parametrize("first,second", [(1, 1), (5, 16), (17, 64), (65, 40), (128, 257), (300, 129)])
 @pytest.mark.parametrize("gate", [True, False])
@@ -35,6 +35,12 @@ def test_native_portions_equal_the_launches_one_by_one(first, second, gate, monk
     assert torch.equal(s, s2) and torch.equal(t, t2)
     for x, y in ((a, a2), (b, b2)):
         assert torch.equal(x[0], y[0]) and torch.equal(x[1], y[1]) and x[2] == y[2]
+
+
+# both sides of the widest tile of one CTA
+@pytest.mark.parametrize("first,second", [(127, 128), (129, 66)])
+def test_portions_around_the_widest_single_tile(first, second, monkeypatch):
+    test_native_portions_equal_the_launches_one_by_one(first, second, True, monkeypatch)
 
 
 def test_portions_do_not_wait_for_the_device():
