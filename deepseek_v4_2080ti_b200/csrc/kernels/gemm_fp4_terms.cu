@@ -23,9 +23,9 @@
 // to tensor memory, two groups by turns (one group: 200 tokens 486 us for 444, 2000 tokens 779 for 738).  All waits are bounded.
 //
 // Measured, us for [gate | up] 4096 x 4096 and down 4096 x 2048 of 256 experts, top 6 (reading the experts that get a token once takes,
-// at 6.43 TB/s, 8 and 4 for one token, 355 and 178 from 200 tokens on): 1 token 24.5, 17.6; 200 tokens 444, 238; 2000 tokens 717, 410.
+// at 6.43 TB/s, 8 and 4 for one token, 355 and 178 from 200 tokens on): 1 token 25, 17; 200 tokens 433, 230; 2000 tokens 670, 381.
 // gemm_wdec_kernel.cuh, which turns every weight into bf16 on the CUDA cores: 1 token 47, 47; 2000 tokens 2218 together.
-// What bounds it: one token, the fixed part of a launch and the sums of cut tiles; 200 tokens, the weight stream (5.1 TB/s) and the chain
+// What bounds it: one token, the fixed part of a launch and the sums of cut tiles; 200 tokens, the weight stream (5.3 TB/s) and the chain
 // copy - spread - product of a stage; 2000 tokens, the same chain, with rows of 13 KB beside 17 KB of weights per stage.
 #include <cuda_bf16.h>
 #include <string.h>

@@ -222,10 +222,11 @@ def _expanded_bf16(w: "PackedLinear", device, gate_up: bool = False) -> "PackedL
 
 
 def expands(t: int, w: "PackedLinear") -> bool:
-    """Does a ``t``-token product expand FP8 matrix ``w`` to bf16 first?  Prefill-sized batches, ragged or not: against
-    ``linear_terms``, whose products need no expansion, a ragged prompt through eight layers took 16.9 ms for 14.7 to 16.8 at 2049
-    tokens, as long at 3001, 29.0 for 30.6 at 4095, 41.8 for 46.4 at 6001 and 55.7 for 63.5 at 8191 (the expansion runs beside the
-    product before it), and the CTA-pair bf16 kernel tiles the even ones."""
+    """Does a ``t``-token product expand FP8 matrix ``w`` to bf16 first?  Prefill-sized batches, ragged or not.  ms of a prompt through
+    eight layers, expanded (beside the product before) / with ``linear_terms``, whose products need no expansion: even ones, which
+    the CTA-pair bf16 kernel tiles, 12.9 / 13.5 at 2048 tokens, 14.0 / 15.2 at 2304, 18.3 / 19.7 at 3072, 22.7 / 26.5 at 4096; ragged
+    ones 16.5 / 14.8 at 2049, 21.8 / 20.0 at 3001, 28.0 / 26.5 at 4095, 40.3 / 40.2 at 6001 (the line is older than the terms' present
+    speed, and theirs would lie near 6000)."""
     return w.wfmt == WF_FP8_B128 and t >= PREDECODE_MIN_T
 
 
