@@ -535,6 +535,7 @@ int b200_add(void* y, const void* x, long long n, cudaStream_t stream) {
 int b200_conv_silu(const void* x, int ldx, const void* w, void* tail, void* y, int ldy, int T, int C,
                    int kw, int update_tail, cudaStream_t stream) {
   if (kw != 4 || C % 8) return -6;
+  if (T <= 0) return 0;       // no tokens: the tail stays as it is
   const int threads = 128;
   const int cblocks = (C / 8 + threads - 1) / threads;
   // Short runs: a thread walks its tokens one after the other (64 at a time: 30 us at 333 tokens of 8192 channels).  us of a convolution and
