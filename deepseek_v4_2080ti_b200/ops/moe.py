@@ -33,8 +33,10 @@ def prepack_fp4(packed: torch.Tensor, scale_e8m0: torch.Tensor, out: torch.Tenso
         scale_e8m0 = torch.cat([scale_e8m0, scale_e8m0.new_zeros(npad - n, k // 32)])
     mt, bk = npad // 128, 128 if k % 128 == 0 else 64
     codes = bk * 64
+    shape = (mt, k // bk, codes + bk * 4)
     if out is None:
-        out = packed.new_empty(mt, k // bk, codes + bk * 4)
+        out = packed.new_empty(shape)
+    assert out.shape == shape, "matrices of one stack have one shape"      # (a copy would repeat a smaller one)
     # one pass over the codes and one over the scales, straight to their places
     if bk == 128:
         out[..., :codes].unflatten(-1, (4, 128, 16)).copy_(packed.view(mt, 128, k // 128, 4, 16).permute(0, 2, 3, 1, 4))
