@@ -115,7 +115,7 @@ struct Int {
 template <int G, int KV>
 __global__ void __launch_bounds__(THREADS)
 gqa_decode_kernel(DecodeParams p) {
-  constexpr int U = G > 5 ? 2 : 3;
+  constexpr int U = G > 5 ? 2 : 4;
   __shared__ float s_m[NSTATE][G], s_l[NSTATE][G];
   __shared__ float s_o[NSTATE][G][D];
   b200::pdl_grid_trigger();
@@ -150,10 +150,10 @@ gqa_decode_kernel(DecodeParams p) {
   }
 
   // U keys of a half-warp at a time: their page numbers, then their rows, are asked for together, and the running maximum and the
-  // sums are rescaled once for all of them; a rest of up to eight keys goes one key a half-warp.  One after the other, a key is two
-  // trips to memory and a chain of shuffles and exponentials.  us for 5 x 8 heads, rows x keys, one key at a time / U = 3: 1 x 24 4.9 /
-  // 4.5, 32 x 60 11 / 7, 64 x 1024 180 / 120, 32 x 4096 663 / 420.  U = 4 takes registers that four blocks an SM do not have (64 x 1024
-  // 207), as does U = 3 from six heads on.  A third of it was the division by the page size.
+  // sums are rescaled once for all of them; a rest of up to eight keys goes one key a half-warp, with the same results as in a whole
+  // chunk.  One after the other, a key is two trips to memory and a chain of shuffles and exponentials.  us for 5 x 8 heads, rows x keys,
+  // one key at a time / U = 4: 1 x 24 4.4 / 2.8, 32 x 60 10.7 / 6.5, 64 x 1024 172 / 108, 32 x 4096 656 / 264 (U = 3: 2.6, 6.8, 116, 275;
+  // from six heads on U = 4 does not fit the registers).  A division for the page of a key and a whole chunk for the rest: 3.3, 7.8, 184, 413.
   const int mine = warp * 2 + half;
   auto key_at = [&](int kk) {                  // rows past the range contribute nothing: they repeat the first one
     const int kc = kk < k1 ? kk : k0;
@@ -205,14 +205,13 @@ gqa_decode_kernel(DecodeParams p) {
         if constexpr (KV != 0) s[u][g] *= row[u].ks;
         if (valid[u]) mn = fmaxf(mn, s[u][g]);
       }
-      const float alpha = exp2f(m[g] - mn);
-      l[g] *= alpha;
+      const float alpha = exp2f(m[g] - mn);     // (products and sums below: one rounding order in every chunk)
 #pragma unroll
-      for (int i = 0; i < 8; ++i) acc[g][i] *= alpha;
+      for (int i = 0; i < 8; ++i) acc[g][i] = __fmul_rn(acc[g][i], alpha);
 #pragma unroll
       for (int u = 0; u < N; ++u) {
         s[u][g] = valid[u] ? exp2f(s[u][g] - mn) : 0.f;
-        l[g] += s[u][g];
+        l[g] = u == 0 ? __fmaf_rn(l[g], alpha, s[u][g]) : __fadd_rn(l[g], s[u][g]);
       }
       m[g] = mn;
     }
@@ -224,7 +223,7 @@ gqa_decode_kernel(DecodeParams p) {
 #pragma unroll
       for (int g = 0; g < G; ++g)
 #pragma unroll
-        for (int i = 0; i < 8; ++i) acc[g][i] += s[u][g] * vf[i];
+        for (int i = 0; i < 8; ++i) acc[g][i] = __fmaf_rn(s[u][g], vf[i], acc[g][i]);
     }
   };
   // warp-uniform: every lane runs the shuffles

@@ -83,3 +83,34 @@ def test_every_cache_format_and_page_size(group, fmt, bs):
         torch.cuda.synchronize()
         _lib.check_status()
         assert ((out.double() - want).abs() <= 2 ** -8 * want.abs() + 2 ** -12).all()       # as above
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("group", [1, 5])
+def test_four_keys_of_a_half_warp_share_one_maximum(group):
+    """Up to five heads a group, the first four keys of a half-warp are weighted by 2^(score - the largest of the four): one that lies 140
+    below it has no weight at all (2^-140 is flushed), and none by way of a key between the two either."""
+    import ctypes
+
+    import numpy as np
+
+    from deepseek_v4_2080ti_b200.ops import _lib
+    log2e, near = np.float32(1.4426950408889634), np.float32(0.6931472)
+    scale = next(x for x in (near, np.nextafter(near, np.float32(0)), np.nextafter(near, np.float32(1))) if x * log2e == np.float32(1))
+    n, per, bs = 64, 32, 16
+    k, v = torch.zeros(n // bs, 1, bs, 128), torch.zeros(n // bs, 1, bs, 128)
+    k[..., 0] = -1000.0                                    # scores: nothing beside those of the first half-warp's keys
+    for key, score in ((0, -140.0), (8, -120.0), (16, -1000.0), (24, 0.0)):
+        k[key // bs, 0, key % bs, 0] = score
+    for key in (0, 8):
+        v[key // bs, 0, key % bs] = 1.0
+    q = torch.zeros(1, group, 128)
+    q[..., 0] = 1.0
+    q, k, v = (x.to("cuda", torch.bfloat16) for x in (q, k, v))
+    bt, kv_len = torch.arange(n // bs, dtype=torch.int32, device="cuda"), torch.tensor([n], dtype=torch.int32, device="cuda")
+    out, part = torch.empty_like(q), torch.full((group, n // per, 130), 7.0, device="cuda")
+    p = _lib.ptr
+    _lib.check(_lib.lib().b200_gqa_decode(p(q), p(k), p(v), p(out), None, p(bt), p(kv_len), p(part), 1, n // bs, bs, group, 1, n // per,
+                                          ctypes.c_float(float(scale)), _lib.stream()), "gqa_decode")
+    torch.cuda.synchronize()
+    assert (part[:, 0, :128] == 2.0 ** -120).all() and (part[:, 0, 128] == 0).all() and (part[:, 0, 129] == 1).all()
