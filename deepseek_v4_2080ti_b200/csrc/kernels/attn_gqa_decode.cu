@@ -154,6 +154,7 @@ gqa_decode_kernel(DecodeParams p) {
   // chunk.  One after the other, a key is two trips to memory and a chain of shuffles and exponentials.  us for 5 x 8 heads, rows x keys,
   // one key at a time / U = 4: 1 x 24 4.4 / 2.8, 32 x 60 10.7 / 6.5, 64 x 1024 172 / 108, 32 x 4096 656 / 264 (U = 3: 2.6, 6.8, 116, 275;
   // from six heads on U = 4 does not fit the registers).  A division for the page of a key and a whole chunk for the rest: 3.3, 7.8, 184, 413.
+  // Three blocks fit an SM where four did, which costs contexts under 18 keys: 64 x 8 4.4 / 5.1, 64 x 24 6.4 / 6.2.
   const int mine = warp * 2 + half;
   auto key_at = [&](int kk) {                  // rows past the range contribute nothing: they repeat the first one
     const int kc = kk < k1 ? kk : k0;
